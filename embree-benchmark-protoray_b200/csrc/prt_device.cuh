@@ -682,29 +682,38 @@ __device__ __forceinline__ void trav_step(TravState& s, const SceneDev& sc, cons
 // With one-triangle leaves a node visit finds a triangle for only a few lanes
 // of a warp, so testing triangles in the visiting lane runs the test with ~3 of
 // 32 lanes.  In the deferred mode a node visit only queues its hit triangles
-// (leaf-order index + owner lane) in a per-warp ring in shared memory; once 32
-// are pending, the whole warp tests them, one per lane, with the owner's ray
+// (leaf-order index + owner lane) in a per-warp list in shared memory; once 32
+// are pending, the whole warp tests the oldest 32, one per lane, and the rest
+// moves to the front of the list; the owner's ray is
 // fetched by shuffles, and the owners' closest hits are merged with one 64-bit
 // shared-memory atomicMin on (t bits, primitive id): positive floats order as
 // their bit patterns and the id breaks exact ties the way tri_test does.  Node
 // culling uses the owner's tHit as of the last merge, which can only be larger
 // than the final one, so no node that holds the closest hit is skipped.
+// The list holds the largest possible step and nothing more, and the
+// barycentrics live in an array of their own that only closest-hit queries
+// allocate: a block of the bounce kernel takes 14 KB of shared memory, 8 blocks
+// fit the 132 KB carveout, and L1 keeps 124 of the SM's 256 KB for nodes and
+// triangles.  (A 512-entry ring beside the barycentrics took 18.5 KB a block
+// and left L1 92 KB: bounces 1-5 of a 33M-path terrain wave 17.32 -> 16.86 ms,
+// 4M incoherent closest-hit queries 1.302 -> 1.274 ms.)
 #ifndef PRT_DEFER_TRIS
 #define PRT_DEFER_TRIS 1
 #endif
-#ifndef PRT_DEFER_FLUSH
-#define PRT_DEFER_FLUSH 32
-#endif
 
-constexpr uint32_t kTriQCap = 512;   // > 31 pending + 8 triangles x 32 lanes from one step
-constexpr uint32_t kTriQMask = kTriQCap - 1;
+constexpr uint32_t kTriQCap = 288;   // >= 31 pending + 8 triangles x 32 lanes from one step
 
 struct TriQueue
 {
     unsigned long long key[32];   // per owner lane: (t bits << 32) | primitive id
-    uint32_t tri[kTriQCap];       // leaf-order triangle index << 5 | owner lane
-    float u[32], v[32];
+    uint32_t tri[kTriQCap];       // oldest first: leaf-order triangle index << 5 | owner lane
     int ti[32];
+};
+
+// Barycentrics of the merged hits, kept only by kernels that return them.
+struct TriQueueUV
+{
+    float u[32], v[32];
 };
 
 __device__ __forceinline__ unsigned long long hit_key(float t, int prim)
@@ -713,13 +722,8 @@ __device__ __forceinline__ unsigned long long hit_key(float t, int prim)
 }
 
 // One node visit of the deferred mode: returns the node's hit triangles
-// (tbase + set bits of tbits) instead of testing them.
-#ifndef PRT_LEAF1_HITS
-#define PRT_LEAF1_HITS 1
-#endif
-
-// tbits: the hit leaf slots (PRT_LEAF1_HITS) with the node's leaf-slot mask in
-// leafMask, or triangle offset bits with leafMask = 0.
+// (tbase and tbits, the hit leaf slots, with the node's leaf-slot mask in
+// leafMask) instead of testing them.
 template <bool kPair = false>
 __device__ __forceinline__ void trav_visit(TravState& s, const SceneDev& sc, const TravRay& r, float tnear, TravStack& st,
                                            uint32_t& tbase, uint32_t& tbits, uint32_t& leafMask,
@@ -736,16 +740,7 @@ __device__ __forceinline__ void trav_visit(TravState& s, const SceneDev& sc, con
     uint4 q[5];
 #pragma unroll
     for (int k = 0; k < 5; ++k) q[k] = __ldg(qp + k);
-    uint32_t hits;
-    if (PRT_LEAF1_HITS)
-    {
-        hits = node_hits1<kPair>(r, q, tnear, s.tHit, leafMask, r.octinv);
-    }
-    else
-    {
-        hits = node_hits(r, q, tnear, s.tHit);
-        leafMask = 0;
-    }
+    const uint32_t hits = node_hits1<kPair>(r, q, tnear, s.tHit, leafMask, r.octinv);
     if (nodeVisits) ++*nodeVisits;
     ng = make_uint2(q[1].x, (hits & 0xff000000u) | (q[0].w >> 24));
     tbits = hits & 0x00ffffffu;
@@ -763,49 +758,49 @@ __device__ __forceinline__ void trav_visit(TravState& s, const SceneDev& sc, con
     s.ng = ng;
 }
 
-// Warp-collective: appends every lane's triangles to the ring at tail
-// (leafMask != 0: tbits are leaf slots, see trav_visit).
-__device__ __forceinline__ void triq_push(TriQueue& q, uint32_t& tail, uint32_t tbase, uint32_t tbits, uint32_t leafMask,
+// Warp-collective: appends every lane's triangles to the n queued ones.  One
+// triangle of each lane that has one per round, placed by the ballot of those
+// lanes: a visit leaves 0.2 triangles per lane, so most calls take two or three
+// rounds of about ten instructions, fewer than a prefix sum of the lanes'
+// counts needs before its first store.
+__device__ __forceinline__ void triq_push(TriQueue& q, uint32_t& n, uint32_t tbase, uint32_t tbits, uint32_t leafMask,
                                           unsigned lane)
 {
-    const unsigned FULL = 0xffffffffu;
-    const uint32_t n = __popc(tbits);
-    uint32_t x = n;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1)
+    const uint32_t lt = (1u << lane) - 1u;
+    for (;;)
     {
-        const uint32_t y = __shfl_up_sync(FULL, x, off);
-        if ((int)lane >= off) x += y;
+        const unsigned m = __ballot_sync(0xffffffffu, tbits != 0);
+        if (!m) break;
+        if (tbits)
+        {
+            const uint32_t low = tbits & (0u - tbits);
+            tbits ^= low;
+            q.tri[n + __popc(m & lt)] = ((tbase + __popc(leafMask & (low - 1u))) << 5) | lane;
+        }
+        n += __popc(m);
     }
-    uint32_t pos = tail + x - n;
-    while (tbits)
-    {
-        const uint32_t bit = __ffs(tbits) - 1u;
-        tbits &= tbits - 1u;
-        q.tri[pos & kTriQMask] = ((tbase + (leafMask ? __popc(leafMask & ((1u << bit) - 1u)) : bit)) << 5) | lane;
-        ++pos;
-    }
-    tail += __shfl_sync(FULL, x, 31);
 }
 
-// Warp-collective: tests the m (<= 32) oldest queued triangles, one per lane,
-// and merges each owner's closest hit into its traversal state.  The owner's
+// Warp-collective: tests the m (<= 32) queued triangles from `first`, one per
+// lane, and merges each owner's closest hit into its traversal state.  The owner's
 // ray, tnear and triangle array (lanes of a batch may traverse different
 // scenes) come from the owner lane by shuffles.
-__device__ __forceinline__ void triq_flush(TriQueue& q, uint32_t& head, uint32_t m, const TriRec* tris, const TravRay& r,
-                                           float tnear, TravState& ts, unsigned lane, uint32_t* triTests = nullptr)
+template <bool kUV>
+__device__ __forceinline__ void triq_flush(TriQueue& q, uint32_t first, uint32_t m, const TriRec* tris, const TravRay& r,
+                                           float tnear, TravState& ts, unsigned lane, TriQueueUV* uv,
+                                           uint32_t* triTests = nullptr)
 {
     const unsigned FULL = 0xffffffffu;
     const bool act = lane < m;
     uint32_t tri = 0;
     int own = 0;
+    __syncwarp();
     if (act)
     {
-        const uint32_t e = q.tri[(head + lane) & kTriQMask];
+        const uint32_t e = q.tri[first + lane];
         tri = e >> 5;
         own = (int)(e & 31u);
     }
-    head += m;
     TravRay o;
     o.org.x = __shfl_sync(FULL, r.org.x, own);
     o.org.y = __shfl_sync(FULL, r.org.y, own);
@@ -840,8 +835,11 @@ __device__ __forceinline__ void triq_flush(TriQueue& q, uint32_t& head, uint32_t
     __syncwarp();
     if (hit && q.key[own] == hit_key(t, prim))
     {
-        q.u[own] = u;
-        q.v[own] = v;
+        if (kUV)
+        {
+            uv->u[own] = u;
+            uv->v[own] = v;
+        }
         q.ti[own] = (int)tri;
     }
     __syncwarp();
@@ -850,8 +848,11 @@ __device__ __forceinline__ void triq_flush(TriQueue& q, uint32_t& head, uint32_t
     {
         ts.tHit = __uint_as_float((uint32_t)(k >> 32));
         ts.primHit = (int)(uint32_t)k;
-        ts.uHit = q.u[lane];
-        ts.vHit = q.v[lane];
+        if (kUV)
+        {
+            ts.uHit = uv->u[lane];
+            ts.vHit = uv->v[lane];
+        }
         ts.triHit = q.ti[lane];
     }
     __syncwarp();
@@ -865,16 +866,17 @@ __device__ __forceinline__ void triq_flush(TriQueue& q, uint32_t& head, uint32_t
 // tests are still merged, which can only move the hit nearer).  The counter
 // pointers (node visits, triangle tests per lane; steps, running-lane steps and
 // flushes per warp) may be null.
-template <bool kPair = false>
+template <bool kPair = false, bool kUV = false>
 __device__ __forceinline__ void warp_trav_deferred(TriQueue& q, TravState& ts, const SceneDev& sc, const TravRay& r,
                                                    float tnear, TravStack& st, bool active, bool mayStop, int refillMin,
                                                    unsigned lane, uint32_t* cNodes = nullptr, uint32_t* cTris = nullptr,
                                                    unsigned long long* cSteps = nullptr,
                                                    unsigned long long* cLaneSteps = nullptr,
-                                                   unsigned long long* cFlushes = nullptr, bool anyHit = false)
+                                                   unsigned long long* cFlushes = nullptr, bool anyHit = false,
+                                                   TriQueueUV* uv = nullptr)
 {
     const unsigned FULL = 0xffffffffu;
-    uint32_t head = 0, tail = 0;
+    uint32_t n = 0;   // queued triangles
     for (;;)
     {
         uint32_t tbase = 0, tbits = 0, lmask = 0;
@@ -884,20 +886,28 @@ __device__ __forceinline__ void warp_trav_deferred(TriQueue& q, TravState& ts, c
             *cSteps += 1;
         }
         if (active && !ts.done) trav_visit<kPair>(ts, sc, r, tnear, st, tbase, tbits, lmask, cNodes);
-        if (__any_sync(FULL, tbits != 0)) triq_push(q, tail, tbase, tbits, lmask, lane);
-        while (tail - head >= (uint32_t)PRT_DEFER_FLUSH)
+        triq_push(q, n, tbase, tbits, lmask, lane);
+        if (n >= 32u)
         {
-            triq_flush(q, head, min(32u, tail - head), sc.tris, r, tnear, ts, lane, cTris);
-            if (cFlushes) *cFlushes += 1;
+            uint32_t first = 0;
+            do
+            {
+                triq_flush<kUV>(q, first, 32u, sc.tris, r, tnear, ts, lane, uv, cTris);
+                if (cFlushes) *cFlushes += 1;
+                first += 32u;
+            } while (n - first >= 32u);
             if (anyHit && ts.triHit >= 0) ts.done = true;
+            // the rest moves to the front
+            n -= first;
+            if (lane < n) q.tri[lane] = q.tri[first + lane];
         }
         const unsigned running = __ballot_sync(FULL, active && !ts.done);
         if (running == 0) break;
         if (mayStop && 32 - __popc(running) >= refillMin) break;
     }
-    while (tail != head)
+    if (n)
     {
-        triq_flush(q, head, min(32u, tail - head), sc.tris, r, tnear, ts, lane, cTris);
+        triq_flush<kUV>(q, 0, n, sc.tris, r, tnear, ts, lane, uv, cTris);
         if (cFlushes) *cFlushes += 1;
     }
 }

@@ -978,7 +978,10 @@ __global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_intersect(SceneD
     st.sh = s_stack + threadIdx.x;
     st.stride = blockDim.x;
     st.overflow = false;
-    TriQueue* tq = reinterpret_cast<TriQueue*>(s_stack + kShared * blockDim.x) + (threadIdx.x >> 5);   // deferTris
+    // deferTris: the warps' triangle queues, then (closest hit) their barycentrics
+    TriQueue* tq = reinterpret_cast<TriQueue*>(s_stack + kShared * blockDim.x) + (threadIdx.x >> 5);
+    TriQueueUV* tuv = reinterpret_cast<TriQueueUV*>(reinterpret_cast<TriQueue*>(s_stack + kShared * blockDim.x) +
+                                                    (blockDim.x >> 5)) + (threadIdx.x >> 5);
     const unsigned FULL = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned ltMask = (1u << lane) - 1u;
@@ -1018,8 +1021,8 @@ __global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_intersect(SceneD
         if (PRT_DEFER_ISECT && sc.deferTris)
         {
             constexpr bool kPair = kAnyHit && PRT_PAIRED_QUERY;
-            warp_trav_deferred<kPair>(*tq, ts, sc, r, tnear, st, has, !exhausted, kRefillMin, lane, nullptr, nullptr,
-                                      nullptr, nullptr, nullptr, kAnyHit);
+            warp_trav_deferred<kPair, !kAnyHit>(*tq, ts, sc, r, tnear, st, has, !exhausted, kRefillMin, lane, nullptr,
+                                                nullptr, nullptr, nullptr, nullptr, kAnyHit, tuv);
         }
         else
         for (;;)
@@ -1614,7 +1617,8 @@ int launch_intersect(const SceneDev& sc, const RayRec* rays, HitRec* hits, int n
     if (n <= 0) return 0;
     const int block = 128;
     size_t shmem = sizeof(uint2) * kShared * block;
-    if (PRT_DEFER_ISECT && sc.deferTris) shmem += sizeof(TriQueue) * (block / 32);
+    if (PRT_DEFER_ISECT && sc.deferTris)
+        shmem += (sizeof(TriQueue) + (anyHit ? 0 : sizeof(TriQueueUV))) * (block / 32);
     LaunchCfg cfg;
     auto go = [&](auto kernel) {
         // no more warps than rays: 32 rays per warp
