@@ -15,7 +15,7 @@
 //   * the frame may hold at most kNoAllocMaxPaths pixels after rounding up to
 //     8x8 tiles (524288, e.g. 1024x512 or 960x544); larger frames are
 //     rejected with PRT_EINVAL;
-//   * g_scratch occupies 40 MiB on every GPU that loads the library, until the
+//   * g_scratch occupies 20 MiB on every GPU that loads the library, until the
 //     process exits;
 //   * all calls on a device share g_scratch, which keeps the last call's
 //     contents: each call clears the counters it needs before using them, and
@@ -43,9 +43,9 @@ constexpr int kNoAllocCounters = 64 + 2;   // one slot per bounce depth (max dep
 
 struct NoAllocScratch
 {
-    PathRec queue[2][kNoAllocMaxPaths];
-    float thr[2][kNoAllocMaxPaths];   // per-path throughput (per-triangle albedo)
-    float L[2][kNoAllocMaxPaths];     // radiance gathered so far (next-event estimation)
+    PathRec queue[kNoAllocMaxPaths];   // the paths of depth 1
+    float thr[kNoAllocMaxPaths];       // per-path throughput (per-triangle albedo)
+    float L[kNoAllocMaxPaths];         // radiance gathered so far (next-event estimation)
     int counts[kNoAllocCounters];
     int fetch[kNoAllocCounters];
     unsigned long long rays;
@@ -221,18 +221,23 @@ extern "C" int prt_render_noalloc(prt_ctx* ctx, const prt_camera* cam, int width
         a.passOffset = pass0 + p0;
         a.passes = std::min(passesPerWave, spp - p0);
         e = cudaMemsetAsync(s->counts, 0, sizeof(int) * 2 * kNoAllocCounters, stream);
-        for (int d = 0; d <= maxDepth && e == cudaSuccess; ++d)
+        if (e != cudaSuccess) break;
+        a.qin = nullptr;
+        a.qout = s->queue;
+        a.thrIn = nullptr;
+        a.thrOut = albedo ? s->thr : nullptr;
+        a.Lin = nullptr;
+        a.Lout = nee ? s->L : nullptr;
+        a.thrConst = 1.0f;
+        launch_bounce(a, 0, cfg, numSMs, stream);
+        e = cudaGetLastError();
+        if (maxDepth > 0 && e == cudaSuccess)
         {
-            a.qin = d == 0 ? nullptr : s->queue[(d - 1) & 1];
-            a.qout = s->queue[d & 1];
-            a.thrIn = albedo && d > 0 ? s->thr[(d - 1) & 1] : nullptr;
-            a.thrOut = albedo ? s->thr[d & 1] : nullptr;
-            a.Lin = nee && d > 0 ? s->L[(d - 1) & 1] : nullptr;
-            a.Lout = nee ? s->L[d & 1] : nullptr;
-            float t = 1.0f;
-            for (int k = 0; k < d; ++k) t *= 0.8f;
-            a.thrConst = t;
-            launch_bounce(a, d, cfg, numSMs, stream);
+            a.qin = a.qout;
+            a.thrIn = a.thrOut;
+            a.Lin = a.Lout;
+            a.thrConst = 0.8f;
+            launch_paths(a, cfg, numSMs, stream);
             e = cudaGetLastError();
         }
     }

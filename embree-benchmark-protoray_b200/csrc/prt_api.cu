@@ -76,11 +76,14 @@ struct prt_ctx
     // render state
     int* dPass = nullptr;                 // device pass counter
     unsigned long long* dRays = nullptr;  // rays of the current call
-    int* dCounts = nullptr;               // [kMaxChains][kMaxDepthCap + 2]
-    int* dFetch = nullptr;                // [kMaxChains][kMaxDepthCap + 2]
-    PathRec* q[kMaxChains][2] = {};       // ping-pong path queues of each concurrent wave chain
+    int* dCounts = nullptr;               // per chain: path counts and work counters per depth (chain_counts)
+    unsigned long long* hRays = nullptr;  // pinned: the call's ray count on the host
+    // path queues of each concurrent wave chain: [0] takes the paths of depth 1;
+    // [1] is the other half of the per-depth ping-pong of prt_render_profile
+    PathRec* q[kMaxChains][2] = {};
     float* thr[kMaxChains][2] = {};
     float* Lq[kMaxChains][2] = {};        // next-event estimation: gathered radiance per path
+    int queueBuffers = 0;                 // of q, thr and Lq allocated per chain
     long long queueCap = 0;
     bool queueL = false;
     int integrator = PRT_INTEGRATOR_DIFFUSE;
@@ -228,13 +231,15 @@ void release_queues(prt_ctx* ctx)
     clear_graphs(ctx);
     ctx->queueCap = 0;
     ctx->queueChains = 0;
+    ctx->queueBuffers = 0;
     ctx->queueThr = false;
     ctx->queueL = false;
 }
 
-int ensure_queues(prt_ctx* ctx, long long paths, bool withThr, int chains = 1, bool withL = false)
+int ensure_queues(prt_ctx* ctx, long long paths, bool withThr, int chains = 1, bool withL = false, int buffers = 1)
 {
-    if (paths <= ctx->queueCap && chains <= ctx->queueChains && (!withThr || ctx->queueThr) && (!withL || ctx->queueL))
+    if (paths <= ctx->queueCap && chains <= ctx->queueChains && buffers <= ctx->queueBuffers &&
+        (!withThr || ctx->queueThr) && (!withL || ctx->queueL))
         return PRT_OK;
     for (int c = 0; c < kMaxChains; ++c)
         for (int i = 0; i < 2; ++i)
@@ -249,12 +254,14 @@ int ensure_queues(prt_ctx* ctx, long long paths, bool withThr, int chains = 1, b
     clear_graphs(ctx);
     long long cap = std::max(paths, ctx->queueCap);
     int nch = std::max(chains, ctx->queueChains);
+    int nbuf = std::max(buffers, ctx->queueBuffers);
     bool thr = withThr || ctx->queueThr;
     bool lq = withL || ctx->queueL;
     ctx->queueCap = 0;
     ctx->queueChains = 0;
+    ctx->queueBuffers = 0;
     for (int c = 0; c < nch; ++c)
-        for (int i = 0; i < 2; ++i)
+        for (int i = 0; i < nbuf; ++i)
         {
             CK(dev_malloc(&ctx->q[c][i], sizeof(PathRec) * (size_t)cap));
             if (thr) CK(dev_malloc(&ctx->thr[c][i], sizeof(float) * (size_t)cap));
@@ -262,6 +269,7 @@ int ensure_queues(prt_ctx* ctx, long long paths, bool withThr, int chains = 1, b
         }
     ctx->queueCap = cap;
     ctx->queueChains = nch;
+    ctx->queueBuffers = nbuf;
     ctx->queueThr = thr;
     ctx->queueL = lq;
     return PRT_OK;
@@ -283,6 +291,16 @@ float const_throughput(int depth)
     float t = 1.0f;
     for (int d = 0; d < depth; ++d) t *= 0.8f;
     return t;
+}
+
+// Counters of a wave chain: paths entering each depth, then the work counters
+// of the persistent loops, cleared together.
+int* chain_counts(const prt_ctx* ctx, int chain) { return ctx->dCounts + chain * 2 * kCounterStride; }
+int* chain_fetch(const prt_ctx* ctx, int chain) { return chain_counts(ctx, chain) + kCounterStride; }
+
+cudaError_t clear_chain(const prt_ctx* ctx, int chain, cudaStream_t s)
+{
+    return cudaMemsetAsync(chain_counts(ctx, chain), 0, sizeof(int) * 2 * kCounterStride, s);
 }
 
 int chains_for(const prt_ctx* ctx) { return std::max(1, std::min(kMaxChains, ctx->cfg.chains)); }
@@ -334,24 +352,27 @@ int record_render(prt_ctx* ctx, int spp, int maxDepth, int accumulate, int& laun
     {
         const int c = w % chains;
         cudaStream_t s = chains > 1 ? ctx->side[c] : ctx->stream;
-        int* counts = ctx->dCounts + c * kCounterStride;
-        int* fetch = ctx->dFetch + c * kCounterStride;
-        a.counts = counts;
-        a.fetch = fetch;
+        a.counts = chain_counts(ctx, c);
+        a.fetch = chain_fetch(ctx, c);
         a.passOffset = w * passesPerWave;
         a.passes = std::min(passesPerWave, spp - w * passesPerWave);
-        CK(cudaMemsetAsync(counts, 0, sizeof(int) * kCounterStride, s));
-        CK(cudaMemsetAsync(fetch, 0, sizeof(int) * kCounterStride, s));
-        for (int d = 0; d <= maxDepth; ++d)
+        CK(clear_chain(ctx, c, s));
+        // depth 0 fills the chain's queue, one launch carries its paths to their ends
+        a.qin = nullptr;
+        a.qout = ctx->q[c][0];
+        a.thrIn = nullptr;
+        a.thrOut = albedo ? ctx->thr[c][0] : nullptr;
+        a.Lin = nullptr;
+        a.Lout = nee ? ctx->Lq[c][0] : nullptr;
+        a.thrConst = const_throughput(0);
+        launches += launch_bounce(a, 0, ctx->cfg, ctx->numSMs, s);
+        if (maxDepth > 0)
         {
-            a.qin = d == 0 ? nullptr : ctx->q[c][(d - 1) & 1];
-            a.qout = ctx->q[c][d & 1];
-            a.thrIn = albedo && d > 0 ? ctx->thr[c][(d - 1) & 1] : nullptr;
-            a.thrOut = albedo ? ctx->thr[c][d & 1] : nullptr;
-            a.Lin = nee && d > 0 ? ctx->Lq[c][(d - 1) & 1] : nullptr;
-            a.Lout = nee ? ctx->Lq[c][d & 1] : nullptr;
-            a.thrConst = const_throughput(d);
-            launches += launch_bounce(a, d, ctx->cfg, ctx->numSMs, s);
+            a.qin = a.qout;
+            a.thrIn = a.thrOut;
+            a.Lin = a.Lout;
+            a.thrConst = const_throughput(1);
+            launches += launch_paths(a, ctx->cfg, ctx->numSMs, s);
         }
     }
     if (chains > 1)
@@ -401,9 +422,9 @@ int run_graph(prt_ctx* ctx, const std::string& key, const std::function<int(int&
 int finish_stats(prt_ctx* ctx, prt_render_stats* stats, int passes)
 {
     CK(cudaEventRecord(ctx->ev1, ctx->stream));
-    CK(cudaEventSynchronize(ctx->ev1));
-    unsigned long long rays = 0;
-    CK(cudaMemcpy(&rays, ctx->dRays, sizeof(rays), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpyAsync(ctx->hRays, ctx->dRays, sizeof(*ctx->hRays), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    const unsigned long long rays = *ctx->hRays;
     float ms = 0;
     CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
     if (stats)
@@ -685,7 +706,7 @@ prt_ctx::~prt_ctx()
     cudaFree(dPass);
     cudaFree(dRays);
     cudaFree(dCounts);
-    cudaFree(dFetch);
+    if (hRays) cudaFreeHost(hRays);
     for (int c = 0; c < kMaxChains; ++c)
     {
         for (int i = 0; i < 2; ++i)
@@ -733,8 +754,8 @@ int prt_create(int device, prt_ctx** out)
     CK(dev_malloc(&ctx->dPass, sizeof(int)));
     CK(cudaMemset(ctx->dPass, 0, sizeof(int)));
     CK(dev_malloc(&ctx->dRays, sizeof(unsigned long long)));
-    CK(dev_malloc(&ctx->dCounts, sizeof(int) * kCounterStride * kMaxChains));
-    CK(dev_malloc(&ctx->dFetch, sizeof(int) * kCounterStride * kMaxChains));
+    CK(dev_malloc(&ctx->dCounts, sizeof(int) * 2 * kCounterStride * kMaxChains));
+    CK(host_pinned_alloc(reinterpret_cast<char**>(&ctx->hRays), sizeof(*ctx->hRays)));
     CK(cudaEventCreateWithFlags(&ctx->forkEv, cudaEventDisableTiming));
     for (int c = 0; c < kMaxChains; ++c)
     {
@@ -810,15 +831,20 @@ int prt_set_albedo(prt_ctx* ctx, const float* albedo, int triCount)
     if (!ctx) return PRT_EINVAL;
     if (!ctx->haveMesh) return fail(ctx, PRT_ESTATE, "no scene loaded");
     CK(cudaSetDevice(ctx->device));
-    clear_graphs(ctx);
     if (!albedo)
     {
+        clear_graphs(ctx);
         cudaFree(ctx->dAlbedo);
         ctx->dAlbedo = nullptr;
         return PRT_OK;
     }
     if (triCount != ctx->nt) return fail(ctx, PRT_EINVAL, "albedo count differs from the triangle count");
-    if (!ctx->dAlbedo) CK(dev_malloc(&ctx->dAlbedo, sizeof(float) * (size_t)std::max(ctx->nt, 1)));
+    // captured graphs hold the array's address, so new values in the same array keep them
+    if (!ctx->dAlbedo)
+    {
+        clear_graphs(ctx);
+        CK(dev_malloc(&ctx->dAlbedo, sizeof(float) * (size_t)std::max(ctx->nt, 1)));
+    }
     if (ctx->nt)
         CK(cudaMemcpyAsync(ctx->dAlbedo, albedo, sizeof(float) * (size_t)ctx->nt, cudaMemcpyDefault, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
@@ -839,8 +865,8 @@ int prt_set_sky(prt_ctx* ctx, float sky)
 {
     if (!ctx) return PRT_EINVAL;
     if (!std::isfinite(sky)) return fail(ctx, PRT_EINVAL, "sky radiance must be finite");
+    if (std::memcmp(&ctx->sky, &sky, sizeof(sky)) != 0) clear_graphs(ctx);   // a kernel argument of captured graphs
     ctx->sky = sky;
-    clear_graphs(ctx);
     return PRT_OK;
 }
 
@@ -1054,7 +1080,7 @@ int prt_render_profile(prt_ctx* ctx, int spp, int maxDepth, double* msPerDepth, 
     const int ppw = passes_per_wave(ctx, spp);
     const bool albedo = ctx->dAlbedo != nullptr;
     const bool nee = ctx->integrator == PRT_INTEGRATOR_DIFFUSE2;
-    st = ensure_queues(ctx, (long long)ppw * perPass, albedo, 1, nee);
+    st = ensure_queues(ctx, (long long)ppw * perPass, albedo, 1, nee, 2);
     if (st != PRT_OK) return st;
     for (int d = 0; d <= maxDepth; ++d)
     {
@@ -1067,8 +1093,8 @@ int prt_render_profile(prt_ctx* ctx, int spp, int maxDepth, double* msPerDepth, 
     a.scene = scene_dev(ctx);
     a.cam = camera_dev(ctx->cam, W, H);
     a.accum = ctx->dAccum;
-    a.counts = ctx->dCounts;
-    a.fetch = ctx->dFetch;
+    a.counts = chain_counts(ctx, 0);
+    a.fetch = chain_fetch(ctx, 0);
     a.rays = ctx->dRays;
     a.passBase = ctx->dPass;
     a.tilesX = tilesX;
@@ -1080,8 +1106,7 @@ int prt_render_profile(prt_ctx* ctx, int spp, int maxDepth, double* msPerDepth, 
     {
         a.passOffset = p0;
         a.passes = std::min(ppw, spp - p0);
-        CK(cudaMemsetAsync(ctx->dCounts, 0, sizeof(int) * (kMaxDepthCap + 2), ctx->stream));
-        CK(cudaMemsetAsync(ctx->dFetch, 0, sizeof(int) * (kMaxDepthCap + 2), ctx->stream));
+        CK(clear_chain(ctx, 0, ctx->stream));
         CK(cudaEventRecord(ev[0], ctx->stream));
         for (int d = 0; d <= maxDepth; ++d)
         {
@@ -1097,7 +1122,7 @@ int prt_render_profile(prt_ctx* ctx, int spp, int maxDepth, double* msPerDepth, 
         }
         CK(cudaGetLastError());
         std::vector<int> counts((size_t)maxDepth + 2);
-        CK(cudaMemcpyAsync(counts.data(), ctx->dCounts, sizeof(int) * counts.size(), cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaMemcpyAsync(counts.data(), a.counts, sizeof(int) * counts.size(), cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
         for (int d = 0; d <= maxDepth; ++d)
         {
@@ -1194,9 +1219,9 @@ int prt_render_replay(prt_ctx* ctx, int pass0, int spp, int maxDepth, prt_render
     CK(cudaSetDevice(ctx->device));
     CK(cudaEventRecord(ctx->ev0, ctx->stream));
     CK(cudaMemsetAsync(ctx->dRays, 0, sizeof(unsigned long long), ctx->stream));
-    CK(cudaMemsetAsync(ctx->dFetch, 0, sizeof(unsigned long long), ctx->stream));
+    CK(clear_chain(ctx, 0, ctx->stream));
     ctx->launches += launch_replay(scene_dev(ctx), camera_dev(ctx->cam, ctx->W, ctx->H), ctx->dAccum, pass0, spp,
-                                   maxDepth, ctx->sky, nullptr, nullptr, nullptr, ctx->dRays, ctx->dFetch, false,
+                                   maxDepth, ctx->sky, nullptr, nullptr, nullptr, ctx->dRays, chain_fetch(ctx, 0), false,
                                    ctx->numSMs, ctx->stream);
     CK(cudaGetLastError());
     return finish_stats(ctx, stats, spp);
@@ -1228,9 +1253,9 @@ int prt_render_backward(prt_ctx* ctx, int pass0, int spp, int maxDepth, const fl
     else CK(dev_malloc(&gS, sizeof(float)));
     CK(cudaMemsetAsync(gA, 0, sizeof(float) * (size_t)ctx->nt, ctx->stream));
     CK(cudaMemsetAsync(gS, 0, sizeof(float), ctx->stream));
-    CK(cudaMemsetAsync(ctx->dFetch, 0, sizeof(unsigned long long), ctx->stream));
+    CK(clear_chain(ctx, 0, ctx->stream));
     ctx->launches += launch_replay(scene_dev(ctx), camera_dev(ctx->cam, ctx->W, ctx->H), ctx->dAccum, pass0, spp,
-                                   maxDepth, ctx->sky, gL, gA, gS, nullptr, ctx->dFetch, true, ctx->numSMs,
+                                   maxDepth, ctx->sky, gL, gA, gS, nullptr, chain_fetch(ctx, 0), true, ctx->numSMs,
                                    ctx->stream);
     CK(cudaGetLastError());
     if (!devA) CK(cudaMemcpyAsync(d_albedo, gA, sizeof(float) * (size_t)ctx->nt, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1341,17 +1366,18 @@ int prt_render_batch(prt_ctx* ctx, const prt_request* reqs, int n, prt_render_st
         {
             const int c = (int)(w % chains);
             cudaStream_t s = chains > 1 ? ctx->side[c] : ctx->stream;
-            a.counts = ctx->dCounts + c * kCounterStride;
-            a.fetch = ctx->dFetch + c * kCounterStride;
+            a.counts = chain_counts(ctx, c);
+            a.fetch = chain_fetch(ctx, c);
             a.waveBegin = w0;
             a.waveEnd = std::min(total, w0 + ppw);
-            CK(cudaMemsetAsync(a.counts, 0, sizeof(int) * kCounterStride, s));
-            CK(cudaMemsetAsync(a.fetch, 0, sizeof(int) * kCounterStride, s));
-            for (int d = 0; d <= maxDepth; ++d)
+            CK(clear_chain(ctx, c, s));
+            a.qin = nullptr;
+            a.qout = ctx->q[c][0];
+            launches += launch_batch_first(a, ctx->cfg, ctx->numSMs, s);
+            if (maxDepth > 0)
             {
-                a.qin = d == 0 ? nullptr : ctx->q[c][(d - 1) & 1];
-                a.qout = ctx->q[c][d & 1];
-                launches += launch_batch_bounce(a, d, ctx->cfg, ctx->numSMs, s);
+                a.qin = a.qout;
+                launches += launch_batch_paths(a, ctx->cfg, ctx->numSMs, s);
             }
         }
         if (chains > 1)

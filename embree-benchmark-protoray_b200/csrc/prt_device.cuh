@@ -521,7 +521,7 @@ __device__ __forceinline__ uint32_t node_hits1(const TravRay& r, const uint4* q,
 // node visit pushes at most one node group and one postponed triangle group,
 // so a tree of L 8-wide levels needs at most 2L entries.
 #ifndef PRT_STACK_SHARED
-#define PRT_STACK_SHARED 8
+#define PRT_STACK_SHARED 6
 #endif
 constexpr int kShared = PRT_STACK_SHARED;
 constexpr int kLocal = 64 - PRT_STACK_SHARED;

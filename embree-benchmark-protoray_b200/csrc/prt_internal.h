@@ -208,7 +208,7 @@ struct WaveArgs
     CameraDev cam;
     float4* accum;             // width*height sums (r,g,b,weight)
     PathRec* qin;              // input queue (depth >= 1)
-    PathRec* qout;             // output queue
+    PathRec* qout;             // output queue (depth 0, and the per-depth kernels)
     float* thrIn;              // per-path throughput (albedo mode), or nullptr
     float* thrOut;
     int* counts;               // counts[d]: paths entering bounce d (d >= 1)
@@ -265,6 +265,8 @@ struct LaunchCfg
 
 // Kernel launchers (render.cu).  Each returns the number of launches issued.
 int launch_bounce(const WaveArgs& a, int depth, const LaunchCfg& cfg, int numSMs, cudaStream_t s);
+// every bounce from depth 1 on (a.qin: the depth-1 queue, counts[1] paths)
+int launch_paths(const WaveArgs& a, const LaunchCfg& cfg, int numSMs, cudaStream_t s);
 // fetch: a zeroed work counter on the device, used by this launch only
 int launch_intersect(const SceneDev& sc, const RayRec* rays, HitRec* hits, int n, bool anyHit, float* anyOut,
                      int* fetch, int numSMs, cudaStream_t s);
@@ -277,7 +279,8 @@ int launch_query(const SceneDev& sc, const RayRec* ray, HitRec* hit, float* pNg,
 int launch_replay(const SceneDev& sc, const CameraDev& cam, float4* accum, int pass0, int spp, int maxDepth, float sky,
                   const float* dL, float* dAlbedo, float* dSky, unsigned long long* rays, int* fetch, bool backward,
                   int numSMs, cudaStream_t s);
-int launch_batch_bounce(const BatchArgs& a, int depth, const LaunchCfg& cfg, int numSMs, cudaStream_t s);
+int launch_batch_first(const BatchArgs& a, const LaunchCfg& cfg, int numSMs, cudaStream_t s);
+int launch_batch_paths(const BatchArgs& a, const LaunchCfg& cfg, int numSMs, cudaStream_t s);
 int launch_fill(float4* p, size_t n, cudaStream_t s);
 
 } // namespace prt_b200

@@ -2,11 +2,13 @@
 //
 // The reference GPU path (render/diffuse_renderer_cuda.cu:159-212) runs, per
 // pass: generateRaysKernel -> { OptiX Prime closest hit -> cudaMemcpy(counter)
-// -> shadeRaysKernel -> cudaMemcpy(count) } per bounce.  Here one persistent
-// kernel per bounce does traversal, shading, queue compaction and
-// accumulation together; primary rays are generated inside the first bounce
-// kernel; queue sizes stay on the device, so a whole render is launched
+// -> shadeRaysKernel -> cudaMemcpy(count) } per bounce.  Here a wave takes two
+// persistent kernels: the first generates, traces and shades the primary rays
+// and queues the paths that go on, the second (k_paths) carries those paths
+// to their ends.  Queue sizes stay on the device, so a whole render is launched
 // without host synchronisation (and is captured as a CUDA graph by the API).
+// k_bounce and k_bounce_nee with kFirst = false do one bounce of all paths
+// per launch, for prt_render_profile's times per depth.
 #include <algorithm>
 
 #include "prt_internal.h"
@@ -86,9 +88,12 @@ __device__ __forceinline__ int warp_append(bool pred, int* counter)
 #endif
 
 // Lanes refill once at least this many of a warp's 32 lanes are idle
-// (persistent threads with dynamic ray fetch, Aila & Laine, HPG 2009).
+// (persistent threads with dynamic ray fetch, Aila & Laine, HPG 2009): fewer
+// shade with emptier warps, more traverse with them.  14 against 12: primaries
+// per lane of a 33M-path terrain wave 8.10 -> 8.00 ms, a 32-request batch 31.45
+// -> 30.95 ms; 16 and 18 lose 0.5-2% on the 1080p terrain.
 #ifndef PRT_REFILL_MIN
-#define PRT_REFILL_MIN 12
+#define PRT_REFILL_MIN 14
 #endif
 constexpr int kRefillMin = PRT_REFILL_MIN;
 
@@ -354,6 +359,150 @@ __global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_bounce(WaveArgs 
             atomicAdd(&g_counters[5], cTriIters);
         }
     }
+}
+
+// All bounces after the first in one launch, for a wave (WaveArgs) or for a
+// wave of a batch (BatchArgs).  A lane takes a path from the depth-1 queue and
+// carries it to its end, bouncing in place, then takes the next one.  One
+// launch per bounce ends in a tail of its own, 60-100 us in which the longest
+// rays of that depth run on an emptying chip, and writes and compacts every
+// path; here a wave has one tail and a path is written once.  Rays of mixed
+// depths share a warp, which costs little: from the second ray on a path's
+// neighbours have scattered.  What a path needs only when it is shaded lives in
+// shared memory (kPathWords words per lane), so the registers hold what
+// traversal needs; with 6 stack entries per lane a block takes 15 KB, within
+// the step that leaves L1 124 KB.
+// Measured against one launch per bounce: 1080p terrain frame of 1 pass 2.12 ->
+// 1.88 ms and of 32 passes 46.4 -> 45.2, 256x256 and 16 passes of 82K triangles
+// 0.765 -> 0.63 ms, 10.24M-triangle field at 4 passes and 9 bounces 5.17 -> 4.72.
+constexpr int kPathWords = 7;   // tag (pixel; in a batch request << 24 | pixel), depth, RNG, throughput, direction
+
+__device__ __forceinline__ const SceneDev& path_scene(const WaveArgs& a, int) { return a.scene; }
+__device__ __forceinline__ float4* path_accum(const WaveArgs& a, uint32_t tag) { return a.accum + tag; }
+__device__ __forceinline__ int path_max_depth(const WaveArgs& a, int) { return a.maxDepth; }
+__device__ __forceinline__ const SceneDev& path_scene(const BatchArgs& a, int req) { return a.reqs[req].scene; }
+__device__ __forceinline__ float4* path_accum(const BatchArgs& a, uint32_t tag)
+{
+    return a.reqs[tag >> 24].accum + (tag & 0xffffffu);
+}
+__device__ __forceinline__ int path_max_depth(const BatchArgs& a, int req) { return a.reqs[req].maxDepth; }
+__device__ __forceinline__ bool path_deferred(const WaveArgs& a) { return a.scene.deferTris != 0; }
+__device__ __forceinline__ bool path_deferred(const BatchArgs& a) { return a.leaf1 != 0; }
+
+// Idle lanes of a warp at which it leaves traversal, act of its lanes holding a
+// ray: kRefillMin of a full warp, the same share of a partly filled one.
+__device__ __forceinline__ int stop_idle(unsigned act)
+{
+    const int n = __popc(act);
+    return 32 - n + max(1, n * kRefillMin / 32);
+}
+
+template <class Args, bool kBatch, bool kAlbedo>
+__global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_paths(Args a)
+{
+    extern __shared__ uint2 s_stack[];
+    TravStack st;
+    st.sh = s_stack + threadIdx.x;
+    st.stride = blockDim.x;
+    st.overflow = false;
+    uint32_t* s_path = reinterpret_cast<uint32_t*>(s_stack + kShared * blockDim.x);
+    uint32_t* path = s_path + threadIdx.x;   // word k of this lane's path at path[k * bd]
+    TriQueue* tq = reinterpret_cast<TriQueue*>(s_path + kPathWords * blockDim.x) + (threadIdx.x >> 5);   // deferred
+    const int bd = blockDim.x;
+    const unsigned FULL = 0xffffffffu;
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned ltMask = (1u << lane) - 1u;
+    const int total = *(volatile int*)&a.counts[1];
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(a.rays, (unsigned long long)total);
+    unsigned long long more = 0;   // rays of depth 2 and on, per warp
+
+    bool has = false;         // this lane holds a path
+    bool exhausted = false;   // warp-uniform: every queued path has been claimed
+    int req = 0;              // kBatch: the request of this lane's path
+    TravRay r;
+    TravState ts;
+    ts.done = true;
+    for (;;)
+    {
+        // --- lanes whose ray is traced: the path ends or bounces -----------------
+        bool fresh = false;   // this lane has a new ray (org, dir)
+        float3 org, dir;
+        if (has && ts.done)
+        {
+            const int depth = (int)path[bd];
+            float thr = __uint_as_float(path[3 * bd]);
+            if (ts.triHit < 0 || depth == path_max_depth(a, req))
+            {
+                const float c = ts.triHit < 0 ? __fmul_rn(thr, a.sky) : 0.0f;
+                red_add_v4(path_accum(a, path[0]), c, c, c, 1.0f);
+                has = false;
+            }
+            else
+            {
+                const SceneDev& sc = path_scene(a, req);
+                uint32_t rng = path[2 * bd];
+                org = r.org;
+                dir = f3(__uint_as_float(path[4 * bd]), __uint_as_float(path[5 * bd]), __uint_as_float(path[6 * bd]));
+                thr = __fmul_rn(thr, kAlbedo && sc.albedo ? __ldg(sc.albedo + ts.primHit) : 0.8f);
+                diffuse_bounce(sc.tris, ts.triHit, org, dir, ts.tHit, rng);
+                path[bd] = (uint32_t)(depth + 1);
+                path[2 * bd] = rng;
+                path[3 * bd] = __float_as_uint(thr);
+                fresh = true;
+            }
+        }
+        more += __popc(__ballot_sync(FULL, fresh));
+        // --- lanes without a path take the next ones ------------------------------
+        const unsigned idle = __ballot_sync(FULL, !has);
+        if (!exhausted && idle)
+        {
+            const int n = __popc(idle);
+            int base = 0;
+            if (lane == 0) base = atomicAdd(&a.fetch[1], n);
+            base = __shfl_sync(FULL, base, 0);
+            exhausted = base + n >= total;
+            const int i = base + __popc(idle & ltMask);
+            if (!has && i < total)
+            {
+                const PathRec pr = load_path(a.qin, i);
+                org = f3(pr.w0.x, pr.w0.y, pr.w0.z);
+                dir = f3(pr.w1.x, pr.w1.y, pr.w1.z);
+                const uint32_t tag = __float_as_uint(pr.w0.w);
+                if (kBatch) req = (int)(tag >> 24);
+                float thr = 0.8f;
+                if constexpr (!kBatch) thr = kAlbedo ? __ldcs(a.thrIn + i) : a.thrConst;
+                path[0] = tag;
+                path[bd] = 1u;
+                path[2 * bd] = __float_as_uint(pr.w1.w);
+                path[3 * bd] = __float_as_uint(thr);
+                has = fresh = true;
+            }
+        }
+        const unsigned act = __ballot_sync(FULL, has);
+        if (act == 0) break;   // every lane asked for a path above and the queue had none
+        if (fresh)
+        {
+            path[4 * bd] = __float_as_uint(dir.x);
+            path[5 * bd] = __float_as_uint(dir.y);
+            path[6 * bd] = __float_as_uint(dir.z);
+            trav_setup(r, org, dir);
+            trav_init(ts, path_scene(a, req), FLT_MAX, st);
+        }
+        // --- traverse until enough of the warp's rays are done ---------------------
+        const int stopIdle = stop_idle(act);
+        if (PRT_DEFER_TRIS && path_deferred(a))
+        {
+            warp_trav_deferred<PRT_PAIRED_LATER>(*tq, ts, path_scene(a, req), r, 0.0f, st, has, true, stopIdle, lane);
+        }
+        else
+        for (;;)
+        {
+            if (has && !ts.done) trav_step<false>(ts, path_scene(a, req), r, 0.0f, st);
+            const unsigned running = __ballot_sync(FULL, has && !ts.done);
+            if (32 - __popc(running) >= stopIdle) break;
+        }
+    }
+    if (lane == 0 && more) atomicAdd(a.rays, more);
 }
 
 // Primary rays as warp packets (trees with one-triangle leaves).  A warp takes
@@ -962,12 +1111,145 @@ __global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_bounce_nee(WaveA
     if (lane == 0 && shadowRays) atomicAdd(a.rays, shadowRays);
 }
 
+// k_paths for the next-event-estimation integrator: at a hit before maxDepth a
+// lane samples its shadow and extension rays from the same frame, traces the
+// shadow ray first (any hit; +0.5 * throughput * sky if it escapes) while the
+// extension ray waits in shared memory, then the extension ray.
+constexpr int kNeeWords = 11;   // pixel, depth | shadow << 8, RNG, throughput, radiance, direction, extension origin
+
+template <bool kAlbedo>
+__global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_paths_nee(WaveArgs a)
+{
+    extern __shared__ uint2 s_stack[];
+    TravStack st;
+    st.sh = s_stack + threadIdx.x;
+    st.stride = blockDim.x;
+    st.overflow = false;
+    uint32_t* s_path = reinterpret_cast<uint32_t*>(s_stack + kShared * blockDim.x);
+    uint32_t* path = s_path + threadIdx.x;   // word k of this lane's path at path[k * bd]
+    TriQueue* tq = reinterpret_cast<TriQueue*>(s_path + kNeeWords * blockDim.x) + (threadIdx.x >> 5);   // deferTris
+    const int bd = blockDim.x;
+    const unsigned FULL = 0xffffffffu;
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned ltMask = (1u << lane) - 1u;
+    const int total = *(volatile int*)&a.counts[1];
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(a.rays, (unsigned long long)total);
+    unsigned long long more = 0;   // shadow rays and extension rays of depth 2 and on, per warp
+
+    bool has = false, exhausted = false;
+    bool shadow = false;      // this lane's ray is a shadow ray
+    TravRay r;
+    TravState ts;
+    ts.done = true;
+    for (;;)
+    {
+        // --- lanes whose ray is traced ---------------------------------------------
+        bool fresh = false;   // this lane has a new ray (org, dir)
+        float3 org, dir;
+        if (has && ts.done)
+        {
+            const int depth = (int)(path[bd] & 0xffu);
+            float thr = __uint_as_float(path[3 * bd]), L = __uint_as_float(path[4 * bd]);
+            dir = f3(__uint_as_float(path[5 * bd]), __uint_as_float(path[6 * bd]), __uint_as_float(path[7 * bd]));
+            if (shadow)
+            {
+                if (ts.triHit < 0) L = __fadd_rn(L, __fmul_rn(__fmul_rn(thr, a.sky), 0.5f));
+                path[4 * bd] = __float_as_uint(L);
+                path[bd] = (uint32_t)(depth + 1);
+                org = f3(__uint_as_float(path[8 * bd]), __uint_as_float(path[9 * bd]), __uint_as_float(path[10 * bd]));
+                shadow = false;
+                fresh = true;
+            }
+            else if (ts.triHit < 0 || depth == a.maxDepth)
+            {
+                if (ts.triHit < 0) L = __fadd_rn(L, __fmul_rn(__fmul_rn(thr, a.sky), 0.5f));
+                red_add_v4(a.accum + path[0], L, L, L, 1.0f);
+                has = false;
+            }
+            else
+            {
+                thr = __fmul_rn(thr, kAlbedo && a.scene.albedo ? __ldg(a.scene.albedo + ts.primHit) : 0.8f);
+                uint32_t rng = path[2 * bd];
+                const HitFrame hf = hit_frame(a.scene.tris, ts.triHit, r.org, dir, ts.tHit);
+                float3 eo, ed;
+                sample_bounce(hf, rng, org, dir);   // shadow ray
+                sample_bounce(hf, rng, eo, ed);     // extension ray
+                path[bd] = (uint32_t)depth | 0x100u;
+                path[2 * bd] = rng;
+                path[3 * bd] = __float_as_uint(thr);
+                path[5 * bd] = __float_as_uint(ed.x);
+                path[6 * bd] = __float_as_uint(ed.y);
+                path[7 * bd] = __float_as_uint(ed.z);
+                path[8 * bd] = __float_as_uint(eo.x);
+                path[9 * bd] = __float_as_uint(eo.y);
+                path[10 * bd] = __float_as_uint(eo.z);
+                shadow = true;
+                fresh = true;
+            }
+        }
+        more += __popc(__ballot_sync(FULL, fresh));
+        // --- lanes without a path take the next ones ------------------------------
+        const unsigned idle = __ballot_sync(FULL, !has);
+        if (!exhausted && idle)
+        {
+            const int n = __popc(idle);
+            int base = 0;
+            if (lane == 0) base = atomicAdd(&a.fetch[1], n);
+            base = __shfl_sync(FULL, base, 0);
+            exhausted = base + n >= total;
+            const int i = base + __popc(idle & ltMask);
+            if (!has && i < total)
+            {
+                const PathRec pr = load_path(a.qin, i);
+                org = f3(pr.w0.x, pr.w0.y, pr.w0.z);
+                dir = f3(pr.w1.x, pr.w1.y, pr.w1.z);
+                path[0] = __float_as_uint(pr.w0.w);
+                path[bd] = 1u;
+                path[2 * bd] = __float_as_uint(pr.w1.w);
+                path[3 * bd] = __float_as_uint(kAlbedo ? __ldcs(a.thrIn + i) : a.thrConst);
+                path[4 * bd] = __float_as_uint(__ldcs(a.Lin + i));
+                path[5 * bd] = __float_as_uint(dir.x);
+                path[6 * bd] = __float_as_uint(dir.y);
+                path[7 * bd] = __float_as_uint(dir.z);
+                shadow = false;
+                has = fresh = true;
+            }
+        }
+        const unsigned act = __ballot_sync(FULL, has);
+        if (act == 0) break;   // every lane asked for a path above and the queue had none
+        if (fresh)
+        {
+            trav_setup(r, org, dir);
+            trav_init(ts, a.scene, FLT_MAX, st);
+        }
+        // --- traverse until enough of the warp's rays are done ---------------------
+        const int stopIdle = stop_idle(act);
+        if (PRT_DEFER_NEE && a.scene.deferTris)
+        {
+            warp_trav_deferred<PRT_PAIRED_NEE>(*tq, ts, a.scene, r, 0.0f, st, has, true, stopIdle, lane, nullptr, nullptr,
+                                               nullptr, nullptr, nullptr, shadow);
+        }
+        else
+        for (;;)
+        {
+            if (has && !ts.done) trav_step<false>(ts, a.scene, r, 0.0f, st, nullptr, nullptr, shadow);
+            const unsigned running = __ballot_sync(FULL, has && !ts.done);
+            if (32 - __popc(running) >= stopIdle) break;
+        }
+    }
+    if (lane == 0 && more) atomicAdd(a.rays, more);
+}
+
 // The IntersectorStreamCuda seam (core/intersector_stream_cuda.h:32-33):
 // closest or any hit for n ray records.  Persistent warps with the same
 // dynamic per-lane refill as k_bounce: a lane whose query is complete writes
-// its hit record, and once kRefillMin lanes of the warp are free they claim
+// its hit record, and once kQueryRefill lanes of the warp are free they claim
 // the next rays from the call's work counter, so incoherent queries of very
 // different lengths keep the warp's lanes busy.
+// Idle lanes at which the query kernel refills: writing a hit costs less than a
+// bounce (4M incoherent closest-hit queries 1.277 ms; 1.305 with 14).
+constexpr int kQueryRefill = 12;
+
 template <bool kAnyHit>
 __global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_intersect(SceneDev sc, const RayRec* __restrict__ rays,
                                                                          HitRec* __restrict__ hits,
@@ -994,7 +1276,7 @@ __global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_intersect(SceneD
     for (;;)
     {
         unsigned idle = __ballot_sync(FULL, !has);
-        if (!exhausted && (__popc(idle) >= kRefillMin || idle == FULL))
+        if (!exhausted && (__popc(idle) >= kQueryRefill || idle == FULL))
         {
             int cnt = __popc(idle);
             int base = 0;
@@ -1021,7 +1303,7 @@ __global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_intersect(SceneD
         if (PRT_DEFER_ISECT && sc.deferTris)
         {
             constexpr bool kPair = kAnyHit && PRT_PAIRED_QUERY;
-            warp_trav_deferred<kPair, !kAnyHit>(*tq, ts, sc, r, tnear, st, has, !exhausted, kRefillMin, lane, nullptr,
+            warp_trav_deferred<kPair, !kAnyHit>(*tq, ts, sc, r, tnear, st, has, !exhausted, kQueryRefill, lane, nullptr,
                                                 nullptr, nullptr, nullptr, nullptr, kAnyHit, tuv);
         }
         else
@@ -1030,7 +1312,7 @@ __global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_intersect(SceneD
             if (has && !ts.done) trav_step<kAnyHit>(ts, sc, r, tnear, st);
             unsigned running = __ballot_sync(FULL, has && !ts.done);
             if (running == 0) break;
-            if (!exhausted && 32 - __popc(running) >= kRefillMin) break;
+            if (!exhausted && 32 - __popc(running) >= kQueryRefill) break;
         }
         if (has && ts.done)
         {
@@ -1265,13 +1547,12 @@ __global__ void __launch_bounds__(128, 8) k_replay(SceneDev sc, CameraDev cam, f
     }
 }
 
-// Batched bounce: the paths of many requests share one queue.  Item i of the
-// first bounce is a global path index resolved to (request, pass, tile,
-// Morton index) by a binary search over the requests' path ranges; later
-// bounces carry (request << 24 | pixel) in the path record.  Lanes refill
-// dynamically as in k_bounce.
-template <bool kFirst>
-__global__ void __launch_bounds__(128, 8) k_batch_bounce(BatchArgs a, int depth)
+// First bounce of the batched renderer: the paths of many requests share one
+// queue.  Item i of a wave is a global path index resolved to (request, pass,
+// tile, Morton index) by a binary search over the requests' path ranges; the
+// queued path records carry (request << 24 | pixel).  Lanes refill dynamically
+// as in k_bounce; k_paths takes the queue.
+__global__ void __launch_bounds__(128, 8) k_batch_first(BatchArgs a)
 {
     extern __shared__ uint2 s_dyn[];
     uint2* s_stack = s_dyn;
@@ -1286,17 +1567,13 @@ __global__ void __launch_bounds__(128, 8) k_batch_bounce(BatchArgs a, int depth)
     const unsigned FULL = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned ltMask = (1u << lane) - 1u;
-    const long long total = kFirst ? (a.waveEnd - a.waveBegin) : (long long)*(volatile int*)&a.counts[depth];
-    if (!kFirst && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(a.rays, (unsigned long long)total);
+    const long long total = a.waveEnd - a.waveBegin;
     unsigned long long myRays = 0;
-    float thrDepth = 1.0f;
-    for (int d = 0; d < depth; ++d) thrDepth = __fmul_rn(thrDepth, 0.8f);
 
     bool has = false;
     bool exhausted = false;
     int pixel = 0, req = 0;
     uint32_t rng = 0;
-    int qi = 0;               // input-queue index of this lane's path (PRT_RELOAD_PATH)
     TravRay r;
     TravState ts;
     ts.done = true;
@@ -1307,7 +1584,7 @@ __global__ void __launch_bounds__(128, 8) k_batch_bounce(BatchArgs a, int depth)
         {
             int n = __popc(idle);
             int base = 0;
-            if (lane == 0) base = atomicAdd(&a.fetch[depth], n);
+            if (lane == 0) base = atomicAdd(&a.fetch[0], n);
             base = __shfl_sync(FULL, base, 0);
             if (base + n >= total) exhausted = true;
             int i = base + __popc(idle & ltMask);
@@ -1315,55 +1592,31 @@ __global__ void __launch_bounds__(128, 8) k_batch_bounce(BatchArgs a, int depth)
             {
                 float3 org, dir;
                 bool ok = true;
-                if (kFirst)
+                long long gi = a.waveBegin + i;
+                int lo = 0, hi = a.nreq - 1;
+                while (lo < hi)
                 {
-                    long long gi = a.waveBegin + i;
-                    int lo = 0, hi = a.nreq - 1;
-                    while (lo < hi)
-                    {
-                        int mid = (lo + hi + 1) >> 1;
-                        if (s_begin[mid] <= gi) lo = mid;
-                        else hi = mid - 1;
-                    }
-                    req = lo;
-                    const BatchReq& R = a.reqs[req];
-                    long long local = gi - s_begin[req];
-                    int perPass = R.tilesX * R.tilesY * 64;
-                    int pass = (int)(local / perPass);
-                    int x, y;
-                    if (!wave_item_pixel((int)(local - (long long)pass * perPass), R.tilesX, R.cam.width,
-                                         R.cam.height, x, y))
-                    {
-                        ok = false;
-                    }
-                    else
-                    {
-                        pixel = x + y * R.cam.width;
-                        rng = rng_seed(pass, pixel);
-                        camera_ray(R.cam, x, y, rng, org, dir);
-                        ++myRays;
-                    }
+                    int mid = (lo + hi + 1) >> 1;
+                    if (s_begin[mid] <= gi) lo = mid;
+                    else hi = mid - 1;
                 }
-                else if (PRT_RELOAD_PATH)
+                req = lo;
+                const BatchReq& R = a.reqs[req];
+                long long local = gi - s_begin[req];
+                int perPass = R.tilesX * R.tilesY * 64;
+                int pass = (int)(local / perPass);
+                int x, y;
+                if (!wave_item_pixel((int)(local - (long long)pass * perPass), R.tilesX, R.cam.width,
+                                     R.cam.height, x, y))
                 {
-                    // as in k_bounce: pixel, RNG and direction are read again when
-                    // the lane shades; the request id stays (it selects the scene)
-                    const float4* p = reinterpret_cast<const float4*>(a.qin + i);
-                    const float4 w0 = __ldcg(p), w1 = __ldcg(p + 1);
-                    org = f3(w0.x, w0.y, w0.z);
-                    dir = f3(w1.x, w1.y, w1.z);
-                    req = (int)((uint32_t)__float_as_int(w0.w) >> 24);
-                    qi = i;
+                    ok = false;
                 }
                 else
                 {
-                    PathRec pr = load_path(a.qin, i);
-                    org = f3(pr.w0.x, pr.w0.y, pr.w0.z);
-                    int tag = __float_as_int(pr.w0.w);
-                    req = (int)((uint32_t)tag >> 24);
-                    pixel = tag & 0xffffff;
-                    dir = f3(pr.w1.x, pr.w1.y, pr.w1.z);
-                    rng = __float_as_uint(pr.w1.w);
+                    pixel = x + y * R.cam.width;
+                    rng = rng_seed(pass, pixel);
+                    camera_ray(R.cam, x, y, rng, org, dir);
+                    ++myRays;
                 }
                 if (ok)
                 {
@@ -1380,8 +1633,7 @@ __global__ void __launch_bounds__(128, 8) k_batch_bounce(BatchArgs a, int depth)
         }
         if (PRT_DEFER_TRIS && a.leaf1)
         {
-            constexpr bool kPair = !kFirst && PRT_RELOAD_PATH && PRT_PAIRED_LATER;
-            warp_trav_deferred<kPair>(*tq, ts, a.reqs[req].scene, r, 0.0f, st, has, !exhausted, kRefillMin, lane);
+            warp_trav_deferred(*tq, ts, a.reqs[req].scene, r, 0.0f, st, has, !exhausted, kRefillMin, lane);
         }
         else
         for (;;)
@@ -1394,47 +1646,28 @@ __global__ void __launch_bounds__(128, 8) k_batch_bounce(BatchArgs a, int depth)
         const bool fin = has && ts.done;
         bool cont = false;
         float contrib = 0.f;
-        int fpix = 0;
-        uint32_t frng = 0;
-        float3 forg = r.org, fdir = f3(0.f, 0.f, 0.f);
+        float3 forg = r.org, fdir = r.dir;
         if (fin)
         {
-            if (!kFirst && PRT_RELOAD_PATH)
-            {
-                const float4* p = reinterpret_cast<const float4*>(a.qin + qi);
-                const float4 w1 = __ldcs(p + 1);
-                fpix = __float_as_int(__ldcs(reinterpret_cast<const float*>(p) + 3)) & 0xffffff;
-                fdir = f3(w1.x, w1.y, w1.z);
-                frng = __float_as_uint(w1.w);
-            }
-            else
-            {
-                fpix = pixel;
-                fdir = r.dir;
-                frng = rng;
-            }
             const BatchReq& R = a.reqs[req];
             if (ts.triHit < 0)
             {
-                contrib = __fmul_rn(thrDepth, a.sky);
+                contrib = a.sky;   // throughput 1
             }
-            else if (depth < R.maxDepth)
+            else if (R.maxDepth > 0)
             {
-                diffuse_bounce(R.scene.tris, ts.triHit, forg, fdir, ts.tHit, frng);
+                diffuse_bounce(R.scene.tris, ts.triHit, forg, fdir, ts.tHit, rng);
                 cont = true;
             }
         }
-        int o = warp_append(cont, &a.counts[depth + 1]);
-        if (cont) store_path(a.qout, o, forg, (req << 24) | fpix, fdir, frng);
-        else if (fin) red_add_v4(a.reqs[req].accum + fpix, contrib, contrib, contrib, 1.0f);
+        int o = warp_append(cont, &a.counts[1]);
+        if (cont) store_path(a.qout, o, forg, (req << 24) | pixel, fdir, rng);
+        else if (fin) red_add_v4(a.reqs[req].accum + pixel, contrib, contrib, contrib, 1.0f);
         if (fin) has = false;
     }
-    if (kFirst)
-    {
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) myRays += __shfl_down_sync(FULL, myRays, off);
-        if (lane == 0 && myRays) atomicAdd(a.rays, myRays);
-    }
+    for (int off = 16; off > 0; off >>= 1) myRays += __shfl_down_sync(FULL, myRays, off);
+    if (lane == 0 && myRays) atomicAdd(a.rays, myRays);
 }
 
 // Depth 0 of the batched renderer as warp packets (k_primary_packet's
@@ -1587,15 +1820,45 @@ int launch_bounce(const WaveArgs& a, int depth, const LaunchCfg& cfg, int numSMs
     return 1;
 }
 
-int launch_batch_bounce(const BatchArgs& a, int depth, const LaunchCfg& cfg, int numSMs, cudaStream_t s)
+namespace {
+
+template <class Args, class Kernel>
+void run_paths(Kernel kernel, const Args& a, int words, bool deferred, const LaunchCfg& cfg, int numSMs, cudaStream_t s)
+{
+    size_t shmem = (sizeof(uint2) * kShared + sizeof(uint32_t) * words) * cfg.block;
+    if (deferred) shmem += sizeof(TriQueue) * (cfg.block / 32);
+    const int grid = grid_for(kernel, cfg.block, shmem, numSMs, cfg);
+    kernel<<<grid, cfg.block, shmem, s>>>(a);
+}
+
+} // namespace
+
+int launch_paths(const WaveArgs& a, const LaunchCfg& cfg, int numSMs, cudaStream_t s)
+{
+    const bool albedo = a.thrIn != nullptr, deferred = PRT_DEFER_TRIS && a.scene.deferTris;
+    if (a.Lin)
+    {
+        const bool deferredNee = PRT_DEFER_NEE && a.scene.deferTris;
+        if (albedo) run_paths(k_paths_nee<true>, a, kNeeWords, deferredNee, cfg, numSMs, s);
+        else run_paths(k_paths_nee<false>, a, kNeeWords, deferredNee, cfg, numSMs, s);
+        return 1;
+    }
+    if (albedo) run_paths(k_paths<WaveArgs, false, true>, a, kPathWords, deferred, cfg, numSMs, s);
+    else run_paths(k_paths<WaveArgs, false, false>, a, kPathWords, deferred, cfg, numSMs, s);
+    return 1;
+}
+
+int launch_batch_paths(const BatchArgs& a, const LaunchCfg& cfg, int numSMs, cudaStream_t s)
+{
+    run_paths(k_paths<BatchArgs, true, false>, a, kPathWords, PRT_DEFER_TRIS && a.leaf1, cfg, numSMs, s);
+    return 1;
+}
+
+int launch_batch_first(const BatchArgs& a, const LaunchCfg& cfg, int numSMs, cudaStream_t s)
 {
     size_t shmem = sizeof(uint2) * kShared * cfg.block + sizeof(long long) * a.nreq;
     if (PRT_DEFER_TRIS && a.leaf1) shmem += sizeof(TriQueue) * (cfg.block / 32);
-    auto go = [&](auto kernel) {
-        int grid = grid_for(kernel, cfg.block, shmem, numSMs, cfg);
-        kernel<<<grid, cfg.block, shmem, s>>>(a, depth);
-    };
-    if (depth == 0 && PRT_PACKET_PRIMARY && cfg.packet && a.packet)
+    if (PRT_PACKET_PRIMARY && cfg.packet && a.packet)
     {
         const size_t pshmem = sizeof(long long) * a.nreq + sizeof(uint2) * kPacketStack * (cfg.block / 32);
         auto goPacket = [&](auto kernel) {
@@ -1606,8 +1869,8 @@ int launch_batch_bounce(const BatchArgs& a, int depth, const LaunchCfg& cfg, int
         else goPacket(k_batch_primary_packet<false>);
         return 1;
     }
-    if (depth == 0) go(k_batch_bounce<true>);
-    else go(k_batch_bounce<false>);
+    const int grid = grid_for(k_batch_first, cfg.block, shmem, numSMs, cfg);
+    k_batch_first<<<grid, cfg.block, shmem, s>>>(a);
     return 1;
 }
 

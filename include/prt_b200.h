@@ -274,7 +274,7 @@ int prt_get_tune(prt_ctx* ctx, prt_tune* tune);
  * callers that cannot allocate device memory at render time (an application
  * that owns the GPU's memory through its own pool, or a frame loop that cannot
  * afford cudaMalloc's implicit synchronisation).  Its path queues live in one
- * fixed 40 MiB device array per GPU, so frames are limited to 524288 pixels
+ * fixed 20 MiB device array per GPU, so frames are limited to 524288 pixels
  * after rounding up to 8x8 tiles (larger ones return PRT_EINVAL).  `accum`
  * must be 16-byte aligned device (or managed) memory of the context's GPU,
  * else PRT_EINVAL.  All calls on a device share that array: calls that overlap
