@@ -931,8 +931,12 @@ int build_bvh8_tree(const float* dPos, int nv, const int* dIdx, int nt, Bvh8Devi
 {
     (void)nv;
     int status = PRT_OK;
-    out.release();
-    if (nt <= 0) return PRT_OK;   // empty scene: no root
+    out.nodeCount = out.triCount = out.levels = 0;
+    if (nt <= 0)
+    {
+        out.release();
+        return PRT_OK;   // empty scene: no root
+    }
 
     const int n = nt;
     const int nInternal = n > 1 ? n - 1 : 0;
@@ -997,12 +1001,20 @@ int build_bvh8_tree(const float* dPos, int nv, const int* dIdx, int nt, Bvh8Devi
     carve(block);
     {
         const size_t nodeBytes = (sizeof(Bvh8Node) * (size_t)nodeCapacity + 255) & ~(size_t)255;
-        out.bytes = nodeBytes + sizeof(TriRec) * (size_t)n;
-        char* blk = nullptr;
-        BUILD_CHECK(dev_malloc(&blk, out.bytes));
-        out.block = blk;
-        out.nodes = reinterpret_cast<Bvh8Node*>(blk);
-        out.tris = reinterpret_cast<TriRec*>(blk + nodeBytes);
+        // a rebuild writes into the block of the last build if it fits: freeing
+        // and allocating hundreds of MB costs up to milliseconds and a device
+        // synchronisation
+        const size_t need = nodeBytes + sizeof(TriRec) * (size_t)n;
+        if (!out.block || out.bytes < need || out.bytes > 2 * need)
+        {
+            out.release();
+            char* blk = nullptr;
+            BUILD_CHECK(dev_malloc(&blk, need));
+            out.block = blk;
+            out.bytes = need;
+        }
+        out.nodes = reinterpret_cast<Bvh8Node*>(out.block);
+        out.tris = reinterpret_cast<TriRec*>(static_cast<char*>(out.block) + nodeBytes);
     }
 
     k_tri_boxes<<<boundBlocks, 256, 0, stream>>>(dPos, dIdx, n, triBox, partial);
@@ -1013,8 +1025,10 @@ int build_bvh8_tree(const float* dPos, int nv, const int* dIdx, int nt, Bvh8Devi
     {
         if (rebuild)
         {
-            top.tmp = keysB;   // free after the sort
-            BUILD_CHECK(sah_build_tree(n, triBox, cbounds, valsA, child, range, parent, top, numSMs, stream));
+            top.order[0] = keysA;   // free after the sort
+            top.order[1] = keysB;
+            BUILD_CHECK(sah_build_tree(n, triBox, cbounds, valsA, valsB, child, range, parent, top, numSMs, stream));
+            std::swap(valsA, valsB);
         }
         else
         {

@@ -121,27 +121,28 @@ int build_bvh8(const float* dPos, int nv, const int* dIdx, int nt, Bvh8Device& o
                DeviceScratch* scratch = nullptr);
 
 // Full SAH binary tree for the high-quality build (sah_build.cu): scratch
-// carved by sah_tree_carve (tmp: n free words the caller supplies), then
-// sah_build_tree writes child / range / parent of the n - 1 internal nodes
-// (root 0, leaves ~p for position p of perm) and reorders perm.
+// carved by sah_tree_carve (order: two arrays of n words the caller supplies),
+// then sah_build_tree writes child / range / parent of the n - 1 internal nodes
+// (root 0, leaves ~p for position p of out) and out, the triangles of perm in
+// the tree's order.
 struct TopTask;
 struct TopSplit;
 struct SahTreeBuffers
 {
     TopTask* task[2];
+    int4* chunks[2];
+    uint32_t* bins[2];
     TopSplit* splits;
-    uint32_t* bins;
-    uint32_t* leftCount;   // per chunk, then its exclusive scan
-    uint32_t* scanSums;
+    uint16_t* cum;
     int* small;
     int* counters;
-    int4* chunks;
-    uint32_t* tmp;
+    uint32_t* order[2];
     int maxTasks, maxChunks;
 };
 void sah_tree_carve(Carve& c, int n, SahTreeBuffers& B);
-cudaError_t sah_build_tree(int n, const float* triBox, const float* cbounds, uint32_t* perm, int2* child, int2* range,
-                           int* parent, const SahTreeBuffers& B, int numSMs, cudaStream_t stream);
+cudaError_t sah_build_tree(int n, const float* triBox, const float* cbounds, const uint32_t* perm, uint32_t* out,
+                           int2* child, int2* range, int* parent, const SahTreeBuffers& B, int numSMs,
+                           cudaStream_t stream);
 
 // Sort and scan primitives (sort_scan.cu).  radix_sort_pairs sorts (key, value)
 // pairs stably on key bits [0, bits); the sorted pairs end in keys/vals (the

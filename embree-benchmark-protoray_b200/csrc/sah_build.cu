@@ -21,8 +21,10 @@ namespace prt_b200 {
 // Task and split records of the top-down phase (declared in prt_internal.h).
 struct TopTask
 {
-    int lo, hi, node, pad;
-    float cmin[3], cmax[3];   // centroid bounds
+    int lo, hi, node;
+    int firstChunk, chunks;            // its chunks in the level's chunk list
+    int bins;                          // of several chunks: its merged bins
+    uint32_t cmin[3], cmax[3];         // centroid bounds as order-preserving bits (ford)
 };
 
 struct TopSplit
@@ -30,15 +32,10 @@ struct TopSplit
     int axis;       // -1: no bin separates the centroids; split the range in the middle
     int bin;        // left: bins 0..bin
     int nl;         // triangles going left
-    int pad;
-    // centroid bounds of the two halves, as order-preserving bits (ford):
-    // reduced with integer atomics by k_top_count
-    uint32_t cmin[2][3], cmax[2][3];
+    int task[2];    // the halves' tasks in the next level, -1: a subtree or a leaf
 };
 
 namespace {
-
-inline int div_up(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 __device__ __forceinline__ float box_half_area_lh(const float* lo, const float* hi)
 {
@@ -379,18 +376,32 @@ __global__ void __launch_bounds__(kSahLeaves) k_sah_rebuild(int n, const int* __
 // The high-quality build makes a full SAH tree instead of the Morton
 // hierarchy.  From the root (the triangles in Morton order), every task (a
 // node and its contiguous range of triangles) with more than kSahLeaves
-// triangles is split by the least SAH cost over
-// kTopBins centroid bins per axis (bin boxes and counts gathered per chunk of
-// the range in shared memory, then merged with atomics), its triangles are
-// partitioned into the two halves of the range, and the halves become the
-// next level's tasks, k_sah_rebuild's subtrees (2..kSahLeaves triangles) or
-// leaves.  The halves' centroid bounds (the next level's bin ranges) are
-// gathered by the counting pass over the split, not per bin.  One host
-// read-back per level (the next tasks' count and ranges) sizes the next
-// level's launches.
+// triangles is split by the least SAH cost over kTopBins centroid bins per axis,
+// its triangles are partitioned into the two halves of the range, and the
+// halves become the next level's tasks, k_sah_rebuild's subtrees
+// (2..kSahLeaves triangles) or leaves.
+//
+// A level is two launches over the chunks (kTopChunk triangles) of its tasks:
+//   k_top_bin        gathers the bins; the block that brings a task's last chunk
+//                    evaluates the split and makes the children, with their
+//                    tasks and chunks
+//   k_top_partition  moves the triangles to their halves, in order, and gathers
+//                    the halves' centroid bounds (the next level's bin ranges)
+// Task and chunk lists are made on the device, so levels are launched without
+// waiting for the host, which reads the task count back once per batch of
+// levels.  A level is a few tens of microseconds of work at 1.4M triangles, so
+// launches, host round trips and passes over the triangles are what bounds it.
+// Measured against nine launches per level (bins, split, count, children, a
+// scan, partition, copy back), a read-back per level and a new output block per
+// build: prt_build_accel of 82K triangles 2.78 -> 0.96 ms, 1.38M triangles 5.80
+// -> 3.25, 10.24M triangles 28.8 -> 21.4.
 constexpr int kTopBins = 32;
-constexpr int kTopChunk = 4096;        // triangles per block of the binning and partition passes
+constexpr int kTopChunk = 2048;        // triangles per block of the two passes
+constexpr int kTopBlock = 256;
 constexpr int kBinWords = 7;           // count, box lo, box hi (order-preserving float bits)
+constexpr int kTaskBins = 3 * kTopBins * kBinWords;
+constexpr int kTopSlots = 4;           // level l counts its tasks, chunks and merged bins in slot l & 3
+constexpr int kTopCounts = 3;
 
 __device__ __forceinline__ uint32_t ford(float f)
 {
@@ -413,191 +424,111 @@ __device__ __forceinline__ float top_scale(float cmin, float cmax)
     return e > 0.f ? (float)kTopBins * 0.99999f / e : 0.f;
 }
 
-__global__ void k_top_init_bins(uint32_t* bins, int words)
+// The empty value of word i of a task's bins: count 0; lo fields (1-3) start at
+// the largest value, hi fields (4-6) at 0.
+__device__ __forceinline__ uint32_t bin_empty(int i)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < words; i += gridDim.x * blockDim.x)
-    {
-        const int w = i % kBinWords;
-        // count 0; lo fields (1-3) start at the largest value, hi fields (4-6) at 0
-        bins[i] = w == 0 ? 0u : (w <= 3 ? 0xffffffffu : 0u);
-    }
+    const int w = i % kBinWords;
+    return w >= 1 && w <= 3 ? 0xffffffffu : 0u;
 }
 
-// Chunk c: task chunks[c].x, triangles [chunks[c].y, chunks[c].z].
-__global__ void __launch_bounds__(256) k_top_bin(const int4* __restrict__ chunks, const TopTask* __restrict__ tasks,
-                                                 const uint32_t* __restrict__ perm, const float* __restrict__ triBox,
-                                                 uint32_t* bins)
+// What a level reads and what it makes for the next one.
+struct TopArgs
 {
-    __shared__ uint32_t sb[3 * kTopBins * kBinWords];
-    const int4 ch = chunks[blockIdx.x];
-    const TopTask tk = tasks[ch.x];
-    for (int i = threadIdx.x; i < 3 * kTopBins * kBinWords; i += blockDim.x)
-    {
-        const int w = i % kBinWords;
-        sb[i] = w == 0 ? 0u : (w <= 3 ? 0xffffffffu : 0u);
-    }
-    __syncthreads();
-    float sc[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) sc[k] = top_scale(tk.cmin[k], tk.cmax[k]);
-    const unsigned lane = threadIdx.x & 31u;
-    for (int i0 = ch.y; i0 <= ch.z; i0 += blockDim.x)
-    {
-        // the lanes of a warp that fall into one bin (neighbours in the
-        // triangle order often do) merge their boxes with warp reductions and
-        // one lane updates the bin
-        const int i = i0 + threadIdx.x;
-        const bool valid = i <= ch.z;
-        uint32_t lo[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, hi[3] = {0, 0, 0};
-        float c[3] = {0.f, 0.f, 0.f};
-        if (valid)
-        {
-            const uint32_t tri = perm[i];
-#pragma unroll
-            for (int k = 0; k < 3; ++k)
-            {
-                const float bl = triBox[6 * (size_t)tri + k], bh = triBox[6 * (size_t)tri + 3 + k];
-                lo[k] = ford(bl);
-                hi[k] = ford(bh);
-                c[k] = 0.5f * (bl + bh);
-            }
-        }
-#pragma unroll
-        for (int ax = 0; ax < 3; ++ax)
-        {
-            const int bin = valid ? top_bin(c[ax], tk.cmin[ax], sc[ax]) : -1;
-            const unsigned peers = __match_any_sync(0xffffffffu, bin);
-            uint32_t r[7];
-            r[0] = __popc(peers);
-#pragma unroll
-            for (int k = 0; k < 3; ++k)
-            {
-                r[1 + k] = __reduce_min_sync(peers, lo[k]);
-                r[4 + k] = __reduce_max_sync(peers, hi[k]);
-            }
-            if (valid && lane == (unsigned)(__ffs(peers) - 1))
-            {
-                uint32_t* w = sb + (ax * kTopBins + bin) * kBinWords;
-                atomicAdd(w, r[0]);
-#pragma unroll
-                for (int k = 0; k < 3; ++k)
-                {
-                    atomicMin(w + 1 + k, r[1 + k]);
-                    atomicMax(w + 4 + k, r[4 + k]);
-                }
-            }
-        }
-    }
-    __syncthreads();
-    uint32_t* g = bins + (size_t)ch.x * 3 * kTopBins * kBinWords;
-    for (int i = threadIdx.x; i < 3 * kTopBins * kBinWords; i += blockDim.x)
-    {
-        const int w = i % kBinWords;
-        if (w == 0)
-        {
-            if (sb[i]) atomicAdd(g + i, sb[i]);
-        }
-        else if (w <= 3)
-        {
-            if (sb[i] != 0xffffffffu) atomicMin(g + i, sb[i]);
-        }
-        else if (sb[i])
-        {
-            atomicMax(g + i, sb[i]);
-        }
-    }
-}
+    int n;
+    const float* triBox;
+    const uint32_t* src;        // the level's triangles
+    uint32_t* dst;              // the next level's
+    uint32_t* out;              // the final order: subtrees and leaves
+    const TopTask* tasks;
+    const int4* chunks;         // {task, first triangle, last triangle, index in the task}
+    TopTask* nextTasks;
+    int4* nextChunks;
+    const int* count;           // [0] tasks, [1] chunks, [2] tasks of several chunks of this level
+    int* nextCount;             // of the next level
+    int* clearCount;            // of the level after it
+    TopSplit* splits;           // per task
+    uint32_t* bins;             // merged bins of the tasks of several chunks, last word: the chunks that have arrived
+    uint32_t* nextBins;
+    uint16_t* cum;              // per chunk of a task of several: [axis][bin] triangles in bins 0..bin
+    int* small;                 // subtree roots
+    int* numSmall;
+    int* nodeCounter;
+    int2* child;
+    int2* range;
+    int* parent;
+};
 
 __device__ __forceinline__ float shfl_ud(float v, int off, bool down)
 {
     return down ? __shfl_down_sync(0xffffffffu, v, off) : __shfl_up_sync(0xffffffffu, v, off);
 }
 
-// One warp per task, lane b = bin b: the least-cost split over the bins of
-// the three axes (prefix and suffix boxes by warp scans; ties to the lower
-// axis, then the lower bin).  The halves' centroid bounds start empty here
-// and are gathered by k_top_count.
-__global__ void k_top_split(const TopTask* __restrict__ tasks, int numTasks, const uint32_t* __restrict__ bins,
-                            TopSplit* splits)
+// Least-cost split over the bins of one axis (a warp, lane = bin; prefix and
+// suffix boxes by warp scans): (cost bits << 32) | (axis * 32 + bin), ~0 if no
+// bin separates the triangles.
+__device__ __forceinline__ unsigned long long axis_split(const uint32_t* bins, int ax, int lane)
 {
-    static_assert(kTopBins == 32, "one lane per bin");
-    const int ti = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (ti >= numTasks) return;   // warp-uniform
-    const int lane = threadIdx.x & 31;
-    const TopTask tk = tasks[ti];
-    const uint32_t* g = bins + (size_t)ti * 3 * kTopBins * kBinWords;
-    unsigned long long best = ~0ull;   // (cost bits << 32) | (axis * 32 + bin)
-    for (int ax = 0; ax < 3; ++ax)
+    const uint32_t* w = bins + (ax * kTopBins + lane) * kBinWords;
+    const int cnt = (int)w[0];
+    // left: inclusive prefix over bins 0..lane; right: suffix over lane..31
+    int lc = cnt, rc = cnt;
+    float llo[3], lhi[3], rlo[3], rhi[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
     {
-        const uint32_t* w = g + (ax * kTopBins + lane) * kBinWords;
-        const int cnt = (int)w[0];
-        float lo[3], hi[3];
+        llo[k] = rlo[k] = cnt ? funord(w[1 + k]) : FLT_MAX;
+        lhi[k] = rhi[k] = cnt ? funord(w[4 + k]) : -FLT_MAX;
+    }
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1)
+    {
+        const int ulc = __shfl_up_sync(0xffffffffu, lc, off);
+        const int drc = __shfl_down_sync(0xffffffffu, rc, off);
+        float ul[3], uh[3], dl[3], dh[3];
 #pragma unroll
         for (int k = 0; k < 3; ++k)
         {
-            lo[k] = cnt ? funord(w[1 + k]) : FLT_MAX;
-            hi[k] = cnt ? funord(w[4 + k]) : -FLT_MAX;
+            ul[k] = shfl_ud(llo[k], off, false);
+            uh[k] = shfl_ud(lhi[k], off, false);
+            dl[k] = shfl_ud(rlo[k], off, true);
+            dh[k] = shfl_ud(rhi[k], off, true);
         }
-        // left: inclusive prefix over bins 0..lane; right: suffix over lane..31
-        int lc = cnt, rc = cnt;
-        float llo[3], lhi[3], rlo[3], rhi[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
+        if (lane >= off)
         {
-            llo[k] = rlo[k] = lo[k];
-            lhi[k] = rhi[k] = hi[k];
-        }
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1)
-        {
-            const int ulc = __shfl_up_sync(0xffffffffu, lc, off);
-            const int drc = __shfl_down_sync(0xffffffffu, rc, off);
-            float ul[3], uh[3], dl[3], dh[3];
+            lc += ulc;
 #pragma unroll
             for (int k = 0; k < 3; ++k)
             {
-                ul[k] = shfl_ud(llo[k], off, false);
-                uh[k] = shfl_ud(lhi[k], off, false);
-                dl[k] = shfl_ud(rlo[k], off, true);
-                dh[k] = shfl_ud(rhi[k], off, true);
-            }
-            if (lane >= off)
-            {
-                lc += ulc;
-#pragma unroll
-                for (int k = 0; k < 3; ++k)
-                {
-                    llo[k] = fminf(llo[k], ul[k]);
-                    lhi[k] = fmaxf(lhi[k], uh[k]);
-                }
-            }
-            if (lane + off < 32)
-            {
-                rc += drc;
-#pragma unroll
-                for (int k = 0; k < 3; ++k)
-                {
-                    rlo[k] = fminf(rlo[k], dl[k]);
-                    rhi[k] = fmaxf(rhi[k], dh[k]);
-                }
+                llo[k] = fminf(llo[k], ul[k]);
+                lhi[k] = fmaxf(lhi[k], uh[k]);
             }
         }
-        // split after bin `lane`: the suffix from lane + 1
-        const int nrc = __shfl_down_sync(0xffffffffu, rc, 1);
-        float nlo[3], nhi[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
+        if (lane + off < 32)
         {
-            nlo[k] = __shfl_down_sync(0xffffffffu, rlo[k], 1);
-            nhi[k] = __shfl_down_sync(0xffffffffu, rhi[k], 1);
+            rc += drc;
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+            {
+                rlo[k] = fminf(rlo[k], dl[k]);
+                rhi[k] = fmaxf(rhi[k], dh[k]);
+            }
         }
-        if (lane < 31 && lc > 0 && nrc > 0)
-        {
-            const float c = box_half_area_lh(llo, lhi) * (float)lc + box_half_area_lh(nlo, nhi) * (float)nrc;
-            const unsigned long long key = ((unsigned long long)__float_as_uint(fmaxf(c, 0.f)) << 32) |
-                                           (unsigned)(ax * kTopBins + lane);
-            best = key < best ? key : best;
-        }
+    }
+    // split after bin `lane`: the suffix from lane + 1
+    const int nrc = __shfl_down_sync(0xffffffffu, rc, 1);
+    float nlo[3], nhi[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+    {
+        nlo[k] = __shfl_down_sync(0xffffffffu, rlo[k], 1);
+        nhi[k] = __shfl_down_sync(0xffffffffu, rhi[k], 1);
+    }
+    unsigned long long best = ~0ull;
+    if (lane < 31 && lc > 0 && nrc > 0)
+    {
+        const float c = box_half_area_lh(llo, lhi) * (float)lc + box_half_area_lh(nlo, nhi) * (float)nrc;
+        best = ((unsigned long long)__float_as_uint(fmaxf(c, 0.f)) << 32) | (unsigned)(ax * kTopBins + lane);
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1)
@@ -605,327 +536,518 @@ __global__ void k_top_split(const TopTask* __restrict__ tasks, int numTasks, con
         const unsigned long long o = __shfl_xor_sync(0xffffffffu, best, off);
         best = o < best ? o : best;
     }
-    TopSplit sp;
-    sp.pad = 0;
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-        {
-            sp.cmin[h][k] = 0xffffffffu;
-            sp.cmax[h][k] = 0u;
-        }
-    if (best == ~0ull)
-    {
-        sp.axis = -1;
-        sp.bin = 0;
-        sp.nl = (tk.hi - tk.lo + 1) / 2;
-    }
-    else
-    {
-        const int code = (int)(best & 0xffffffffu);
-        sp.axis = code / kTopBins;
-        sp.bin = code % kTopBins;
-        const uint32_t* w = g + (sp.axis * kTopBins + lane) * kBinWords;
-        const int cnt = (int)w[0];
-        sp.nl = __reduce_add_sync(0xffffffffu, lane <= sp.bin ? cnt : 0);
-    }
-    if (lane == 0) splits[ti] = sp;
+    return best;
 }
 
-// One thread per task: the two halves become internal nodes (next-level tasks
-// or rebuild subtrees) or leaves.
-__global__ void k_top_children(const TopTask* __restrict__ tasks, int numTasks, const TopSplit* __restrict__ splits,
-                               int n, TopTask* nextTasks, int* numNext,
-                               int* small, int* numSmall, int* nodeCounter, int2* child, int2* range, int* parent)
+// Adds the warp's triangles to the bins of one axis.  Neighbours in the
+// triangle order fall into few bins near the root and into many near the
+// leaves: up to four bins, each is reduced over the warp and one lane updates
+// it; beyond that the lanes update their bins themselves, since atomics on
+// different words run side by side and on the same word one by one.
+__device__ __forceinline__ void warp_bin(uint32_t* axisBins, int bin, const uint32_t* lo, const uint32_t* hi, unsigned lane)
 {
-    const int ti = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ti >= numTasks) return;
-    const TopTask tk = tasks[ti];
-    const TopSplit sp = splits[ti];
-    const int lo[2] = {tk.lo, tk.lo + sp.nl}, hi[2] = {tk.lo + sp.nl - 1, tk.hi};
-    int refs[2];
-    for (int side = 0; side < 2; ++side)
+    const unsigned FULL = 0xffffffffu;
+    const unsigned peers = __match_any_sync(FULL, bin);
+    unsigned leaders = __ballot_sync(FULL, bin >= 0 && lane == (unsigned)(__ffs(peers) - 1));
+    if (__popc(leaders) <= 4)
     {
-        const int size = hi[side] - lo[side] + 1;
-        if (size == 1)
+        while (leaders)
         {
-            refs[side] = ~lo[side];
-            parent[(n - 1) + lo[side]] = tk.node;
-            continue;
-        }
-        const int id = atomicAdd(nodeCounter, 1);
-        refs[side] = id;
-        parent[id] = tk.node;
-        range[id] = make_int2(lo[side], hi[side]);
-        if (size <= kSahLeaves)
-        {
-            small[atomicAdd(numSmall, 1)] = id;
-            continue;
-        }
-        TopTask c;
-        c.lo = lo[side];
-        c.hi = hi[side];
-        c.node = id;
-        c.pad = 0;
-        for (int k = 0; k < 3; ++k)
-        {
-            c.cmin[k] = funord(sp.cmin[side][k]);
-            c.cmax[k] = funord(sp.cmax[side][k]);
-        }
-        nextTasks[atomicAdd(numNext, 1)] = c;
-    }
-    child[tk.node] = make_int2(refs[0], refs[1]);
-}
-
-__device__ __forceinline__ int top_side(const TopTask& tk, const TopSplit& sp, float sc, int i, uint32_t tri,
-                                        const float* __restrict__ triBox)
-{
-    if (sp.axis < 0) return i - tk.lo < sp.nl ? 0 : 1;
-    const float c = 0.5f * (triBox[6 * (size_t)tri + sp.axis] + triBox[6 * (size_t)tri + 3 + sp.axis]);
-    return top_bin(c, tk.cmin[sp.axis], sc) <= sp.bin ? 0 : 1;
-}
-
-// Triangles of each chunk that go left, and the centroid bounds of the two
-// halves (merged into the task's split record with integer atomics on the
-// order-preserving bits).
-__global__ void __launch_bounds__(256) k_top_count(const int4* __restrict__ chunks, const TopTask* __restrict__ tasks,
-                                                   TopSplit* splits, const uint32_t* __restrict__ perm,
-                                                   const float* __restrict__ triBox, uint32_t* leftCount)
-{
-    __shared__ int warpCount[8];
-    const int4 ch = chunks[blockIdx.x];
-    const TopTask tk = tasks[ch.x];
-    TopSplit sp;
-    sp.axis = splits[ch.x].axis;
-    sp.bin = splits[ch.x].bin;
-    sp.nl = splits[ch.x].nl;
-    const float sc = sp.axis >= 0 ? top_scale(tk.cmin[sp.axis], tk.cmax[sp.axis]) : 0.f;
-    int mine = 0;
-    uint32_t cmin[2][3], cmax[2][3];
+            const int l = __ffs(leaders) - 1;
+            leaders &= leaders - 1;
+            const unsigned grp = __shfl_sync(FULL, peers, l);
+            const bool in = (grp >> lane) & 1u;
+            uint32_t r[6];
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-        {
-            cmin[h][k] = 0xffffffffu;
-            cmax[h][k] = 0u;
-        }
-    for (int i = ch.y + threadIdx.x; i <= ch.z; i += blockDim.x)
-    {
-        const uint32_t tri = perm[i];
-        const int side = top_side(tk, sp, sc, i, tri, triBox);
-        mine += side == 0;
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-        {
-            const uint32_t c = ford(0.5f * (triBox[6 * (size_t)tri + k] + triBox[6 * (size_t)tri + 3 + k]));
-            if (side == 0)
+            for (int k = 0; k < 3; ++k)
             {
-                cmin[0][k] = min(cmin[0][k], c);
-                cmax[0][k] = max(cmax[0][k], c);
+                r[k] = __reduce_min_sync(FULL, in ? lo[k] : 0xffffffffu);
+                r[3 + k] = __reduce_max_sync(FULL, in ? hi[k] : 0u);
+            }
+            if ((int)lane == l)
+            {
+                uint32_t* w = axisBins + bin * kBinWords;
+                atomicAdd(w, (uint32_t)__popc(grp));
+#pragma unroll
+                for (int k = 0; k < 3; ++k)
+                {
+                    atomicMin(w + 1 + k, r[k]);
+                    atomicMax(w + 4 + k, r[3 + k]);
+                }
+            }
+        }
+    }
+    else if (bin >= 0)
+    {
+        uint32_t* w = axisBins + bin * kBinWords;
+        atomicAdd(w, 1u);
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+        {
+            atomicMin(w + 1 + k, lo[k]);
+            atomicMax(w + 4 + k, hi[k]);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kTopBlock) k_top_bin(TopArgs a)
+{
+    __shared__ uint32_t sb[kTaskBins];
+    __shared__ unsigned long long s_best[3];
+    __shared__ int s_last, s_task[2], s_chunk[2], s_bins[2];
+    const unsigned lane = threadIdx.x & 31u;
+    const int warp = threadIdx.x >> 5;
+    const int numChunks = a.count[1];
+    for (int c = blockIdx.x; c < numChunks; c += gridDim.x)
+    {
+        const int4 ch = a.chunks[c];
+        const TopTask tk = a.tasks[ch.x];
+        float cmin[3], sc[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+        {
+            cmin[k] = funord(tk.cmin[k]);
+            sc[k] = top_scale(cmin[k], funord(tk.cmax[k]));
+        }
+        for (int i = threadIdx.x; i < kTaskBins; i += kTopBlock) sb[i] = bin_empty(i);
+        __syncthreads();
+        for (int i0 = ch.y; i0 <= ch.z; i0 += kTopBlock)
+        {
+            const int i = i0 + (int)threadIdx.x;
+            const bool valid = i <= ch.z;
+            uint32_t lo[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, hi[3] = {0, 0, 0};
+            int bin[3] = {-1, -1, -1};
+            if (valid)
+            {
+                const uint32_t tri = a.src[i];
+                const float2* bp = reinterpret_cast<const float2*>(a.triBox + 6 * (size_t)tri);
+                const float2 b0 = __ldg(bp), b1 = __ldg(bp + 1), b2 = __ldg(bp + 2);
+                const float bl[3] = {b0.x, b0.y, b1.x}, bh[3] = {b1.y, b2.x, b2.y};
+#pragma unroll
+                for (int k = 0; k < 3; ++k)
+                {
+                    lo[k] = ford(bl[k]);
+                    hi[k] = ford(bh[k]);
+                    bin[k] = top_bin(0.5f * (bl[k] + bh[k]), cmin[k], sc[k]);
+                }
+            }
+            if (__any_sync(0xffffffffu, valid))
+            {
+#pragma unroll
+                for (int ax = 0; ax < 3; ++ax) warp_bin(sb + ax * kTopBins * kBinWords, bin[ax], lo, hi, lane);
+            }
+        }
+        __syncthreads();
+        // a task of several chunks: the partition pass needs each chunk's
+        // counts, and the task's bins are merged in global memory
+        bool last = true;
+        if (tk.chunks > 1)
+        {
+            if (warp < 3)
+            {
+                int x = (int)sb[(warp * kTopBins + (int)lane) * kBinWords];
+#pragma unroll
+                for (int off = 1; off < 32; off <<= 1)
+                {
+                    const int y = __shfl_up_sync(0xffffffffu, x, off);
+                    if ((int)lane >= off) x += y;
+                }
+                a.cum[(size_t)c * 3 * kTopBins + warp * kTopBins + lane] = (uint16_t)x;
+            }
+            uint32_t* g = a.bins + (size_t)tk.bins * (kTaskBins + 1);
+            for (int i = threadIdx.x; i < kTaskBins; i += kTopBlock)
+            {
+                const uint32_t v = sb[i];
+                if (v == bin_empty(i)) continue;
+                const int w = i % kBinWords;
+                if (w == 0) atomicAdd(g + i, v);
+                else if (w <= 3) atomicMin(g + i, v);
+                else atomicMax(g + i, v);
+            }
+            __threadfence();
+            __syncthreads();
+            if (threadIdx.x == 0) s_last = atomicAdd(g + kTaskBins, 1u) == (uint32_t)tk.chunks - 1u;
+            __syncthreads();
+            last = s_last != 0;
+            if (last)
+            {
+                __threadfence();
+                for (int i = threadIdx.x; i < kTaskBins; i += kTopBlock) sb[i] = __ldcg(g + i);
+            }
+            __syncthreads();
+        }
+        if (!last) continue;   // block-uniform
+        // --- the split ----------------------------------------------------------
+        if (warp < 3)
+        {
+            const unsigned long long b = axis_split(sb, warp, (int)lane);
+            if (lane == 0) s_best[warp] = b;
+        }
+        __syncthreads();
+        if (warp == 0)
+        {
+            unsigned long long best = s_best[0];
+            if (s_best[1] < best) best = s_best[1];
+            if (s_best[2] < best) best = s_best[2];
+            TopSplit sp;
+            if (best == ~0ull)
+            {
+                sp.axis = -1;
+                sp.bin = 0;
+                sp.nl = (tk.hi - tk.lo + 1) / 2;
             }
             else
             {
-                cmin[1][k] = min(cmin[1][k], c);
-                cmax[1][k] = max(cmax[1][k], c);
+                const int code = (int)(best & 0xffffffffu);
+                sp.axis = code / kTopBins;
+                sp.bin = code % kTopBins;
+                const int cnt = (int)sb[(sp.axis * kTopBins + (int)lane) * kBinWords];
+                sp.nl = __reduce_add_sync(0xffffffffu, (int)lane <= sp.bin ? cnt : 0);
             }
-        }
-    }
-    mine = __reduce_add_sync(0xffffffffu, mine);
-    if ((threadIdx.x & 31) == 0) warpCount[threadIdx.x >> 5] = mine;
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-        {
-            const uint32_t lo = __reduce_min_sync(0xffffffffu, cmin[h][k]);
-            const uint32_t hi = __reduce_max_sync(0xffffffffu, cmax[h][k]);
-            if ((threadIdx.x & 31) == 0)
+            // --- the two halves: next-level tasks, subtrees or leaves -----------
+            if (lane < 2)
             {
-                if (lo != 0xffffffffu) atomicMin(&splits[ch.x].cmin[h][k], lo);
-                if (hi != 0u) atomicMax(&splits[ch.x].cmax[h][k], hi);
+                const int side = (int)lane;
+                const int lo = side == 0 ? tk.lo : tk.lo + sp.nl, hi = side == 0 ? tk.lo + sp.nl - 1 : tk.hi;
+                const int size = hi - lo + 1;
+                int ref = ~lo, task = -1, chunk = 0, bins = -1;
+                if (size == 1)
+                {
+                    a.parent[(a.n - 1) + lo] = tk.node;
+                }
+                else
+                {
+                    ref = atomicAdd(a.nodeCounter, 1);
+                    a.parent[ref] = tk.node;
+                    a.range[ref] = make_int2(lo, hi);
+                    if (size <= kSahLeaves)
+                    {
+                        a.small[atomicAdd(a.numSmall, 1)] = ref;
+                    }
+                    else
+                    {
+                        const int nch = (size + kTopChunk - 1) / kTopChunk;
+                        task = atomicAdd(a.nextCount, 1);
+                        chunk = atomicAdd(a.nextCount + 1, nch);
+                        if (nch > 1) bins = atomicAdd(a.nextCount + 2, 1);
+                        TopTask t;
+                        t.lo = lo;
+                        t.hi = hi;
+                        t.node = ref;
+                        t.firstChunk = chunk;
+                        t.chunks = nch;
+                        t.bins = bins;
+#pragma unroll
+                        for (int k = 0; k < 3; ++k)
+                        {
+                            t.cmin[k] = 0xffffffffu;
+                            t.cmax[k] = 0u;
+                        }
+                        a.nextTasks[task] = t;
+                    }
+                }
+                const int other = __shfl_xor_sync(0x3u, ref, 1);
+                const int otherTask = __shfl_xor_sync(0x3u, task, 1);
+                s_task[side] = task;
+                s_chunk[side] = chunk;
+                s_bins[side] = bins;
+                if (side == 0)
+                {
+                    a.child[tk.node] = make_int2(ref, other);
+                    sp.task[0] = task;
+                    sp.task[1] = otherTask;
+                    a.splits[ch.x] = sp;
+                }
+            }
+            if (lane == 0) s_last = sp.nl;
+        }
+        __syncthreads();
+        // the tasks' chunks, and empty bins for those of several
+        const int nl = s_last;
+        for (int side = 0; side < 2; ++side)
+        {
+            const int task = s_task[side], chunk = s_chunk[side];
+            if (task < 0) continue;
+            const int lo = side == 0 ? tk.lo : tk.lo + nl, hi = side == 0 ? tk.lo + nl - 1 : tk.hi;
+            const int nch = (hi - lo + kTopChunk) / kTopChunk;
+            for (int k = threadIdx.x; k < nch; k += kTopBlock)
+                a.nextChunks[chunk + k] =
+                    make_int4(task, lo + k * kTopChunk, min(hi, lo + (k + 1) * kTopChunk - 1), k);
+            if (nch > 1)
+                for (int i = threadIdx.x; i <= kTaskBins; i += kTopBlock)
+                    a.nextBins[(size_t)s_bins[side] * (kTaskBins + 1) + i] = i == kTaskBins ? 0u : bin_empty(i);
+        }
+        __syncthreads();
+    }
+}
+
+// The triangles of each chunk to their half of the task's range, in their
+// order: a half that is a task goes to dst, a subtree or a leaf to its place in
+// the final order.  The halves' centroid bounds go to their tasks with integer
+// atomics on the order-preserving bits.
+__global__ void __launch_bounds__(kTopBlock) k_top_partition(TopArgs a)
+{
+    __shared__ int warpCount[2][kTopBlock / 32];
+    __shared__ int s_before;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int numChunks = a.count[1];
+    if (blockIdx.x == 0 && threadIdx.x < kTopCounts) a.clearCount[threadIdx.x] = 0;
+    for (int c = blockIdx.x; c < numChunks; c += gridDim.x)
+    {
+        const int4 ch = a.chunks[c];
+        const TopTask tk = a.tasks[ch.x];
+        const TopSplit sp = a.splits[ch.x];
+        float cmin = 0.f, sc = 0.f;
+        if (sp.axis >= 0)
+        {
+            cmin = funord(tk.cmin[sp.axis]);
+            sc = top_scale(cmin, funord(tk.cmax[sp.axis]));
+        }
+        // left triangles of the task before this chunk
+        if (threadIdx.x == 0) s_before = 0;
+        __syncthreads();
+        if (sp.axis < 0)
+        {
+            if (threadIdx.x == 0) s_before = min(ch.y - tk.lo, sp.nl);
+        }
+        else if (ch.w > 0)
+        {
+            int sum = 0;
+            for (int k = threadIdx.x; k < ch.w; k += kTopBlock)
+                sum += a.cum[(size_t)(tk.firstChunk + k) * 3 * kTopBins + sp.axis * kTopBins + sp.bin];
+            sum = __reduce_add_sync(0xffffffffu, sum);
+            if (lane == 0 && sum) atomicAdd(&s_before, sum);
+        }
+        __syncthreads();
+        int baseL = s_before, baseR = (ch.y - tk.lo) - s_before;
+        uint32_t bmin[2][3], bmax[2][3];
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+            {
+                bmin[h][k] = 0xffffffffu;
+                bmax[h][k] = 0u;
+            }
+        uint32_t* const toL = sp.task[0] >= 0 ? a.dst : a.out;
+        uint32_t* const toR = sp.task[1] >= 0 ? a.dst : a.out;
+        for (int i0 = ch.y; i0 <= ch.z; i0 += kTopBlock)
+        {
+            const int i = i0 + (int)threadIdx.x;
+            const bool valid = i <= ch.z;
+            uint32_t tri = 0;
+            int side = 0;
+            if (valid)
+            {
+                tri = a.src[i];
+                const float2* bp = reinterpret_cast<const float2*>(a.triBox + 6 * (size_t)tri);
+                const float2 b0 = __ldg(bp), b1 = __ldg(bp + 1), b2 = __ldg(bp + 2);
+                const float cen[3] = {0.5f * (b0.x + b1.y), 0.5f * (b0.y + b2.x), 0.5f * (b1.x + b2.y)};
+                if (sp.axis < 0) side = i - tk.lo < sp.nl ? 0 : 1;
+                else
+                {
+                    const float cx = sp.axis == 0 ? cen[0] : (sp.axis == 1 ? cen[1] : cen[2]);
+                    side = top_bin(cx, cmin, sc) <= sp.bin ? 0 : 1;
+                }
+#pragma unroll
+                for (int k = 0; k < 3; ++k)
+                {
+                    const uint32_t o = ford(cen[k]);
+                    if (side == 0)
+                    {
+                        bmin[0][k] = min(bmin[0][k], o);
+                        bmax[0][k] = max(bmax[0][k], o);
+                    }
+                    else
+                    {
+                        bmin[1][k] = min(bmin[1][k], o);
+                        bmax[1][k] = max(bmax[1][k], o);
+                    }
+                }
+            }
+            const unsigned left = __ballot_sync(0xffffffffu, valid && side == 0);
+            const unsigned right = __ballot_sync(0xffffffffu, valid && side == 1);
+            if (lane == 0)
+            {
+                warpCount[0][warp] = __popc(left);
+                warpCount[1][warp] = __popc(right);
+            }
+            __syncthreads();
+            int before = 0, tl = 0, tr = 0;
+#pragma unroll
+            for (int w = 0; w < kTopBlock / 32; ++w)
+            {
+                if (w == warp) before = side == 0 ? tl : tr;
+                tl += warpCount[0][w];
+                tr += warpCount[1][w];
+            }
+            if (valid)
+            {
+                const unsigned m = side == 0 ? left : right;
+                const int r = (side == 0 ? baseL : baseR) + before + __popc(m & ((1u << lane) - 1u));
+                const int at = side == 0 ? tk.lo + r : tk.lo + sp.nl + r;
+                if (at <= tk.hi) (side == 0 ? toL : toR)[at] = tri;
+            }
+            baseL += tl;
+            baseR += tr;
+            __syncthreads();
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+        {
+            if (sp.task[h] < 0) continue;   // block-uniform
+            TopTask* t = a.nextTasks + sp.task[h];
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+            {
+                const uint32_t lo = __reduce_min_sync(0xffffffffu, bmin[h][k]);
+                const uint32_t hi = __reduce_max_sync(0xffffffffu, bmax[h][k]);
+                if (lane == 0)
+                {
+                    if (lo != 0xffffffffu) atomicMin(&t->cmin[k], lo);
+                    if (hi != 0u) atomicMax(&t->cmax[k], hi);
+                }
             }
         }
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-        int tot = 0;
-        for (int w = 0; w < 8; ++w) tot += warpCount[w];
-        leftCount[blockIdx.x] = (uint32_t)tot;
     }
-}
-
-// The triangles of each chunk to their half of the task's range (in tmp), in
-// their order: leftBase = the chunk's left triangles before it in its task
-// (exclusive scan of k_top_count's counts minus the scan at the task's first
-// chunk, chunks[c].w).
-__global__ void __launch_bounds__(256) k_top_partition(const int4* __restrict__ chunks,
-                                                       const TopTask* __restrict__ tasks,
-                                                       const TopSplit* __restrict__ splits,
-                                                       const uint32_t* __restrict__ perm,
-                                                       const float* __restrict__ triBox,
-                                                       const uint32_t* __restrict__ leftScan, uint32_t* tmp)
-{
-    __shared__ int warpCount[2][8];
-    const int4 ch = chunks[blockIdx.x];
-    const TopTask tk = tasks[ch.x];
-    const TopSplit sp = splits[ch.x];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const float sc = sp.axis >= 0 ? top_scale(tk.cmin[sp.axis], tk.cmax[sp.axis]) : 0.f;
-    int base[2];
-    base[0] = (int)(leftScan[blockIdx.x] - leftScan[ch.w]);
-    base[1] = (ch.y - tk.lo) - base[0];
-    for (int i0 = ch.y; i0 <= ch.z; i0 += blockDim.x)
-    {
-        const int i = i0 + threadIdx.x;
-        const bool valid = i <= ch.z;
-        uint32_t tri = 0;
-        int side = 0;
-        if (valid)
-        {
-            tri = perm[i];
-            side = top_side(tk, sp, sc, i, tri, triBox);
-        }
-        const unsigned left = __ballot_sync(0xffffffffu, valid && side == 0);
-        const unsigned right = __ballot_sync(0xffffffffu, valid && side == 1);
-        if (lane == 0)
-        {
-            warpCount[0][warp] = __popc(left);
-            warpCount[1][warp] = __popc(right);
-        }
-        __syncthreads();
-        if (valid)
-        {
-            int before = 0;
-            for (int w = 0; w < warp; ++w) before += warpCount[side][w];
-            const unsigned m = side == 0 ? left : right;
-            const int r = base[side] + before + __popc(m & ((1u << lane) - 1u));
-            const int dst = side == 0 ? tk.lo + r : tk.lo + sp.nl + r;
-            if (dst <= tk.hi) tmp[dst] = tri;
-        }
-        int tl = 0, tr = 0;
-        for (int w = 0; w < 8; ++w)
-        {
-            tl += warpCount[0][w];
-            tr += warpCount[1][w];
-        }
-        base[0] += tl;
-        base[1] += tr;
-        __syncthreads();
-    }
-}
-
-__global__ void k_top_copy(const int4* __restrict__ chunks, const uint32_t* __restrict__ tmp, uint32_t* perm)
-{
-    const int4 ch = chunks[blockIdx.x];
-    for (int i = ch.y + threadIdx.x; i <= ch.z; i += blockDim.x) perm[i] = tmp[i];
 }
 
 // The root: node 0 over all n triangles, a task (n > kSahLeaves) or a rebuild
-// subtree.  counters: [0] next-level tasks, [1] rebuild subtrees, [2] nodes.
-__global__ void k_top_root(const float* __restrict__ cbounds, int n, TopTask* tasks, int* small, int* counters,
-                           int2* range, int* parent)
+// subtree.  counters: [0] rebuild subtrees, [1] nodes, then the levels' slots.
+__global__ void k_top_root(const float* __restrict__ cbounds, int n, TopTask* tasks, int4* chunks, uint32_t* bins,
+                           int* small, int* counters, int2* range, int* parent)
 {
-    range[0] = make_int2(0, n - 1);
-    parent[0] = -1;
-    counters[0] = 0;
-    counters[1] = 0;
-    counters[2] = 1;
-    if (n <= kSahLeaves)
+    const int nch = (n + kTopChunk - 1) / kTopChunk;
+    if (threadIdx.x == 0)
     {
-        small[0] = 0;
+        range[0] = make_int2(0, n - 1);
+        parent[0] = -1;
+        counters[0] = n <= kSahLeaves ? 1 : 0;
         counters[1] = 1;
-        return;
+        for (int i = 0; i < kTopCounts * kTopSlots; ++i) counters[2 + i] = 0;
+        if (n <= kSahLeaves)
+        {
+            small[0] = 0;
+        }
+        else
+        {
+            counters[2] = 1;
+            counters[3] = nch;
+            counters[4] = 1;
+            TopTask t;
+            t.lo = 0;
+            t.hi = n - 1;
+            t.node = 0;
+            t.firstChunk = 0;
+            t.chunks = nch;
+            t.bins = 0;
+            for (int k = 0; k < 3; ++k)
+            {
+                t.cmin[k] = ford(cbounds[k]);
+                t.cmax[k] = ford(cbounds[3 + k]);
+            }
+            tasks[0] = t;
+        }
     }
-    TopTask t;
-    t.lo = 0;
-    t.hi = n - 1;
-    t.node = 0;
-    t.pad = 0;
-    for (int k = 0; k < 3; ++k)
-    {
-        t.cmin[k] = cbounds[k];
-        t.cmax[k] = cbounds[3 + k];
-    }
-    tasks[0] = t;
+    if (n <= kSahLeaves) return;
+    for (int k = threadIdx.x; k < nch; k += blockDim.x)
+        chunks[k] = make_int4(0, k * kTopChunk, min(n - 1, (k + 1) * kTopChunk - 1), k);
+    for (int i = threadIdx.x; i <= kTaskBins; i += blockDim.x) bins[i] = i == kTaskBins ? 0u : bin_empty(i);
 }
 
 } // namespace
 
 void sah_tree_carve(Carve& c, int n, SahTreeBuffers& B)
 {
+    // a level's tasks are disjoint ranges of more than kSahLeaves triangles, each
+    // with at most one partly filled chunk; those of several chunks have more
+    // than kTopChunk triangles
     B.maxTasks = n / (kSahLeaves + 1) + 2;
     B.maxChunks = n / kTopChunk + B.maxTasks + 2;
-    B.task[0] = c.take<TopTask>(B.maxTasks);
-    B.task[1] = c.take<TopTask>(B.maxTasks);
+    const int maxBins = n / (kTopChunk + 1) + 2;
+    for (int i = 0; i < 2; ++i)
+    {
+        B.task[i] = c.take<TopTask>(B.maxTasks);
+        B.chunks[i] = c.take<int4>(B.maxChunks);
+        B.bins[i] = c.take<uint32_t>((size_t)maxBins * (kTaskBins + 1));
+    }
     B.splits = c.take<TopSplit>(B.maxTasks);
-    B.bins = c.take<uint32_t>((size_t)B.maxTasks * 3 * kTopBins * kBinWords);
-    B.leftCount = c.take<uint32_t>(B.maxChunks);
-    B.scanSums = c.take<uint32_t>(scan_sums_entries(B.maxChunks));
+    B.cum = c.take<uint16_t>((size_t)B.maxChunks * 3 * kTopBins);
     B.small = c.take<int>((size_t)n / 2 + 1);
-    B.counters = c.take<int>(3);
-    B.chunks = c.take<int4>(B.maxChunks);
+    B.counters = c.take<int>(2 + kTopCounts * kTopSlots);
 }
 
-
 // Top-down binned SAH from the root down to subtrees of kSahLeaves triangles,
-// then k_sah_rebuild for those.  perm: the triangles (reordered in place).
-cudaError_t sah_build_tree(int n, const float* triBox, const float* cbounds, uint32_t* perm, int2* child, int2* range,
-                           int* parent, const SahTreeBuffers& B, int numSMs, cudaStream_t stream)
+// then k_sah_rebuild for those.  perm: the triangles in their starting order;
+// out: in the tree's order.
+cudaError_t sah_build_tree(int n, const float* triBox, const float* cbounds, const uint32_t* perm, uint32_t* out,
+                           int2* child, int2* range, int* parent, const SahTreeBuffers& B, int numSMs,
+                           cudaStream_t stream)
 {
-    k_top_root<<<1, 1, 0, stream>>>(cbounds, n, B.task[0], B.small, B.counters, range, parent);
+    k_top_root<<<1, 256, 0, stream>>>(cbounds, n, B.task[0], B.chunks[0], B.bins[0], B.small, B.counters, range, parent);
     cudaError_t e = cudaGetLastError();
-    int numTasks = n > kSahLeaves ? 1 : 0;
-    int cur = 0;
-    std::vector<TopTask> host(1);   // the tasks' ranges (the root's is known)
-    host[0].lo = 0;
-    host[0].hi = n - 1;
-    std::vector<int4> chunks;
-    while (e == cudaSuccess && numTasks > 0)
+    if (n <= kSahLeaves)
     {
-        if (numTasks > B.maxTasks) return cudaErrorInvalidValue;
-        chunks.clear();
-        for (int ti = 0; ti < numTasks; ++ti)
-        {
-            const int first = (int)chunks.size();
-            for (int s = host[ti].lo; s <= host[ti].hi; s += kTopChunk)
-                chunks.push_back(make_int4(ti, s, std::min(host[ti].hi, s + kTopChunk - 1), first));
-        }
-        const int nch = (int)chunks.size();
-        if (nch > B.maxChunks) return cudaErrorInvalidValue;
-        e = cudaMemcpyAsync(B.chunks, chunks.data(), sizeof(int4) * nch, cudaMemcpyHostToDevice, stream);
-        if (e != cudaSuccess) break;
-        const int words = numTasks * 3 * kTopBins * kBinWords;
-        k_top_init_bins<<<std::min(div_up(words, 256), 4 * numSMs), 256, 0, stream>>>(B.bins, words);
-        k_top_bin<<<nch, 256, 0, stream>>>(B.chunks, B.task[cur], perm, triBox, B.bins);
-        k_top_split<<<div_up(numTasks, 4), 128, 0, stream>>>(B.task[cur], numTasks, B.bins, B.splits);
-        k_top_count<<<nch, 256, 0, stream>>>(B.chunks, B.task[cur], B.splits, perm, triBox, B.leftCount);
-        e = cudaMemsetAsync(B.counters, 0, sizeof(int), stream);
-        if (e != cudaSuccess) break;
-        k_top_children<<<div_up(numTasks, 128), 128, 0, stream>>>(B.task[cur], numTasks, B.splits, n,
-                                                                   B.task[cur ^ 1], B.counters, B.small,
-                                                                   B.counters + 1, B.counters + 2, child, range,
-                                                                   parent);
-        exclusive_scan_u32(B.leftCount, B.leftCount, B.scanSums, nch, stream);
-        k_top_partition<<<nch, 256, 0, stream>>>(B.chunks, B.task[cur], B.splits, perm, triBox, B.leftCount, B.tmp);
-        k_top_copy<<<nch, 256, 0, stream>>>(B.chunks, B.tmp, perm);
-        e = cudaGetLastError();
-        // one read-back per level: the count and the ranges of the next tasks
-        // (at most two per task)
-        const int cap = std::min(B.maxTasks, 2 * numTasks);
-        host.resize(cap);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&numTasks, B.counters, sizeof(int), cudaMemcpyDeviceToHost, stream);
         if (e == cudaSuccess)
-            e = cudaMemcpyAsync(host.data(), B.task[cur ^ 1], sizeof(TopTask) * cap, cudaMemcpyDeviceToHost, stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-        cur ^= 1;
+            e = cudaMemcpyAsync(out, perm, sizeof(uint32_t) * (size_t)n, cudaMemcpyDeviceToDevice, stream);
+    }
+    else
+    {
+        int binSM = 1, partSM = 1;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&binSM, k_top_bin, kTopBlock, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&partSM, k_top_partition, kTopBlock, 0);
+        // enough levels for SAH splits of ordinary scenes, then more at a time
+        int batch = 4;
+        for (int m = n; m > kSahLeaves; m >>= 1) ++batch;
+        int level = 0;
+        for (;;)
+        {
+            for (int l = 0; l < batch && e == cudaSuccess; ++l, ++level)
+            {
+                TopArgs a;
+                a.n = n;
+                a.triBox = triBox;
+                a.src = level == 0 ? perm : B.order[(level - 1) & 1];
+                a.dst = B.order[level & 1];
+                a.out = out;
+                a.tasks = B.task[level & 1];
+                a.chunks = B.chunks[level & 1];
+                a.nextTasks = B.task[(level + 1) & 1];
+                a.nextChunks = B.chunks[(level + 1) & 1];
+                a.count = B.counters + 2 + kTopCounts * (level & (kTopSlots - 1));
+                a.nextCount = B.counters + 2 + kTopCounts * ((level + 1) & (kTopSlots - 1));
+                a.clearCount = B.counters + 2 + kTopCounts * ((level + 2) & (kTopSlots - 1));
+                a.splits = B.splits;
+                a.bins = B.bins[level & 1];
+                a.nextBins = B.bins[(level + 1) & 1];
+                a.cum = B.cum;
+                a.small = B.small;
+                a.numSmall = B.counters;
+                a.nodeCounter = B.counters + 1;
+                a.child = child;
+                a.range = range;
+                a.parent = parent;
+                const long long bound =
+                    std::min<long long>(B.maxChunks, (long long)n / kTopChunk + 1 + (level < 30 ? 1ll << level : 1ll << 30));
+                k_top_bin<<<(int)std::min<long long>(bound, (long long)binSM * numSMs), kTopBlock, 0, stream>>>(a);
+                k_top_partition<<<(int)std::min<long long>(bound, (long long)partSM * numSMs), kTopBlock, 0, stream>>>(a);
+                e = cudaGetLastError();
+            }
+            int numTasks = 0;
+            if (e == cudaSuccess)
+                e = cudaMemcpyAsync(&numTasks, B.counters + 2 + kTopCounts * (level & (kTopSlots - 1)), sizeof(int),
+                                    cudaMemcpyDeviceToHost, stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+            if (e != cudaSuccess || numTasks == 0) break;
+            if (numTasks > B.maxTasks) return cudaErrorInvalidValue;
+            batch = 8;
+        }
     }
     if (e != cudaSuccess) return e;
     int perSM = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_sah_rebuild, kSahLeaves, 0);
-    k_sah_rebuild<<<std::max(1, perSM) * numSMs, kSahLeaves, 0, stream>>>(n, B.small, B.counters + 1, triBox, perm,
-                                                                       child, range, parent, B.counters + 2);
+    k_sah_rebuild<<<std::max(1, perSM) * numSMs, kSahLeaves, 0, stream>>>(n, B.small, B.counters, triBox, out, child,
+                                                                       range, parent, B.counters + 1);
     return cudaGetLastError();
 }
 
