@@ -43,330 +43,397 @@ __device__ __forceinline__ float box_half_area_lh(const float* lo, const float* 
     return dx * dy + dy * dz + dz * dx;
 }
 
-// --- subtrees of at most kSahLeaves triangles: exact sweep SAH, one block each -
+__device__ __forceinline__ uint32_t ford(float f)
+{
+    const uint32_t u = __float_as_uint(f);
+    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float funord(uint32_t u)
+{
+    return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
+}
+
+// --- subtrees of at most kSahLeaves triangles: exact sweep SAH, three warps each -
 //
 // A subtree of 2..kSahLeaves triangles covers a contiguous range [a, b] of the
-// triangle order; one block builds it top-down to single-triangle leaves, all
-// nodes of a depth at once, permuting the triangles only inside [a, b].
+// triangle order; one block of three warps, a warp per axis, builds it top-down
+// to single-triangle leaves, all nodes of a depth at once, permuting the
+// triangles only inside [a, b].
 // Splits: for each axis the range's triangles sorted by centroid, the split
 // after position p costs area(left box) x |left| + area(right box) x |right|;
 // the least cost wins (ties to the more balanced split, then the lower axis
 // and position).
+// The nodes of a depth are segments of the position range.  A warp walks its
+// axis' positions in windows of 32, with segmented shuffle scans inside a window
+// and a carry between windows, and windows whose segments are all single
+// triangles are skipped; the warps meet at five barriers per depth.  The latency
+// of the scans bounds it; element indices, segment ids and segment ends are
+// bytes, so a subtree takes 15 KB of shared memory and an SM holds 14 of them.
+// Measured against one 256-thread block per subtree, whose scans stepped over
+// shared memory with two barriers a step: prt_build_accel of 1.38M triangles 3.25
+// -> 2.55 ms, 10.24M triangles 21.4 -> 15.7 (one warp for all three axes: 2.81 and
+// 17.2, and 82K triangles 12% slower).
 constexpr int kSahLeaves = 256;
 
 struct SahShared
 {
-    float box[6][kSahLeaves];         // triangle boxes of the range (lo xyz, hi xyz)
-    float cen[3][kSahLeaves];         // doubled centroids
-    int list[2][3][kSahLeaves];       // per axis: elements in centroid order (double buffered)
-    float scan[6][kSahLeaves];        // prefix / suffix boxes of one axis list
-    float preArea[kSahLeaves];        // area of the prefix box ending at each position
-    unsigned long long best[kSahLeaves];   // per segment: least split key
-    int segStart[kSahLeaves], segEnd[kSahLeaves], segNode[kSahLeaves], segRight[kSahLeaves];
-    int segOf[kSahLeaves];            // per position: its segment
-    int rank[3][kSahLeaves];          // segmented scan of the left marks, per axis list
-    int orig[kSahLeaves];             // triangle id of each element
-    int pool[kSahLeaves];             // internal node indices of the subtree (root first)
-    unsigned char mark[kSahLeaves];   // element goes left
-    int nseg, poolNext, splitting, rootPos;   // rootPos: the first new node index
-    int maxSeg, nextMaxSeg;   // largest segment of this depth / of the next
+    float box[6][kSahLeaves];           // triangle boxes of the range (lo xyz, hi xyz)
+    float suffix[3][kSahLeaves];        // per axis list: area of the box from each position to its segment's end
+    unsigned long long best[kSahLeaves];    // per segment: least split key, ~0 for a single triangle
+    uint8_t list[2][3][kSahLeaves];     // per axis: elements in centroid order (double buffered)
+    uint8_t segOf[kSahLeaves];          // per position: its segment
+    uint8_t mark[kSahLeaves];           // per element: it goes left
+    // per segment: first and last position, node (0: the root, k: the k-th new
+    // one), the segment of its right half; per axis: left marks before its start
+    uint8_t segStart[kSahLeaves], segEnd[kSahLeaves], segNode[kSahLeaves], segRight[kSahLeaves];
+    uint8_t segBase[3][kSahLeaves];
+    int first, nseg, maxSeg;            // node index of pool entry 1; segments, and the largest, of this depth
 };
 
-__device__ __forceinline__ float area6(float lx, float ly, float lz, float hx, float hy, float hz)
+__device__ __forceinline__ float area6(const float* v)
 {
-    const float dx = hx - lx, dy = hy - ly, dz = hz - lz;
+    const float dx = v[3] - v[0], dy = v[4] - v[1], dz = v[5] - v[2];
     return dx * dy + dy * dz + dz * dx;
+}
+
+__device__ __forceinline__ void box_merge(float* v, const float* w)
+{
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+    {
+        v[k] = fminf(v[k], w[k]);
+        v[3 + k] = fmaxf(v[3 + k], w[3 + k]);
+    }
+}
+
+// Sorts the kSahLeaves (key, idx) pairs of a warp, pair lane * 8 + r in
+// register r, by key then idx (bitonic; strides below 8 inside a lane).
+__device__ __forceinline__ void warp_sort256(uint32_t* key, uint32_t* idx, int lane)
+{
+#pragma unroll
+    for (int size = 2; size <= kSahLeaves; size <<= 1)
+    {
+#pragma unroll
+        for (int stride = size >> 1; stride > 0; stride >>= 1)
+        {
+            if (stride >= 8)
+            {
+                const bool lower = (lane & (stride >> 3)) == 0;
+#pragma unroll
+                for (int r = 0; r < 8; ++r)
+                {
+                    const uint32_t ko = __shfl_xor_sync(0xffffffffu, key[r], stride >> 3);
+                    const uint32_t io = __shfl_xor_sync(0xffffffffu, idx[r], stride >> 3);
+                    const bool up = ((lane * 8) & size) == 0;
+                    const bool greater = key[r] > ko || (key[r] == ko && idx[r] > io);
+                    if (greater == (lower == up))
+                    {
+                        key[r] = ko;
+                        idx[r] = io;
+                    }
+                }
+            }
+            else
+            {
+#pragma unroll
+                for (int r = 0; r < 8; ++r)
+                {
+                    if (r & stride) continue;
+                    const bool up = ((lane * 8 + r) & size) == 0;
+                    const uint32_t k0 = key[r], k1 = key[r + stride], i0 = idx[r], i1 = idx[r + stride];
+                    const bool greater = k0 > k1 || (k0 == k1 && i0 > i1);
+                    if (greater == up)
+                    {
+                        key[r] = k1;
+                        key[r + stride] = k0;
+                        idx[r] = i1;
+                        idx[r + stride] = i0;
+                    }
+                }
+            }
+        }
+    }
 }
 
 // One subtree per block: roots[i] is its root (an internal node whose range
 // holds 2..kSahLeaves triangles); its other internal nodes take new indices
 // from *nodeCounter.
-__global__ void __launch_bounds__(kSahLeaves) k_sah_rebuild(int n, const int* __restrict__ roots,
-                                                          const int* __restrict__ numRoots,
-                                                          const float* __restrict__ triBox, uint32_t* vals,
-                                                          int2* child, int2* range, int* parent, int* nodeCounter)
+__global__ void __launch_bounds__(96) k_sah_subtrees(int n, const int* __restrict__ roots,
+                                                   const int* __restrict__ numRoots, const float* __restrict__ triBox,
+                                                   uint32_t* vals, int2* child, int2* range, int* parent,
+                                                   int* nodeCounter)
 {
     __shared__ SahShared S;
-    const int t = threadIdx.x;
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int ax = threadIdx.x >> 5;   // this warp's axis
+    const unsigned lt = (1u << lane) - 1u;
     const int count = *numRoots;
     for (int ri = blockIdx.x; ri < count; ri += gridDim.x)
     {
         const int u = roots[ri];
         const int2 rg = range[u];
         const int a = rg.x, ns = rg.y - rg.x + 1;   // 2 <= ns <= kSahLeaves
-        if (t == 0) S.rootPos = ns > 2 ? atomicAdd(nodeCounter, ns - 2) : 0;   // first new index
+        const int nw = (ns + 31) >> 5;
         // --- load the range ---------------------------------------------------
-        if (t < ns)
+        for (int t = threadIdx.x; t < ns; t += 96)
         {
             const uint32_t tri = vals[a + t];
-            S.orig[t] = (int)tri;
-#pragma unroll
-            for (int k = 0; k < 6; ++k) S.box[k][t] = triBox[6 * (size_t)tri + k];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) S.cen[k][t] = S.box[k][t] + S.box[3 + k][t];
+            const float2* bp = reinterpret_cast<const float2*>(triBox + 6 * (size_t)tri);
+            const float2 b0 = __ldg(bp), b1 = __ldg(bp + 1), b2 = __ldg(bp + 2);
+            S.box[0][t] = b0.x;
+            S.box[1][t] = b0.y;
+            S.box[2][t] = b1.x;
+            S.box[3][t] = b1.y;
+            S.box[4][t] = b2.x;
+            S.box[5][t] = b2.y;
             S.segOf[t] = 0;
         }
-        if (t == 0)
+        if (threadIdx.x == 0)
         {
-            S.nseg = 1;
+            S.first = ns > 2 ? atomicAdd(nodeCounter, ns - 2) : 0;
             S.segStart[0] = 0;
-            S.segEnd[0] = ns - 1;
-            S.poolNext = 1;
-        }
-        __syncthreads();
-        if (t < ns - 1) S.pool[t] = t == 0 ? u : S.rootPos + t - 1;
-        if (t == 0) S.segNode[0] = u;
-        // --- per axis: elements sorted by centroid (bitonic, ties by element;
-        //     the three axes side by side) ---------------------------------------
-#pragma unroll
-        for (int ax = 0; ax < 3; ++ax)
-        {
-            S.scan[ax][t] = t < ns ? S.cen[ax][t] : FLT_MAX;
-            S.list[0][ax][t] = t < ns ? t : kSahLeaves + t;
-        }
-        __syncthreads();
-        for (int size = 2; size <= kSahLeaves; size <<= 1)
-            for (int stride = size >> 1; stride > 0; stride >>= 1)
-            {
-                const int o = t ^ stride;
-                const bool up = (t & size) == 0;
-                const bool lower = t < o;
-                float ko[3];
-                int io[3];
-                bool take[3];
-#pragma unroll
-                for (int ax = 0; ax < 3; ++ax)
-                {
-                    ko[ax] = S.scan[ax][o];
-                    io[ax] = S.list[0][ax][o];
-                    const float km = S.scan[ax][t];
-                    const int im = S.list[0][ax][t];
-                    const bool mGreater = km > ko[ax] || (km == ko[ax] && im > io[ax]);
-                    take[ax] = lower ? (up ? mGreater : !mGreater) : (up ? !mGreater : mGreater);
-                }
-                __syncthreads();
-#pragma unroll
-                for (int ax = 0; ax < 3; ++ax)
-                    if (take[ax])
-                    {
-                        S.scan[ax][t] = ko[ax];
-                        S.list[0][ax][t] = io[ax];
-                    }
-                __syncthreads();
-            }
-        int cur = 0;
-        if (t == 0)
-        {
-            S.splitting = 0;
+            S.segEnd[0] = (uint8_t)(ns - 1);
+            S.segNode[0] = 0;
+            S.nseg = 1;
             S.maxSeg = ns;
         }
         __syncthreads();
-        // --- one depth of the subtree per pass -------------------------------------
-        for (int depth = 0; depth < kSahLeaves; ++depth)
+        // --- the axis' elements sorted by (doubled) centroid, ties by element -----
         {
-            if (t < S.nseg)
+            uint32_t key[8], idx[8];
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
             {
-                S.best[t] = ~0ull;
-                if (S.segEnd[t] > S.segStart[t]) S.splitting = 1;
+                const int i = lane * 8 + r;
+                idx[r] = (uint32_t)i;
+                // + 0: a negative zero ties with a positive one
+                key[r] = i < ns ? ford(S.box[ax][i] + S.box[3 + ax][i] + 0.0f) : 0xffffffffu;
             }
+            warp_sort256(key, idx, lane);
+            uint2 packed;
+            packed.x = idx[0] | (idx[1] << 8) | (idx[2] << 16) | (idx[3] << 24);
+            packed.y = idx[4] | (idx[5] << 8) | (idx[6] << 16) | (idx[7] << 24);
+            *reinterpret_cast<uint2*>(&S.list[0][ax][lane * 8]) = packed;
+            __syncwarp();
+        }
+        int cur = 0, pool = 1;   // pool: warp 0
+        // --- one depth of the subtree per pass ------------------------------------
+        for (;;)
+        {
+            const int maxSeg = S.maxSeg, nseg = S.nseg;
+            if (maxSeg <= 1) break;
+            const int span = min(maxSeg, 32);   // scans inside a window need log2(span) steps
+            for (int i = threadIdx.x; i < nseg; i += 96) S.best[i] = ~0ull;
             __syncthreads();
-            if (!S.splitting) break;
-            const int s = t < ns ? S.segOf[t] : 0;
-            const int st0 = t < ns ? S.segStart[s] : 0, en0 = t < ns ? S.segEnd[s] : 0;
-            const int span = S.maxSeg;   // scans within segments need log2(span) steps
-            if (t == 0) S.nextMaxSeg = 1;
-            for (int ax = 0; ax < 3; ++ax)
+            // suffix areas, last window first
+            float carry[6] = {FLT_MAX, FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX};
+            for (int w = nw - 1; w >= 0; --w)
             {
-                // prefix boxes along the axis list, within segments
+                const int t = 32 * w + lane;
+                const int s = t < ns ? S.segOf[t] : 0;
+                const int st = S.segStart[s], en = S.segEnd[s];
+                const bool act = t < ns && en > st;
+                if (!__any_sync(FULL, act)) continue;
+                const int room = act ? min(en, 32 * w + 31) - t : 0;   // lanes to the segment's end in this window
                 float v[6];
-                if (t < ns)
+                const int e = act ? S.list[cur][ax][t] : 0;
+#pragma unroll
+                for (int k = 0; k < 6; ++k) v[k] = S.box[k][e];
+#pragma unroll
+                for (int off = 1; off < 32; off <<= 1)
                 {
-                    const int e = S.list[cur][ax][t];
+                    if (off >= span) break;
+                    float o[6];
 #pragma unroll
-                    for (int k = 0; k < 6; ++k) v[k] = S.box[k][e];
-#pragma unroll
-                    for (int k = 0; k < 6; ++k) S.scan[k][t] = v[k];
+                    for (int k = 0; k < 6; ++k) o[k] = __shfl_down_sync(FULL, v[k], off);
+                    if (off <= room) box_merge(v, o);
                 }
-                __syncthreads();
-                for (int off = 1; off < span; off <<= 1)
+                if (act && en >= 32 * (w + 1)) box_merge(v, carry);
+                S.suffix[ax][t] = area6(v);
+#pragma unroll
+                for (int k = 0; k < 6; ++k) carry[k] = __shfl_sync(FULL, v[k], 0);
+            }
+            __syncwarp();
+            // prefix areas, the costs, and each segment's least
+            for (int w = 0; w < nw; ++w)
+            {
+                const int t = 32 * w + lane;
+                const int s = t < ns ? S.segOf[t] : 0;
+                const int st = S.segStart[s], en = S.segEnd[s];
+                const bool act = t < ns && en > st;
+                if (!__any_sync(FULL, act)) continue;
+                const int back = act ? t - max(st, 32 * w) : 0;
+                const int room = act ? min(en, 32 * w + 31) - t : 0;
+                float v[6];
+                const int e = act ? S.list[cur][ax][t] : 0;
+#pragma unroll
+                for (int k = 0; k < 6; ++k) v[k] = S.box[k][e];
+#pragma unroll
+                for (int off = 1; off < 32; off <<= 1)
                 {
-                    const bool take = t < ns && t - off >= st0;
-                    float w[6];
-                    if (take)
+                    if (off >= span) break;
+                    float o[6];
 #pragma unroll
-                        for (int k = 0; k < 6; ++k) w[k] = S.scan[k][t - off];
-                    __syncthreads();
-                    if (take)
-                    {
-#pragma unroll
-                        for (int k = 0; k < 3; ++k)
-                        {
-                            v[k] = fminf(v[k], w[k]);
-                            v[3 + k] = fmaxf(v[3 + k], w[3 + k]);
-                            S.scan[k][t] = v[k];
-                            S.scan[3 + k][t] = v[3 + k];
-                        }
-                    }
-                    __syncthreads();
+                    for (int k = 0; k < 6; ++k) o[k] = __shfl_up_sync(FULL, v[k], off);
+                    if (off <= back) box_merge(v, o);
                 }
-                if (t < ns) S.preArea[t] = area6(v[0], v[1], v[2], v[3], v[4], v[5]);
-                // suffix boxes
-                if (t < ns)
+                if (act && st < 32 * w) box_merge(v, carry);
+                unsigned long long key = ~0ull;
+                if (act && t < en)
                 {
-                    const int e = S.list[cur][ax][t];
-#pragma unroll
-                    for (int k = 0; k < 6; ++k) v[k] = S.box[k][e];
-                }
-                __syncthreads();
-                if (t < ns)
-#pragma unroll
-                    for (int k = 0; k < 6; ++k) S.scan[k][t] = v[k];
-                __syncthreads();
-                for (int off = 1; off < span; off <<= 1)
-                {
-                    const bool take = t < ns && t + off <= en0;
-                    float w[6];
-                    if (take)
-#pragma unroll
-                        for (int k = 0; k < 6; ++k) w[k] = S.scan[k][t + off];
-                    __syncthreads();
-                    if (take)
-                    {
-#pragma unroll
-                        for (int k = 0; k < 3; ++k)
-                        {
-                            v[k] = fminf(v[k], w[k]);
-                            v[3 + k] = fmaxf(v[3 + k], w[3 + k]);
-                            S.scan[k][t] = v[k];
-                            S.scan[3 + k][t] = v[3 + k];
-                        }
-                    }
-                    __syncthreads();
-                }
-                // cost of the split after position t (the suffix from t + 1)
-                if (t < ns && t < en0)
-                {
-                    const float sa = area6(S.scan[0][t + 1], S.scan[1][t + 1], S.scan[2][t + 1], S.scan[3][t + 1],
-                                           S.scan[4][t + 1], S.scan[5][t + 1]);
-                    const int nl = t - st0 + 1, nr = en0 - t;
-                    const float c = S.preArea[t] * (float)nl + sa * (float)nr;
+                    // the split after position t
+                    const int nl = t - st + 1, nr = en - t;
+                    const float c = area6(v) * (float)nl + S.suffix[ax][t + 1] * (float)nr;
                     const unsigned imbalance = (unsigned)abs(nl - nr);
-                    const unsigned long long key = ((unsigned long long)__float_as_uint(fmaxf(c, 0.f)) << 32) |
-                                                   ((unsigned long long)imbalance << 16) | ((unsigned)ax << 8) |
-                                                   (unsigned)(t - st0);
-                    atomicMin(&S.best[s], key);
+                    key = ((unsigned long long)__float_as_uint(fmaxf(c, 0.f)) << 32) |
+                          ((unsigned long long)imbalance << 16) | ((unsigned)ax << 8) | (unsigned)(t - st);
                 }
-                __syncthreads();
+#pragma unroll
+                for (int k = 0; k < 6; ++k) carry[k] = __shfl_sync(FULL, v[k], 31);
+#pragma unroll
+                for (int off = 1; off < 32; off <<= 1)
+                {
+                    if (off >= span) break;
+                    const unsigned long long o = __shfl_down_sync(FULL, key, off);
+                    if (off <= room && o < key) key = o;
+                }
+                // the first lane of a segment's part in this window holds the part's least
+                if (act && back == 0 && key != ~0ull) atomicMin(&S.best[s], key);
             }
+            __syncthreads();
             // marks: the chosen axis list's prefix goes left
-            if (t < ns && en0 > st0)
+            for (int t = threadIdx.x; t < ns; t += 96)
             {
+                const int s = S.segOf[t];
                 const unsigned long long b = S.best[s];
-                const int ax = (int)((b >> 8) & 0xff), sp = st0 + (int)(b & 0xff);
-                S.mark[S.list[cur][ax][t]] = t <= sp ? 1 : 0;
+                if (b == ~0ull) continue;
+                const int sp = S.segStart[s] + (int)(b & 0xff);
+                S.mark[S.list[cur][(int)((b >> 8) & 0xff)][t]] = t <= sp ? 1 : 0;
             }
             __syncthreads();
-            // stable partition of the three lists within the splitting segments
-            int m[3] = {0, 0, 0};
-            if (t < ns && en0 > st0)
-#pragma unroll
-                for (int ax = 0; ax < 3; ++ax) m[ax] = S.mark[S.list[cur][ax][t]];
-            int incl[3] = {m[0], m[1], m[2]};
-            if (t < ns)
-#pragma unroll
-                for (int ax = 0; ax < 3; ++ax) S.rank[ax][t] = incl[ax];
-            __syncthreads();
-            for (int off = 1; off < span; off <<= 1)
+            // stable partition of the axis' list within the splitting segments
             {
-                const bool take = t < ns && t - off >= st0;
-                int w[3] = {0, 0, 0};
-                if (take)
-#pragma unroll
-                    for (int ax = 0; ax < 3; ++ax) w[ax] = S.rank[ax][t - off];
-                __syncthreads();
-                if (take)
-#pragma unroll
-                    for (int ax = 0; ax < 3; ++ax)
-                    {
-                        incl[ax] += w[ax];
-                        S.rank[ax][t] = incl[ax];
-                    }
-                __syncthreads();
-            }
-            if (t < ns)
-            {
-                if (en0 > st0)
+                int run = 0;   // left marks in the windows before
+                for (int w = 0; w < nw; ++w)
                 {
+                    const int t = 32 * w + lane;
+                    const int s = t < ns ? S.segOf[t] : 0;
                     const unsigned long long b = S.best[s];
-                    const int nl = (int)(b & 0xff) + 1;
-#pragma unroll
-                    for (int ax = 0; ax < 3; ++ax)
+                    const int st = S.segStart[s];
+                    const bool act = t < ns && b != ~0ull;
+                    const int e = t < ns ? S.list[cur][ax][t] : 0;
+                    const bool left = act && S.mark[e];
+                    const unsigned m = __ballot_sync(FULL, left);
+                    const int before = run + __popc(m & lt);
+                    run += __popc(m);
+                    if (act && t == st) S.segBase[ax][s] = (uint8_t)before;
+                    __syncwarp();
+                    if (t < ns)
                     {
-                        const int before = incl[ax] - m[ax];   // left elements before t in the segment
-                        const int np = m[ax] ? st0 + before : st0 + nl + (t - st0 - before);
-                        S.list[cur ^ 1][ax][np] = S.list[cur][ax][t];
+                        int np = t;
+                        if (act)
+                        {
+                            const int rank = before - S.segBase[ax][s];   // left elements before t in the segment
+                            np = left ? st + rank : st + (int)(b & 0xff) + 1 + (t - st - rank);
+                        }
+                        S.list[cur ^ 1][ax][np] = (uint8_t)e;
                     }
-                }
-                else
-                {
-#pragma unroll
-                    for (int ax = 0; ax < 3; ++ax) S.list[cur ^ 1][ax][t] = S.list[cur][ax][t];
                 }
             }
             __syncthreads();
             // nodes: each splitting segment is an internal node with two children
-            const int nsegOld = S.nseg;
-            __syncthreads();
-            if (t < nsegOld && S.segEnd[t] > S.segStart[t])
+            if (ax == 0)
             {
-                const int st = S.segStart[t], en = S.segEnd[t], node = S.segNode[t];
-                const int sp = st + (int)(S.best[t] & 0xff);
-                int refs[2];
-                const int cs[2] = {st, sp + 1}, ce[2] = {sp, en};
-                const int right = atomicAdd(&S.nseg, 1);
-#pragma unroll
-                for (int c = 0; c < 2; ++c)
+                int newMax = 1, next = nseg;
+                const int first = S.first;
+                for (int i0 = 0; i0 < nseg; i0 += 32)
                 {
-                    const int segId = c == 0 ? t : right;
-                    if (ce[c] == cs[c])
+                    const int i = i0 + lane;
+                    const unsigned long long b = i < nseg ? S.best[i] : ~0ull;
+                    const bool split = b != ~0ull;
+                    int st = 0, en = 0, sp = 0;
+                    if (split)
                     {
-                        refs[c] = ~(a + cs[c]);
-                        parent[(n - 1) + a + cs[c]] = node;
-                        S.segNode[segId] = -1;
+                        st = S.segStart[i];
+                        en = S.segEnd[i];
+                        sp = st + (int)(b & 0xff);
                     }
-                    else
+                    const int ls = sp - st + 1, rs = en - sp;
+                    const unsigned ms = __ballot_sync(FULL, split);
+                    const unsigned ml = __ballot_sync(FULL, split && ls > 1), mr = __ballot_sync(FULL, split && rs > 1);
+                    if (split)
                     {
-                        const int id = S.pool[atomicAdd(&S.poolNext, 1)];
-                        refs[c] = id;
-                        parent[id] = node;
-                        range[id] = make_int2(a + cs[c], a + ce[c]);
-                        S.segNode[segId] = id;
+                        const int right = next + __popc(ms & lt);
+                        const int pl = pool + __popc(ml & lt) + __popc(mr & lt), pr = pl + (ls > 1 ? 1 : 0);
+                        const int me = S.segNode[i];
+                        const int node = me == 0 ? u : first + me - 1;
+                        int2 refs;
+                        if (ls > 1)
+                        {
+                            refs.x = first + pl - 1;
+                            parent[refs.x] = node;
+                            range[refs.x] = make_int2(a + st, a + sp);
+                        }
+                        else
+                        {
+                            refs.x = ~(a + st);
+                            parent[(n - 1) + a + st] = node;
+                        }
+                        if (rs > 1)
+                        {
+                            refs.y = first + pr - 1;
+                            parent[refs.y] = node;
+                            range[refs.y] = make_int2(a + sp + 1, a + en);
+                        }
+                        else
+                        {
+                            refs.y = ~(a + en);
+                            parent[(n - 1) + a + en] = node;
+                        }
+                        child[node] = refs;
+                        S.segEnd[i] = (uint8_t)sp;
+                        S.segNode[i] = (uint8_t)pl;   // of no use when the half is a single triangle
+                        S.segRight[i] = (uint8_t)right;
+                        S.segStart[right] = (uint8_t)(sp + 1);
+                        S.segEnd[right] = (uint8_t)en;
+                        S.segNode[right] = (uint8_t)pr;
+                        newMax = max(newMax, max(ls, rs));
                     }
+                    next += __popc(ms);
+                    pool += __popc(ml) + __popc(mr);
                 }
-                child[node] = make_int2(refs[0], refs[1]);
-                atomicMax(&S.nextMaxSeg, max(sp - st + 1, en - sp));
-                S.segRight[t] = right;
-                S.segStart[right] = sp + 1;
-                S.segEnd[right] = en;
-                S.segEnd[t] = sp;
+                newMax = __reduce_max_sync(FULL, newMax);
+                if (lane == 0)
+                {
+                    S.maxSeg = newMax;
+                    S.nseg = next;
+                }
             }
             __syncthreads();
-            if (t < ns && en0 > st0)
+            for (int t = threadIdx.x; t < ns; t += 96)
             {
-                const unsigned long long b = S.best[s];
-                const int sp = st0 + (int)(b & 0xff);
-                if (t > sp) S.segOf[t] = S.segRight[s];
-            }
-            if (t == 0)
-            {
-                S.splitting = 0;
-                S.maxSeg = S.nextMaxSeg;
+                const int s = S.segOf[t];
+                if (S.best[s] != ~0ull && t > S.segEnd[s]) S.segOf[t] = S.segRight[s];
             }
             cur ^= 1;
             __syncthreads();
         }
         // the triangles in their new order
-        if (t < ns) vals[a + t] = (uint32_t)S.orig[S.list[cur][0][t]];
+        uint32_t tri[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+        {
+            const int t = threadIdx.x + 96 * k;
+            tri[k] = t < ns ? vals[a + S.list[cur][0][t]] : 0u;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+        {
+            const int t = threadIdx.x + 96 * k;
+            if (t < ns) vals[a + t] = tri[k];
+        }
         __syncthreads();
     }
 }
@@ -378,7 +445,7 @@ __global__ void __launch_bounds__(kSahLeaves) k_sah_rebuild(int n, const int* __
 // node and its contiguous range of triangles) with more than kSahLeaves
 // triangles is split by the least SAH cost over kTopBins centroid bins per axis,
 // its triangles are partitioned into the two halves of the range, and the
-// halves become the next level's tasks, k_sah_rebuild's subtrees
+// halves become the next level's tasks, k_sah_subtrees' subtrees
 // (2..kSahLeaves triangles) or leaves.
 //
 // A level is two launches over the chunks (kTopChunk triangles) of its tasks:
@@ -402,16 +469,6 @@ constexpr int kBinWords = 7;           // count, box lo, box hi (order-preservin
 constexpr int kTaskBins = 3 * kTopBins * kBinWords;
 constexpr int kTopSlots = 4;           // level l counts its tasks, chunks and merged bins in slot l & 3
 constexpr int kTopCounts = 3;
-
-__device__ __forceinline__ uint32_t ford(float f)
-{
-    const uint32_t u = __float_as_uint(f);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float funord(uint32_t u)
-{
-    return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
-}
 
 __device__ __forceinline__ int top_bin(float c, float cmin, float scale)
 {
@@ -978,7 +1035,7 @@ void sah_tree_carve(Carve& c, int n, SahTreeBuffers& B)
 }
 
 // Top-down binned SAH from the root down to subtrees of kSahLeaves triangles,
-// then k_sah_rebuild for those.  perm: the triangles in their starting order;
+// then k_sah_subtrees for those.  perm: the triangles in their starting order;
 // out: in the tree's order.
 cudaError_t sah_build_tree(int n, const float* triBox, const float* cbounds, const uint32_t* perm, uint32_t* out,
                            int2* child, int2* range, int* parent, const SahTreeBuffers& B, int numSMs,
@@ -1045,9 +1102,9 @@ cudaError_t sah_build_tree(int n, const float* triBox, const float* cbounds, con
     }
     if (e != cudaSuccess) return e;
     int perSM = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_sah_rebuild, kSahLeaves, 0);
-    k_sah_rebuild<<<std::max(1, perSM) * numSMs, kSahLeaves, 0, stream>>>(n, B.small, B.counters, triBox, out, child,
-                                                                       range, parent, B.counters + 1);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_sah_subtrees, 96, 0);
+    k_sah_subtrees<<<std::max(1, perSM) * numSMs, 96, 0, stream>>>(n, B.small, B.counters, triBox, out, child, range,
+                                                                parent, B.counters + 1);
     return cudaGetLastError();
 }
 
