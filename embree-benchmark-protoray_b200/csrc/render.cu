@@ -1375,7 +1375,9 @@ __global__ void k_resolve_ldr(const float4* __restrict__ accum, uint32_t* __rest
 __global__ void k_advance_pass(int* passBase, int spp) { *passBase += spp; }
 
 constexpr int kReplayMaxDepth = 16;
-constexpr int kAggSlots = 1024;   // block-private gradient slots of the adjoint
+constexpr int kAggSlots = 256;             // block-private gradient slots of the adjoint
+constexpr int kReplayWords = 7;            // pixel, depth, RNG, throughput, direction (as k_paths)
+constexpr int kBackwardWords = 9;          // and dL/d(radiance) of the pixel, this lane's sky gradient
 
 // Path-replay megakernel: each lane carries whole paths (pass, pixel), from
 // the camera ray to escape or maxDepth.  The forward mode accumulates the
@@ -1385,10 +1387,15 @@ constexpr int kAggSlots = 1024;   // block-private gradient slots of the adjoint
 //   radiance = sky * prod_k albedo[prim_k]
 //   d radiance / d albedo[prim_k] = radiance / albedo[prim_k]
 //   d radiance / d sky            = prod_k albedo[prim_k]
-// Paths are regenerated per lane (a lane whose path ends takes the next one
-// once kRefillMin lanes of its warp are free), and traversal advances one node
-// per step, as in k_bounce.  The bounce arithmetic is the same device code as
-// the wavefront renderer's, so both compute bit-identical paths.
+// Paths bounce in their lane and are replaced when they end, with the path's
+// state in shared memory, as in k_paths.  The bounce arithmetic is the same
+// device code as the wavefront renderer's, so both compute bit-identical paths.
+// Both modes defer triangle tests and test nodes with paired FMAs; the backward
+// mode affords the queues with 256 gradient slots (1024: 6% slower for the shared
+// memory).  Traversal latency and issue bound it, as k_paths.  512x512, 16
+// passes, 82K triangles: forward 1.94 -> 1.67 ms, backward 2.29 -> 1.95 ms against
+// lanes that kept the path in registers, refilled at 12 idle lanes only and (in
+// the backward mode) tested triangles in the lane.
 template <bool kBackward>
 __global__ void __launch_bounds__(128, 8) k_replay(SceneDev sc, CameraDev cam, float4* accum, int pass0, int spp,
                                                    int maxDepth, float sky, const float* __restrict__ dL,
@@ -1415,108 +1422,66 @@ __global__ void __launch_bounds__(128, 8) k_replay(SceneDev sc, CameraDev cam, f
     st.sh = s_stack + threadIdx.x;
     st.stride = blockDim.x;
     st.overflow = false;
-    TriQueue* tq = reinterpret_cast<TriQueue*>(s_stack + kShared * blockDim.x) + (threadIdx.x >> 5);   // forward, deferTris
+    constexpr int kWords = kBackward ? kBackwardWords : kReplayWords;
+    uint32_t* s_path = reinterpret_cast<uint32_t*>(s_stack + kShared * blockDim.x);
+    uint32_t* path = s_path + threadIdx.x;   // word k of this lane's path at path[k * bd]
+    TriQueue* tq = reinterpret_cast<TriQueue*>(s_path + ((kWords + 1) & ~1) * blockDim.x) + (threadIdx.x >> 5);   // deferTris
+    const int bd = blockDim.x;
     const unsigned FULL = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned ltMask = (1u << lane) - 1u;
-    const int W = cam.width, H = cam.height;
-    const long long npix = (long long)W * H;
+    const int W = cam.width;
+    const long long npix = (long long)W * cam.height;
     const long long total = (long long)spp * npix;
-    float skyGrad = 0.f;
-    unsigned long long myRays = 0;
+    if (kBackward) path[8 * bd] = 0u;   // sky gradient 0
+    unsigned long long traced = 0;      // rays, per warp
 
-    bool has = false;
-    bool exhausted = false;
-    int pixel = 0, depth = 0, np = 0;
-    uint32_t rng = 0;
-    float thr = 1.f, g = 0.f;
-    int prims[kBackward ? kReplayMaxDepth : 1];
+    bool has = false, exhausted = false;
+    int prims[kBackward ? kReplayMaxDepth : 1];   // the triangles the path bounced off
     TravRay r;
     TravState ts;
     ts.done = true;
     for (;;)
     {
-        unsigned idle = __ballot_sync(FULL, !has);
-        if (!exhausted && (__popc(idle) >= kRefillMin || idle == FULL))
-        {
-            int n = __popc(idle);
-            long long base = 0;
-            if (lane == 0) base = (long long)atomicAdd(reinterpret_cast<unsigned long long*>(fetch), (unsigned long long)n);
-            base = __shfl_sync(FULL, base, 0);
-            if (base + n >= total) exhausted = true;
-            long long gi = base + __popc(idle & ltMask);
-            if (!has && gi < total)
-            {
-                int pass = (int)(gi / npix);
-                pixel = (int)(gi - (long long)pass * npix);
-                bool ok = true;
-                if (kBackward)
-                {
-                    g = dL[3 * (size_t)pixel] + dL[3 * (size_t)pixel + 1] + dL[3 * (size_t)pixel + 2];
-                    ok = g != 0.f;
-                }
-                if (ok)
-                {
-                    rng = rng_seed(pass0 + pass, pixel);
-                    float3 org, dir;
-                    camera_ray(cam, pixel % W, pixel / W, rng, org, dir);
-                    trav_setup(r, org, dir);
-                    trav_init(ts, sc, FLT_MAX, st);
-                    thr = 1.0f;
-                    depth = 0;
-                    np = 0;
-                    has = true;
-                }
-            }
-        }
-        if (__ballot_sync(FULL, has) == 0)
-        {
-            if (exhausted) break;
-            continue;
-        }
-        if (PRT_DEFER_REPLAY && !kBackward && sc.deferTris)
-        {
-            warp_trav_deferred(*tq, ts, sc, r, 0.0f, st, has, true, kRefillMin, lane);
-        }
-        else
-        for (;;)
-        {
-            if (has && !ts.done) trav_step<false>(ts, sc, r, 0.0f, st);
-            unsigned running = __ballot_sync(FULL, has && !ts.done);
-            if (running == 0) break;
-            if (32 - __popc(running) >= kRefillMin) break;
-        }
+        // --- lanes whose ray is traced: the path ends or bounces -----------------
+        bool fresh = false;   // this lane has a new ray (org, dir)
+        float3 org, dir;
+        traced += __popc(__ballot_sync(FULL, has && ts.done));
         if (has && ts.done)
         {
-            ++myRays;
-            bool escaped = ts.triHit < 0;
+            const int depth = (int)path[bd];
+            float thr = __uint_as_float(path[3 * bd]);
+            const bool escaped = ts.triHit < 0;
             if (!escaped && depth < maxDepth)
             {
-                // continue the path in this lane
+                uint32_t rng = path[2 * bd];
+                org = r.org;
+                dir = f3(__uint_as_float(path[4 * bd]), __uint_as_float(path[5 * bd]), __uint_as_float(path[6 * bd]));
                 thr = __fmul_rn(thr, sc.albedo ? __ldg(sc.albedo + ts.primHit) : 0.8f);
-                if (kBackward) prims[np++] = ts.primHit;
-                float3 org = r.org, dir = r.dir;
+                if (kBackward) prims[depth] = ts.primHit;
                 diffuse_bounce(sc.tris, ts.triHit, org, dir, ts.tHit, rng);
-                trav_setup(r, org, dir);
-                trav_init(ts, sc, FLT_MAX, st);
-                ++depth;
+                path[bd] = (uint32_t)(depth + 1);
+                path[2 * bd] = rng;
+                path[3 * bd] = __float_as_uint(thr);
+                fresh = true;
             }
             else
             {
-                float c = escaped ? __fmul_rn(thr, sky) : 0.0f;
+                const float c = escaped ? __fmul_rn(thr, sky) : 0.0f;
                 if (!kBackward)
                 {
-                    red_add_v4(accum + pixel, c, c, c, 1.0f);
+                    red_add_v4(accum + path[0], c, c, c, 1.0f);
                 }
                 else if (escaped)
                 {
-                    skyGrad += g * thr;
-                    float gc = g * c;
-                    for (int k = 0; k < np; ++k)
+                    const float g = __uint_as_float(path[7 * bd]);
+                    path[8 * bd] = __float_as_uint(__uint_as_float(path[8 * bd]) + g * thr);
+                    const float gc = g * c;
+                    for (int k = 0; k < depth; ++k)
                     {
                         const int pk = prims[k];
-                        float al = sc.albedo ? __ldg(sc.albedo + pk) : 0.8f;
-                        float v = gc / al;
+                        const float al = sc.albedo ? __ldg(sc.albedo + pk) : 0.8f;
+                        const float v = gc / al;
                         const int slot = pk & (kAggSlots - 1);
                         int key = s_key[slot];
                         if (key == -1) key = atomicCAS(&s_key[slot], -1, pk);   // -1: claimed by us
@@ -1527,18 +1492,74 @@ __global__ void __launch_bounds__(128, 8) k_replay(SceneDev sc, CameraDev cam, f
                 has = false;
             }
         }
+        // --- lanes without a path take the next ones ------------------------------
+        const unsigned idle = __ballot_sync(FULL, !has);
+        if (!exhausted && idle)
+        {
+            const int n = __popc(idle);
+            long long base = 0;
+            if (lane == 0) base = (long long)atomicAdd(reinterpret_cast<unsigned long long*>(fetch), (unsigned long long)n);
+            base = __shfl_sync(FULL, base, 0);
+            exhausted = base + n >= total;
+            const long long gi = base + __popc(idle & ltMask);
+            if (!has && gi < total)
+            {
+                const int pass = (int)(gi / npix);
+                const int pixel = (int)(gi - (long long)pass * npix);
+                float g = 1.f;
+                if (kBackward)
+                {
+                    g = dL[3 * (size_t)pixel] + dL[3 * (size_t)pixel + 1] + dL[3 * (size_t)pixel + 2];
+                    path[7 * bd] = __float_as_uint(g);
+                }
+                if (g != 0.f)   // a pixel without a gradient has nothing to replay
+                {
+                    uint32_t rng = rng_seed(pass0 + pass, pixel);
+                    camera_ray(cam, pixel % W, pixel / W, rng, org, dir);
+                    path[0] = (uint32_t)pixel;
+                    path[bd] = 0u;
+                    path[2 * bd] = rng;
+                    path[3 * bd] = __float_as_uint(1.0f);
+                    has = fresh = true;
+                }
+            }
+        }
+        const unsigned act = __ballot_sync(FULL, has);
+        if (act == 0)
+        {
+            if (exhausted) break;
+            continue;
+        }
+        if (fresh)
+        {
+            path[4 * bd] = __float_as_uint(dir.x);
+            path[5 * bd] = __float_as_uint(dir.y);
+            path[6 * bd] = __float_as_uint(dir.z);
+            trav_setup(r, org, dir);
+            trav_init(ts, sc, FLT_MAX, st);
+        }
+        // --- traverse until enough of the warp's rays are done ---------------------
+        const int stopIdle = stop_idle(act);
+        if (PRT_DEFER_REPLAY && sc.deferTris)
+        {
+            warp_trav_deferred<PRT_PAIRED_LATER>(*tq, ts, sc, r, 0.0f, st, has, true, stopIdle, lane);
+        }
+        else
+        for (;;)
+        {
+            if (has && !ts.done) trav_step<false>(ts, sc, r, 0.0f, st);
+            const unsigned running = __ballot_sync(FULL, has && !ts.done);
+            if (32 - __popc(running) >= stopIdle) break;
+        }
     }
+    if (kBackward)
+    {
+        float skyGrad = __uint_as_float(path[8 * bd]);
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1)
-    {
-        skyGrad += __shfl_down_sync(FULL, skyGrad, off);
-        myRays += __shfl_down_sync(FULL, myRays, off);
+        for (int off = 16; off > 0; off >>= 1) skyGrad += __shfl_down_sync(FULL, skyGrad, off);
+        if (lane == 0 && skyGrad != 0.f) atomicAdd(dSky, skyGrad);
     }
-    if (lane == 0)
-    {
-        if (kBackward && skyGrad != 0.f) atomicAdd(dSky, skyGrad);
-        if (rays) atomicAdd(rays, myRays);
-    }
+    if (lane == 0 && rays) atomicAdd(rays, traced);
     if (kBackward)
     {
         __syncthreads();
@@ -1953,10 +1974,9 @@ int launch_replay(const SceneDev& sc, const CameraDev& cam, float4* accum, int p
     long long total = (long long)spp * cam.width * cam.height;
     if (total <= 0) return 0;
     const int block = 128;
-    size_t shmem = sizeof(uint2) * kShared * block;
-    // the backward kernel keeps in-lane triangle tests: with its gradient table
-    // in shared memory the queues would cost it occupancy (measured 17% slower)
-    if (PRT_DEFER_REPLAY && !backward && sc.deferTris) shmem += sizeof(TriQueue) * (block / 32);
+    const int words = ((backward ? kBackwardWords : kReplayWords) + 1) & ~1;   // the queues after them are 8-byte aligned
+    size_t shmem = (sizeof(uint2) * kShared + sizeof(uint32_t) * words) * block;
+    if (PRT_DEFER_REPLAY && sc.deferTris) shmem += sizeof(TriQueue) * (block / 32);
     LaunchCfg cfg;
     auto go = [&](auto kernel) {
         int grid = grid_for(kernel, block, shmem, numSMs, cfg);
