@@ -1170,7 +1170,7 @@ int prt_intersect(prt_ctx* ctx, const prt_ray* rays, prt_hit* hits, int n, void*
     CK(cudaSetDevice(ctx->device));
     cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
     int* fetch = nullptr;
-    st = isect_counter(ctx, s, &fetch);
+    if (!intersect_few(n, false, ctx->numSMs)) st = isect_counter(ctx, s, &fetch);
     if (st != PRT_OK) return st;
     ctx->launches += launch_intersect(scene_dev(ctx), (const RayRec*)rays, (HitRec*)hits, n, false, nullptr, fetch, ctx->numSMs, s);
     CK(cudaGetLastError());
@@ -1202,7 +1202,7 @@ int prt_occluded(prt_ctx* ctx, const prt_ray* rays, float* out, int n, void* str
     CK(cudaSetDevice(ctx->device));
     cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
     int* fetch = nullptr;
-    st = isect_counter(ctx, s, &fetch);
+    if (!intersect_few(n, true, ctx->numSMs)) st = isect_counter(ctx, s, &fetch);
     if (st != PRT_OK) return st;
     ctx->launches += launch_intersect(scene_dev(ctx), (const RayRec*)rays, nullptr, n, true, out, fetch, ctx->numSMs, s);
     CK(cudaGetLastError());

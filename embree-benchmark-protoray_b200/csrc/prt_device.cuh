@@ -912,22 +912,6 @@ __device__ __forceinline__ void warp_trav_deferred(TriQueue& q, TravState& ts, c
     }
 }
 
-// Closest hit (anyHit = false) or any hit (anyHit = true) over (tnear, tfar].
-// Returns the leaf-order triangle index of the hit (or -1), with t/u/v/prim.
-template <bool anyHit>
-__device__ __forceinline__ int traverse(const SceneDev& sc, const TravRay& r, float tnear, float tfar, TravStack& st,
-                                        float& tHit, int& primHit, float& uHit, float& vHit)
-{
-    TravState s;
-    trav_init(s, sc, tfar, st);
-    while (!s.done) trav_step<anyHit>(s, sc, r, tnear, st);
-    tHit = s.tHit;
-    primHit = s.primHit;
-    uHit = s.uHit;
-    vHit = s.vHit;
-    return s.triHit;
-}
-
 // Post-intersection shading and the diffuse bounce
 // (geometry/triangle_mesh.cpp:59-100 + render/diffuse_integrator_single.h:57-63):
 // hit point, eps = max(t, max|p|) * 0x1.fp-18 (core/ray.h:71-76), geometric

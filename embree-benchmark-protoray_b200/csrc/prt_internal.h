@@ -268,7 +268,9 @@ struct LaunchCfg
 int launch_bounce(const WaveArgs& a, int depth, const LaunchCfg& cfg, int numSMs, cudaStream_t s);
 // every bounce from depth 1 on (a.qin: the depth-1 queue, counts[1] paths)
 int launch_paths(const WaveArgs& a, const LaunchCfg& cfg, int numSMs, cudaStream_t s);
-// fetch: a zeroed work counter on the device, used by this launch only
+// whether launch_intersect takes n rays without a work counter
+bool intersect_few(int n, bool anyHit, int numSMs);
+// fetch: a zeroed work counter on the device, used by this launch only (unused when intersect_few)
 int launch_intersect(const SceneDev& sc, const RayRec* rays, HitRec* hits, int n, bool anyHit, float* anyOut,
                      int* fetch, int numSMs, cudaStream_t s);
 int launch_resolve_ldr(const float4* accum, uint32_t* out, int n, cudaStream_t s);

@@ -1328,20 +1328,164 @@ __global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_intersect(SceneD
     }
 }
 
-// Hit point and geometric normal of one query ray (Renderer::queryRay).
+// Closest or any hit of one ray by a group of 8 lanes, lane j testing child j of
+// the node the ray is at and the triangles of that child if it is a leaf (trees
+// of any leaf size).  Every lane of the group holds the ray and the traversal
+// state; stk: the group's kPacketStack entries of shared memory.  Returns the
+// leaf-order index of the hit triangle, or -1, in every lane.
+template <bool kAnyHit>
+__device__ __forceinline__ int group_trace(const SceneDev& sc, const TravRay& r, float tnear, uint2* stk, unsigned lane,
+                                           float& tHit, int& primHit, float& uHit, float& vHit)
+{
+    const int j = (int)(lane & 7u);
+    const unsigned gshift = lane & 24u, gmask = 0xffu << gshift;
+    int triHit = -1;
+    if (!sc.hasRoot) return -1;
+    // byte offsets of this lane's near and far planes in a node
+    const int nX = (r.inv.x < 0.f ? 56 : 32) + j, fX = (r.inv.x < 0.f ? 32 : 56) + j;
+    const int nY = (r.inv.y < 0.f ? 64 : 40) + j, fY = (r.inv.y < 0.f ? 40 : 64) + j;
+    const int nZ = (r.inv.z < 0.f ? 72 : 48) + j, fZ = (r.inv.z < 0.f ? 48 : 72) + j;
+    int sp = 0;
+    uint2 ng = make_uint2(0u, 0x80000000u);   // the root: one internal child at base 0
+    for (;;)
+    {
+        const uint32_t b = 31u - __clz(ng.y & 0xff000000u);
+        ng.y &= ~(1u << b);
+        const uint32_t slot = (b - 24u) ^ r.octinv;
+        const uint32_t nodeIdx = ng.x + __popc((ng.y & 0xffu) & ((1u << slot) - 1u));
+        if ((ng.y & 0xff000000u) && sp < kPacketStack)
+        {
+            if (j == 0) stk[sp] = ng;
+            ++sp;
+        }
+        const uint4* qp = reinterpret_cast<const uint4*>(sc.nodes + nodeIdx);
+        const unsigned char* bp = reinterpret_cast<const unsigned char*>(qp);
+        const uint4 q0 = __ldg(qp), q1 = __ldg(qp + 1);
+        const uint32_t bnX = __ldg(bp + nX), bfX = __ldg(bp + fX), bnY = __ldg(bp + nY), bfY = __ldg(bp + fY),
+                       bnZ = __ldg(bp + nZ), bfZ = __ldg(bp + fZ);
+        // this child's slab test, as node_hits does it
+        const uint32_t e = q0.w;
+        const float aix = __uint_as_float(((e & 0xffu) + 15u) << 23) * r.inv.x;
+        const float aiy = __uint_as_float((((e >> 8) & 0xffu) + 15u) << 23) * r.inv.y;
+        const float aiz = __uint_as_float((((e >> 16) & 0xffu) + 15u) << 23) * r.inv.z;
+        const float aox = (__uint_as_float(q0.x) - r.org.x) * r.inv.x - aix;
+        const float aoy = (__uint_as_float(q0.y) - r.org.y) * r.inv.y - aiy;
+        const float aoz = (__uint_as_float(q0.z) - r.org.z) * r.inv.z - aiz;
+        const float t0 = fmax3(fmaf(byte_unit(bnX, 0), aix, aox), fmaf(byte_unit(bnY, 0), aiy, aoy),
+                               fmaxf(fmaf(byte_unit(bnZ, 0), aiz, aoz), tnear));
+        const float t1 = fmin3(fmaf(byte_unit(bfX, 0), aix, aox), fmaf(byte_unit(bfY, 0), aiy, aoy),
+                               fminf(fmaf(byte_unit(bfZ, 0), aiz, aoz), tHit * 1.0000004f));
+        const uint32_t meta = ((j < 4 ? q1.z : q1.w) >> (8 * (j & 3))) & 0xffu;
+        const bool hit = meta != 0 && t0 <= t1 * 1.0000008f;
+        const uint32_t imask = e >> 24;
+        const uint32_t c8 = (__ballot_sync(gmask, hit) >> gshift) & 0xffu;
+        if (c8 & ~imask)
+        {
+            // the hit leaves' triangles, each lane its own; the group keeps the
+            // nearest (ties to the lower primitive id)
+            unsigned long long key = hit_key(tHit, primHit);
+            const unsigned long long before = key;
+            float u = 0.f, v = 0.f;
+            int ti = 0;
+            if (hit && !((imask >> j) & 1u))
+            {
+                float tb = tHit;
+                int pb = primHit;
+                for (uint32_t k = 0; k < (uint32_t)__popc(meta >> 5); ++k)
+                {
+                    const int idx = (int)(q1.y + (meta & 0x1fu) + k);
+                    const float4* tp = reinterpret_cast<const float4*>(sc.tris + idx);
+                    const float4 v0 = __ldg(tp), v1 = __ldg(tp + 1), v2 = __ldg(tp + 2);
+                    const int prim = __float_as_int(v0.w);
+                    float t, uu, vv;
+                    if (tri_test(r, f3(v0.x, v0.y, v0.z), f3(v1.x, v1.y, v1.z), f3(v2.x, v2.y, v2.z), tnear, tb, prim, pb,
+                                 t, uu, vv))
+                    {
+                        tb = t;
+                        pb = prim;
+                        u = uu;
+                        v = vv;
+                        ti = idx;
+                        key = hit_key(t, prim);
+                    }
+                }
+            }
+            const unsigned long long mine = key;
+#pragma unroll
+            for (int off = 1; off < 8; off <<= 1)
+            {
+                const unsigned long long o = __shfl_xor_sync(gmask, key, off);
+                key = o < key ? o : key;
+            }
+            if (key != before)
+            {
+                const int win = __ffs(__ballot_sync(gmask, mine == key)) - 1;
+                tHit = __uint_as_float((uint32_t)(key >> 32));
+                primHit = (int)(uint32_t)key;
+                uHit = __shfl_sync(gmask, u, win);
+                vHit = __shfl_sync(gmask, v, win);
+                triHit = __shfl_sync(gmask, ti, win);
+                if (kAnyHit) return triHit;
+            }
+        }
+        // internal hits: bit slot -> bit slot ^ octinv, as node_hits1 orders them
+        uint32_t in8 = c8 & imask;
+        uint32_t sw = ((in8 & 0x55u) << 1) | ((in8 >> 1) & 0x55u);
+        in8 = (r.octinv & 1u) ? sw : in8;
+        sw = ((in8 & 0x33u) << 2) | ((in8 >> 2) & 0x33u);
+        in8 = (r.octinv & 2u) ? sw : in8;
+        sw = ((in8 & 0x0fu) << 4) | ((in8 >> 4) & 0x0fu);
+        in8 = (r.octinv & 4u) ? sw : in8;
+        ng = make_uint2(q1.x, (in8 << 24) | imask);
+        if (!(ng.y & 0xff000000u))
+        {
+            if (sp == 0) return triHit;
+            __syncwarp(gmask);
+            ng = stk[--sp];
+            __syncwarp(gmask);
+        }
+    }
+}
+
+// Few rays: a group of 8 lanes per ray.  One lane per ray leaves the chip idle
+// while the longest ray's chain of node visits runs, each some 300 dependent
+// instructions and a cache miss; eight lanes cut a visit to about a fifth of
+// that.  perWarp (1, 2 or 4) rays share a warp.
+template <bool kAnyHit>
+__global__ void __launch_bounds__(128) k_intersect_few(SceneDev sc, const RayRec* __restrict__ rays,
+                                                     HitRec* __restrict__ hits, float* __restrict__ anyOut, int n,
+                                                     int perWarp)
+{
+    __shared__ uint2 s_stk[16 * kPacketStack];
+    const unsigned lane = threadIdx.x & 31u;
+    const int group = (int)(lane >> 3);
+    const long long i = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * perWarp + group;
+    if (group >= perWarp || i >= n) return;
+    const float4* rp = reinterpret_cast<const float4*>(rays + i);
+    const float4 a = __ldg(rp), b = __ldg(rp + 1);
+    TravRay r;
+    trav_setup(r, f3(a.x, a.y, a.z), f3(b.x, b.y, b.z));
+    float t = b.w, u = 0.f, v = 0.f;
+    int prim = 0x7fffffff;
+    const int tri = group_trace<kAnyHit>(sc, r, a.w, s_stk + (threadIdx.x >> 3) * kPacketStack, lane, t, prim, u, v);
+    if ((lane & 7u) != 0) return;
+    if (kAnyHit) anyOut[i] = tri >= 0 ? t : -1.0f;
+    else reinterpret_cast<float4*>(hits)[i] = tri >= 0 ? make_float4(t, __int_as_float(prim), u, v)
+                                                       : make_float4(-1.0f, __int_as_float(-1), 0.f, 0.f);
+}
+
+// Hit point and geometric normal of one query ray (Renderer::queryRay), by one
+// group of 8 lanes.
 __global__ void k_query(SceneDev sc, const RayRec* ray, HitRec* hit, float* pNg)
 {
-    __shared__ uint2 s_stack[kShared];
-    TravStack st;
-    st.sh = s_stack;
-    st.stride = 1;
-    st.overflow = false;
-    RayRec rr = *ray;
+    __shared__ uint2 s_stk[kPacketStack];
+    const RayRec rr = *ray;
     TravRay r;
     trav_setup(r, f3(rr.ox, rr.oy, rr.oz), f3(rr.dx, rr.dy, rr.dz));
-    float t, u, v;
-    int prim;
-    int ti = traverse<false>(sc, r, rr.tnear, rr.tfar, st, t, prim, u, v);
+    float t = rr.tfar, u = 0.f, v = 0.f;
+    int prim = 0x7fffffff;
+    const int ti = group_trace<false>(sc, r, rr.tnear, s_stk, threadIdx.x, t, prim, u, v);
+    if (threadIdx.x != 0) return;
     if (ti < 0)
     {
         *hit = HitRec{-1.0f, -1, 0.f, 0.f};
@@ -1895,11 +2039,28 @@ int launch_batch_first(const BatchArgs& a, const LaunchCfg& cfg, int numSMs, cud
     return 1;
 }
 
+// Up to about 256 (closest) or 512 (any hit) rays per SM the longest ray's chain
+// of node visits takes longer than the work does, and eight lanes per ray win;
+// beyond that their emptier lanes cost more than they save.  Incoherent
+// closest-hit calls, one lane -> eight lanes: 1000 rays on 82K triangles 54 -> 39
+// us, on 1.38M 81 -> 43; 40000 on 1.38M 110 -> 94; 80000 on 1.38M 128 -> 148 (any
+// hit: 112 -> 114).
+bool intersect_few(int n, bool anyHit, int numSMs) { return n <= (anyHit ? 512 : 256) * numSMs; }
+
 int launch_intersect(const SceneDev& sc, const RayRec* rays, HitRec* hits, int n, bool anyHit, float* anyOut,
                      int* fetch, int numSMs, cudaStream_t s)
 {
     if (n <= 0) return 0;
     const int block = 128;
+    if (intersect_few(n, anyHit, numSMs))
+    {
+        // rays of one warp wait for one another, so they share it only once the chip is full
+        const int perWarp = n <= 4 * numSMs ? 1 : (n <= 16 * numSMs ? 2 : 4);
+        const int blocks = (n + 4 * perWarp - 1) / (4 * perWarp);
+        if (anyHit) k_intersect_few<true><<<blocks, block, 0, s>>>(sc, rays, hits, anyOut, n, perWarp);
+        else k_intersect_few<false><<<blocks, block, 0, s>>>(sc, rays, hits, anyOut, n, perWarp);
+        return 1;
+    }
     size_t shmem = sizeof(uint2) * kShared * block;
     if (PRT_DEFER_ISECT && sc.deferTris)
         shmem += (sizeof(TriQueue) + (anyHit ? 0 : sizeof(TriQueueUV))) * (block / 32);
@@ -1916,7 +2077,7 @@ int launch_intersect(const SceneDev& sc, const RayRec* rays, HitRec* hits, int n
 
 int launch_query(const SceneDev& sc, const RayRec* ray, HitRec* hit, float* pNg, cudaStream_t s)
 {
-    k_query<<<1, 1, 0, s>>>(sc, ray, hit, pNg);
+    k_query<<<1, 8, 0, s>>>(sc, ray, hit, pNg);
     return 1;
 }
 
