@@ -455,8 +455,8 @@ int build_mesh_gpu(const prt_soup_triangle* hostTris, int n, cudaStream_t stream
     if (n > 0)
     {
         if (soupOnDevice) soup = const_cast<float*>(reinterpret_cast<const float*>(hostTris));
-        if (!soupOnDevice)
-            MB_CHECK(cudaMemcpyAsync(soup, hostTris, sizeof(prt_soup_triangle) * (size_t)n, cudaMemcpyDefault, stream));
+        else
+            MB_CHECK(stage_upload(soup, hostTris, sizeof(prt_soup_triangle) * (size_t)n, stream));
     }
     MB_CHECK(cudaMemsetAsync(small, 0, sizeof(unsigned) * 2, stream));
     MB_CHECK(cudaEventRecord(ev0, stream));
@@ -597,13 +597,14 @@ int build_mesh_gpu_indexed(const SoupIndexed& s, cudaStream_t stream, BuiltMesh&
         e = dev_malloc(&block, carve(nullptr));
     }
     if (e == cudaSuccess) carve(block);
-    if (e == cudaSuccess && s.nv) e = cudaMemcpyAsync(dv, s.v, sizeof(float) * 3 * (size_t)s.nv, cudaMemcpyHostToDevice, stream);
-    if (e == cudaSuccess && s.nvt)
-        e = cudaMemcpyAsync(dvt, s.vt, sizeof(float) * 2 * (size_t)s.nvt, cudaMemcpyHostToDevice, stream);
-    if (e == cudaSuccess && s.nvn)
-        e = cudaMemcpyAsync(dvn, s.vn, sizeof(float) * 3 * (size_t)s.nvn, cudaMemcpyHostToDevice, stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dcorners, s.corners, sizeof(int) * cornerInts, cudaMemcpyHostToDevice, stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dmat, s.mat, sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, stream);
+    auto put = [&](void* dst, const void* src, size_t bytes) {
+        if (e == cudaSuccess && bytes) e = stage_upload(dst, src, bytes, stream);
+    };
+    put(dv, s.v, sizeof(float) * 3 * (size_t)s.nv);
+    put(dvt, s.vt, sizeof(float) * 2 * (size_t)s.nvt);
+    put(dvn, s.vn, sizeof(float) * 3 * (size_t)s.nvn);
+    put(dcorners, s.corners, sizeof(int) * cornerInts);
+    put(dmat, s.mat, sizeof(int) * (size_t)n);
     if (e == cudaSuccess)
     {
         k_soup_expand<<<div_up(n, 256), 256, 0, stream>>>(dv, dvt, dvn, dcorners, s.cornerInts, dmat, n, dsoup);

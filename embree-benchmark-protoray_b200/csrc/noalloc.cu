@@ -37,6 +37,36 @@
 namespace prt_b200 {
 
 namespace {
+using CtxGetCurrentFn = CUresult (*)(CUcontext*);
+using CtxGetIdFn = CUresult (*)(CUcontext, unsigned long long*);
+} // namespace
+
+// Id of the CUDA context current on this thread, through the driver entry
+// points the runtime hands out (no link against libcuda needed).
+cudaError_t current_context_id(unsigned long long* id)
+{
+    static CtxGetCurrentFn getCurrent = nullptr;
+    static CtxGetIdFn getId = nullptr;
+    if (!getCurrent || !getId)
+    {
+        void* f0 = nullptr;
+        void* f1 = nullptr;
+        cudaDriverEntryPointQueryResult q0, q1;
+        cudaError_t e = cudaGetDriverEntryPoint("cuCtxGetCurrent", &f0, cudaEnableDefault, &q0);
+        if (e == cudaSuccess) e = cudaGetDriverEntryPoint("cuCtxGetId", &f1, cudaEnableDefault, &q1);
+        if (e != cudaSuccess) return e;
+        if (q0 != cudaDriverEntryPointSuccess || q1 != cudaDriverEntryPointSuccess || !f0 || !f1)
+            return cudaErrorSymbolNotFound;
+        getCurrent = reinterpret_cast<CtxGetCurrentFn>(f0);
+        getId = reinterpret_cast<CtxGetIdFn>(f1);
+    }
+    CUcontext c = nullptr;
+    if (getCurrent(&c) != CUDA_SUCCESS || !c) return cudaErrorDeviceUninitialized;
+    if (getId(c, id) != CUDA_SUCCESS) return cudaErrorDeviceUninitialized;
+    return cudaSuccess;
+}
+
+namespace {
 
 constexpr long long kNoAllocMaxPaths = 1LL << 19;
 constexpr int kNoAllocCounters = 64 + 2;   // one slot per bounce depth (max depth 64) + 2
@@ -64,34 +94,6 @@ struct AddressCache
 
 std::mutex g_lock;
 AddressCache g_cache[kMaxDevices];
-
-using CtxGetCurrentFn = CUresult (*)(CUcontext*);
-using CtxGetIdFn = CUresult (*)(CUcontext, unsigned long long*);
-
-// Id of the CUDA context current on this thread, through the driver entry
-// points the runtime hands out (no link against libcuda needed).
-cudaError_t current_context_id(unsigned long long* id)
-{
-    static CtxGetCurrentFn getCurrent = nullptr;
-    static CtxGetIdFn getId = nullptr;
-    if (!getCurrent || !getId)
-    {
-        void* f0 = nullptr;
-        void* f1 = nullptr;
-        cudaDriverEntryPointQueryResult q0, q1;
-        cudaError_t e = cudaGetDriverEntryPoint("cuCtxGetCurrent", &f0, cudaEnableDefault, &q0);
-        if (e == cudaSuccess) e = cudaGetDriverEntryPoint("cuCtxGetId", &f1, cudaEnableDefault, &q1);
-        if (e != cudaSuccess) return e;
-        if (q0 != cudaDriverEntryPointSuccess || q1 != cudaDriverEntryPointSuccess || !f0 || !f1)
-            return cudaErrorSymbolNotFound;
-        getCurrent = reinterpret_cast<CtxGetCurrentFn>(f0);
-        getId = reinterpret_cast<CtxGetIdFn>(f1);
-    }
-    CUcontext c = nullptr;
-    if (getCurrent(&c) != CUDA_SUCCESS || !c) return cudaErrorDeviceUninitialized;
-    if (getId(c, id) != CUDA_SUCCESS) return cudaErrorDeviceUninitialized;
-    return cudaSuccess;
-}
 
 // Device address of g_scratch in the current context of `device` (which is
 // current); looked up once per context.

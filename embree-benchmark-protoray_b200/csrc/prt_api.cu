@@ -63,6 +63,7 @@ struct prt_ctx
     Bvh8Device bvh;
     DeviceScratch buildScratch;   // BVH and mesh build scratch, reused by later builds
     DeviceScratch uploadScratch;  // a parsed OBJ's lists on the device, reused by later mesh builds
+    bool staged = false;          // counted among the device's users of the staging slots
     bool built = false;
     int leafMax = kDefaultLeafMax;
     bool highQuality = true;   // SAH grouping into 8-wide nodes
@@ -446,14 +447,15 @@ int check_ready(prt_ctx* ctx, bool needFrame)
     return PRT_OK;
 }
 
-__global__ void k_deinterleave(const float* __restrict__ attrs, int stride, int nv, float* __restrict__ pos)
+// Floats [first, first + width) of nv records of stride floats, packed.
+__global__ void k_column(const float* __restrict__ attrs, int stride, int first, int width, int nv,
+                         float* __restrict__ out)
 {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < 3LL * nv;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)width * nv;
          i += (long long)gridDim.x * blockDim.x)
     {
-        long long v = i / 3;
-        int k = (int)(i - 3 * v);
-        pos[i] = attrs[v * stride + k];
+        const long long v = i / width;
+        out[i] = attrs[v * stride + first + (int)(i - width * v)];
     }
 }
 
@@ -660,7 +662,7 @@ int load_mesh_file(prt_ctx* ctx, const char* path, float outLo[3], float outHi[3
         e = cudaMemcpyAsync(dAttr, pinned + idxBytes, attrBytes, cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess && stride != 3 && vert)
     {
-        k_deinterleave<<<512, 256, 0, ctx->stream>>>(dAttr, stride, vert, dPos);
+        k_column<<<512, 256, 0, ctx->stream>>>(dAttr, stride, 0, 3, vert, dPos);
         ctx->launches++;
         e = cudaGetLastError();
     }
@@ -699,6 +701,7 @@ prt_ctx::~prt_ctx()
     bvh.release();
     buildScratch.release();
     uploadScratch.release();
+    if (staged) stage_release(device);
     cudaFree(dPos);
     cudaFree(dIdx);
     cudaFree(dAlbedo);
@@ -748,6 +751,8 @@ int prt_create(int device, prt_ctx** out)
     CK(cudaGetDeviceProperties(&prop, device));
     ctx->numSMs = prop.multiProcessorCount;
     ctx->name = prop.name;
+    stage_retain(device);
+    ctx->staged = true;
     CK(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
     CK(cudaEventCreate(&ctx->ev0));
     CK(cudaEventCreate(&ctx->ev1));
@@ -798,9 +803,9 @@ int prt_load_mesh(prt_ctx* ctx, const int* indices, int triCount, const float* p
     cudaError_t e = dev_malloc(&dPos, sizeof(float) * 3 * (size_t)std::max(vertCount, 1));
     if (e == cudaSuccess) e = dev_malloc(&dIdx, sizeof(int) * 3 * (size_t)std::max(triCount, 1));
     if (e == cudaSuccess && vertCount)
-        e = cudaMemcpyAsync(dPos, positions, sizeof(float) * 3 * (size_t)vertCount, cudaMemcpyDefault, ctx->stream);
+        e = stage_upload(dPos, positions, sizeof(float) * 3 * (size_t)vertCount, ctx->stream);
     if (e == cudaSuccess && triCount)
-        e = cudaMemcpyAsync(dIdx, indices, sizeof(int) * 3 * (size_t)triCount, cudaMemcpyDefault, ctx->stream);
+        e = stage_upload(dIdx, indices, sizeof(int) * 3 * (size_t)triCount, ctx->stream);
     if (e != cudaSuccess)
     {
         cudaFree(dPos);
@@ -1009,8 +1014,7 @@ int prt_read_accum(prt_ctx* ctx, float* rgbw)
     if (!ctx || !rgbw) return PRT_EINVAL;
     if (!ctx->dAccum) return fail(ctx, PRT_ESTATE, "frame not initialised (prt_init_frame)");
     CK(cudaSetDevice(ctx->device));
-    CK(cudaMemcpyAsync(rgbw, ctx->dAccum, sizeof(float4) * (size_t)ctx->W * ctx->H, cudaMemcpyDefault, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
+    CK(stage_download(rgbw, ctx->dAccum, sizeof(float4) * (size_t)ctx->W * ctx->H, ctx->stream));
     return PRT_OK;
 }
 
@@ -1681,21 +1685,29 @@ int prt_read_built_mesh(prt_ctx* ctx, int* indices, int* materialIds, float* pos
     CK(cudaSetDevice(ctx->device));
     if (m.triCount)
     {
-        CK(cudaMemcpyAsync(indices, m.idx, sizeof(int) * 3 * (size_t)m.triCount, cudaMemcpyDefault, ctx->stream));
-        CK(cudaMemcpyAsync(materialIds, m.mat, sizeof(int) * (size_t)m.triCount, cudaMemcpyDefault, ctx->stream));
+        CK(stage_download(indices, m.idx, sizeof(int) * 3 * (size_t)m.triCount, ctx->stream));
+        CK(stage_download(materialIds, m.mat, sizeof(int) * (size_t)m.triCount, ctx->stream));
     }
-    if (m.vertCount)
+    if (m.vertCount && m.stride == 3)
     {
-        // de-interleave with strided copies: position, normal and texcoord columns
-        const size_t pitch = sizeof(float) * m.stride;
-        CK(cudaMemcpy2DAsync(positions, 12, m.attr, pitch, 12, m.vertCount, cudaMemcpyDefault, ctx->stream));
-        if (m.hasNormals)
-            CK(cudaMemcpy2DAsync(normals, 12, m.attr + 3, pitch, 12, m.vertCount, cudaMemcpyDefault, ctx->stream));
-        if (m.hasTexcoords)
-            CK(cudaMemcpy2DAsync(texcoords, 8, m.attr + (m.hasNormals ? 6 : 3), pitch, 8, m.vertCount,
-                                 cudaMemcpyDefault, ctx->stream));
+        CK(stage_download(positions, m.attr, sizeof(float) * 3 * (size_t)m.vertCount, ctx->stream));
     }
-    CK(cudaStreamSynchronize(ctx->stream));
+    else if (m.vertCount)
+    {
+        // the position, normal and texcoord columns, gathered in the build's scratch
+        const size_t nv = (size_t)m.vertCount;
+        CK(ctx->buildScratch.reserve(sizeof(float) * 3 * nv));
+        float* tmp = static_cast<float*>(ctx->buildScratch.p);
+        auto column = [&](float* out, int first, int width) -> cudaError_t {
+            k_column<<<512, 256, 0, ctx->stream>>>(m.attr, m.stride, first, width, m.vertCount, tmp);
+            ctx->launches++;
+            cudaError_t e = cudaGetLastError();
+            return e == cudaSuccess ? stage_download(out, tmp, sizeof(float) * width * nv, ctx->stream) : e;
+        };
+        CK(column(positions, 0, 3));
+        if (m.hasNormals) CK(column(normals, 3, 3));
+        if (m.hasTexcoords) CK(column(texcoords, m.hasNormals ? 6 : 3, 2));
+    }
     return PRT_OK;
 }
 

@@ -108,6 +108,23 @@ struct DeviceScratch
     }
 };
 
+// Id of the CUDA context current on this thread (noalloc.cu); a device has
+// another one after cudaDeviceReset.
+cudaError_t current_context_id(unsigned long long* id);
+
+// Bulk copies between pageable host memory and the current device through
+// pinned slots filled by several threads (host_copy.cu); copies of pinned or
+// device memory and small ones go to cudaMemcpyAsync.  The slots (8 MB) are
+// shared by the contexts of a device: made at the first large copy, freed with
+// the device's last context; a copy that finds them in use by another thread
+// goes to cudaMemcpyAsync.
+void stage_retain(int device);    // a context on the device begins
+void stage_release(int device);   // and ends
+// returns when src has been read; the copies are enqueued on stream
+cudaError_t stage_upload(void* dst, const void* src, size_t bytes, cudaStream_t stream);
+// returns when dst is complete
+cudaError_t stage_download(void* dst, const void* src, size_t bytes, cudaStream_t stream);
+
 struct BuildInfo
 {
     double buildMs = 0;
