@@ -138,6 +138,13 @@ constexpr int kRefillMin = PRT_REFILL_MIN;
 #ifndef PRT_BOUNCE_MIN_BLOCKS
 #define PRT_BOUNCE_MIN_BLOCKS 8
 #endif
+// The kernels that carry more per lane (a batch's request, shadow rays,
+// gradients, barycentrics) spill at 64 registers and are faster with 72 and 7
+// blocks: 32-request batch 30.8 -> 29.9 ms, diffuse2 1080p 4 passes 11.08 -> 10.93,
+// 4M closest-hit queries 1.280 -> 1.265, adjoint 512x512 16 passes 1.95 -> 1.93.  The
+// others lose 0.2% (any hit 1.3%, packets 3.5%); 6 blocks lose 1-3%, 9 blocks (56
+// registers) 5%.
+constexpr int kWideBlocks = 7;
 
 // One bounce of the wavefront over the queue of paths entering `depth`.
 // kFirst: the queue is implicit — item i is (pass, 8x8 tile, Morton index)
@@ -398,7 +405,7 @@ __device__ __forceinline__ int stop_idle(unsigned act)
 }
 
 template <class Args, bool kBatch, bool kAlbedo>
-__global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_paths(Args a)
+__global__ void __launch_bounds__(128, kBatch ? kWideBlocks : PRT_BOUNCE_MIN_BLOCKS) k_paths(Args a)
 {
     extern __shared__ uint2 s_stack[];
     TravStack st;
@@ -912,7 +919,7 @@ __global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_primary_packet(W
 // escaping extension ray adds throughput * sky weighted 1 from the camera and
 // 0.5 after a bounce.  Shadow rays are counted as rays.
 template <bool kFirst, bool kAlbedo>
-__global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_bounce_nee(WaveArgs a, int depth)
+__global__ void __launch_bounds__(128, kWideBlocks) k_bounce_nee(WaveArgs a, int depth)
 {
     extern __shared__ uint2 s_stack[];
     TravStack st;
@@ -1118,7 +1125,7 @@ __global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_bounce_nee(WaveA
 constexpr int kNeeWords = 11;   // pixel, depth | shadow << 8, RNG, throughput, radiance, direction, extension origin
 
 template <bool kAlbedo>
-__global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_paths_nee(WaveArgs a)
+__global__ void __launch_bounds__(128, kWideBlocks) k_paths_nee(WaveArgs a)
 {
     extern __shared__ uint2 s_stack[];
     TravStack st;
@@ -1251,7 +1258,7 @@ __global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_paths_nee(WaveAr
 constexpr int kQueryRefill = 12;
 
 template <bool kAnyHit>
-__global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_intersect(SceneDev sc, const RayRec* __restrict__ rays,
+__global__ void __launch_bounds__(128, kAnyHit ? PRT_BOUNCE_MIN_BLOCKS : kWideBlocks) k_intersect(SceneDev sc, const RayRec* __restrict__ rays,
                                                                          HitRec* __restrict__ hits,
                                                                          float* __restrict__ anyOut, int n, int* fetch)
 {
@@ -1541,7 +1548,7 @@ constexpr int kBackwardWords = 9;          // and dL/d(radiance) of the pixel, t
 // lanes that kept the path in registers, refilled at 12 idle lanes only and (in
 // the backward mode) tested triangles in the lane.
 template <bool kBackward>
-__global__ void __launch_bounds__(128, 8) k_replay(SceneDev sc, CameraDev cam, float4* accum, int pass0, int spp,
+__global__ void __launch_bounds__(128, kWideBlocks) k_replay(SceneDev sc, CameraDev cam, float4* accum, int pass0, int spp,
                                                    int maxDepth, float sky, const float* __restrict__ dL,
                                                    float* dAlbedo, float* dSky, unsigned long long* rays,
                                                    int* fetch)
@@ -1717,7 +1724,7 @@ __global__ void __launch_bounds__(128, 8) k_replay(SceneDev sc, CameraDev cam, f
 // tile, Morton index) by a binary search over the requests' path ranges; the
 // queued path records carry (request << 24 | pixel).  Lanes refill dynamically
 // as in k_bounce; k_paths takes the queue.
-__global__ void __launch_bounds__(128, 8) k_batch_first(BatchArgs a)
+__global__ void __launch_bounds__(128, kWideBlocks) k_batch_first(BatchArgs a)
 {
     extern __shared__ uint2 s_dyn[];
     uint2* s_stack = s_dyn;
