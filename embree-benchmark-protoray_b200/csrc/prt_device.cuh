@@ -863,10 +863,15 @@ __device__ __forceinline__ void triq_flush(TriQueue& q, uint32_t first, uint32_t
 // or, when mayStop, until refillMin lanes are idle; every queued test is merged
 // before it returns.  active: this lane holds a ray.  anyHit: this lane's ray
 // is an occlusion query, which stops at the first merged hit (its later queued
-// tests are still merged, which can only move the hit nearer).  The counter
+// tests are still merged, which can only move the hit nearer).  kEager: a flush
+// takes as many tests as lanes were traversing (at most 32) instead of 32, so
+// that hits are known soon when few rays are left or when a hit ends the ray.
+// Ray queries gain (4M incoherent rays: any hit 1.000 -> 0.925 ms, closest 1.262
+// -> 1.240; 100000 rays, closest 0.152 -> 0.117); the path kernels, with shorter
+// rays and lanes that go on bouncing, lose 0.5-2%.  The counter
 // pointers (node visits, triangle tests per lane; steps, running-lane steps and
 // flushes per warp) may be null.
-template <bool kPair = false, bool kUV = false>
+template <bool kPair = false, bool kUV = false, bool kEager = false>
 __device__ __forceinline__ void warp_trav_deferred(TriQueue& q, TravState& ts, const SceneDev& sc, const TravRay& r,
                                                    float tnear, TravStack& st, bool active, bool mayStop, int refillMin,
                                                    unsigned lane, uint32_t* cNodes = nullptr, uint32_t* cTris = nullptr,
@@ -876,7 +881,8 @@ __device__ __forceinline__ void warp_trav_deferred(TriQueue& q, TravState& ts, c
                                                    TriQueueUV* uv = nullptr)
 {
     const unsigned FULL = 0xffffffffu;
-    uint32_t n = 0;   // queued triangles
+    uint32_t n = 0;       // queued triangles
+    uint32_t full = 32;   // of a flush
     for (;;)
     {
         uint32_t tbase = 0, tbits = 0, lmask = 0;
@@ -887,15 +893,16 @@ __device__ __forceinline__ void warp_trav_deferred(TriQueue& q, TravState& ts, c
         }
         if (active && !ts.done) trav_visit<kPair>(ts, sc, r, tnear, st, tbase, tbits, lmask, cNodes);
         triq_push(q, n, tbase, tbits, lmask, lane);
-        if (n >= 32u)
+        if (n >= full)
         {
             uint32_t first = 0;
             do
             {
-                triq_flush<kUV>(q, first, 32u, sc.tris, r, tnear, ts, lane, uv, cTris);
+                const uint32_t m = kEager ? min(32u, n - first) : 32u;
+                triq_flush<kUV>(q, first, m, sc.tris, r, tnear, ts, lane, uv, cTris);
                 if (cFlushes) *cFlushes += 1;
-                first += 32u;
-            } while (n - first >= 32u);
+                first += m;
+            } while (n - first >= full);
             if (anyHit && ts.triHit >= 0) ts.done = true;
             // the rest moves to the front
             n -= first;
@@ -903,6 +910,7 @@ __device__ __forceinline__ void warp_trav_deferred(TriQueue& q, TravState& ts, c
         }
         const unsigned running = __ballot_sync(FULL, active && !ts.done);
         if (running == 0) break;
+        if (kEager) full = (uint32_t)__popc(running);
         if (mayStop && 32 - __popc(running) >= refillMin) break;
     }
     if (n)

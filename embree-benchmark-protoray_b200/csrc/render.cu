@@ -1310,7 +1310,7 @@ __global__ void __launch_bounds__(128, kAnyHit ? PRT_BOUNCE_MIN_BLOCKS : kWideBl
         if (PRT_DEFER_ISECT && sc.deferTris)
         {
             constexpr bool kPair = kAnyHit && PRT_PAIRED_QUERY;
-            warp_trav_deferred<kPair, !kAnyHit>(*tq, ts, sc, r, tnear, st, has, !exhausted, kQueryRefill, lane, nullptr,
+            warp_trav_deferred<kPair, !kAnyHit, true>(*tq, ts, sc, r, tnear, st, has, !exhausted, kQueryRefill, lane, nullptr,
                                                 nullptr, nullptr, nullptr, nullptr, kAnyHit, tuv);
         }
         else
@@ -2046,13 +2046,13 @@ int launch_batch_first(const BatchArgs& a, const LaunchCfg& cfg, int numSMs, cud
     return 1;
 }
 
-// Up to about 256 (closest) or 512 (any hit) rays per SM the longest ray's chain
+// Up to about 192 (closest) or 320 (any hit) rays per SM the longest ray's chain
 // of node visits takes longer than the work does, and eight lanes per ray win;
 // beyond that their emptier lanes cost more than they save.  Incoherent
 // closest-hit calls, one lane -> eight lanes: 1000 rays on 82K triangles 54 -> 39
-// us, on 1.38M 81 -> 43; 40000 on 1.38M 110 -> 94; 80000 on 1.38M 128 -> 148 (any
-// hit: 112 -> 114).
-bool intersect_few(int n, bool anyHit, int numSMs) { return n <= (anyHit ? 512 : 256) * numSMs; }
+// us, on 1.38M 66 -> 42; 28000 on 1.38M 84 -> 79, 40000 86 -> 94 (any hit: 82 -> 72,
+// and 80000 96 -> 114).
+bool intersect_few(int n, bool anyHit, int numSMs) { return n <= (anyHit ? 320 : 192) * numSMs; }
 
 int launch_intersect(const SceneDev& sc, const RayRec* rays, HitRec* hits, int n, bool anyHit, float* anyOut,
                      int* fetch, int numSMs, cudaStream_t s)

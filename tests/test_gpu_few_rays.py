@@ -9,7 +9,7 @@ torch = pytest.importorskip("torch")
 
 pytestmark = pytest.mark.gpu
 
-MANY = 200000   # above 512 rays per SM
+MANY = 200000   # above 320 rays per SM
 
 
 def _calls(c, rays, n):
@@ -43,7 +43,8 @@ def test_few_rays_equal_many(small, leaf, reach):
     torch.cuda.synchronize()
     hits, occ = _calls(c, rays, MANY)
     assert (hits[:, 1] >= 0).any() and (hits[:, 1] < 0).any()
-    for n in (1, 3, 4, 5, 31, 4 * sms, 4 * sms + 1, 16 * sms + 1, 256 * sms, 256 * sms + 1, 512 * sms, 512 * sms + 1):
+    for n in (1, 3, 4, 5, 31, 4 * sms, 4 * sms + 1, 16 * sms + 1, 192 * sms, 192 * sms + 1, 320 * sms, 320 * sms + 1,
+              512 * sms):
         h, o = _calls(c, rays, n)
         np.testing.assert_array_equal(h, hits[:n])
         np.testing.assert_array_equal(o >= 0, occ[:n] >= 0)
