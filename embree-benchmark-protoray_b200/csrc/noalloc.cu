@@ -69,13 +69,13 @@ cudaError_t current_context_id(unsigned long long* id)
 namespace {
 
 constexpr long long kNoAllocMaxPaths = 1LL << 19;
+constexpr long long kNoAllocMaxItems = 1LL << 30;   // of one launch without a queue: its 32-bit counter
 constexpr int kNoAllocCounters = 64 + 2;   // one slot per bounce depth (max depth 64) + 2
 
 struct NoAllocScratch
 {
     PathRec queue[kNoAllocMaxPaths];   // the paths of depth 1
     float thr[kNoAllocMaxPaths];       // per-path throughput (per-triangle albedo)
-    float L[kNoAllocMaxPaths];         // radiance gathered so far (next-event estimation)
     int counts[kNoAllocCounters];
     int fetch[kNoAllocCounters];
     unsigned long long rays;
@@ -191,7 +191,9 @@ extern "C" int prt_render_noalloc(prt_ctx* ctx, const prt_camera* cam, int width
     e = scratch_address(device, &s);
     if (e != cudaSuccess) return ctx_fail(ctx, PRT_ECUDA, cudaGetErrorString(e));
 
-    const int passesPerWave = (int)std::max<long long>(1, kNoAllocMaxPaths / perPass);
+    // packets need the queue; otherwise waves without one are as large as they come
+    const bool whole = nee || !packet_primaries(scene.leafTris, cfg);
+    const int passesPerWave = (int)std::max<long long>(1, (whole ? kNoAllocMaxItems : kNoAllocMaxPaths) / perPass);
     WaveArgs a;
     a.scene = scene;
     a.cam.origin = make_float3(cam->origin[0], cam->origin[1], cam->origin[2]);
@@ -225,19 +227,22 @@ extern "C" int prt_render_noalloc(prt_ctx* ctx, const prt_camera* cam, int width
         e = cudaMemsetAsync(s->counts, 0, sizeof(int) * 2 * kNoAllocCounters, stream);
         if (e != cudaSuccess) break;
         a.qin = nullptr;
-        a.qout = s->queue;
         a.thrIn = nullptr;
-        a.thrOut = albedo ? s->thr : nullptr;
-        a.Lin = nullptr;
-        a.Lout = nee ? s->L : nullptr;
         a.thrConst = 1.0f;
+        if (whole)
+        {
+            launch_whole(a, albedo, nee, cfg, numSMs, stream);
+            e = cudaGetLastError();
+            continue;
+        }
+        a.qout = s->queue;
+        a.thrOut = albedo ? s->thr : nullptr;
         launch_bounce(a, 0, cfg, numSMs, stream);
         e = cudaGetLastError();
         if (maxDepth > 0 && e == cudaSuccess)
         {
             a.qin = a.qout;
             a.thrIn = a.thrOut;
-            a.Lin = a.Lout;
             a.thrConst = 0.8f;
             launch_paths(a, cfg, numSMs, stream);
             e = cudaGetLastError();

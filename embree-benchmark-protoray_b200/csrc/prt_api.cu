@@ -40,6 +40,9 @@ constexpr int kMaxChains = 4;
 #define PRT_LEAF_MAX 1
 #endif
 constexpr int kDefaultLeafMax = PRT_LEAF_MAX;
+// Items (pixels of all passes, rounded up to tiles) of one launch: its 32-bit
+// counter also takes the requests of every lane past the end.
+constexpr long long kMaxItems = 1LL << 30;
 constexpr int kCounterStride = 64 + 2;   // counters per chain: one per bounce depth (<= 64) + 2
 
 struct prt_ctx
@@ -75,7 +78,7 @@ struct prt_ctx
     float4* dAccum = nullptr;
 
     // render state
-    int* dPass = nullptr;                 // device pass counter
+    int* dPass = nullptr;                 // first pass of the current render call, and of the next one
     unsigned long long* dRays = nullptr;  // rays of the current call
     int* dCounts = nullptr;               // per chain: path counts and work counters per depth (chain_counts)
     unsigned long long* hRays = nullptr;  // pinned: the call's ray count on the host
@@ -313,25 +316,45 @@ int passes_per_wave(const prt_ctx* ctx, int spp)
     return (int)std::max<long long>(1, std::min<long long>(spp, ppw / perPass));
 }
 
-// Records every device operation of one render call on ctx->stream (the
-// queues are allocated beforehand: no allocation happens during capture).
-int record_render(prt_ctx* ctx, int spp, int maxDepth, int accumulate, int& launches)
+// The waves of one render call.
+struct WavePlan
+{
+    long long perPass;   // items of a pass: the frame rounded up to 8x8 tiles
+    int passes;          // per wave
+    int waves, chains;
+    bool whole;          // each wave is one launch without queues (whole_paths)
+};
+
+WavePlan plan_waves(const prt_ctx* ctx, int spp)
+{
+    WavePlan p;
+    const bool nee = ctx->integrator == PRT_INTEGRATOR_DIFFUSE2;
+    p.perPass = (long long)((ctx->W + 7) / 8) * ((ctx->H + 7) / 8) * 64;
+    p.passes = passes_per_wave(ctx, spp);
+    p.whole = whole_paths(p.passes * p.perPass, ctx->bvh.leafMax, ctx->cfg, nee, ctx->numSMs);
+    // without queues nothing but the item counter bounds a wave
+    if (nee && ctx->cfg.pathsPerWave == 0) p.passes = (int)std::max<long long>(1, std::min<long long>(spp, kMaxItems / p.perPass));
+    p.waves = (spp + p.passes - 1) / p.passes;
+    p.chains = std::max(1, std::min(chains_for(ctx), p.waves));
+    return p;
+}
+
+// Issues every device operation of one render call on ctx->stream (the
+// queues are allocated beforehand, so that the call can be captured).
+int record_render(prt_ctx* ctx, const WavePlan& plan, int spp, int maxDepth, int accumulate, int& launches)
 {
     const int W = ctx->W, H = ctx->H;
     const int tilesX = (W + 7) / 8, tilesY = (H + 7) / 8;
-    const long long perPass = (long long)tilesX * tilesY * 64;
-    const int passesPerWave = passes_per_wave(ctx, spp);
+    const int passesPerWave = plan.passes, waves = plan.waves, chains = plan.chains;
     const bool albedo = ctx->dAlbedo != nullptr;
-    const int waves = (spp + passesPerWave - 1) / passesPerWave;
-    const int chains = std::max(1, std::min(chains_for(ctx), waves));
     const bool nee = ctx->integrator == PRT_INTEGRATOR_DIFFUSE2;
-    if (ctx->queueCap < (long long)passesPerWave * perPass || ctx->queueChains < chains ||
-        (albedo && !ctx->queueThr) || (nee && !ctx->queueL))
+    if (!plan.whole && (ctx->queueCap < passesPerWave * plan.perPass || ctx->queueChains < chains ||
+                        (albedo && !ctx->queueThr)))
         return fail(ctx, PRT_EINTERNAL, "path queues too small");
 
     launches = 0;
     if (!accumulate) CK(cudaMemsetAsync(ctx->dAccum, 0, sizeof(float4) * (size_t)W * H, ctx->stream));
-    CK(cudaMemsetAsync(ctx->dRays, 0, sizeof(unsigned long long), ctx->stream));
+    launches += launch_begin_render(ctx->dPass, spp, ctx->dRays, ctx->dCounts, kMaxChains * 2 * kCounterStride, ctx->stream);
     // waves are dealt round-robin to `chains` streams, so the tail of one
     // wave's bounce kernel overlaps the work of another wave
     if (chains > 1)
@@ -357,21 +380,24 @@ int record_render(prt_ctx* ctx, int spp, int maxDepth, int accumulate, int& laun
         a.fetch = chain_fetch(ctx, c);
         a.passOffset = w * passesPerWave;
         a.passes = std::min(passesPerWave, spp - w * passesPerWave);
-        CK(clear_chain(ctx, c, s));
-        // depth 0 fills the chain's queue, one launch carries its paths to their ends
+        if (w >= chains) CK(clear_chain(ctx, c, s));   // launch_begin_render has cleared the first waves'
         a.qin = nullptr;
-        a.qout = ctx->q[c][0];
         a.thrIn = nullptr;
-        a.thrOut = albedo ? ctx->thr[c][0] : nullptr;
         a.Lin = nullptr;
-        a.Lout = nee ? ctx->Lq[c][0] : nullptr;
         a.thrConst = const_throughput(0);
+        if (plan.whole)
+        {
+            launches += launch_whole(a, albedo, nee, ctx->cfg, ctx->numSMs, s);
+            continue;
+        }
+        // depth 0 fills the chain's queue, one launch carries its paths to their ends
+        a.qout = ctx->q[c][0];
+        a.thrOut = albedo ? ctx->thr[c][0] : nullptr;
         launches += launch_bounce(a, 0, ctx->cfg, ctx->numSMs, s);
         if (maxDepth > 0)
         {
             a.qin = a.qout;
             a.thrIn = a.thrOut;
-            a.Lin = a.Lout;
             a.thrConst = const_throughput(1);
             launches += launch_paths(a, ctx->cfg, ctx->numSMs, s);
         }
@@ -382,7 +408,6 @@ int record_render(prt_ctx* ctx, int spp, int maxDepth, int accumulate, int& laun
             CK(cudaEventRecord(ctx->joinEv[c], ctx->side[c]));
             CK(cudaStreamWaitEvent(ctx->stream, ctx->joinEv[c], 0));
         }
-    launches += launch_advance_pass(ctx->dPass, spp, ctx->stream);
     CK(cudaGetLastError());
     return PRT_OK;
 }
@@ -756,8 +781,8 @@ int prt_create(int device, prt_ctx** out)
     CK(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
     CK(cudaEventCreate(&ctx->ev0));
     CK(cudaEventCreate(&ctx->ev1));
-    CK(dev_malloc(&ctx->dPass, sizeof(int)));
-    CK(cudaMemset(ctx->dPass, 0, sizeof(int)));
+    CK(dev_malloc(&ctx->dPass, sizeof(int) * 2));
+    CK(cudaMemset(ctx->dPass, 0, sizeof(int) * 2));
     CK(dev_malloc(&ctx->dRays, sizeof(unsigned long long)));
     CK(dev_malloc(&ctx->dCounts, sizeof(int) * 2 * kCounterStride * kMaxChains));
     CK(host_pinned_alloc(reinterpret_cast<char**>(&ctx->hRays), sizeof(*ctx->hRays)));
@@ -986,7 +1011,7 @@ int prt_clear(prt_ctx* ctx)
     if (!ctx->dAccum) return fail(ctx, PRT_ESTATE, "frame not initialised (prt_init_frame)");
     CK(cudaSetDevice(ctx->device));
     CK(cudaMemsetAsync(ctx->dAccum, 0, sizeof(float4) * (size_t)ctx->W * ctx->H, ctx->stream));
-    CK(cudaMemsetAsync(ctx->dPass, 0, sizeof(int), ctx->stream));
+    CK(cudaMemsetAsync(ctx->dPass, 0, sizeof(int) * 2, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     return PRT_OK;
 }
@@ -995,7 +1020,7 @@ int prt_set_pass(prt_ctx* ctx, int pass)
 {
     if (!ctx || pass < 0) return PRT_EINVAL;
     CK(cudaSetDevice(ctx->device));
-    CK(cudaMemcpyAsync(ctx->dPass, &pass, sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(ctx->dPass + 1, &pass, sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     return PRT_OK;
 }
@@ -1004,7 +1029,7 @@ int prt_get_pass(prt_ctx* ctx, int* pass)
 {
     if (!ctx || !pass) return PRT_EINVAL;
     CK(cudaSetDevice(ctx->device));
-    CK(cudaMemcpyAsync(pass, ctx->dPass, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaMemcpyAsync(pass, ctx->dPass + 1, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     return PRT_OK;
 }
@@ -1042,25 +1067,34 @@ int prt_render(prt_ctx* ctx, int spp, int maxDepth, int accumulate, prt_render_s
     if (st != PRT_OK) return st;
     if (spp < 0 || maxDepth < 0 || maxDepth > kMaxDepthCap) return fail(ctx, PRT_EINVAL, "invalid spp or maxDepth");
     CK(cudaSetDevice(ctx->device));
+    WavePlan plan{};
     if (spp > 0)
     {
-        const long long perPass = (long long)((ctx->W + 7) / 8) * ((ctx->H + 7) / 8) * 64;
-        const int ppw = passes_per_wave(ctx, spp);
-        const int waves = (spp + ppw - 1) / ppw;
-        st = ensure_queues(ctx, (long long)ppw * perPass, ctx->dAlbedo != nullptr,
-                           std::max(1, std::min(chains_for(ctx), waves)),
-                           ctx->integrator == PRT_INTEGRATOR_DIFFUSE2);
-        if (st != PRT_OK) return st;
+        plan = plan_waves(ctx, spp);
+        if (!plan.whole)
+        {
+            st = ensure_queues(ctx, plan.passes * plan.perPass, ctx->dAlbedo != nullptr, plan.chains);
+            if (st != PRT_OK) return st;
+        }
     }
     CK(cudaEventRecord(ctx->ev0, ctx->stream));
     if (spp > 0)
     {
-        std::ostringstream key;
-        key << "render:" << ctx->integrator << ":" << spp << ":" << maxDepth << ":" << accumulate << ":" << ctx->cfg.block << ":"
-            << ctx->cfg.blocksPerSM << ":" << ctx->cfg.pathsPerWave;
         int launches = 0;
-        st = run_graph(ctx, key.str(), [&](int& l) { return record_render(ctx, spp, maxDepth, accumulate, l); },
-                       launches);
+        if (plan.waves == 1)
+        {
+            // two or three launches: cheaper than a graph of them, and nothing to
+            // record again when the camera or the scene changes
+            st = record_render(ctx, plan, spp, maxDepth, accumulate, launches);
+        }
+        else
+        {
+            std::ostringstream key;
+            key << "render:" << ctx->integrator << ":" << spp << ":" << maxDepth << ":" << accumulate << ":" << ctx->cfg.block
+                << ":" << ctx->cfg.blocksPerSM << ":" << ctx->cfg.pathsPerWave;
+            st = run_graph(ctx, key.str(),
+                           [&](int& l) { return record_render(ctx, plan, spp, maxDepth, accumulate, l); }, launches);
+        }
         if (st != PRT_OK) return st;
         ctx->launches += launches;
     }
@@ -1106,6 +1140,7 @@ int prt_render_profile(prt_ctx* ctx, int spp, int maxDepth, double* msPerDepth, 
     a.maxDepth = maxDepth;
     a.sky = ctx->sky;
     CK(cudaMemsetAsync(ctx->dAccum, 0, sizeof(float4) * (size_t)W * H, ctx->stream));
+    ctx->launches += launch_begin_render(ctx->dPass, spp, ctx->dRays, ctx->dCounts, kMaxChains * 2 * kCounterStride, ctx->stream);
     for (int p0 = 0; p0 < spp; p0 += ppw)
     {
         a.passOffset = p0;
@@ -1136,8 +1171,6 @@ int prt_render_profile(prt_ctx* ctx, int spp, int maxDepth, double* msPerDepth, 
             raysPerDepth[d] += d == 0 ? (long long)a.passes * W * H : counts[(size_t)d];
         }
     }
-    launch_advance_pass(ctx->dPass, spp, ctx->stream);
-    ctx->launches++;
     CK(cudaStreamSynchronize(ctx->stream));
     for (auto& e : ev) cudaEventDestroy(e);
     return PRT_OK;
@@ -1504,7 +1537,7 @@ int prt_autotune(prt_ctx* ctx, int spp, int maxDepth, prt_tune* best)
         for (int rep = 0; rep < 4; ++rep)
         {
             prt_render_stats rs;
-            CK(cudaMemsetAsync(ctx->dPass, 0, sizeof(int), ctx->stream));
+            CK(cudaMemsetAsync(ctx->dPass, 0, sizeof(int) * 2, ctx->stream));
             int s2 = prt_render(ctx, spp, maxDepth, 0, &rs);
             if (s2 != PRT_OK) return s2;
             if (rep > 0) *mray = std::max(*mray, rs.mray);

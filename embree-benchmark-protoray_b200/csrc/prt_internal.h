@@ -285,13 +285,20 @@ struct LaunchCfg
 int launch_bounce(const WaveArgs& a, int depth, const LaunchCfg& cfg, int numSMs, cudaStream_t s);
 // every bounce from depth 1 on (a.qin: the depth-1 queue, counts[1] paths)
 int launch_paths(const WaveArgs& a, const LaunchCfg& cfg, int numSMs, cudaStream_t s);
+// Whether waves of `paths` paths are best rendered by one launch from their
+// camera rays on (launch_whole, which needs no queue).  albedo: paths carry
+// per-triangle albedo; nee: next-event estimation.
+bool packet_primaries(int leafTris, const LaunchCfg& cfg);
+bool whole_paths(long long paths, int leafTris, const LaunchCfg& cfg, bool nee, int numSMs);
+int launch_whole(const WaveArgs& a, bool albedo, bool nee, const LaunchCfg& cfg, int numSMs, cudaStream_t s);
 // whether launch_intersect takes n rays without a work counter
 bool intersect_few(int n, bool anyHit, int numSMs);
 // fetch: a zeroed work counter on the device, used by this launch only (unused when intersect_few)
 int launch_intersect(const SceneDev& sc, const RayRec* rays, HitRec* hits, int n, bool anyHit, float* anyOut,
                      int* fetch, int numSMs, cudaStream_t s);
 int launch_resolve_ldr(const float4* accum, uint32_t* out, int n, cudaStream_t s);
-int launch_advance_pass(int* passBase, int spp, cudaStream_t s);
+// pass: this call's first pass, then the next call's; counters: the chains' words, cleared
+int launch_begin_render(int* pass, int spp, unsigned long long* rays, int* counters, int words, cudaStream_t s);
 // primary rays of pass `pass` for every pixel of cam's frame (row-major)
 int launch_primary_rays(const CameraDev& cam, int pass, RayRec* out, cudaStream_t s);
 int launch_query(const SceneDev& sc, const RayRec* ray, HitRec* hit, float* pNg, cudaStream_t s);

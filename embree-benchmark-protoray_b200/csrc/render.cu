@@ -5,7 +5,7 @@
 // -> shadeRaysKernel -> cudaMemcpy(count) } per bounce.  Here a wave takes two
 // persistent kernels: the first generates, traces and shades the primary rays
 // and queues the paths that go on, the second (k_paths) carries those paths
-// to their ends.  Queue sizes stay on the device, so a whole render is launched
+// to their ends; small waves and next-event estimation take one.  Queue sizes stay on the device, so a whole render is launched
 // without host synchronisation (and is captured as a CUDA graph by the API).
 // k_bounce and k_bounce_nee with kFirst = false do one bounce of all paths
 // per launch, for prt_render_profile's times per depth.
@@ -382,6 +382,8 @@ __global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_bounce(WaveArgs 
 // Measured against one launch per bounce: 1080p terrain frame of 1 pass 2.12 ->
 // 1.88 ms and of 32 passes 46.4 -> 45.2, 256x256 and 16 passes of 82K triangles
 // 0.765 -> 0.63 ms, 10.24M-triangle field at 4 passes and 9 bounces 5.17 -> 4.72.
+// kPrimary: the lanes generate their paths' camera rays too, so a small wave is
+// one launch with one tail and needs no queue (whole_paths below).
 constexpr int kPathWords = 7;   // tag (pixel; in a batch request << 24 | pixel), depth, RNG, throughput, direction
 
 __device__ __forceinline__ const SceneDev& path_scene(const WaveArgs& a, int) { return a.scene; }
@@ -404,9 +406,10 @@ __device__ __forceinline__ int stop_idle(unsigned act)
     return 32 - n + max(1, n * kRefillMin / 32);
 }
 
-template <class Args, bool kBatch, bool kAlbedo>
-__global__ void __launch_bounds__(128, kBatch ? kWideBlocks : PRT_BOUNCE_MIN_BLOCKS) k_paths(Args a)
+template <class Args, bool kBatch, bool kAlbedo, bool kPrimary>
+__global__ void __launch_bounds__(128, kBatch || kPrimary ? kWideBlocks : PRT_BOUNCE_MIN_BLOCKS) k_paths(Args a)
 {
+    static_assert(!(kBatch && kPrimary), "a batch's primary rays have their own kernels");
     extern __shared__ uint2 s_stack[];
     TravStack st;
     st.sh = s_stack + threadIdx.x;
@@ -419,9 +422,22 @@ __global__ void __launch_bounds__(128, kBatch ? kWideBlocks : PRT_BOUNCE_MIN_BLO
     const unsigned FULL = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned ltMask = (1u << lane) - 1u;
-    const int total = *(volatile int*)&a.counts[1];
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(a.rays, (unsigned long long)total);
-    unsigned long long more = 0;   // rays of depth 2 and on, per warp
+    int total, perPass = 0, pass0 = 0;
+    if constexpr (kPrimary)
+    {
+        perPass = a.tilesX * a.tilesY * 64;
+        total = a.passes * perPass;
+        pass0 = *a.passBase + a.passOffset;
+        if (blockIdx.x == 0 && threadIdx.x == 0)
+            atomicAdd(a.rays, (unsigned long long)a.passes * (unsigned long long)a.cam.width *
+                                  (unsigned long long)a.cam.height);
+    }
+    else
+    {
+        total = *(volatile int*)&a.counts[1];
+        if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(a.rays, (unsigned long long)total);
+    }
+    unsigned long long more = 0;   // rays of bounces in this kernel, per warp
 
     bool has = false;         // this lane holds a path
     bool exhausted = false;   // warp-uniform: every queued path has been claimed
@@ -465,28 +481,51 @@ __global__ void __launch_bounds__(128, kBatch ? kWideBlocks : PRT_BOUNCE_MIN_BLO
         {
             const int n = __popc(idle);
             int base = 0;
-            if (lane == 0) base = atomicAdd(&a.fetch[1], n);
+            if (lane == 0) base = atomicAdd(&a.fetch[kPrimary ? 0 : 1], n);
             base = __shfl_sync(FULL, base, 0);
             exhausted = base + n >= total;
             const int i = base + __popc(idle & ltMask);
             if (!has && i < total)
             {
-                const PathRec pr = load_path(a.qin, i);
-                org = f3(pr.w0.x, pr.w0.y, pr.w0.z);
-                dir = f3(pr.w1.x, pr.w1.y, pr.w1.z);
-                const uint32_t tag = __float_as_uint(pr.w0.w);
-                if (kBatch) req = (int)(tag >> 24);
-                float thr = 0.8f;
-                if constexpr (!kBatch) thr = kAlbedo ? __ldcs(a.thrIn + i) : a.thrConst;
-                path[0] = tag;
-                path[bd] = 1u;
-                path[2 * bd] = __float_as_uint(pr.w1.w);
-                path[3 * bd] = __float_as_uint(thr);
-                has = fresh = true;
+                if constexpr (kPrimary)
+                {
+                    const int pass = i / perPass;
+                    int x, y;
+                    if (wave_item_pixel(i - pass * perPass, a.tilesX, a.cam.width, a.cam.height, x, y))
+                    {
+                        const int pixel = x + y * a.cam.width;
+                        uint32_t rng = rng_seed(pass0 + pass, pixel);
+                        camera_ray(a.cam, x, y, rng, org, dir);
+                        path[0] = (uint32_t)pixel;
+                        path[bd] = 0u;
+                        path[2 * bd] = rng;
+                        path[3 * bd] = __float_as_uint(1.0f);
+                        has = fresh = true;
+                    }
+                }
+                else
+                {
+                    const PathRec pr = load_path(a.qin, i);
+                    org = f3(pr.w0.x, pr.w0.y, pr.w0.z);
+                    dir = f3(pr.w1.x, pr.w1.y, pr.w1.z);
+                    const uint32_t tag = __float_as_uint(pr.w0.w);
+                    if (kBatch) req = (int)(tag >> 24);
+                    float thr = 0.8f;
+                    if constexpr (!kBatch) thr = kAlbedo ? __ldcs(a.thrIn + i) : a.thrConst;
+                    path[0] = tag;
+                    path[bd] = 1u;
+                    path[2 * bd] = __float_as_uint(pr.w1.w);
+                    path[3 * bd] = __float_as_uint(thr);
+                    has = fresh = true;
+                }
             }
         }
         const unsigned act = __ballot_sync(FULL, has);
-        if (act == 0) break;   // every lane asked for a path above and the queue had none
+        if (act == 0)
+        {
+            if (exhausted) break;
+            continue;   // kPrimary: a tile's items outside the frame
+        }
         if (fresh)
         {
             path[4 * bd] = __float_as_uint(dir.x);
@@ -1118,10 +1157,14 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_bounce_nee(WaveArgs a, int
     if (lane == 0 && shadowRays) atomicAdd(a.rays, shadowRays);
 }
 
-// k_paths for the next-event-estimation integrator: at a hit before maxDepth a
+// A whole wave of the next-event-estimation integrator, from the camera rays on,
+// as k_paths<kPrimary>: at a hit before maxDepth a
 // lane samples its shadow and extension rays from the same frame, traces the
 // shadow ray first (any hit; +0.5 * throughput * sky if it escapes) while the
-// extension ray waits in shared memory, then the extension ray.
+// extension ray waits in shared memory, then the extension ray.  Camera rays are a
+// small part of this integrator's rays, so starting them here wins at every size:
+// against a first launch that queued the paths (k_bounce_nee), terrain 256x256 1
+// pass 0.76 -> 0.64 ms, 1001x563 16 passes 11.92 -> 11.54, 1080p 32 passes 86.5 -> 82.6.
 constexpr int kNeeWords = 11;   // pixel, depth | shadow << 8, RNG, throughput, radiance, direction, extension origin
 
 template <bool kAlbedo>
@@ -1139,9 +1182,13 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_paths_nee(WaveArgs a)
     const unsigned FULL = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned ltMask = (1u << lane) - 1u;
-    const int total = *(volatile int*)&a.counts[1];
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(a.rays, (unsigned long long)total);
-    unsigned long long more = 0;   // shadow rays and extension rays of depth 2 and on, per warp
+    const int perPass = a.tilesX * a.tilesY * 64;
+    const int total = a.passes * perPass;
+    const int pass0 = *a.passBase + a.passOffset;
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        atomicAdd(a.rays, (unsigned long long)a.passes * (unsigned long long)a.cam.width *
+                              (unsigned long long)a.cam.height);
+    unsigned long long more = 0;   // shadow rays and extension rays after the camera's, per warp
 
     bool has = false, exhausted = false;
     bool shadow = false;      // this lane's ray is a shadow ray
@@ -1169,7 +1216,8 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_paths_nee(WaveArgs a)
             }
             else if (ts.triHit < 0 || depth == a.maxDepth)
             {
-                if (ts.triHit < 0) L = __fadd_rn(L, __fmul_rn(__fmul_rn(thr, a.sky), 0.5f));
+                if (ts.triHit < 0)
+                    L = __fadd_rn(L, __fmul_rn(__fmul_rn(thr, a.sky), depth == 0 ? 1.0f : 0.5f));
                 red_add_v4(a.accum + path[0], L, L, L, 1.0f);
                 has = false;
             }
@@ -1201,29 +1249,38 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_paths_nee(WaveArgs a)
         {
             const int n = __popc(idle);
             int base = 0;
-            if (lane == 0) base = atomicAdd(&a.fetch[1], n);
+            if (lane == 0) base = atomicAdd(&a.fetch[0], n);
             base = __shfl_sync(FULL, base, 0);
             exhausted = base + n >= total;
             const int i = base + __popc(idle & ltMask);
             if (!has && i < total)
             {
-                const PathRec pr = load_path(a.qin, i);
-                org = f3(pr.w0.x, pr.w0.y, pr.w0.z);
-                dir = f3(pr.w1.x, pr.w1.y, pr.w1.z);
-                path[0] = __float_as_uint(pr.w0.w);
-                path[bd] = 1u;
-                path[2 * bd] = __float_as_uint(pr.w1.w);
-                path[3 * bd] = __float_as_uint(kAlbedo ? __ldcs(a.thrIn + i) : a.thrConst);
-                path[4 * bd] = __float_as_uint(__ldcs(a.Lin + i));
-                path[5 * bd] = __float_as_uint(dir.x);
-                path[6 * bd] = __float_as_uint(dir.y);
-                path[7 * bd] = __float_as_uint(dir.z);
-                shadow = false;
-                has = fresh = true;
+                const int pass = i / perPass;
+                int x, y;
+                if (wave_item_pixel(i - pass * perPass, a.tilesX, a.cam.width, a.cam.height, x, y))
+                {
+                    const int pixel = x + y * a.cam.width;
+                    uint32_t rng = rng_seed(pass0 + pass, pixel);
+                    camera_ray(a.cam, x, y, rng, org, dir);
+                    path[0] = (uint32_t)pixel;
+                    path[bd] = 0u;
+                    path[2 * bd] = rng;
+                    path[3 * bd] = __float_as_uint(1.0f);
+                    path[4 * bd] = 0u;
+                    path[5 * bd] = __float_as_uint(dir.x);
+                    path[6 * bd] = __float_as_uint(dir.y);
+                    path[7 * bd] = __float_as_uint(dir.z);
+                    shadow = false;
+                    has = fresh = true;
+                }
             }
         }
         const unsigned act = __ballot_sync(FULL, has);
-        if (act == 0) break;   // every lane asked for a path above and the queue had none
+        if (act == 0)
+        {
+            if (exhausted) break;
+            continue;   // a tile's items outside the frame
+        }
         if (fresh)
         {
             trav_setup(r, org, dir);
@@ -1523,7 +1580,18 @@ __global__ void k_resolve_ldr(const float4* __restrict__ accum, uint32_t* __rest
     out[i] = (uint32_t)b | ((uint32_t)gg << 8) | ((uint32_t)r << 16);
 }
 
-__global__ void k_advance_pass(int* passBase, int spp) { *passBase += spp; }
+// Start of a render call: its first pass is the next one (pass[1]), the call
+// after it begins spp later; the ray count and the wave counters start at 0.
+__global__ void k_begin_render(int* pass, int spp, unsigned long long* rays, int* counters, int words)
+{
+    if (threadIdx.x == 0)
+    {
+        pass[0] = pass[1];
+        pass[1] += spp;
+        *rays = 0;
+    }
+    for (int i = threadIdx.x; i < words; i += blockDim.x) counters[i] = 0;
+}
 
 constexpr int kReplayMaxDepth = 16;
 constexpr int kAggSlots = 256;             // block-private gradient slots of the adjoint
@@ -1960,7 +2028,7 @@ int launch_bounce(const WaveArgs& a, int depth, const LaunchCfg& cfg, int numSMs
         }
         return 1;
     }
-    if (depth == 0 && PRT_PACKET_PRIMARY && cfg.packet && a.scene.leafTris == 1)
+    if (depth == 0 && packet_primaries(a.scene.leafTris, cfg))
     {
         const size_t pshmem = sizeof(uint2) * kPacketStack * (cfg.block / 32);
         auto goPacket = [&](auto kernel) {
@@ -1994,6 +2062,15 @@ int launch_bounce(const WaveArgs& a, int depth, const LaunchCfg& cfg, int numSMs
 
 namespace {
 
+// Paths per SM up to which a wave's primary rays start in k_paths itself.  A
+// small wave is mostly tail (the last rays of each launch run on an emptying
+// chip) and one tail beats two; a large one loses more by mixing camera rays with
+// later bounces, whose neighbours have scattered.  Two launches -> one, 82K / 1.38M
+// / 450K triangles: 65K paths 0.29 / 0.46 / 0.28 -> 0.25 / 0.40 / 0.23 ms, 1M paths
+// 0.62 / 1.19 / 0.62 -> 0.59 / 1.16 / 0.57, 2.1M 0.93 / 1.93 / 0.95 -> 0.93 / 1.94 / 0.92,
+// 4.2M 1.57 / 3.46 / 1.63 -> 1.64 / 3.57 / 1.65.
+constexpr int kWholePaths = 10240;
+
 template <class Args, class Kernel>
 void run_paths(Kernel kernel, const Args& a, int words, bool deferred, const LaunchCfg& cfg, int numSMs, cudaStream_t s)
 {
@@ -2005,24 +2082,36 @@ void run_paths(Kernel kernel, const Args& a, int words, bool deferred, const Lau
 
 } // namespace
 
+bool packet_primaries(int leafTris, const LaunchCfg& cfg) { return PRT_PACKET_PRIMARY && cfg.packet && leafTris == 1; }
+
+bool whole_paths(long long paths, int leafTris, const LaunchCfg& cfg, bool nee, int numSMs)
+{
+    // primary rays as packets have their own kernel (not with next-event estimation)
+    return nee || (!packet_primaries(leafTris, cfg) && paths <= (long long)kWholePaths * numSMs);
+}
+
+int launch_whole(const WaveArgs& a, bool albedo, bool nee, const LaunchCfg& cfg, int numSMs, cudaStream_t s)
+{
+    const bool deferred = (nee ? PRT_DEFER_NEE : PRT_DEFER_TRIS) && a.scene.deferTris;
+    auto go = [&](auto kernel, int words) { run_paths(kernel, a, words, deferred, cfg, numSMs, s); };
+    if (nee && albedo) go(k_paths_nee<true>, kNeeWords);
+    else if (nee) go(k_paths_nee<false>, kNeeWords);
+    else if (albedo) go(k_paths<WaveArgs, false, true, true>, kPathWords);
+    else go(k_paths<WaveArgs, false, false, true>, kPathWords);
+    return 1;
+}
+
 int launch_paths(const WaveArgs& a, const LaunchCfg& cfg, int numSMs, cudaStream_t s)
 {
-    const bool albedo = a.thrIn != nullptr, deferred = PRT_DEFER_TRIS && a.scene.deferTris;
-    if (a.Lin)
-    {
-        const bool deferredNee = PRT_DEFER_NEE && a.scene.deferTris;
-        if (albedo) run_paths(k_paths_nee<true>, a, kNeeWords, deferredNee, cfg, numSMs, s);
-        else run_paths(k_paths_nee<false>, a, kNeeWords, deferredNee, cfg, numSMs, s);
-        return 1;
-    }
-    if (albedo) run_paths(k_paths<WaveArgs, false, true>, a, kPathWords, deferred, cfg, numSMs, s);
-    else run_paths(k_paths<WaveArgs, false, false>, a, kPathWords, deferred, cfg, numSMs, s);
+    const bool deferred = PRT_DEFER_TRIS && a.scene.deferTris;
+    if (a.thrIn) run_paths(k_paths<WaveArgs, false, true, false>, a, kPathWords, deferred, cfg, numSMs, s);
+    else run_paths(k_paths<WaveArgs, false, false, false>, a, kPathWords, deferred, cfg, numSMs, s);
     return 1;
 }
 
 int launch_batch_paths(const BatchArgs& a, const LaunchCfg& cfg, int numSMs, cudaStream_t s)
 {
-    run_paths(k_paths<BatchArgs, true, false>, a, kPathWords, PRT_DEFER_TRIS && a.leaf1, cfg, numSMs, s);
+    run_paths(k_paths<BatchArgs, true, false, false>, a, kPathWords, PRT_DEFER_TRIS && a.leaf1, cfg, numSMs, s);
     return 1;
 }
 
@@ -2129,9 +2218,9 @@ int launch_primary_rays(const CameraDev& cam, int pass, RayRec* out, cudaStream_
     return 1;
 }
 
-int launch_advance_pass(int* passBase, int spp, cudaStream_t s)
+int launch_begin_render(int* pass, int spp, unsigned long long* rays, int* counters, int words, cudaStream_t s)
 {
-    k_advance_pass<<<1, 1, 0, s>>>(passBase, spp);
+    k_begin_render<<<1, 256, 0, s>>>(pass, spp, rays, counters, words);
     return 1;
 }
 
