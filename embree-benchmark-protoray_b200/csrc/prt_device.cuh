@@ -200,39 +200,105 @@ struct SceneDev
 // other 5 bits of a queue entry hold the owner lane).
 constexpr int kDeferMaxTris = 1 << 27;
 
-// Per-ray constants for traversal.
+// Per-ray constants of the node tests.  oct: oct_code of the direction's octant.
 struct TravRay
 {
     float3 org;
-    float3 dir;
     float3 inv;
-    uint32_t octinv;   // 7 - octant of dir
-    int kx, ky, kz;    // watertight shear axes
-    float Sx, Sy, Sz;
+    uint32_t oct;
 };
 
-__device__ __forceinline__ void trav_setup(TravRay& r, float3 org, float3 dir)
+// Per-ray constants of the watertight triangle test: shear axes and factors.
+// Kernels with deferred tests keep them in shared memory (kShearWords words per
+// lane), since only flushes read them, usually another lane's.
+struct Shear
 {
-    r.org = org;
-    r.dir = dir;
-    const float tiny = 1e-30f;
-    r.inv.x = 1.0f / (fabsf(dir.x) > tiny ? dir.x : copysignf(tiny, dir.x));
-    r.inv.y = 1.0f / (fabsf(dir.y) > tiny ? dir.y : copysignf(tiny, dir.y));
-    r.inv.z = 1.0f / (fabsf(dir.z) > tiny ? dir.z : copysignf(tiny, dir.z));
-    uint32_t oct = (dir.x < 0.f ? 1u : 0u) | (dir.y < 0.f ? 2u : 0u) | (dir.z < 0.f ? 4u : 0u);
-    r.octinv = 7u - oct;
+    int kx, ky, kz;
+    float Sx, Sy, Sz;
+};
+constexpr int kShearWords = 4;
+
+__device__ __forceinline__ Shear shear_of(float3 dir)
+{
+    Shear s;
     float ax = fabsf(dir.x), ay = fabsf(dir.y), az = fabsf(dir.z);
     int kz = (ax > ay) ? (ax > az ? 0 : 2) : (ay > az ? 1 : 2);
     int kx = kz + 1; if (kx == 3) kx = 0;
     int ky = kx + 1; if (ky == 3) ky = 0;
     float dkz = kz == 0 ? dir.x : (kz == 1 ? dir.y : dir.z);
     if (dkz < 0.f) { int t = kx; kx = ky; ky = t; }
-    r.kx = kx; r.ky = ky; r.kz = kz;
+    s.kx = kx; s.ky = ky; s.kz = kz;
     float dkx = kx == 0 ? dir.x : (kx == 1 ? dir.y : dir.z);
     float dky = ky == 0 ? dir.x : (ky == 1 ? dir.y : dir.z);
-    r.Sx = dkx / dkz;
-    r.Sy = dky / dkz;
-    r.Sz = 1.0f / dkz;
+    s.Sx = dkx / dkz;
+    s.Sy = dky / dkz;
+    s.Sz = 1.0f / dkz;
+    return s;
+}
+
+// Word k of a lane's shear terms at w[k * stride].
+__device__ __forceinline__ void shear_store(uint32_t* w, int stride, const Shear& s)
+{
+    w[0] = __float_as_uint(s.Sx);
+    w[stride] = __float_as_uint(s.Sy);
+    w[2 * stride] = __float_as_uint(s.Sz);
+    w[3 * stride] = (uint32_t)(s.kx | (s.ky << 2) | (s.kz << 4));
+}
+
+__device__ __forceinline__ Shear shear_load(const uint32_t* w, int stride)
+{
+    Shear s;
+    s.Sx = __uint_as_float(w[0]);
+    s.Sy = __uint_as_float(w[stride]);
+    s.Sz = __uint_as_float(w[2 * stride]);
+    const int k = (int)w[3 * stride];
+    s.kx = k & 3;
+    s.ky = (k >> 2) & 3;
+    s.kz = k >> 4;
+    return s;
+}
+
+// Octant code: delta-swap masks that move bit s of an 8-bit mask to bit
+// s ^ octinv (permute_octant; a byte each in bits 0..23), and 24 ^ octinv in
+// bits 24..28 (next_child), where octinv = 7 - octant of the direction.
+__device__ __forceinline__ uint32_t oct_code(float3 dir)
+{
+    const uint32_t octinv = 7u - ((dir.x < 0.f ? 1u : 0u) | (dir.y < 0.f ? 2u : 0u) | (dir.z < 0.f ? 4u : 0u));
+    return ((octinv & 1u) ? 0x55u : 0u) | ((octinv & 2u) ? 0x3300u : 0u) | ((octinv & 4u) ? 0x0f0000u : 0u) |
+           ((24u ^ octinv) << 24);
+}
+
+__device__ __forceinline__ uint32_t oct_inv(uint32_t oct) { return 24u ^ (oct >> 24); }
+
+__device__ __forceinline__ uint32_t permute_octant(uint32_t x, uint32_t oct)
+{
+    uint32_t t = (x ^ (x >> 1)) & oct;   // x has 8 bits: only the lowest mask counts
+    x ^= t * 3u;
+    t = (x ^ (x >> 2)) & (oct >> 8);
+    x ^= t * 5u;
+    t = (x ^ (x >> 4)) & (oct >> 16);
+    return x ^ (t * 17u);
+}
+
+// Next child of a node group: the highest of its hit bits 24..31, cleared in
+// ng.y; returns the child's node index (base + rank among the internal slots
+// below it).
+__device__ __forceinline__ uint32_t next_child(uint2& ng, uint32_t oct)
+{
+    const uint32_t b = 31u - __clz(ng.y);      // >= 24: bits 24..31 are not all 0
+    ng.y ^= 1u << b;
+    const uint32_t slot = b ^ (oct >> 24);
+    return ng.x + __popc(ng.y & ((1u << slot) - 1u));   // imask is in bits 0..7, slot <= 7
+}
+
+__device__ __forceinline__ void trav_setup(TravRay& r, float3 org, float3 dir)
+{
+    r.org = org;
+    const float tiny = 1e-30f;
+    r.inv.x = 1.0f / (fabsf(dir.x) > tiny ? dir.x : copysignf(tiny, dir.x));
+    r.inv.y = 1.0f / (fabsf(dir.y) > tiny ? dir.y : copysignf(tiny, dir.y));
+    r.inv.z = 1.0f / (fabsf(dir.z) > tiny ? dir.z : copysignf(tiny, dir.z));
+    r.oct = oct_code(dir);
 }
 
 __device__ __forceinline__ float comp(float3 v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : v.z); }
@@ -242,10 +308,10 @@ __device__ __forceinline__ float comp(float3 v, int k) { return k == 0 ? v.x : (
 // that exact ties resolve the same way in every traversal order.  On a hit
 // returns true and sets t (and the barycentrics b1 -> u, b2 -> v, the
 // reference's convention, geometry/triangle_mesh.cpp:69-71).
-__device__ __forceinline__ bool tri_test(const TravRay& r, float3 v0, float3 v1, float3 v2, float tnear, float tbest,
-                                         int prim, int bestPrim, float& t, float& u, float& v)
+__device__ __forceinline__ bool tri_test(float3 org, const Shear& r, float3 v0, float3 v1, float3 v2, float tnear,
+                                         float tbest, int prim, int bestPrim, float& t, float& u, float& v)
 {
-    float3 A = sub(v0, r.org), B = sub(v1, r.org), C = sub(v2, r.org);
+    float3 A = sub(v0, org), B = sub(v1, org), C = sub(v2, org);
     float Akz = comp(A, r.kz), Bkz = comp(B, r.kz), Ckz = comp(C, r.kz);
     float Ax = comp(A, r.kx) - r.Sx * Akz, Ay = comp(A, r.ky) - r.Sy * Akz;
     float Bx = comp(B, r.kx) - r.Sx * Bkz, By = comp(B, r.ky) - r.Sy * Bkz;
@@ -360,7 +426,7 @@ __device__ __forceinline__ uint32_t node_hits(const TravRay& r, const uint4* q, 
     uint32_t loX[2] = {q[2].x, q[2].y}, loY[2] = {q[2].z, q[2].w}, loZ[2] = {q[3].x, q[3].y};
     uint32_t hiX[2] = {q[3].z, q[3].w}, hiY[2] = {q[4].x, q[4].y}, hiZ[2] = {q[4].z, q[4].w};
     uint32_t meta[2] = {q[1].z, q[1].w};
-    const uint32_t octinv4 = r.octinv * 0x01010101u;
+    const uint32_t octinv4 = oct_inv(r.oct) * 0x01010101u;
     uint32_t hits = 0;
     const float tfarp = tfar * 1.0000004f;
 #pragma unroll
@@ -435,16 +501,27 @@ __device__ __forceinline__ uint32_t node_hits(const TravRay& r, const uint4* q, 
 // slot order, so the triangle of leaf slot j is triBase + popc(leafMask below j).
 // Returns internal hits at bits 24 + (slot ^ octinv) as node_hits does, leaf
 // hits as slot bits 0..7, and the node's leaf-slot mask in leafMask.
-// octinv: the octant code that orders the internal hit bits (the ray's own in
-// per-lane traversal; one shared by a warp in packet traversal).  kPair: the
-// planes of two children per paired FP32 FMA (fma.rn.f32x2); faster where the
-// kernel has registers to spare for the paired coefficients, slower where they
-// make it spill heavily (closest-hit ray queries, the first bounce of the
-// diffuse2 kernel).  Both give the same results: each lane of a paired FMA is
+// oct: the octant code that orders the internal hit bits (the ray's own in
+// per-lane traversal; one shared by a warp in packet traversal).
+// kPair: the planes of two children per paired FP32 FMA (fma.rn.f32x2); faster
+// where the kernel has registers to spare for the paired coefficients, slower
+// where they make it spill heavily (closest-hit ray queries, the first bounce of
+// the diffuse2 kernel).  Both give the same results: each lane of a paired FMA is
 // rounded once, as fmaf is.
+// The integer and min/max pipe, at half the issue rate, is the busiest of this
+// test, so a child's comparison is an FMA whose sign bit is shifted into the mask
+// of misses (t1 * (1 + slack) - t0 < 0) instead of a compare and a bit set, and
+// the octant order is three delta swaps (packet kernel of a 33M-ray terrain wave
+// 8.03 -> 7.94 ms, 1 spp HD frame 1.870 -> 1.853; the loops with incoherent rays
+// wait for memory and keep their times).
+__device__ __forceinline__ uint32_t child_miss(uint32_t misses, float t0, float t1)
+{
+    return __funnelshift_l(__float_as_uint(fmaf(t1, 1.0000008f, -t0)), misses, 1);
+}
+
 template <bool kPair = false>
 __device__ __forceinline__ uint32_t node_hits1(const TravRay& r, const uint4* q, float tnear, float tfar,
-                                               uint32_t& leafMask, uint32_t octinv)
+                                               uint32_t& leafMask, uint32_t oct)
 {
     float px = __uint_as_float(q[0].x), py = __uint_as_float(q[0].y), pz = __uint_as_float(q[0].z);
     uint32_t e = q[0].w;
@@ -457,9 +534,9 @@ __device__ __forceinline__ uint32_t node_hits1(const TravRay& r, const uint4* q,
     uint32_t loX[2] = {q[2].x, q[2].y}, loY[2] = {q[2].z, q[2].w}, loZ[2] = {q[3].x, q[3].y};
     uint32_t hiX[2] = {q[3].z, q[3].w}, hiY[2] = {q[4].x, q[4].y}, hiZ[2] = {q[4].z, q[4].w};
     const float tfarp = tfar * 1.0000004f;
-    uint32_t c8 = 0;
+    uint32_t misses = 0;   // children 7 down to 0: child j ends in bit j
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
+    for (int h = 1; h >= 0; --h)
     {
         uint32_t nearX = nx ? hiX[h] : loX[h], farX = nx ? loX[h] : hiX[h];
         uint32_t nearY = ny ? hiY[h] : loY[h], farY = ny ? loY[h] : hiY[h];
@@ -467,7 +544,7 @@ __device__ __forceinline__ uint32_t node_hits1(const TravRay& r, const uint4* q,
         if constexpr (kPair)
         {
 #pragma unroll
-            for (int j = 0; j < 4; j += 2)
+            for (int j = 2; j >= 0; j -= 2)
             {
                 const float2 nX = ffma2(byte_unit(nearX, j), byte_unit(nearX, j + 1), aix, aox);
                 const float2 nY = ffma2(byte_unit(nearY, j), byte_unit(nearY, j + 1), aiy, aoy);
@@ -477,14 +554,14 @@ __device__ __forceinline__ uint32_t node_hits1(const TravRay& r, const uint4* q,
                 const float2 fZ = ffma2(byte_unit(farZ, j), byte_unit(farZ, j + 1), aiz, aoz);
                 const float t0a = fmax3(nX.x, nY.x, fmaxf(nZ.x, tnear)), t1a = fmin3(fX.x, fY.x, fminf(fZ.x, tfarp));
                 const float t0b = fmax3(nX.y, nY.y, fmaxf(nZ.y, tnear)), t1b = fmin3(fX.y, fY.y, fminf(fZ.y, tfarp));
-                if (t0a <= t1a * 1.0000008f) c8 |= 1u << (4 * h + j);
-                if (t0b <= t1b * 1.0000008f) c8 |= 1u << (4 * h + j + 1);
+                misses = child_miss(misses, t0b, t1b);
+                misses = child_miss(misses, t0a, t1a);
             }
         }
         else
         {
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
+            for (int j = 3; j >= 0; --j)
             {
                 float tnx = fmaf(byte_unit(nearX, j), aix, aox);
                 float tny = fmaf(byte_unit(nearY, j), aiy, aoy);
@@ -494,26 +571,17 @@ __device__ __forceinline__ uint32_t node_hits1(const TravRay& r, const uint4* q,
                 float tfz = fmaf(byte_unit(farZ, j), aiz, aoz);
                 float t0 = fmax3(tnx, tny, fmaxf(tnz, tnear));
                 float t1 = fmin3(tfx, tfy, fminf(tfz, tfarp));
-                if (t0 <= t1 * 1.0000008f) c8 |= 1u << (4 * h + j);
+                misses = child_miss(misses, t0, t1);
             }
         }
     }
     // bit 5 of each meta byte -> one bit per slot (multiply gathers bytes 0..3 into bits 24..27)
     const uint32_t ne = ((((q[1].z >> 5) & 0x01010101u) * 0x01020408u) >> 24) |
                         (((((q[1].w >> 5) & 0x01010101u) * 0x01020408u) >> 24) << 4);
-    c8 &= ne;
+    const uint32_t c8 = ne & ~misses;
     const uint32_t imask = q[0].w >> 24;
     leafMask = ne & ~imask;
-    // internal hits: bit slot -> bit slot ^ octinv (three conditional swaps)
-    uint32_t in8 = c8 & imask;
-    const uint32_t o = octinv;
-    uint32_t sw = ((in8 & 0x55u) << 1) | ((in8 >> 1) & 0x55u);
-    in8 = (o & 1u) ? sw : in8;
-    sw = ((in8 & 0x33u) << 2) | ((in8 >> 2) & 0x33u);
-    in8 = (o & 2u) ? sw : in8;
-    sw = ((in8 & 0x0fu) << 4) | ((in8 >> 4) & 0x0fu);
-    in8 = (o & 4u) ? sw : in8;
-    return (in8 << 24) | (c8 & leafMask);
+    return (permute_octant(c8 & imask, oct) << 24) | (c8 & leafMask);
 }
 
 // Traversal stack: the first kShared entries of each thread live in shared
@@ -592,7 +660,8 @@ __device__ __forceinline__ void trav_init(TravState& s, const SceneDev& sc, floa
 #endif
 
 template <bool anyHit>
-__device__ __forceinline__ void trav_step(TravState& s, const SceneDev& sc, const TravRay& r, float tnear, TravStack& st,
+__device__ __forceinline__ void trav_step(TravState& s, const SceneDev& sc, const TravRay& r, const Shear& sh, float tnear,
+                                          TravStack& st,
                                           uint32_t* nodeVisits = nullptr, uint32_t* triTests = nullptr,
                                           bool anyHitRt = false)
 {
@@ -601,11 +670,7 @@ __device__ __forceinline__ void trav_step(TravState& s, const SceneDev& sc, cons
     if (ng.y & 0xff000000u)
     {
         // visit the next child node of the group
-        uint32_t b = 31u - __clz(ng.y & 0xff000000u);
-        ng.y &= ~(1u << b);
-        uint32_t slot = (b - 24u) ^ r.octinv;
-        uint32_t rel = __popc((ng.y & 0xffu) & ((1u << slot) - 1u));
-        uint32_t nodeIdx = ng.x + rel;
+        const uint32_t nodeIdx = next_child(ng, r.oct);
         if (ng.y & 0xff000000u) st.push(ng);
         const uint4* qp = reinterpret_cast<const uint4*>(sc.nodes + nodeIdx);
         uint4 q[5];
@@ -618,7 +683,7 @@ __device__ __forceinline__ void trav_step(TravState& s, const SceneDev& sc, cons
         {
             // start fetching the child visited next while the triangles are tested
             uint32_t nb = 31u - __clz(ng.y & 0xff000000u);
-            uint32_t ns = (nb - 24u) ^ r.octinv;
+            uint32_t ns = nb ^ (r.oct >> 24);
             uint32_t nidx = ng.x + __popc((ng.y & 0xffu) & ((1u << ns) - 1u));
             const char* np = reinterpret_cast<const char*>(sc.nodes + nidx);
             asm volatile("prefetch.global.L1 [%0];" ::"l"(np));
@@ -650,7 +715,7 @@ __device__ __forceinline__ void trav_step(TravState& s, const SceneDev& sc, cons
         int prim = __float_as_int(a.w);
         float t, u, v;
         if (triTests) ++*triTests;
-        if (tri_test(r, f3(a.x, a.y, a.z), f3(bq.x, bq.y, bq.z), f3(c.x, c.y, c.z), tnear, s.tHit, prim, s.primHit,
+        if (tri_test(r.org, sh, f3(a.x, a.y, a.z), f3(bq.x, bq.y, bq.z), f3(c.x, c.y, c.z), tnear, s.tHit, prim, s.primHit,
                      t, u, v))
         {
             s.tHit = t;
@@ -690,18 +755,22 @@ __device__ __forceinline__ void trav_step(TravState& s, const SceneDev& sc, cons
 // their bit patterns and the id breaks exact ties the way tri_test does.  Node
 // culling uses the owner's tHit as of the last merge, which can only be larger
 // than the final one, so no node that holds the closest hit is skipped.
-// The list holds the largest possible step and nothing more, and the
-// barycentrics live in an array of their own that only closest-hit queries
-// allocate: a block of the bounce kernel takes 14 KB of shared memory, 8 blocks
-// fit the 132 KB carveout, and L1 keeps 124 of the SM's 256 KB for nodes and
-// triangles.  (A 512-entry ring beside the barycentrics took 18.5 KB a block
-// and left L1 92 KB: bounces 1-5 of a 33M-path terrain wave 17.32 -> 16.86 ms,
-// 4M incoherent closest-hit queries 1.302 -> 1.274 ms.)
+// The list holds the largest step on top of what may wait, the barycentrics live
+// in an array of their own that only closest-hit queries allocate, and a ray's
+// shear terms lie in shared memory, where whichever lane tests for it reads them:
+// in registers, six per lane that only flushes need, they made the loops spill
+// (a local load or store for every one or two node loads of the whole-path
+// kernel).  Together with the loops' per-path state there (pixel, RNG, direction):
+// bounces 1-5 of a 33M-path terrain wave 16.90 -> 16.66 ms, 4M incoherent
+// closest-hit queries 1.243 -> 1.212, any hit 0.922 -> 0.890, next-event terrain
+// frame 10.65 -> 10.38, 256x256 at 16 spp on the small scene 0.590 -> 0.571.
+// (A 64-entry queue flushed between the rounds of appends made the bounces 4%
+// slower: the flush is then inlined into the loop around them.)
 #ifndef PRT_DEFER_TRIS
 #define PRT_DEFER_TRIS 1
 #endif
 
-constexpr uint32_t kTriQCap = 288;   // >= 31 pending + 8 triangles x 32 lanes from one step
+constexpr uint32_t kTriQCap = 288;   // 31 waiting and eight of each lane
 
 struct TriQueue
 {
@@ -730,17 +799,13 @@ __device__ __forceinline__ void trav_visit(TravState& s, const SceneDev& sc, con
                                            uint32_t* nodeVisits = nullptr)
 {
     uint2 ng = s.ng;
-    uint32_t b = 31u - __clz(ng.y & 0xff000000u);
-    ng.y &= ~(1u << b);
-    uint32_t slot = (b - 24u) ^ r.octinv;
-    uint32_t rel = __popc((ng.y & 0xffu) & ((1u << slot) - 1u));
-    uint32_t nodeIdx = ng.x + rel;
+    const uint32_t nodeIdx = next_child(ng, r.oct);
     if (ng.y & 0xff000000u) st.push(ng);
     const uint4* qp = reinterpret_cast<const uint4*>(sc.nodes + nodeIdx);
     uint4 q[5];
 #pragma unroll
     for (int k = 0; k < 5; ++k) q[k] = __ldg(qp + k);
-    const uint32_t hits = node_hits1<kPair>(r, q, tnear, s.tHit, leafMask, r.octinv);
+    const uint32_t hits = node_hits1<kPair>(r, q, tnear, s.tHit, leafMask, r.oct);
     if (nodeVisits) ++*nodeVisits;
     ng = make_uint2(q[1].x, (hits & 0xff000000u) | (q[0].w >> 24));
     tbits = hits & 0x00ffffffu;
@@ -758,37 +823,15 @@ __device__ __forceinline__ void trav_visit(TravState& s, const SceneDev& sc, con
     s.ng = ng;
 }
 
-// Warp-collective: appends every lane's triangles to the n queued ones.  One
-// triangle of each lane that has one per round, placed by the ballot of those
-// lanes: a visit leaves 0.2 triangles per lane, so most calls take two or three
-// rounds of about ten instructions, fewer than a prefix sum of the lanes'
-// counts needs before its first store.
-__device__ __forceinline__ void triq_push(TriQueue& q, uint32_t& n, uint32_t tbase, uint32_t tbits, uint32_t leafMask,
-                                          unsigned lane)
-{
-    const uint32_t lt = (1u << lane) - 1u;
-    for (;;)
-    {
-        const unsigned m = __ballot_sync(0xffffffffu, tbits != 0);
-        if (!m) break;
-        if (tbits)
-        {
-            const uint32_t low = tbits & (0u - tbits);
-            tbits ^= low;
-            q.tri[n + __popc(m & lt)] = ((tbase + __popc(leafMask & (low - 1u))) << 5) | lane;
-        }
-        n += __popc(m);
-    }
-}
-
-// Warp-collective: tests the m (<= 32) queued triangles from `first`, one per
+// Warp-collective: tests the first m (<= 32) queued triangles, one per
 // lane, and merges each owner's closest hit into its traversal state.  The owner's
 // ray, tnear and triangle array (lanes of a batch may traverse different
-// scenes) come from the owner lane by shuffles.
+// scenes) come from the owner lane by shuffles, its shear terms from its words of
+// shared memory (shw: this lane's).
 template <bool kUV>
 __device__ __forceinline__ void triq_flush(TriQueue& q, uint32_t first, uint32_t m, const TriRec* tris, const TravRay& r,
-                                           float tnear, TravState& ts, unsigned lane, TriQueueUV* uv,
-                                           uint32_t* triTests = nullptr)
+                                           const uint32_t* shw, int stride, float tnear, TravState& ts, unsigned lane,
+                                           TriQueueUV* uv, uint32_t* triTests = nullptr)
 {
     const unsigned FULL = 0xffffffffu;
     const bool act = lane < m;
@@ -801,17 +844,11 @@ __device__ __forceinline__ void triq_flush(TriQueue& q, uint32_t first, uint32_t
         tri = e >> 5;
         own = (int)(e & 31u);
     }
-    TravRay o;
-    o.org.x = __shfl_sync(FULL, r.org.x, own);
-    o.org.y = __shfl_sync(FULL, r.org.y, own);
-    o.org.z = __shfl_sync(FULL, r.org.z, own);
-    o.Sx = __shfl_sync(FULL, r.Sx, own);
-    o.Sy = __shfl_sync(FULL, r.Sy, own);
-    o.Sz = __shfl_sync(FULL, r.Sz, own);
-    const int kp = __shfl_sync(FULL, r.kx | (r.ky << 2) | (r.kz << 4), own);
-    o.kx = kp & 3;
-    o.ky = (kp >> 2) & 3;
-    o.kz = kp >> 4;
+    float3 org;
+    org.x = __shfl_sync(FULL, r.org.x, own);
+    org.y = __shfl_sync(FULL, r.org.y, own);
+    org.z = __shfl_sync(FULL, r.org.z, own);
+    const Shear o = shear_load(shw + own - (int)lane, stride);
     const float tb = __shfl_sync(FULL, ts.tHit, own);
     const int bp = __shfl_sync(FULL, ts.primHit, own);
     const float tn = __shfl_sync(FULL, tnear, own);
@@ -829,7 +866,7 @@ __device__ __forceinline__ void triq_flush(TriQueue& q, uint32_t first, uint32_t
         const float4 a = __ldg(tp), bq = __ldg(tp + 1), c = __ldg(tp + 2);
         prim = __float_as_int(a.w);
         if (triTests) ++*triTests;
-        hit = tri_test(o, f3(a.x, a.y, a.z), f3(bq.x, bq.y, bq.z), f3(c.x, c.y, c.z), tn, tb, prim, bp, t, u, v);
+        hit = tri_test(org, o, f3(a.x, a.y, a.z), f3(bq.x, bq.y, bq.z), f3(c.x, c.y, c.z), tn, tb, prim, bp, t, u, v);
         if (hit) atomicMin(&q.key[own], hit_key(t, prim));
     }
     __syncwarp();
@@ -873,8 +910,9 @@ __device__ __forceinline__ void triq_flush(TriQueue& q, uint32_t first, uint32_t
 // flushes per warp) may be null.
 template <bool kPair = false, bool kUV = false, bool kEager = false>
 __device__ __forceinline__ void warp_trav_deferred(TriQueue& q, TravState& ts, const SceneDev& sc, const TravRay& r,
-                                                   float tnear, TravStack& st, bool active, bool mayStop, int refillMin,
-                                                   unsigned lane, uint32_t* cNodes = nullptr, uint32_t* cTris = nullptr,
+                                                   const uint32_t* shw, int stride, float tnear, TravStack& st,
+                                                   bool active, bool mayStop, int refillMin, unsigned lane,
+                                                   uint32_t* cNodes = nullptr, uint32_t* cTris = nullptr,
                                                    unsigned long long* cSteps = nullptr,
                                                    unsigned long long* cLaneSteps = nullptr,
                                                    unsigned long long* cFlushes = nullptr, bool anyHit = false,
@@ -892,19 +930,32 @@ __device__ __forceinline__ void warp_trav_deferred(TriQueue& q, TravState& ts, c
             *cSteps += 1;
         }
         if (active && !ts.done) trav_visit<kPair>(ts, sc, r, tnear, st, tbase, tbits, lmask, cNodes);
-        triq_push(q, n, tbase, tbits, lmask, lane);
+        // One triangle of each lane that has one per round, placed by the ballot
+        // of those lanes (a visit leaves 0.2 triangles per lane, so most steps take
+        // two or three rounds)
+        for (;;)
+        {
+            const unsigned m = __ballot_sync(FULL, tbits != 0);
+            if (!m) break;
+            if (tbits)
+            {
+                const uint32_t low = tbits & (0u - tbits);
+                tbits ^= low;
+                q.tri[n + __popc(m & ((1u << lane) - 1u))] = ((tbase + __popc(lmask & (low - 1u))) << 5) | lane;
+            }
+            n += __popc(m);
+        }
         if (n >= full)
         {
             uint32_t first = 0;
             do
             {
-                const uint32_t m = kEager ? min(32u, n - first) : 32u;
-                triq_flush<kUV>(q, first, m, sc.tris, r, tnear, ts, lane, uv, cTris);
+                const uint32_t k = kEager ? min(32u, n - first) : 32u;
+                triq_flush<kUV>(q, first, k, sc.tris, r, shw, stride, tnear, ts, lane, uv, cTris);
                 if (cFlushes) *cFlushes += 1;
-                first += m;
+                first += k;
             } while (n - first >= full);
             if (anyHit && ts.triHit >= 0) ts.done = true;
-            // the rest moves to the front
             n -= first;
             if (lane < n) q.tri[lane] = q.tri[first + lane];
         }
@@ -915,7 +966,7 @@ __device__ __forceinline__ void warp_trav_deferred(TriQueue& q, TravState& ts, c
     }
     if (n)
     {
-        triq_flush<kUV>(q, 0, n, sc.tris, r, tnear, ts, lane, uv, cTris);
+        triq_flush<kUV>(q, 0, n, sc.tris, r, shw, stride, tnear, ts, lane, uv, cTris);
         if (cFlushes) *cFlushes += 1;
     }
 }

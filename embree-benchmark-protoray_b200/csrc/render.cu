@@ -146,6 +146,9 @@ constexpr int kRefillMin = PRT_REFILL_MIN;
 // registers) 5%.
 constexpr int kWideBlocks = 7;
 
+// Words of shared memory per lane of the per-bounce kernels.
+constexpr int bounce_words(bool first) { return kShearWords + (first || !PRT_RELOAD_PATH ? 5 : 0); }
+
 // One bounce of the wavefront over the queue of paths entering `depth`.
 // kFirst: the queue is implicit — item i is (pass, 8x8 tile, Morton index)
 // and the primary ray is generated in registers.
@@ -163,8 +166,12 @@ __global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_bounce(WaveArgs 
     st.sh = s_stack + threadIdx.x;
     st.stride = blockDim.x;
     st.overflow = false;
-    // this warp's triangle queue, after the block's stack columns
-    TriQueue* tq = reinterpret_cast<TriQueue*>(s_stack + kShared * blockDim.x) + (threadIdx.x >> 5);
+    // the block's stack columns, then its lanes' words (shear terms and, in the
+    // first bounce, pixel, RNG state and direction), then the triangle queues
+    const int bd = blockDim.x;
+    uint32_t* shw = reinterpret_cast<uint32_t*>(s_stack + kShared * blockDim.x) + threadIdx.x;
+    TriQueue* tq = reinterpret_cast<TriQueue*>(reinterpret_cast<uint32_t*>(s_stack + kShared * blockDim.x) +
+                                               bounce_words(kFirst) * blockDim.x) + (threadIdx.x >> 5);
     const unsigned FULL = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned ltMask = (1u << lane) - 1u;
@@ -190,8 +197,6 @@ __global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_bounce(WaveArgs 
     bool exhausted = false;   // warp-uniform: every queue entry has been claimed
     uint32_t cNodes = 0, cTris = 0, cRays = 0;                          // per lane (PRT_COUNTERS)
     unsigned long long cSteps = 0, cLaneSteps = 0, cTriIters = 0;       // per warp (PRT_COUNTERS)
-    int pixel = 0;
-    uint32_t rng = 0;
     int qi = 0;               // input-queue index of this lane's path (PRT_RELOAD_PATH)
     float thr = 0.f;
     TravRay r;
@@ -212,6 +217,8 @@ __global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_bounce(WaveArgs 
             if (!has && i < total)
             {
                 float3 org, dir;
+                int pixel = 0;
+                uint32_t rng = 0;
                 bool ok = true;
                 if (kFirst)
                 {
@@ -252,6 +259,15 @@ __global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_bounce(WaveArgs 
                 if (ok)
                 {
                     has = true;
+                    if (kFirst || !PRT_RELOAD_PATH)
+                    {
+                        shw[4 * bd] = (uint32_t)pixel;
+                        shw[5 * bd] = rng;
+                        shw[6 * bd] = __float_as_uint(dir.x);
+                        shw[7 * bd] = __float_as_uint(dir.y);
+                        shw[8 * bd] = __float_as_uint(dir.z);
+                    }
+                    shear_store(shw, bd, shear_of(dir));
                     trav_setup(r, org, dir);
                     trav_init(ts, a.scene, FLT_MAX, st);
                 }
@@ -268,31 +284,34 @@ __global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_bounce(WaveArgs 
             // node visits queue their triangles; the warp tests them 32 at a
             // time, and every pending test is done before any lane shades
             constexpr bool kPair = kFirst ? PRT_PAIRED_FIRST : (PRT_RELOAD_PATH && PRT_PAIRED_LATER);
-            warp_trav_deferred<kPair>(*tq, ts, a.scene, r, 0.0f, st, has, !exhausted, kRefillMin, lane,
+            warp_trav_deferred<kPair>(*tq, ts, a.scene, r, shw, bd, 0.0f, st, has, !exhausted, kRefillMin, lane,
                                       PRT_COUNTERS ? &cNodes : nullptr, PRT_COUNTERS ? &cTris : nullptr,
                                       PRT_COUNTERS ? &cSteps : nullptr, PRT_COUNTERS ? &cLaneSteps : nullptr,
                                       PRT_COUNTERS ? &cTriIters : nullptr);
         }
         else
-        for (;;)
         {
-            if (PRT_COUNTERS)
+            const Shear sh = shear_load(shw, bd);
+            for (;;)
             {
-                unsigned run0 = __ballot_sync(FULL, has && !ts.done);
-                uint32_t tris = 0;
-                if (has && !ts.done) trav_step<false>(ts, a.scene, r, 0.0f, st, &cNodes, &tris);
-                cTris += tris;
-                cLaneSteps += __popc(run0);
-                cSteps += 1;
-                cTriIters += __reduce_max_sync(FULL, tris);
+                if (PRT_COUNTERS)
+                {
+                    unsigned run0 = __ballot_sync(FULL, has && !ts.done);
+                    uint32_t tris = 0;
+                    if (has && !ts.done) trav_step<false>(ts, a.scene, r, sh, 0.0f, st, &cNodes, &tris);
+                    cTris += tris;
+                    cLaneSteps += __popc(run0);
+                    cSteps += 1;
+                    cTriIters += __reduce_max_sync(FULL, tris);
+                }
+                else if (has && !ts.done)
+                {
+                    trav_step<false>(ts, a.scene, r, sh, 0.0f, st);
+                }
+                unsigned running = __ballot_sync(FULL, has && !ts.done);
+                if (running == 0) break;
+                if (!exhausted && 32 - __popc(running) >= kRefillMin) break;
             }
-            else if (has && !ts.done)
-            {
-                trav_step<false>(ts, a.scene, r, 0.0f, st);
-            }
-            unsigned running = __ballot_sync(FULL, has && !ts.done);
-            if (running == 0) break;
-            if (!exhausted && 32 - __popc(running) >= kRefillMin) break;
         }
         // --- finish the lanes whose traversal is complete ---------------------
         // (the finished path's pixel, RNG state and rays are iteration-local, so
@@ -315,9 +334,9 @@ __global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_bounce(WaveArgs 
             }
             else
             {
-                fpix = pixel;
-                fdir = r.dir;
-                frng = rng;
+                fpix = (int)shw[4 * bd];
+                frng = shw[5 * bd];
+                fdir = f3(__uint_as_float(shw[6 * bd]), __uint_as_float(shw[7 * bd]), __uint_as_float(shw[8 * bd]));
             }
             if (ts.triHit < 0)
             {
@@ -377,14 +396,14 @@ __global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_bounce(WaveArgs 
 // depths share a warp, which costs little: from the second ray on a path's
 // neighbours have scattered.  What a path needs only when it is shaded lives in
 // shared memory (kPathWords words per lane), so the registers hold what
-// traversal needs; with 6 stack entries per lane a block takes 15 KB, within
-// the step that leaves L1 124 KB.
+// traversal needs; a block takes 18 KB.
 // Measured against one launch per bounce: 1080p terrain frame of 1 pass 2.12 ->
 // 1.88 ms and of 32 passes 46.4 -> 45.2, 256x256 and 16 passes of 82K triangles
 // 0.765 -> 0.63 ms, 10.24M-triangle field at 4 passes and 9 bounces 5.17 -> 4.72.
 // kPrimary: the lanes generate their paths' camera rays too, so a small wave is
 // one launch with one tail and needs no queue (whole_paths below).
-constexpr int kPathWords = 7;   // tag (pixel; in a batch request << 24 | pixel), depth, RNG, throughput, direction
+// tag (pixel; in a batch request << 24 | pixel), depth, RNG, throughput, direction, shear terms
+constexpr int kPathWords = 7 + kShearWords;
 
 __device__ __forceinline__ const SceneDev& path_scene(const WaveArgs& a, int) { return a.scene; }
 __device__ __forceinline__ float4* path_accum(const WaveArgs& a, uint32_t tag) { return a.accum + tag; }
@@ -419,6 +438,7 @@ __global__ void __launch_bounds__(128, kBatch || kPrimary ? kWideBlocks : PRT_BO
     uint32_t* path = s_path + threadIdx.x;   // word k of this lane's path at path[k * bd]
     TriQueue* tq = reinterpret_cast<TriQueue*>(s_path + kPathWords * blockDim.x) + (threadIdx.x >> 5);   // deferred
     const int bd = blockDim.x;
+    uint32_t* shw = path + 7 * bd;
     const unsigned FULL = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned ltMask = (1u << lane) - 1u;
@@ -437,7 +457,7 @@ __global__ void __launch_bounds__(128, kBatch || kPrimary ? kWideBlocks : PRT_BO
         total = *(volatile int*)&a.counts[1];
         if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(a.rays, (unsigned long long)total);
     }
-    unsigned long long more = 0;   // rays of bounces in this kernel, per warp
+    uint32_t more = 0;   // rays of bounces in this kernel, per warp
 
     bool has = false;         // this lane holds a path
     bool exhausted = false;   // warp-uniform: every queued path has been claimed
@@ -531,6 +551,7 @@ __global__ void __launch_bounds__(128, kBatch || kPrimary ? kWideBlocks : PRT_BO
             path[4 * bd] = __float_as_uint(dir.x);
             path[5 * bd] = __float_as_uint(dir.y);
             path[6 * bd] = __float_as_uint(dir.z);
+            shear_store(shw, bd, shear_of(dir));
             trav_setup(r, org, dir);
             trav_init(ts, path_scene(a, req), FLT_MAX, st);
         }
@@ -538,17 +559,20 @@ __global__ void __launch_bounds__(128, kBatch || kPrimary ? kWideBlocks : PRT_BO
         const int stopIdle = stop_idle(act);
         if (PRT_DEFER_TRIS && path_deferred(a))
         {
-            warp_trav_deferred<PRT_PAIRED_LATER>(*tq, ts, path_scene(a, req), r, 0.0f, st, has, true, stopIdle, lane);
+            warp_trav_deferred<PRT_PAIRED_LATER>(*tq, ts, path_scene(a, req), r, shw, bd, 0.0f, st, has, true, stopIdle, lane);
         }
         else
-        for (;;)
         {
-            if (has && !ts.done) trav_step<false>(ts, path_scene(a, req), r, 0.0f, st);
-            const unsigned running = __ballot_sync(FULL, has && !ts.done);
-            if (32 - __popc(running) >= stopIdle) break;
+            const Shear sh = shear_load(shw, bd);
+            for (;;)
+            {
+                if (has && !ts.done) trav_step<false>(ts, path_scene(a, req), r, sh, 0.0f, st);
+                const unsigned running = __ballot_sync(FULL, has && !ts.done);
+                if (32 - __popc(running) >= stopIdle) break;
+            }
         }
     }
-    if (lane == 0 && more) atomicAdd(a.rays, more);
+    if (lane == 0 && more) atomicAdd(a.rays, (unsigned long long)more);
 }
 
 // Primary rays as warp packets (trees with one-triangle leaves).  A warp takes
@@ -648,14 +672,14 @@ __device__ __forceinline__ float ia_max(float plane, float omin, float omax, flo
 
 // The traversal loop of packet_closest_hit_ia over the packet's ranges.
 template <bool kPoint>
-__device__ __forceinline__ void packet_ia_loop(const SceneDev& sc, const TravRay& r, bool valid, uint32_t woct,
+__device__ __forceinline__ void packet_ia_loop(const SceneDev& sc, const TravRay& r, const Shear& sh, bool valid, uint32_t woct,
                                                uint2* stk, unsigned lane, float& tHit, int& primHit, int& triHit,
                                                float oxmin, float oxmax, float oymin, float oymax, float ozmin,
                                                float ozmax, float ixmin, float ixmax, float iymin, float iymax,
                                                float izmin, float izmax)
 {
     const unsigned FULL = 0xffffffffu;
-    const uint32_t oct = 7u - woct;   // bit k: negative direction on axis k
+    const uint32_t oct = 7u - oct_inv(woct);   // bit k: negative direction on axis k
     const bool nx = (oct & 1u) != 0u, ny = (oct & 2u) != 0u, nz = (oct & 4u) != 0u;
     const int c = (int)(lane & 7u);
     const int cw = c >> 2, cb = c & 3;
@@ -669,10 +693,7 @@ __device__ __forceinline__ void packet_ia_loop(const SceneDev& sc, const TravRay
     uint2 ng = make_uint2(0u, 0x80000000u);   // the root: one internal child at base 0
     for (;;)
     {
-        const uint32_t b = 31u - __clz(ng.y & 0xff000000u);
-        ng.y &= ~(1u << b);
-        const uint32_t slot = (b - 24u) ^ woct;
-        const uint32_t nodeIdx = ng.x + __popc((ng.y & 0xffu) & ((1u << slot) - 1u));
+        const uint32_t nodeIdx = next_child(ng, woct);
         if ((ng.y & 0xff000000u) && sp < kPacketStack)
         {
             if (lane == 0) stk[sp] = ng;
@@ -749,7 +770,7 @@ __device__ __forceinline__ void packet_ia_loop(const SceneDev& sc, const TravRay
                     const float4 v0 = __ldg(tp), v1 = __ldg(tp + 1), v2 = __ldg(tp + 2);
                     const int prim = __float_as_int(v0.w);
                     float t, u, v;
-                    if (tri_test(r, f3(v0.x, v0.y, v0.z), f3(v1.x, v1.y, v1.z), f3(v2.x, v2.y, v2.z), 0.0f, tHit,
+                    if (tri_test(r.org, sh, f3(v0.x, v0.y, v0.z), f3(v1.x, v1.y, v1.z), f3(v2.x, v2.y, v2.z), 0.0f, tHit,
                                  prim, primHit, t, u, v))
                     {
                         tHit = t;
@@ -761,13 +782,7 @@ __device__ __forceinline__ void packet_ia_loop(const SceneDev& sc, const TravRay
             tfarP = __uint_as_float(__reduce_max_sync(FULL, valid ? __float_as_uint(tHit) : 0u));
         }
         // internal hits: bit slot -> bit slot ^ octinv, as node_hits1 orders them
-        uint32_t in8 = c8 & imask;
-        uint32_t sw = ((in8 & 0x55u) << 1) | ((in8 >> 1) & 0x55u);
-        in8 = (woct & 1u) ? sw : in8;
-        sw = ((in8 & 0x33u) << 2) | ((in8 >> 2) & 0x33u);
-        in8 = (woct & 2u) ? sw : in8;
-        sw = ((in8 & 0x0fu) << 4) | ((in8 >> 4) & 0x0fu);
-        in8 = (woct & 4u) ? sw : in8;
+        const uint32_t in8 = permute_octant(c8 & imask, woct);
         ng = make_uint2(q[1].x, (in8 << 24) | imask);
         if (!(ng.y & 0xff000000u))
         {
@@ -779,8 +794,8 @@ __device__ __forceinline__ void packet_ia_loop(const SceneDev& sc, const TravRay
     }
 }
 
-__device__ __forceinline__ void packet_closest_hit_ia(const SceneDev& sc, const TravRay& r, bool valid,
-                                                      unsigned vmask, uint32_t woct, uint2* stk, unsigned lane,
+__device__ __forceinline__ void packet_closest_hit_ia(const SceneDev& sc, const TravRay& r, const Shear& sh,
+                                                      bool valid, unsigned vmask, uint32_t woct, uint2* stk, unsigned lane,
                                                       float& tHit, int& primHit, int& triHit)
 {
     const unsigned FULL = 0xffffffffu;
@@ -800,10 +815,10 @@ __device__ __forceinline__ void packet_closest_hit_ia(const SceneDev& sc, const 
     const float izmin = warp_min_f(iz), izmax = warp_max_f(iz);
     // pinhole packets share one origin: half the interval products
     if (oxmin == oxmax && oymin == oymax && ozmin == ozmax)
-        packet_ia_loop<true>(sc, r, valid, woct, stk, lane, tHit, primHit, triHit, oxmin, oxmax, oymin, oymax, ozmin,
+        packet_ia_loop<true>(sc, r, sh, valid, woct, stk, lane, tHit, primHit, triHit, oxmin, oxmax, oymin, oymax, ozmin,
                              ozmax, ixmin, ixmax, iymin, iymax, izmin, izmax);
     else
-        packet_ia_loop<false>(sc, r, valid, woct, stk, lane, tHit, primHit, triHit, oxmin, oxmax, oymin, oymax, ozmin,
+        packet_ia_loop<false>(sc, r, sh, valid, woct, stk, lane, tHit, primHit, triHit, oxmin, oxmax, oymin, oymax, ozmin,
                               ozmax, ixmin, ixmax, iymin, iymax, izmin, izmax);
 }
 
@@ -812,28 +827,25 @@ __device__ __forceinline__ void packet_closest_hit_ia(const SceneDev& sc, const 
 // ray; vmask: the ballot of valid; stk: the warp's kPacketStack entries of
 // shared memory.  Returns this lane's closest hit (triHit -1: none).
 template <bool kPair, bool kIA>
-__device__ __forceinline__ void packet_closest_hit(const SceneDev& sc, const TravRay& r, bool valid, unsigned vmask,
-                                                   uint2* stk, unsigned lane, float& tHit, int& primHit, int& triHit)
+__device__ __forceinline__ void packet_closest_hit(const SceneDev& sc, const TravRay& r, const Shear& sh, bool valid,
+                                                   unsigned vmask, uint2* stk, unsigned lane, float& tHit, int& primHit, int& triHit)
 {
     const unsigned FULL = 0xffffffffu;
-    const uint32_t woct = __shfl_sync(FULL, r.octinv, __ffs(vmask) - 1);
+    const uint32_t woct = __shfl_sync(FULL, r.oct, __ffs(vmask) - 1);
     tHit = FLT_MAX;
     primHit = 0x7fffffff;
     triHit = -1;
     if (!sc.hasRoot) return;
-    if (kIA && __all_sync(FULL, !valid || r.octinv == woct))
+    if (kIA && __all_sync(FULL, !valid || r.oct == woct))
     {
-        packet_closest_hit_ia(sc, r, valid, vmask, woct, stk, lane, tHit, primHit, triHit);
+        packet_closest_hit_ia(sc, r, sh, valid, vmask, woct, stk, lane, tHit, primHit, triHit);
         return;
     }
     int sp = 0;
     uint2 ng = make_uint2(0u, 0x80000000u);   // the root: one internal child at base 0
     for (;;)
     {
-        const uint32_t b = 31u - __clz(ng.y & 0xff000000u);
-        ng.y &= ~(1u << b);
-        const uint32_t slot = (b - 24u) ^ woct;
-        const uint32_t nodeIdx = ng.x + __popc((ng.y & 0xffu) & ((1u << slot) - 1u));
+        const uint32_t nodeIdx = next_child(ng, woct);
         if ((ng.y & 0xff000000u) && sp < kPacketStack)
         {
             if (lane == 0) stk[sp] = ng;
@@ -856,7 +868,7 @@ __device__ __forceinline__ void packet_closest_hit(const SceneDev& sc, const Tra
             const float4 v0 = __ldg(tp), v1 = __ldg(tp + 1), v2 = __ldg(tp + 2);
             const int prim = __float_as_int(v0.w);
             float t, u, v;
-            if (tri_test(r, f3(v0.x, v0.y, v0.z), f3(v1.x, v1.y, v1.z), f3(v2.x, v2.y, v2.z), 0.0f, tHit, prim,
+            if (tri_test(r.org, sh, f3(v0.x, v0.y, v0.z), f3(v1.x, v1.y, v1.z), f3(v2.x, v2.y, v2.z), 0.0f, tHit, prim,
                          primHit, t, u, v))
             {
                 tHit = t;
@@ -918,7 +930,7 @@ __global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_primary_packet(W
         trav_setup(r, org, dir);
         float tHit;
         int primHit, triHit;
-        packet_closest_hit<PRT_PAIRED_PACKET, kIA>(a.scene, r, valid, vmask, stk, lane, tHit, primHit, triHit);
+        packet_closest_hit<PRT_PAIRED_PACKET, kIA>(a.scene, r, shear_of(dir), valid, vmask, stk, lane, tHit, primHit, triHit);
         // shade / append / accumulate, as k_bounce does at depth 0
         bool cont = false;
         float contrib = 0.f;
@@ -965,7 +977,10 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_bounce_nee(WaveArgs a, int
     st.sh = s_stack + threadIdx.x;
     st.stride = blockDim.x;
     st.overflow = false;
-    TriQueue* tq = reinterpret_cast<TriQueue*>(s_stack + kShared * blockDim.x) + (threadIdx.x >> 5);   // deferTris
+    const int bd = blockDim.x;
+    uint32_t* shw = reinterpret_cast<uint32_t*>(s_stack + kShared * blockDim.x) + threadIdx.x;   // as in k_bounce
+    TriQueue* tq = reinterpret_cast<TriQueue*>(reinterpret_cast<uint32_t*>(s_stack + kShared * blockDim.x) +
+                                               bounce_words(kFirst) * blockDim.x) + (threadIdx.x >> 5);   // deferTris
     const unsigned FULL = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned ltMask = (1u << lane) - 1u;
@@ -989,8 +1004,6 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_bounce_nee(WaveArgs a, int
     const float missWeight = depth > 0 ? 0.5f : 1.0f;
 
     bool has = false, exhausted = false, shadow = false;
-    int pixel = 0;
-    uint32_t rng = 0;
     int qi = 0;               // input-queue index of this lane's path (PRT_RELOAD_PATH)
     int slot = 0;             // output-queue slot of the extension ray while its shadow ray is traced
     float thr = 0.f, L = 0.f;
@@ -1012,6 +1025,8 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_bounce_nee(WaveArgs a, int
             if (!has && i < total)
             {
                 float3 org, dir;
+                int pixel = 0;
+                uint32_t rng = 0;
                 bool ok = true;
                 if (kFirst)
                 {
@@ -1055,6 +1070,15 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_bounce_nee(WaveArgs a, int
                 {
                     has = true;
                     shadow = false;
+                    if (kFirst || !PRT_RELOAD_PATH)
+                    {
+                        shw[4 * bd] = (uint32_t)pixel;
+                        shw[5 * bd] = rng;
+                        shw[6 * bd] = __float_as_uint(dir.x);
+                        shw[7 * bd] = __float_as_uint(dir.y);
+                        shw[8 * bd] = __float_as_uint(dir.z);
+                    }
+                    shear_store(shw, bd, shear_of(dir));
                     trav_setup(r, org, dir);
                     trav_init(ts, a.scene, FLT_MAX, st);
                 }
@@ -1069,16 +1093,19 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_bounce_nee(WaveArgs a, int
         {
             // extension rays (closest hit) and shadow rays (any hit) share the queue
             constexpr bool kPair = !kFirst && PRT_RELOAD_PATH && PRT_PAIRED_NEE;
-            warp_trav_deferred<kPair>(*tq, ts, a.scene, r, 0.0f, st, has, true, kRefillMin, lane, nullptr, nullptr,
+            warp_trav_deferred<kPair>(*tq, ts, a.scene, r, shw, bd, 0.0f, st, has, true, kRefillMin, lane, nullptr, nullptr,
                                       nullptr, nullptr, nullptr, shadow);
         }
         else
-        for (;;)
         {
-            if (has && !ts.done) trav_step<false>(ts, a.scene, r, 0.0f, st, nullptr, nullptr, shadow);
-            unsigned running = __ballot_sync(FULL, has && !ts.done);
-            if (running == 0) break;
-            if (32 - __popc(running) >= kRefillMin) break;
+            const Shear sh = shear_load(shw, bd);
+            for (;;)
+            {
+                if (has && !ts.done) trav_step<false>(ts, a.scene, r, sh, 0.0f, st, nullptr, nullptr, shadow);
+                unsigned running = __ballot_sync(FULL, has && !ts.done);
+                if (running == 0) break;
+                if (32 - __popc(running) >= kRefillMin) break;
+            }
         }
         // Extension-ray lanes that hit sample their shadow and extension rays,
         // append the extension ray at once and keep only its queue slot while
@@ -1104,9 +1131,9 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_bounce_nee(WaveArgs a, int
             }
             else
             {
-                fpix = pixel;
-                fdir = r.dir;
-                frng = rng;
+                fpix = (int)shw[4 * bd];
+                frng = shw[5 * bd];
+                fdir = f3(__uint_as_float(shw[6 * bd]), __uint_as_float(shw[7 * bd]), __uint_as_float(shw[8 * bd]));
             }
             if (ts.triHit < 0)
             {
@@ -1135,6 +1162,7 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_bounce_nee(WaveArgs a, int
             store_path(a.qout, o, eo, fpix, ed, frng);
             if (kAlbedo) __stcs(a.thrOut + o, thr);
             slot = o;
+            shear_store(shw, bd, shear_of(sd));
             trav_setup(r, so, sd);
             trav_init(ts, a.scene, FLT_MAX, st);
             shadow = true;
@@ -1165,7 +1193,8 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_bounce_nee(WaveArgs a, int
 // small part of this integrator's rays, so starting them here wins at every size:
 // against a first launch that queued the paths (k_bounce_nee), terrain 256x256 1
 // pass 0.76 -> 0.64 ms, 1001x563 16 passes 11.92 -> 11.54, 1080p 32 passes 86.5 -> 82.6.
-constexpr int kNeeWords = 11;   // pixel, depth | shadow << 8, RNG, throughput, radiance, direction, extension origin
+// pixel, depth | shadow << 8, RNG, throughput, radiance, direction, extension origin, shear terms
+constexpr int kNeeWords = 11 + kShearWords;
 
 template <bool kAlbedo>
 __global__ void __launch_bounds__(128, kWideBlocks) k_paths_nee(WaveArgs a)
@@ -1179,6 +1208,7 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_paths_nee(WaveArgs a)
     uint32_t* path = s_path + threadIdx.x;   // word k of this lane's path at path[k * bd]
     TriQueue* tq = reinterpret_cast<TriQueue*>(s_path + kNeeWords * blockDim.x) + (threadIdx.x >> 5);   // deferTris
     const int bd = blockDim.x;
+    uint32_t* shw = path + 11 * bd;
     const unsigned FULL = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned ltMask = (1u << lane) - 1u;
@@ -1188,7 +1218,7 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_paths_nee(WaveArgs a)
     if (blockIdx.x == 0 && threadIdx.x == 0)
         atomicAdd(a.rays, (unsigned long long)a.passes * (unsigned long long)a.cam.width *
                               (unsigned long long)a.cam.height);
-    unsigned long long more = 0;   // shadow rays and extension rays after the camera's, per warp
+    uint32_t more = 0;   // shadow rays and extension rays after the camera's, per warp
 
     bool has = false, exhausted = false;
     bool shadow = false;      // this lane's ray is a shadow ray
@@ -1283,6 +1313,7 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_paths_nee(WaveArgs a)
         }
         if (fresh)
         {
+            shear_store(shw, bd, shear_of(dir));
             trav_setup(r, org, dir);
             trav_init(ts, a.scene, FLT_MAX, st);
         }
@@ -1290,18 +1321,21 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_paths_nee(WaveArgs a)
         const int stopIdle = stop_idle(act);
         if (PRT_DEFER_NEE && a.scene.deferTris)
         {
-            warp_trav_deferred<PRT_PAIRED_NEE>(*tq, ts, a.scene, r, 0.0f, st, has, true, stopIdle, lane, nullptr, nullptr,
+            warp_trav_deferred<PRT_PAIRED_NEE>(*tq, ts, a.scene, r, shw, bd, 0.0f, st, has, true, stopIdle, lane, nullptr, nullptr,
                                                nullptr, nullptr, nullptr, shadow);
         }
         else
-        for (;;)
         {
-            if (has && !ts.done) trav_step<false>(ts, a.scene, r, 0.0f, st, nullptr, nullptr, shadow);
-            const unsigned running = __ballot_sync(FULL, has && !ts.done);
-            if (32 - __popc(running) >= stopIdle) break;
+            const Shear sh = shear_load(shw, bd);
+            for (;;)
+            {
+                if (has && !ts.done) trav_step<false>(ts, a.scene, r, sh, 0.0f, st, nullptr, nullptr, shadow);
+                const unsigned running = __ballot_sync(FULL, has && !ts.done);
+                if (32 - __popc(running) >= stopIdle) break;
+            }
         }
     }
-    if (lane == 0 && more) atomicAdd(a.rays, more);
+    if (lane == 0 && more) atomicAdd(a.rays, (unsigned long long)more);
 }
 
 // The IntersectorStreamCuda seam (core/intersector_stream_cuda.h:32-33):
@@ -1324,10 +1358,14 @@ __global__ void __launch_bounds__(128, kAnyHit ? PRT_BOUNCE_MIN_BLOCKS : kWideBl
     st.sh = s_stack + threadIdx.x;
     st.stride = blockDim.x;
     st.overflow = false;
-    // deferTris: the warps' triangle queues, then (closest hit) their barycentrics
-    TriQueue* tq = reinterpret_cast<TriQueue*>(s_stack + kShared * blockDim.x) + (threadIdx.x >> 5);
-    TriQueueUV* tuv = reinterpret_cast<TriQueueUV*>(reinterpret_cast<TriQueue*>(s_stack + kShared * blockDim.x) +
-                                                    (blockDim.x >> 5)) + (threadIdx.x >> 5);
+    // the block's stack columns, its lanes' shear terms and, deferTris, the warps'
+    // triangle queues, then (closest hit) their barycentrics
+    const int bd = blockDim.x;
+    uint32_t* s_words = reinterpret_cast<uint32_t*>(s_stack + kShared * blockDim.x);
+    uint32_t* shw = s_words + threadIdx.x;
+    TriQueue* s_queues = reinterpret_cast<TriQueue*>(s_words + kShearWords * blockDim.x);
+    TriQueue* tq = s_queues + (threadIdx.x >> 5);
+    TriQueueUV* tuv = reinterpret_cast<TriQueueUV*>(s_queues + (blockDim.x >> 5)) + (threadIdx.x >> 5);
     const unsigned FULL = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned ltMask = (1u << lane) - 1u;
@@ -1352,7 +1390,9 @@ __global__ void __launch_bounds__(128, kAnyHit ? PRT_BOUNCE_MIN_BLOCKS : kWideBl
             {
                 const float4* rp = reinterpret_cast<const float4*>(rays + i);
                 float4 a = __ldcs(rp), b = __ldcs(rp + 1);
-                trav_setup(r, f3(a.x, a.y, a.z), f3(b.x, b.y, b.z));
+                const float3 dir = f3(b.x, b.y, b.z);
+                shear_store(shw, bd, shear_of(dir));
+                trav_setup(r, f3(a.x, a.y, a.z), dir);
                 trav_init(ts, sc, b.w, st);
                 tnear = a.w;
                 idx = i;
@@ -1367,16 +1407,19 @@ __global__ void __launch_bounds__(128, kAnyHit ? PRT_BOUNCE_MIN_BLOCKS : kWideBl
         if (PRT_DEFER_ISECT && sc.deferTris)
         {
             constexpr bool kPair = kAnyHit && PRT_PAIRED_QUERY;
-            warp_trav_deferred<kPair, !kAnyHit, true>(*tq, ts, sc, r, tnear, st, has, !exhausted, kQueryRefill, lane, nullptr,
+            warp_trav_deferred<kPair, !kAnyHit, true>(*tq, ts, sc, r, shw, bd, tnear, st, has, !exhausted, kQueryRefill, lane, nullptr,
                                                 nullptr, nullptr, nullptr, nullptr, kAnyHit, tuv);
         }
         else
-        for (;;)
         {
-            if (has && !ts.done) trav_step<kAnyHit>(ts, sc, r, tnear, st);
-            unsigned running = __ballot_sync(FULL, has && !ts.done);
-            if (running == 0) break;
-            if (!exhausted && 32 - __popc(running) >= kQueryRefill) break;
+            const Shear sh = shear_load(shw, bd);
+            for (;;)
+            {
+                if (has && !ts.done) trav_step<kAnyHit>(ts, sc, r, sh, tnear, st);
+                unsigned running = __ballot_sync(FULL, has && !ts.done);
+                if (running == 0) break;
+                if (!exhausted && 32 - __popc(running) >= kQueryRefill) break;
+            }
         }
         if (has && ts.done)
         {
@@ -1398,8 +1441,8 @@ __global__ void __launch_bounds__(128, kAnyHit ? PRT_BOUNCE_MIN_BLOCKS : kWideBl
 // state; stk: the group's kPacketStack entries of shared memory.  Returns the
 // leaf-order index of the hit triangle, or -1, in every lane.
 template <bool kAnyHit>
-__device__ __forceinline__ int group_trace(const SceneDev& sc, const TravRay& r, float tnear, uint2* stk, unsigned lane,
-                                           float& tHit, int& primHit, float& uHit, float& vHit)
+__device__ __forceinline__ int group_trace(const SceneDev& sc, const TravRay& r, const Shear& sh, float tnear, uint2* stk,
+                                           unsigned lane, float& tHit, int& primHit, float& uHit, float& vHit)
 {
     const int j = (int)(lane & 7u);
     const unsigned gshift = lane & 24u, gmask = 0xffu << gshift;
@@ -1413,10 +1456,7 @@ __device__ __forceinline__ int group_trace(const SceneDev& sc, const TravRay& r,
     uint2 ng = make_uint2(0u, 0x80000000u);   // the root: one internal child at base 0
     for (;;)
     {
-        const uint32_t b = 31u - __clz(ng.y & 0xff000000u);
-        ng.y &= ~(1u << b);
-        const uint32_t slot = (b - 24u) ^ r.octinv;
-        const uint32_t nodeIdx = ng.x + __popc((ng.y & 0xffu) & ((1u << slot) - 1u));
+        const uint32_t nodeIdx = next_child(ng, r.oct);
         if ((ng.y & 0xff000000u) && sp < kPacketStack)
         {
             if (j == 0) stk[sp] = ng;
@@ -1462,8 +1502,8 @@ __device__ __forceinline__ int group_trace(const SceneDev& sc, const TravRay& r,
                     const float4 v0 = __ldg(tp), v1 = __ldg(tp + 1), v2 = __ldg(tp + 2);
                     const int prim = __float_as_int(v0.w);
                     float t, uu, vv;
-                    if (tri_test(r, f3(v0.x, v0.y, v0.z), f3(v1.x, v1.y, v1.z), f3(v2.x, v2.y, v2.z), tnear, tb, prim, pb,
-                                 t, uu, vv))
+                    if (tri_test(r.org, sh, f3(v0.x, v0.y, v0.z), f3(v1.x, v1.y, v1.z), f3(v2.x, v2.y, v2.z), tnear, tb, prim,
+                                 pb, t, uu, vv))
                     {
                         tb = t;
                         pb = prim;
@@ -1493,13 +1533,7 @@ __device__ __forceinline__ int group_trace(const SceneDev& sc, const TravRay& r,
             }
         }
         // internal hits: bit slot -> bit slot ^ octinv, as node_hits1 orders them
-        uint32_t in8 = c8 & imask;
-        uint32_t sw = ((in8 & 0x55u) << 1) | ((in8 >> 1) & 0x55u);
-        in8 = (r.octinv & 1u) ? sw : in8;
-        sw = ((in8 & 0x33u) << 2) | ((in8 >> 2) & 0x33u);
-        in8 = (r.octinv & 2u) ? sw : in8;
-        sw = ((in8 & 0x0fu) << 4) | ((in8 >> 4) & 0x0fu);
-        in8 = (r.octinv & 4u) ? sw : in8;
+        const uint32_t in8 = permute_octant(c8 & imask, r.oct);
         ng = make_uint2(q1.x, (in8 << 24) | imask);
         if (!(ng.y & 0xff000000u))
         {
@@ -1528,10 +1562,11 @@ __global__ void __launch_bounds__(128) k_intersect_few(SceneDev sc, const RayRec
     const float4* rp = reinterpret_cast<const float4*>(rays + i);
     const float4 a = __ldg(rp), b = __ldg(rp + 1);
     TravRay r;
-    trav_setup(r, f3(a.x, a.y, a.z), f3(b.x, b.y, b.z));
+    const float3 dir = f3(b.x, b.y, b.z);
+    trav_setup(r, f3(a.x, a.y, a.z), dir);
     float t = b.w, u = 0.f, v = 0.f;
     int prim = 0x7fffffff;
-    const int tri = group_trace<kAnyHit>(sc, r, a.w, s_stk + (threadIdx.x >> 3) * kPacketStack, lane, t, prim, u, v);
+    const int tri = group_trace<kAnyHit>(sc, r, shear_of(dir), a.w, s_stk + (threadIdx.x >> 3) * kPacketStack, lane, t, prim, u, v);
     if ((lane & 7u) != 0) return;
     if (kAnyHit) anyOut[i] = tri >= 0 ? t : -1.0f;
     else reinterpret_cast<float4*>(hits)[i] = tri >= 0 ? make_float4(t, __int_as_float(prim), u, v)
@@ -1545,10 +1580,11 @@ __global__ void k_query(SceneDev sc, const RayRec* ray, HitRec* hit, float* pNg)
     __shared__ uint2 s_stk[kPacketStack];
     const RayRec rr = *ray;
     TravRay r;
-    trav_setup(r, f3(rr.ox, rr.oy, rr.oz), f3(rr.dx, rr.dy, rr.dz));
+    const float3 dir = f3(rr.dx, rr.dy, rr.dz);
+    trav_setup(r, f3(rr.ox, rr.oy, rr.oz), dir);
     float t = rr.tfar, u = 0.f, v = 0.f;
     int prim = 0x7fffffff;
-    const int ti = group_trace<false>(sc, r, rr.tnear, s_stk, threadIdx.x, t, prim, u, v);
+    const int ti = group_trace<false>(sc, r, shear_of(dir), rr.tnear, s_stk, threadIdx.x, t, prim, u, v);
     if (threadIdx.x != 0) return;
     if (ti < 0)
     {
@@ -1556,11 +1592,11 @@ __global__ void k_query(SceneDev sc, const RayRec* ray, HitRec* hit, float* pNg)
         return;
     }
     *hit = HitRec{t, prim, u, v};
-    float3 p = madd(r.org, t, r.dir);
+    float3 p = madd(r.org, t, dir);
     const TriRec tr = sc.tris[ti];
     float3 p0 = f3(tr.v0.x, tr.v0.y, tr.v0.z), p1 = f3(tr.v1.x, tr.v1.y, tr.v1.z), p2 = f3(tr.v2.x, tr.v2.y, tr.v2.z);
     float3 Ng = normalize(cross(sub(p1, p0), sub(p2, p0)));
-    if (dot(Ng, r.dir) > 0.0f) Ng = f3(-Ng.x, -Ng.y, -Ng.z);
+    if (dot(Ng, dir) > 0.0f) Ng = f3(-Ng.x, -Ng.y, -Ng.z);
     pNg[0] = p.x; pNg[1] = p.y; pNg[2] = p.z;
     pNg[3] = Ng.x; pNg[4] = Ng.y; pNg[5] = Ng.z;
 }
@@ -1595,8 +1631,10 @@ __global__ void k_begin_render(int* pass, int spp, unsigned long long* rays, int
 
 constexpr int kReplayMaxDepth = 16;
 constexpr int kAggSlots = 256;             // block-private gradient slots of the adjoint
-constexpr int kReplayWords = 7;            // pixel, depth, RNG, throughput, direction (as k_paths)
-constexpr int kBackwardWords = 9;          // and dL/d(radiance) of the pixel, this lane's sky gradient
+// words per lane: pixel, depth, RNG, throughput, direction (as k_paths), shear terms;
+// backward: and dL/d(radiance) of the pixel, this lane's sky gradient
+constexpr int kReplayWords = 7 + kShearWords;
+constexpr int kBackwardWords = kReplayWords + 2;
 
 // Path-replay megakernel: each lane carries whole paths (pass, pixel), from
 // the camera ray to escape or maxDepth.  The forward mode accumulates the
@@ -1644,16 +1682,18 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_replay(SceneDev sc, Camera
     constexpr int kWords = kBackward ? kBackwardWords : kReplayWords;
     uint32_t* s_path = reinterpret_cast<uint32_t*>(s_stack + kShared * blockDim.x);
     uint32_t* path = s_path + threadIdx.x;   // word k of this lane's path at path[k * bd]
-    TriQueue* tq = reinterpret_cast<TriQueue*>(s_path + ((kWords + 1) & ~1) * blockDim.x) + (threadIdx.x >> 5);   // deferTris
+    TriQueue* tq = reinterpret_cast<TriQueue*>(s_path + kWords * blockDim.x) + (threadIdx.x >> 5);   // deferTris
     const int bd = blockDim.x;
+    uint32_t* shw = path + 7 * bd;
+    uint32_t* grad = path + kReplayWords * bd;   // kBackward
     const unsigned FULL = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned ltMask = (1u << lane) - 1u;
     const int W = cam.width;
     const long long npix = (long long)W * cam.height;
     const long long total = (long long)spp * npix;
-    if (kBackward) path[8 * bd] = 0u;   // sky gradient 0
-    unsigned long long traced = 0;      // rays, per warp
+    if (kBackward) grad[bd] = 0u;   // sky gradient 0
+    uint32_t traced = 0;      // rays, per warp
 
     bool has = false, exhausted = false;
     int prims[kBackward ? kReplayMaxDepth : 1];   // the triangles the path bounced off
@@ -1693,8 +1733,8 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_replay(SceneDev sc, Camera
                 }
                 else if (escaped)
                 {
-                    const float g = __uint_as_float(path[7 * bd]);
-                    path[8 * bd] = __float_as_uint(__uint_as_float(path[8 * bd]) + g * thr);
+                    const float g = __uint_as_float(grad[0]);
+                    grad[bd] = __float_as_uint(__uint_as_float(grad[bd]) + g * thr);
                     const float gc = g * c;
                     for (int k = 0; k < depth; ++k)
                     {
@@ -1729,7 +1769,7 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_replay(SceneDev sc, Camera
                 if (kBackward)
                 {
                     g = dL[3 * (size_t)pixel] + dL[3 * (size_t)pixel + 1] + dL[3 * (size_t)pixel + 2];
-                    path[7 * bd] = __float_as_uint(g);
+                    grad[0] = __float_as_uint(g);
                 }
                 if (g != 0.f)   // a pixel without a gradient has nothing to replay
                 {
@@ -1754,6 +1794,7 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_replay(SceneDev sc, Camera
             path[4 * bd] = __float_as_uint(dir.x);
             path[5 * bd] = __float_as_uint(dir.y);
             path[6 * bd] = __float_as_uint(dir.z);
+            shear_store(shw, bd, shear_of(dir));
             trav_setup(r, org, dir);
             trav_init(ts, sc, FLT_MAX, st);
         }
@@ -1761,24 +1802,27 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_replay(SceneDev sc, Camera
         const int stopIdle = stop_idle(act);
         if (PRT_DEFER_REPLAY && sc.deferTris)
         {
-            warp_trav_deferred<PRT_PAIRED_LATER>(*tq, ts, sc, r, 0.0f, st, has, true, stopIdle, lane);
+            warp_trav_deferred<PRT_PAIRED_LATER>(*tq, ts, sc, r, shw, bd, 0.0f, st, has, true, stopIdle, lane);
         }
         else
-        for (;;)
         {
-            if (has && !ts.done) trav_step<false>(ts, sc, r, 0.0f, st);
-            const unsigned running = __ballot_sync(FULL, has && !ts.done);
-            if (32 - __popc(running) >= stopIdle) break;
+            const Shear sh = shear_load(shw, bd);
+            for (;;)
+            {
+                if (has && !ts.done) trav_step<false>(ts, sc, r, sh, 0.0f, st);
+                const unsigned running = __ballot_sync(FULL, has && !ts.done);
+                if (32 - __popc(running) >= stopIdle) break;
+            }
         }
     }
     if (kBackward)
     {
-        float skyGrad = __uint_as_float(path[8 * bd]);
+        float skyGrad = __uint_as_float(grad[bd]);
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) skyGrad += __shfl_down_sync(FULL, skyGrad, off);
         if (lane == 0 && skyGrad != 0.f) atomicAdd(dSky, skyGrad);
     }
-    if (lane == 0 && rays) atomicAdd(rays, traced);
+    if (lane == 0 && rays) atomicAdd(rays, (unsigned long long)traced);
     if (kBackward)
     {
         __syncthreads();
@@ -1797,7 +1841,11 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_batch_first(BatchArgs a)
     extern __shared__ uint2 s_dyn[];
     uint2* s_stack = s_dyn;
     long long* s_begin = reinterpret_cast<long long*>(s_dyn + kShared * blockDim.x);
-    TriQueue* tq = reinterpret_cast<TriQueue*>(s_begin + a.nreq) + (threadIdx.x >> 5);   // when a.leaf1
+    const int bd = blockDim.x;
+    // per lane, as in k_bounce: shear terms, pixel, RNG state, direction
+    uint32_t* shw = reinterpret_cast<uint32_t*>(s_begin + a.nreq) + threadIdx.x;
+    TriQueue* tq = reinterpret_cast<TriQueue*>(reinterpret_cast<uint32_t*>(s_begin + a.nreq) +
+                                               bounce_words(true) * blockDim.x) + (threadIdx.x >> 5);   // when a.leaf1
     for (int q = threadIdx.x; q < a.nreq; q += blockDim.x) s_begin[q] = a.reqs[q].pathBegin;
     __syncthreads();
     TravStack st;
@@ -1812,8 +1860,7 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_batch_first(BatchArgs a)
 
     bool has = false;
     bool exhausted = false;
-    int pixel = 0, req = 0;
-    uint32_t rng = 0;
+    int req = 0;
     TravRay r;
     TravState ts;
     ts.done = true;
@@ -1831,6 +1878,8 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_batch_first(BatchArgs a)
             if (!has && i < total)
             {
                 float3 org, dir;
+                int pixel = 0;
+                uint32_t rng = 0;
                 bool ok = true;
                 long long gi = a.waveBegin + i;
                 int lo = 0, hi = a.nreq - 1;
@@ -1861,6 +1910,12 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_batch_first(BatchArgs a)
                 if (ok)
                 {
                     has = true;
+                    shw[4 * bd] = (uint32_t)pixel;
+                    shw[5 * bd] = rng;
+                    shw[6 * bd] = __float_as_uint(dir.x);
+                    shw[7 * bd] = __float_as_uint(dir.y);
+                    shw[8 * bd] = __float_as_uint(dir.z);
+                    shear_store(shw, bd, shear_of(dir));
                     trav_setup(r, org, dir);
                     trav_init(ts, a.reqs[req].scene, FLT_MAX, st);
                 }
@@ -1873,22 +1928,30 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_batch_first(BatchArgs a)
         }
         if (PRT_DEFER_TRIS && a.leaf1)
         {
-            warp_trav_deferred(*tq, ts, a.reqs[req].scene, r, 0.0f, st, has, !exhausted, kRefillMin, lane);
+            warp_trav_deferred(*tq, ts, a.reqs[req].scene, r, shw, bd, 0.0f, st, has, !exhausted, kRefillMin, lane);
         }
         else
-        for (;;)
         {
-            if (has && !ts.done) trav_step<false>(ts, a.reqs[req].scene, r, 0.0f, st);
-            unsigned running = __ballot_sync(FULL, has && !ts.done);
-            if (running == 0) break;
-            if (!exhausted && 32 - __popc(running) >= kRefillMin) break;
+            const Shear sh = shear_load(shw, bd);
+            for (;;)
+            {
+                if (has && !ts.done) trav_step<false>(ts, a.reqs[req].scene, r, sh, 0.0f, st);
+                unsigned running = __ballot_sync(FULL, has && !ts.done);
+                if (running == 0) break;
+                if (!exhausted && 32 - __popc(running) >= kRefillMin) break;
+            }
         }
         const bool fin = has && ts.done;
         bool cont = false;
         float contrib = 0.f;
-        float3 forg = r.org, fdir = r.dir;
+        int pixel = 0;
+        uint32_t rng = 0;
+        float3 forg = r.org, fdir = f3(0.f, 0.f, 0.f);
         if (fin)
         {
+            pixel = (int)shw[4 * bd];
+            rng = shw[5 * bd];
+            fdir = f3(__uint_as_float(shw[6 * bd]), __uint_as_float(shw[7 * bd]), __uint_as_float(shw[8 * bd]));
             const BatchReq& R = a.reqs[req];
             if (ts.triHit < 0)
             {
@@ -1968,7 +2031,7 @@ __global__ void __launch_bounds__(128, 8) k_batch_primary_packet(BatchArgs a)
         trav_setup(r, org, dir);
         float tHit;
         int primHit, triHit;
-        packet_closest_hit<PRT_PAIRED_PACKET, kIA>(R.scene, r, valid, vmask, stk, lane, tHit, primHit, triHit);
+        packet_closest_hit<PRT_PAIRED_PACKET, kIA>(R.scene, r, shear_of(dir), valid, vmask, stk, lane, tHit, primHit, triHit);
         bool cont = false;
         float contrib = 0.f;
         if (valid)
@@ -2006,7 +2069,7 @@ int grid_for(Kernel kernel, int block, size_t shmem, int numSMs, const LaunchCfg
 
 int launch_bounce(const WaveArgs& a, int depth, const LaunchCfg& cfg, int numSMs, cudaStream_t s)
 {
-    size_t shmem = sizeof(uint2) * kShared * cfg.block;
+    size_t shmem = (sizeof(uint2) * kShared + sizeof(uint32_t) * bounce_words(depth == 0)) * cfg.block;
     if (a.scene.deferTris && (a.Lout ? PRT_DEFER_NEE : PRT_DEFER_TRIS))
         shmem += sizeof(TriQueue) * (cfg.block / 32);   // the bounce kernels' triangle queues
     bool albedo = a.thrIn != nullptr || a.thrOut != nullptr;
@@ -2117,7 +2180,7 @@ int launch_batch_paths(const BatchArgs& a, const LaunchCfg& cfg, int numSMs, cud
 
 int launch_batch_first(const BatchArgs& a, const LaunchCfg& cfg, int numSMs, cudaStream_t s)
 {
-    size_t shmem = sizeof(uint2) * kShared * cfg.block + sizeof(long long) * a.nreq;
+    size_t shmem = (sizeof(uint2) * kShared + sizeof(uint32_t) * bounce_words(true)) * cfg.block + sizeof(long long) * a.nreq;
     if (PRT_DEFER_TRIS && a.leaf1) shmem += sizeof(TriQueue) * (cfg.block / 32);
     if (PRT_PACKET_PRIMARY && cfg.packet && a.packet)
     {
@@ -2157,7 +2220,7 @@ int launch_intersect(const SceneDev& sc, const RayRec* rays, HitRec* hits, int n
         else k_intersect_few<false><<<blocks, block, 0, s>>>(sc, rays, hits, anyOut, n, perWarp);
         return 1;
     }
-    size_t shmem = sizeof(uint2) * kShared * block;
+    size_t shmem = (sizeof(uint2) * kShared + sizeof(uint32_t) * kShearWords) * block;
     if (PRT_DEFER_ISECT && sc.deferTris)
         shmem += (sizeof(TriQueue) + (anyHit ? 0 : sizeof(TriQueueUV))) * (block / 32);
     LaunchCfg cfg;
@@ -2231,7 +2294,7 @@ int launch_replay(const SceneDev& sc, const CameraDev& cam, float4* accum, int p
     long long total = (long long)spp * cam.width * cam.height;
     if (total <= 0) return 0;
     const int block = 128;
-    const int words = ((backward ? kBackwardWords : kReplayWords) + 1) & ~1;   // the queues after them are 8-byte aligned
+    const int words = backward ? kBackwardWords : kReplayWords;
     size_t shmem = (sizeof(uint2) * kShared + sizeof(uint32_t) * words) * block;
     if (PRT_DEFER_REPLAY && sc.deferTris) shmem += sizeof(TriQueue) * (block / 32);
     LaunchCfg cfg;
