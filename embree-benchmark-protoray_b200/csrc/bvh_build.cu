@@ -409,13 +409,13 @@ struct CollapseArgs
     const int* idx;
     Bvh8Node* nodes;
     TriRec* tris;
-    unsigned long long* alloc;   // 8-wide nodes allocated (high 32 bits), leaf triangles (low 32 bits)
+    // per level: the nodes (high 32 bits) and leaf triangles (low 32 bits) that its
+    // nodes have allocated; then the error flag
+    unsigned long long* alloc;
     int nodeCapacity;
-    int* error;
     int leafMax;          // subtrees of at most this many triangles (1..3) become leaves
     const uint2* dec;     // grouping decisions of k_refit<true>, or nullptr for the greedy grouping
-    int* binRef;          // per 8-wide node: the binary reference it is built from
-    int* marks;           // level l is nodes [marks[l], marks[l + 1]); kCollapseLevels + 2 entries
+    int* binRef;          // per 8-wide node below the root: the binary reference it is built from
 };
 
 // Levels launched; a tree that needs more would overflow the traversal stack
@@ -423,6 +423,12 @@ struct CollapseArgs
 constexpr int kCollapseLevels = kStackMax / 2;
 constexpr int kCollapseBlock = 128;
 constexpr int kGroupsPerBlock = kCollapseBlock / 8;
+static_assert(kCollapseLevels <= 32, "one lane per level in k_collapse");
+
+__device__ __forceinline__ void collapse_error(const CollapseArgs& a)
+{
+    atomicExch(reinterpret_cast<int*>(a.alloc + kCollapseLevels), 1);
+}
 
 __device__ __forceinline__ int ref_count(const CollapseArgs& a, int ref)
 {
@@ -456,32 +462,60 @@ struct __align__(16) CollapseGroup
     int2 front[8];
 };
 
-// One 8-lane group builds 8-wide node nodeIdx from binary reference
-// binRef[nodeIdx]: lane c holds child c of the node.  A binary reference of
-// ~0 with n == 1 is the single-triangle scene.
-__device__ void collapse_node(const CollapseArgs& a, int nodeIdx, int sub, unsigned gmask, CollapseGroup& g)
+// Least and greatest value over an 8-lane group.
+__device__ __forceinline__ uint32_t group_min(uint32_t x)
 {
-    const int bref = a.binRef[nodeIdx];
+#pragma unroll
+    for (int off = 1; off < 8; off <<= 1) x = min(x, __shfl_xor_sync(0xffffffffu, x, off));
+    return x;
+}
+__device__ __forceinline__ uint32_t group_max(uint32_t x)
+{
+#pragma unroll
+    for (int off = 1; off < 8; off <<= 1) x = max(x, __shfl_xor_sync(0xffffffffu, x, off));
+    return x;
+}
+
+// Four nodes per warp, one per 8-lane group: a group with `on` builds 8-wide node
+// nodeIdx from binary reference bref, lane c of it holding child c of the node.
+// (bref = ~0 with n == 1 is the single-triangle scene.)  Its children are
+// allocated from alloc, nodes from firstNode and leaf triangles from firstTri on.
+// All 32 lanes run every step, a group without a node idly: synchronising each
+// group by itself would let the four drift apart and run one after the other. (the
+// collapse of 1.38M triangles so, with a launch per level that noted where the
+// next level ends: 481 us, now 262; prt_build_accel of 82K triangles 0.96 -> 0.82
+// ms, 1.38M 2.55 -> 2.33, 10.24M 15.7 -> 14.7).  A single node takes 9 us, a chain
+// of dependent loads, and the level with most nodes is bound by instructions.
+__device__ void collapse_nodes(const CollapseArgs& a, unsigned long long* alloc, int firstNode, int firstTri, int nodeIdx,
+                               int bref, bool on, int lane, CollapseGroup& g)
+{
+    const unsigned FULL = 0xffffffffu;
+    const int sub = lane & 7, shift = lane & 24;
 
     // 1. children: the roots chosen by the grouping decisions (or greedily
     //    opened), left to right in tree order, child c in lane c
-    int r = 0, nc;
-    if (bref < 0)
+    int r = 0, nc = 0;
+    const bool inner = on && bref >= 0;
+    if (on && !inner)
     {
         r = bref;
         nc = 1;
     }
-    else if (a.dec)
+    if (a.dec)
     {
         // expand the split list breadth-first: an entry (u, i) gives i slots
         // to subtree u; it is final for a triangle or i = 1, else the largest
         // i' <= i without the "no worse with fewer" bit splits it between the
         // binary children (i' = 1: u itself is the root)
-        const int2 c = a.child[bref];
-        const int j = (int)(dec_byte(__ldg(a.dec + bref), 7) & 0x7f);
-        r = sub == 0 ? c.x : c.y;
-        int ri = sub == 0 ? j : 8 - j;
-        nc = 2;
+        int ri = 1;
+        if (inner)
+        {
+            const int2 c = a.child[bref];
+            const int j = (int)(dec_byte(__ldg(a.dec + bref), 7) & 0x7f);
+            r = sub == 0 ? c.x : c.y;
+            ri = sub == 0 ? j : 8 - j;
+            nc = 2;
+        }
         for (int round = 0; round < 8; ++round)
         {
             const bool valid = sub < nc;
@@ -496,14 +530,17 @@ __device__ void collapse_node(const CollapseArgs& a, int nodeIdx, int sub, unsig
             int ii = ri;
             if (expand)
                 while (ii > 1 && (dec_byte(d, ii - 1) & 0x80)) --ii;
-            const bool split = expand && ii > 1;
-            const unsigned splitMask = (__ballot_sync(gmask, split) & gmask) >> (__ffs(gmask) - 1);
-            if (!splitMask) break;
+            bool split = expand && ii > 1;
+            const unsigned splits = __ballot_sync(FULL, split);
+            if (!splits) break;
+            unsigned splitMask = (splits >> shift) & 0xffu;
             if (nc + __popc(splitMask) > 8)
             {
                 // slot counts that do not add up to 8: inconsistent decisions
-                if (sub == 0) atomicExch(a.error, 1);
-                return;
+                if (sub == 0) collapse_error(a);
+                on = split = false;
+                nc = 0;
+                splitMask = 0;
             }
             const int at = min(sub, nc) + __popc(splitMask & ((1u << sub) - 1));
             if (split)
@@ -512,18 +549,18 @@ __device__ void collapse_node(const CollapseArgs& a, int nodeIdx, int sub, unsig
                 g.front[at] = make_int2(cc.x, dj);
                 g.front[at + 1] = make_int2(cc.y, ii - dj);
             }
-            else if (valid)
+            else if (sub < nc)
             {
                 g.front[at] = make_int2(r, expand ? 1 : ri);
             }
             nc += __popc(splitMask);
-            __syncwarp(gmask);
+            __syncwarp();
             if (sub < nc)
             {
                 r = g.front[sub].x;
                 ri = g.front[sub].y;
             }
-            __syncwarp(gmask);
+            __syncwarp();
         }
     }
     else
@@ -531,40 +568,46 @@ __device__ void collapse_node(const CollapseArgs& a, int nodeIdx, int sub, unsig
         // greedy: open the child of largest surface area while fewer than 8
         // (ties to the lower child); the opened child keeps its left half in
         // its lane and the right half goes to lane nc
-        const int2 c = a.child[bref];
-        r = sub == 0 ? c.x : c.y;
-        nc = 2;
+        if (inner)
+        {
+            const int2 c = a.child[bref];
+            r = sub == 0 ? c.x : c.y;
+            nc = 2;
+        }
         bool stale = true;
         uint32_t key = 0;
-        while (nc < 8)
+        for (int round = 0; round < 6; ++round)
         {
             if (stale)
             {
                 key = 0;
-                if (sub < nc && r >= 0 && ref_count(a, r) > a.leafMax)
+                if (inner && sub < nc && r >= 0 && ref_count(a, r) > a.leafMax)
                 {
                     const float ar = half_area(ref_box(a, r));
                     if (ar >= 0.f) key = ((__float_as_uint(ar) | 0x80000000u) & ~7u) | (uint32_t)(7 - sub);
                 }
                 stale = false;
             }
-            const uint32_t top = __reduce_max_sync(gmask, key);
-            if (!top) break;
+            const uint32_t top = group_max(key);
+            if (!__any_sync(FULL, top != 0)) break;
             const int best = 7 - (int)(top & 7u);
             int2 c2 = make_int2(0, 0);
-            if (sub == best) c2 = a.child[r];
-            const int right = __shfl_sync(gmask, c2.y, best, 8);
-            if (sub == best)
+            if (top && sub == best) c2 = a.child[r];
+            const int right = __shfl_sync(FULL, c2.y, best, 8);
+            if (top)
             {
-                r = c2.x;
-                stale = true;
+                if (sub == best)
+                {
+                    r = c2.x;
+                    stale = true;
+                }
+                if (sub == nc)
+                {
+                    r = right;
+                    stale = true;
+                }
+                ++nc;
             }
-            if (sub == nc)
-            {
-                r = right;
-                stale = true;
-            }
-            ++nc;
         }
     }
 
@@ -603,8 +646,8 @@ __device__ void collapse_node(const CollapseArgs& a, int nodeIdx, int sub, unsig
 #pragma unroll
         for (int k = 0; k < 3; ++k)
         {
-            nb[k] = fminf(nb[k], __shfl_xor_sync(gmask, nb[k], off, 8));
-            nb[3 + k] = fmaxf(nb[3 + k], __shfl_xor_sync(gmask, nb[3 + k], off, 8));
+            nb[k] = fminf(nb[k], __shfl_xor_sync(FULL, nb[k], off));
+            nb[3 + k] = fmaxf(nb[3 + k], __shfl_xor_sync(FULL, nb[3 + k], off));
         }
     }
 
@@ -624,7 +667,8 @@ __device__ void collapse_node(const CollapseArgs& a, int nodeIdx, int sub, unsig
     }
     int slot = -1;
     unsigned freeSlots = 0xffu;
-    for (int it = 0; it < nc; ++it)
+    const int ncMax = (int)__reduce_max_sync(FULL, (unsigned)nc);
+    for (int it = 0; it < ncMax; ++it)
     {
         // key: cost (order-preserving bits, 6 low bits dropped), slot, lane;
         // least wins
@@ -647,21 +691,14 @@ __device__ void collapse_node(const CollapseArgs& a, int nodeIdx, int sub, unsig
                 key = (ord & ~63u) | ((uint32_t)bs << 3) | (uint32_t)sub;
             }
         }
-        const uint32_t least = __reduce_min_sync(gmask, key);
-        int bs, bl;
-        if (least != 0xffffffffu)
-        {
-            bs = (int)((least >> 3) & 7u);
-            bl = (int)(least & 7u);
-        }
-        else
-        {
-            // no finite cost left (degenerate boxes): lowest free slot to the
-            // lowest unplaced child
-            bs = __ffs(freeSlots) - 1;
-            const unsigned unplaced = __ballot_sync(gmask, valid && slot < 0) & gmask;
-            bl = __ffs(unplaced >> (__ffs(gmask) - 1)) - 1;
-        }
+        const uint32_t least = group_min(key);
+        const unsigned unplaced = (__ballot_sync(FULL, valid && slot < 0) >> shift) & 0xffu;
+        if (!unplaced) continue;   // a group with fewer children
+        // no finite cost left (degenerate boxes): lowest free slot to the lowest
+        // unplaced child
+        const bool finite = least != 0xffffffffu;
+        const int bs = finite ? (int)((least >> 3) & 7u) : __ffs(freeSlots) - 1;
+        const int bl = finite ? (int)(least & 7u) : __ffs(unplaced) - 1;
         if (sub == bl) slot = bs;
         freeSlots &= ~(1u << bs);
     }
@@ -670,7 +707,7 @@ __device__ void collapse_node(const CollapseArgs& a, int nodeIdx, int sub, unsig
     //    packed in slot order
     if (valid) g.slotRec[slot] = 0x80000000u | (leaf ? 0u : 0x40000000u) | (uint32_t)cnt;
     if ((freeSlots >> sub) & 1u) g.slotRec[sub] = 0;   // the empty slots
-    __syncwarp(gmask);
+    __syncwarp();
     int nInternal = 0, nTris = 0, internalRank = 0, triOff = 0;
     uint32_t imask = 0;
 #pragma unroll
@@ -691,35 +728,26 @@ __device__ void collapse_node(const CollapseArgs& a, int nodeIdx, int sub, unsig
             nTris += c;
         }
     }
-    int childBase = 0, triBase = 0, bad = 0;
-    if (sub == 0)
+    // one atomic for the child nodes and leaf triangles of the warp's groups
+    const unsigned long long req = on ? ((unsigned long long)nInternal << 32) | (unsigned)nTris : 0ull;
+    unsigned long long before = 0, total = 0;
+#pragma unroll
+    for (int l = 0; l < 32; l += 8)
     {
-        // one atomic for the child nodes and leaf triangles of all the groups
-        // of this warp that are here together
-        const unsigned m = __activemask();
-        const int me = threadIdx.x & 31;
-        const unsigned long long req = ((unsigned long long)nInternal << 32) | (unsigned)nTris;
-        unsigned long long before = 0, total = 0;
-        for (unsigned rest = m; rest; rest &= rest - 1)
-        {
-            const int l = __ffs(rest) - 1;
-            const unsigned long long v = __shfl_sync(m, req, l);
-            if (l < me) before += v;
-            total += v;
-        }
-        const int first = __ffs(m) - 1;
-        unsigned long long base = 0;
-        if (me == first) base = atomicAdd(a.alloc, total);
-        base = __shfl_sync(m, base, first) + before;
-        childBase = (int)(base >> 32);
-        triBase = (int)(base & 0xffffffffu);
-        bad = childBase + nInternal > a.nodeCapacity || triBase + nTris > a.n;
-        if (bad) atomicExch(a.error, 1);
+        const unsigned long long v = __shfl_sync(FULL, req, l);
+        if (l < shift) before += v;
+        total += v;
     }
-    const int leader = __ffs(gmask) - 1;
-    if (__shfl_sync(gmask, bad, leader)) return;   // group-uniform
-    childBase = __shfl_sync(gmask, childBase, leader);
-    triBase = __shfl_sync(gmask, triBase, leader);
+    unsigned long long base = 0;
+    if (lane == 0 && total) base = atomicAdd(alloc, total);
+    base = __shfl_sync(FULL, base, 0) + before;
+    const int childBase = firstNode + (int)(base >> 32);
+    const int triBase = firstTri + (int)(base & 0xffffffffu);
+    if (on && (childBase + nInternal > a.nodeCapacity || triBase + nTris > a.n))
+    {
+        if (sub == 0) collapse_error(a);
+        on = false;
+    }
 
     // 6. header: per-axis power-of-two scale s with the node box spanning at
     //    most 253 steps, and origin one step below the box, so every quantized
@@ -770,7 +798,7 @@ __device__ void collapse_node(const CollapseArgs& a, int nodeIdx, int sub, unsig
             g.node[56 + 8 * k + sub] = 0;
         }
     }
-    if (valid)
+    if (on && valid)
     {
 #pragma unroll
         for (int k = 0; k < 3; ++k)
@@ -814,93 +842,92 @@ __device__ void collapse_node(const CollapseArgs& a, int nodeIdx, int sub, unsig
         w[4] = (uint32_t)childBase;
         w[5] = (uint32_t)triBase;
     }
-    __syncwarp(gmask);
-    if (sub < 5) a.nodes[nodeIdx].q[sub] = reinterpret_cast<const uint4*>(g.node)[sub];
-    __syncwarp(gmask);
+    __syncwarp();
+    if (on && sub < 5) a.nodes[nodeIdx].q[sub] = reinterpret_cast<const uint4*>(g.node)[sub];
+    __syncwarp();
 }
 
-// One tree level: nodes [marks[level], marks[level + 1]), one per 8-lane
-// group, grid-strided.
+// One tree level, one node per 8-lane group, grid-strided.  The nodes of a level
+// follow those of the level above, and alloc tells how many each level has: level
+// l + 1 has those that level l allocated.
 __global__ void __launch_bounds__(kCollapseBlock) k_collapse(CollapseArgs a, int level)
 {
     __shared__ CollapseGroup groups[kGroupsPerBlock];
-    if (*(volatile int*)a.error) return;
-    const int begin = *(volatile int*)(a.marks + level);
-    const int end = *(volatile int*)(a.marks + level + 1);
+    if (*reinterpret_cast<const int*>(a.alloc + kCollapseLevels)) return;
     const int lane = threadIdx.x & 31;
-    const int sub = lane & 7;
-    const unsigned gmask = 0xffu << (lane & 24);
+    const unsigned long long above = lane < level ? a.alloc[lane] : 0ull;
+    const unsigned nodesAbove = (unsigned)(above >> 32);
+    const int end = 1 + (int)__reduce_add_sync(0xffffffffu, nodesAbove);   // of this level, the next one's first
+    const int firstTri = (int)__reduce_add_sync(0xffffffffu, (unsigned)above);
+    const int begin = level ? end - (int)__shfl_sync(0xffffffffu, nodesAbove, level - 1) : 0;
     CollapseGroup& g = groups[threadIdx.x >> 3];
     const int stride = gridDim.x * kGroupsPerBlock;
-    for (int w = begin + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 3); w < end; w += stride)
-        collapse_node(a, w, sub, gmask, g);
+    int w = begin + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 3);
+    for (; w - (lane >> 3) < end; w += stride)
+    {
+        const bool on = w < end;
+        const int bref = level ? (on ? a.binRef[w] : 0) : (a.n > 1 ? 0 : ~0);
+        collapse_nodes(a, a.alloc + level, end, firstTri, w, bref, on, lane, g);
+    }
 }
-
-// After level l: the nodes allocated so far end level l + 1.
-__global__ void k_collapse_mark(CollapseArgs a, int level)
-{
-    a.marks[level + 2] = (int)(*(volatile unsigned long long*)a.alloc >> 32);
-}
-
 
 // Runs the collapse from the root, one launch per level, without waiting for
 // the host between levels: launches past the last level find no nodes and
-// return.  The counters are read back after the first kCollapseBatch levels
-// and, for a deeper tree, after the rest.  On success sets the node and
-// triangle counts and the number of 8-wide levels (kCollapseLevels + 1 for a
-// tree deeper than the launches).
-constexpr int kCollapseBatch = 16;
+// return.  The counters are read back after the levels that a tree of n
+// triangles usually has (log8 n and a half more), and after every
+// kCollapseBatch levels of a deeper one.  On success sets the node and triangle
+// counts and the number of 8-wide levels (kCollapseLevels + 1 for a tree deeper
+// than the launches).
+constexpr int kCollapseBatch = 4;
 
 int collapse_levels(const CollapseArgs& a, int n, int numSMs, cudaStream_t stream, int& nodeCount, int& triCount,
                     int& levels, std::string& err)
 {
-    const int root = n > 1 ? 0 : ~0;
-    const unsigned long long alloc0 = 1ull << 32;   // the root
-    const int marks0[2] = {0, 1};
-    int hostErr = 0;
-    unsigned long long hostAlloc = 0;
-    int marks[kCollapseLevels + 2];
-    cudaError_t e = cudaMemcpyAsync(a.binRef, &root, sizeof(int), cudaMemcpyHostToDevice, stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(a.alloc, &alloc0, sizeof(alloc0), cudaMemcpyHostToDevice, stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(a.error, 0, sizeof(int), stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(a.marks, 0, sizeof(int) * (kCollapseLevels + 2), stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(a.marks, marks0, sizeof(marks0), cudaMemcpyHostToDevice, stream);
+    unsigned long long alloc[kCollapseLevels + 1] = {};
+    cudaError_t e = cudaMemsetAsync(a.alloc, 0, sizeof(alloc), stream);
     int perSM = 1;
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_collapse, kCollapseBlock, 0);
     const long long maxBlocks = (long long)std::max(1, numSMs) * std::max(1, perSM);
     long long bound = 1;   // level l holds at most 8^l nodes
+    int log2n = 0;
+    while (log2n < 31 && (1u << log2n) < (unsigned)n) ++log2n;
+    int stop = std::min(kCollapseLevels, log2n / 2 + 1);
     int l = 0;
-    while (e == cudaSuccess && l < kCollapseLevels)
+    bool error = false;
+    while (e == cudaSuccess)
     {
-        const int stop = std::min(kCollapseLevels, l + kCollapseBatch);
         for (; e == cudaSuccess && l < stop; ++l)
         {
             const int blocks = (int)std::min(maxBlocks, (bound + kGroupsPerBlock - 1) / kGroupsPerBlock);
             k_collapse<<<blocks, kCollapseBlock, 0, stream>>>(a, l);
-            k_collapse_mark<<<1, 1, 0, stream>>>(a, l);
             e = cudaGetLastError();
             bound = std::min<long long>(bound * 8, 1ll << 32);
         }
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&hostErr, a.error, sizeof(int), cudaMemcpyDeviceToHost, stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&hostAlloc, a.alloc, sizeof(hostAlloc), cudaMemcpyDeviceToHost, stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(marks, a.marks, sizeof(marks), cudaMemcpyDeviceToHost, stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(alloc, a.alloc, sizeof(alloc), cudaMemcpyDeviceToHost, stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-        if (e == cudaSuccess && (hostErr || marks[l + 1] == marks[l])) break;   // error, or no level l
+        error = alloc[kCollapseLevels] != 0;
+        if (error || !(alloc[l - 1] >> 32) || l == kCollapseLevels) break;
+        stop = std::min(kCollapseLevels, l + kCollapseBatch);
     }
     if (e != cudaSuccess)
     {
         err = std::string("BVH8 collapse: ") + cudaGetErrorString(e);
         return e == cudaErrorMemoryAllocation ? PRT_ENOMEM : PRT_ECUDA;
     }
-    if (hostErr)
+    if (error)
     {
         err = "BVH8 collapse exceeded its node or triangle capacity";
         return PRT_EINTERNAL;
     }
-    levels = 0;
-    while (levels <= kCollapseLevels && marks[levels + 1] > marks[levels]) ++levels;
-    nodeCount = (int)(hostAlloc >> 32);
-    triCount = (int)(hostAlloc & 0xffffffffu);
+    levels = nodeCount = 1;
+    triCount = 0;
+    for (l = 0; l < kCollapseLevels; ++l)
+    {
+        const int below = (int)(alloc[l] >> 32);
+        nodeCount += below;
+        triCount += (int)(alloc[l] & 0xffffffffu);
+        if (below) ++levels;
+    }
     return PRT_OK;
 }
 
@@ -952,7 +979,7 @@ int build_bvh8_tree(const float* dPos, int nv, const int* dIdx, int nt, Bvh8Devi
     float *triBox, *partial, *cbounds, *box;
     uint32_t *keysA, *keysB, *valsA, *valsB, *hist;
     int2 *child, *range;
-    int *parent, *flag, *collapseErr, *marks, *binRef;
+    int *parent, *flag, *binRef;
     SahTreeBuffers top{};
     unsigned long long* collapseAlloc;
     float4* dpCost;
@@ -974,9 +1001,7 @@ int build_bvh8_tree(const float* dPos, int nv, const int* dIdx, int nt, Bvh8Devi
         box = c.take<float>(6 * (size_t)(2 * n));
         binRef = c.take<int>(nodeCapacity);
         if (rebuild) sah_tree_carve(c, n, top);
-        collapseAlloc = c.take<unsigned long long>(1);
-        collapseErr = c.take<int>(1);
-        marks = c.take<int>(kCollapseLevels + 2);
+        collapseAlloc = c.take<unsigned long long>(kCollapseLevels + 1);
         dpCost = group ? c.take<float4>(2 * (size_t)nodeCapacity) : nullptr;
         dpDec = group ? c.take<uint2>(nodeCapacity) : nullptr;
         return c.off;
@@ -1077,11 +1102,9 @@ int build_bvh8_tree(const float* dPos, int nv, const int* dIdx, int nt, Bvh8Devi
         a.tris = out.tris;
         a.alloc = collapseAlloc;
         a.nodeCapacity = nodeCapacity;
-        a.error = collapseErr;
         a.leafMax = std::max(1, std::min(3, leafMax));
         a.dec = dpDec;
         a.binRef = binRef;
-        a.marks = marks;
         int nodeCount = 0, triCount = 0;
         status = collapse_levels(a, n, numSMs, stream, nodeCount, triCount, levels, err);
         if (status == PRT_OK && a.dec && 2 * levels > kStackMax)
