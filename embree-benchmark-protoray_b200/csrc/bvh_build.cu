@@ -30,6 +30,7 @@
 
 #include "prt_device.cuh"
 #include "prt_internal.h"
+#include "refit.cuh"
 
 namespace prt_b200 {
 
@@ -201,9 +202,10 @@ __global__ void k_karras(const uint32_t* __restrict__ keys, int n, int2* __restr
 
 // --- 5. bottom-up refit and SAH-optimal grouping into 8-wide nodes ----------
 //
-// One thread per triangle walks up the tree; the second thread to arrive at
-// a node (atomic counter) computes it from its two finished children, so every
-// node is computed once, after both children.
+// For the Morton tree: one thread per triangle walks up; the second thread to
+// arrive at a node (atomic counter) computes it from its two finished children, so
+// every node is computed once, after both children.  (The SAH tree's nodes are
+// computed by the blocks that build its subtrees, sah_build.cu.)
 //
 // The node box is the union of the children's boxes.  With kGroup the same
 // pass runs the dynamic program of Ylitie, Karras and Laine (HPG 2017,
@@ -217,133 +219,7 @@ __global__ void k_karras(const uint32_t* __restrict__ keys, int n, int2* __restr
 // i = 1 whether u is best a leaf (1) or an 8-wide node (0); for i >= 2 the
 // slots j given to the left child (low 7 bits), with 0x80 set when at most
 // i - 1 roots are no worse.
-#ifndef PRT_WIDE_DP
-#define PRT_WIDE_DP 1
-#endif
-#ifndef PRT_SAH_CTRI
-#define PRT_SAH_CTRI 0.7f
-#endif
-
-__device__ __forceinline__ float box_half_area(const float* b)
-{
-    float dx = b[3] - b[0], dy = b[4] - b[1], dz = b[5] - b[2];
-    return dx * dy + dy * dz + dz * dx;
-}
-
-struct RefitArgs
-{
-    int n;
-    const uint32_t* vals;   // sorted triangle ids
-    const float* triBox;    // 6 floats per triangle, by triangle id
-    const int2* child;
-    const int2* range;
-    const int* parent;
-    float* box;             // 6 floats per node: internal [0, n-1), leaves [n-1, 2n-1)
-    int* flag;              // arrivals per internal node, zeroed
-    float4* cost;           // kGroup: 2 float4 (C(u, 1..8)) per internal node
-    uint2* dec;             // kGroup: 8 decision bytes per internal node
-    int leafMax;
-};
-
-// C(child, 1..8) of a binary child: loaded for an internal node, its area x
-// cTri for a single triangle.
-__device__ __forceinline__ void child_costs(const RefitArgs& a, int ref, const float* b, float* c)
-{
-    if (ref < 0)
-    {
-        const float leafCost = box_half_area(b) * PRT_SAH_CTRI;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) c[i] = leafCost;
-        return;
-    }
-    const float4 lo = __ldcg(a.cost + 2 * (size_t)ref), hi = __ldcg(a.cost + 2 * (size_t)ref + 1);
-    c[0] = lo.x; c[1] = lo.y; c[2] = lo.z; c[3] = lo.w;
-    c[4] = hi.x; c[5] = hi.y; c[6] = hi.z; c[7] = hi.w;
-}
-
-// Node `node` (children ch, triangle range rg) from its two finished
-// children: box, and with kGroup its grouping costs and decisions.
-template <bool kGroup>
-__device__ __forceinline__ void refit_node(const RefitArgs& a, int node, int2 ch, int2 rg)
-{
-    const int n = a.n;
-    const int ia = ch.x >= 0 ? ch.x : (n - 1) + ~ch.x;
-    const int ib = ch.y >= 0 ? ch.y : (n - 1) + ~ch.y;
-    float ba[6], bb[6], r[6];
-#pragma unroll
-    for (int c = 0; c < 6; ++c)
-    {
-        ba[c] = __ldcg(a.box + 6 * (size_t)ia + c);
-        bb[c] = __ldcg(a.box + 6 * (size_t)ib + c);
-    }
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-    {
-        r[c] = fminf(ba[c], bb[c]);
-        r[3 + c] = fmaxf(ba[3 + c], bb[3 + c]);
-    }
-#pragma unroll
-    for (int c = 0; c < 6; ++c) __stcg(a.box + 6 * (size_t)node + c, r[c]);
-    if (kGroup)
-    {
-        float ca[8], cb[8];
-        child_costs(a, ch.x, ba, ca);
-        child_costs(a, ch.y, bb, cb);
-        const float area = box_half_area(r);
-        const int cnt = rg.y - rg.x + 1;
-        float dist[8];
-        uint8_t split[8];
-        dist[0] = FLT_MAX;
-        split[0] = 0;
-#pragma unroll
-        for (int i = 2; i <= 8; ++i)
-        {
-            float best = FLT_MAX;
-            int bj = 1;
-#pragma unroll
-            for (int j = 1; j < i; ++j)
-            {
-                const float v = ca[j - 1] + cb[i - j - 1];
-                if (v < best)
-                {
-                    best = v;
-                    bj = j;
-                }
-            }
-            dist[i - 1] = best;
-            split[i - 1] = (uint8_t)bj;
-        }
-        const float leafOpt = cnt <= a.leafMax ? area * PRT_SAH_CTRI * (float)cnt : FLT_MAX;
-        const float wideOpt = area + dist[7];
-        float cs[8];
-        float c = fminf(leafOpt, wideOpt);
-        cs[0] = c;
-        uint32_t d0 = leafOpt <= wideOpt ? 1u : 0u, d1 = 0;
-#pragma unroll
-        for (int i = 2; i <= 8; ++i)
-        {
-            uint32_t d = split[i - 1];
-            if (c <= dist[i - 1]) d |= 0x80;
-            else c = dist[i - 1];
-            cs[i - 1] = c;
-            if (i <= 4) d0 |= d << (8 * (i - 1));
-            else d1 |= d << (8 * (i - 5));
-        }
-        __stcg(a.cost + 2 * (size_t)node, make_float4(cs[0], cs[1], cs[2], cs[3]));
-        __stcg(a.cost + 2 * (size_t)node + 1, make_float4(cs[4], cs[5], cs[6], cs[7]));
-        __stcg(a.dec + node, make_uint2(d0, d1));
-    }
-}
-
-// Arrival at a node: the atomic increment releases this thread's writes (its
-// child's box and costs) and, for the second arrival, acquires the sibling's.
-__device__ __forceinline__ unsigned arrive(int* flag)
-{
-    unsigned old;
-    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(flag) : "memory");
-    return old;
-}
-
+//
 // The bottom-up walk with lanes refilled: each warp owns a run of consecutive
 // leaves; a lane whose walk ends (first arrival at a node, or the root) takes
 // the warp's next leaf, so the warp's lanes stay busy while the walks that
@@ -389,7 +265,10 @@ __global__ void __launch_bounds__(kRefitBlock) k_refit(RefitArgs a, int leavesPe
             }
             else
             {
-                refit_node<kGroup>(a, node, ch, rg);
+                float ba[6], bb[6];
+                load_box(a, ch.x, ba);
+                load_box(a, ch.y, bb);
+                refit_node<kGroup>(a, node, ch, rg.y - rg.x + 1, ba, bb);
                 node = up;
             }
         }
@@ -1046,39 +925,38 @@ int build_bvh8_tree(const float* dPos, int nv, const int* dIdx, int nt, Bvh8Devi
     k_reduce_bounds<<<1, 256, 0, stream>>>(partial, boundBlocks, cbounds);
     k_morton<<<div_up(n, 256), 256, 0, stream>>>(triBox, n, cbounds, keysA, valsA);
     radix_sort_pairs(keysA, valsA, keysB, valsB, hist, n, 30, stream);
+    RefitArgs ra;
+    ra.n = n;
+    ra.vals = valsA;
+    ra.triBox = triBox;
+    ra.child = child;
+    ra.range = range;
+    ra.parent = parent;
+    ra.box = box;
+    ra.flag = flag;
+    ra.cost = dpCost;
+    ra.dec = dpDec;
+    ra.leafMax = std::max(1, std::min(3, leafMax));
     if (nInternal > 0)
     {
-        if (rebuild)
-        {
-            top.order[0] = keysA;   // free after the sort
-            top.order[1] = keysB;
-            BUILD_CHECK(sah_build_tree(n, triBox, cbounds, valsA, valsB, child, range, parent, top, numSMs, stream));
-            std::swap(valsA, valsB);
-        }
-        else
-        {
-            k_karras<<<div_up(nInternal, 256), 256, 0, stream>>>(keysA, n, child, range, parent);
-        }
         BUILD_CHECK(cudaMemsetAsync(flag, 0, sizeof(int) * (size_t)nInternal, stream));
+        if (!rebuild) k_karras<<<div_up(nInternal, 256), 256, 0, stream>>>(keysA, n, child, range, parent);
     }
     else
     {
         int minus1 = -1;
         BUILD_CHECK(cudaMemcpyAsync(parent, &minus1, sizeof(int), cudaMemcpyHostToDevice, stream));
     }
+    if (rebuild)
     {
-        RefitArgs ra;
-        ra.n = n;
-        ra.vals = valsA;
-        ra.triBox = triBox;
-        ra.child = child;
-        ra.range = range;
-        ra.parent = parent;
-        ra.box = box;
-        ra.flag = flag;
-        ra.cost = dpCost;
-        ra.dec = dpDec;
-        ra.leafMax = std::max(1, std::min(3, leafMax));
+        top.order[0] = keysA;   // free after the sort
+        top.order[1] = keysB;
+        ra.vals = valsB;
+        BUILD_CHECK(sah_build_tree(n, triBox, cbounds, valsA, valsB, child, range, parent, top, ra, numSMs, stream));
+        std::swap(valsA, valsB);
+    }
+    else
+    {
         int perSM = 1;
         if (group) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_refit<true>, kRefitBlock, 0);
         else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_refit<false>, kRefitBlock, 0);

@@ -141,7 +141,9 @@ int build_bvh8(const float* dPos, int nv, const int* dIdx, int nt, Bvh8Device& o
 // carved by sah_tree_carve (order: two arrays of n words the caller supplies),
 // then sah_build_tree writes child / range / parent of the n - 1 internal nodes
 // (root 0, leaves ~p for position p of out) and out, the triangles of perm in
-// the tree's order.
+// the tree's order, and through refit (refit.cuh; its vals is out, its flags are
+// zero) the nodes' boxes and grouping costs.
+struct RefitArgs;
 struct TopTask;
 struct TopSplit;
 struct SahTreeBuffers
@@ -158,8 +160,8 @@ struct SahTreeBuffers
 };
 void sah_tree_carve(Carve& c, int n, SahTreeBuffers& B);
 cudaError_t sah_build_tree(int n, const float* triBox, const float* cbounds, const uint32_t* perm, uint32_t* out,
-                           int2* child, int2* range, int* parent, const SahTreeBuffers& B, int numSMs,
-                           cudaStream_t stream);
+                           int2* child, int2* range, int* parent, const SahTreeBuffers& B, const RefitArgs& refit,
+                           int numSMs, cudaStream_t stream);
 
 // Sort and scan primitives (sort_scan.cu).  radix_sort_pairs sorts (key, value)
 // pairs stably on key bits [0, bits); the sorted pairs end in keys/vals (the

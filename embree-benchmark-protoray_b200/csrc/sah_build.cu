@@ -15,6 +15,7 @@
 
 #include "prt_device.cuh"
 #include "prt_internal.h"
+#include "refit.cuh"
 
 namespace prt_b200 {
 
@@ -66,13 +67,19 @@ __device__ __forceinline__ float funord(uint32_t u)
 // The nodes of a depth are segments of the position range.  A warp walks its
 // axis' positions in windows of 32, with segmented shuffle scans inside a window
 // and a carry between windows, and windows whose segments are all single
-// triangles are skipped; the warps meet at five barriers per depth.  The latency
-// of the scans bounds it; element indices, segment ids and segment ends are
-// bytes, so a subtree takes 15 KB of shared memory and an SM holds 14 of them.
+// triangles are skipped; the warps meet at five barriers per depth.  The scans'
+// shuffles and minima bound it (issue slots 70%, shared-memory pipe 74% in use);
+// element indices, segment ids and segment ends are bytes, so a subtree takes 15
+// KB of shared memory, and an SM holds 12 (by registers).
 // Measured against one 256-thread block per subtree, whose scans stepped over
 // shared memory with two barriers a step: prt_build_accel of 1.38M triangles 3.25
 // -> 2.55 ms, 10.24M triangles 21.4 -> 15.7 (one warp for all three axes: 2.81 and
 // 17.2, and 82K triangles 12% slower).
+// The finished subtree's boxes and grouping costs (refit.cuh) follow, a depth at a
+// time from the last, with the triangles' boxes still in shared memory, and one
+// thread carries on above the root.  As a launch of its own, walking up from every
+// triangle with an atomic per node, that took 222 us for 1.38M triangles; here 107
+// (prt_build_accel 2.23 -> 2.10 ms, 10.24M 14.2 -> 13.4, 82K 0.69 -> 0.67).
 constexpr int kSahLeaves = 256;
 
 struct SahShared
@@ -87,6 +94,7 @@ struct SahShared
     // one), the segment of its right half; per axis: left marks before its start
     uint8_t segStart[kSahLeaves], segEnd[kSahLeaves], segNode[kSahLeaves], segRight[kSahLeaves];
     uint8_t segBase[3][kSahLeaves];
+    uint8_t depthFirst[kSahLeaves + 1];     // per depth: its first node, as in segNode
     int first, nseg, maxSeg;            // node index of pool entry 1; segments, and the largest, of this depth
 };
 
@@ -158,10 +166,10 @@ __device__ __forceinline__ void warp_sort256(uint32_t* key, uint32_t* idx, int l
 // One subtree per block: roots[i] is its root (an internal node whose range
 // holds 2..kSahLeaves triangles); its other internal nodes take new indices
 // from *nodeCounter.
-__global__ void __launch_bounds__(96) k_sah_subtrees(int n, const int* __restrict__ roots,
+__global__ void __launch_bounds__(96, 12) k_sah_subtrees(int n, const int* __restrict__ roots,
                                                    const int* __restrict__ numRoots, const float* __restrict__ triBox,
                                                    uint32_t* vals, int2* child, int2* range, int* parent,
-                                                   int* nodeCounter)
+                                                   int* nodeCounter, RefitArgs refit)
 {
     __shared__ SahShared S;
     const unsigned FULL = 0xffffffffu;
@@ -218,6 +226,7 @@ __global__ void __launch_bounds__(96) k_sah_subtrees(int n, const int* __restric
             __syncwarp();
         }
         int cur = 0, pool = 1;   // pool: warp 0
+        int depth = 0;
         // --- one depth of the subtree per pass ------------------------------------
         for (;;)
         {
@@ -408,6 +417,7 @@ __global__ void __launch_bounds__(96) k_sah_subtrees(int n, const int* __restric
                 {
                     S.maxSeg = newMax;
                     S.nseg = next;
+                    S.depthFirst[depth + 2] = (uint8_t)pool;   // 255 at most
                 }
             }
             __syncthreads();
@@ -417,6 +427,41 @@ __global__ void __launch_bounds__(96) k_sah_subtrees(int n, const int* __restric
                 if (S.best[s] != ~0ull && t > S.segEnd[s]) S.segOf[t] = S.segRight[s];
             }
             cur ^= 1;
+            ++depth;
+            __syncthreads();
+        }
+        // --- bounds and grouping costs, last depth first ----------------------------
+        const uint8_t* order = S.list[cur][0];
+        for (int t = threadIdx.x; t < ns; t += 96)
+        {
+            float* lb = refit.box + 6 * (size_t)((n - 1) + a + t);
+            const int e = order[t];
+#pragma unroll
+            for (int k = 0; k < 6; ++k) __stcg(lb + k, S.box[k][e]);
+        }
+        for (int d = depth - 1; d >= 0; --d)
+        {
+            const int end = d == 0 ? 1 : S.depthFirst[d + 1];
+            for (int i = (d == 0 ? 0 : (d == 1 ? 1 : S.depthFirst[d])) + (int)threadIdx.x; i < end; i += 96)
+            {
+                const int node = i == 0 ? u : S.first + i - 1;
+                const int2 ch = child[node], nr = range[node];
+                float b[2][6];
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                {
+                    const int ref = h == 0 ? ch.x : ch.y;
+                    if (ref >= 0) load_box(refit, ref, b[h]);
+                    else
+                    {
+                        const int e = order[~ref - a];
+#pragma unroll
+                        for (int k = 0; k < 6; ++k) b[h][k] = S.box[k][e];
+                    }
+                }
+                if (refit.cost) refit_node<true>(refit, node, ch, nr.y - nr.x + 1, b[0], b[1]);
+                else refit_node<false>(refit, node, ch, nr.y - nr.x + 1, b[0], b[1]);
+            }
             __syncthreads();
         }
         // the triangles in their new order
@@ -433,6 +478,32 @@ __global__ void __launch_bounds__(96) k_sah_subtrees(int n, const int* __restric
         {
             const int t = threadIdx.x + 96 * k;
             if (t < ns) vals[a + t] = tri[k];
+        }
+        // up from the subtree's root: the second arrival at a node finishes it; a
+        // child that is a single triangle does not arrive
+        if (threadIdx.x == 0)
+        {
+            for (int node = parent[u]; node >= 0; node = parent[node])
+            {
+                const int2 ch = child[node], nr = range[node];
+                const int single = ch.x < 0 ? ch.x : ch.y;
+                float b[2][6];
+                if (single < 0)
+                {
+                    const float* tb = triBox + 6 * (size_t)refit.vals[~single];
+                    float* lb = refit.box + 6 * (size_t)((n - 1) + ~single);
+#pragma unroll
+                    for (int k = 0; k < 6; ++k) __stcg(lb + k, tb[k]);
+                }
+                else if (arrive(refit.flag + node) == 0)
+                {
+                    break;
+                }
+                load_box(refit, ch.x, b[0]);
+                load_box(refit, ch.y, b[1]);
+                if (refit.cost) refit_node<true>(refit, node, ch, nr.y - nr.x + 1, b[0], b[1]);
+                else refit_node<false>(refit, node, ch, nr.y - nr.x + 1, b[0], b[1]);
+            }
         }
         __syncthreads();
     }
@@ -1098,8 +1169,8 @@ void sah_tree_carve(Carve& c, int n, SahTreeBuffers& B)
 // then k_sah_subtrees for those.  perm: the triangles in their starting order;
 // out: in the tree's order.
 cudaError_t sah_build_tree(int n, const float* triBox, const float* cbounds, const uint32_t* perm, uint32_t* out,
-                           int2* child, int2* range, int* parent, const SahTreeBuffers& B, int numSMs,
-                           cudaStream_t stream)
+                           int2* child, int2* range, int* parent, const SahTreeBuffers& B, const RefitArgs& refit,
+                           int numSMs, cudaStream_t stream)
 {
     k_top_root<<<1, 256, 0, stream>>>(cbounds, n, B.task[0], B.chunks[0], B.bins[0], B.small, B.counters, range, parent);
     cudaError_t e = cudaGetLastError();
@@ -1164,7 +1235,7 @@ cudaError_t sah_build_tree(int n, const float* triBox, const float* cbounds, con
     int perSM = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_sah_subtrees, 96, 0);
     k_sah_subtrees<<<std::max(1, perSM) * numSMs, 96, 0, stream>>>(n, B.small, B.counters, triBox, out, child, range,
-                                                                parent, B.counters + 1);
+                                                                parent, B.counters + 1, refit);
     return cudaGetLastError();
 }
 
