@@ -1,0 +1,44 @@
+"""A wave takes all its passes of a pixel in turn, and camera rays of a pixel that
+end together are added as one: a frame of several passes in one call equals the
+sum of one-pass calls to the rounding of a pixel's sum, for passes that do and do
+not divide a warp and pixels that do not fill a tile."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("packets", [0, 1, 2])
+@pytest.mark.parametrize("spp", [2, 3, 32, 33])
+@pytest.mark.parametrize("size,depth,integrator,albedo",
+                         [((37, 23), 3, "diffuse", False), ((61, 9), 0, "diffuse", True),
+                          ((64, 40), 2, "diffuse", True), ((37, 23), 2, "diffuse2", True)])
+def test_passes_in_one_call(small, packets, spp, size, depth, integrator, albedo):
+    import prt
+    import scenes
+    mesh, view = small
+    w, h = size
+    c = prt.Context(0)
+    c.load_mesh(mesh.indices, mesh.positions)
+    c.build()
+    c.set_integrator(integrator)
+    if albedo:
+        c.set_albedo(scenes.albedo_for(mesh))
+    c.init_frame(w, h)
+    c.set_view(view, w, h)
+    c.set_tune(128, 0, 0, 2, packets)
+    rays = 0
+    for _ in range(spp):
+        rays += c.render(1, depth)["ray"]
+    ref = c.read_accum()
+    c.clear()
+    c.set_pass(0)
+    st = c.render(spp, depth)
+    img = c.read_accum()
+    assert st["ray"] == rays
+    np.testing.assert_array_equal(img[..., 3], ref[..., 3])
+    # both sums have at most two terms per ray, of at most 1 each and 2 spp in all
+    terms = 2 * spp * (depth + 1)
+    np.testing.assert_allclose(img[..., :3], ref[..., :3], rtol=0, atol=2.0 ** -23 * terms * 2 * spp)
+    c.close()
