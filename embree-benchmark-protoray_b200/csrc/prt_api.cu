@@ -323,7 +323,16 @@ struct WavePlan
     int passes;          // per wave
     int waves, chains;
     bool whole;          // each wave is one launch without queues (whole_paths)
+    int packet;          // primary rays of a wave with queues, as LaunchCfg::packet
 };
+
+// Without a setting, large waves of many passes take packets, which then span few
+// pixels; smaller ones end in the longest packet.  A 1080p frame of 16 passes (two
+// waves of 16.6M paths), per lane -> packets: 82K triangles 6.30 -> 5.87 ms, 1.38M
+// 23.2 -> 21.5, 10.24M 16.7 -> 15.2, 2M in 2000 spheres 10.1 -> 9.9.  At 7.4M paths the
+// last is 5% slower with packets, at 1.6M 40%.
+constexpr long long kPacketPaths = 81920;   // per SM
+constexpr int kPacketPasses = 8;
 
 WavePlan plan_waves(const prt_ctx* ctx, int spp)
 {
@@ -332,6 +341,8 @@ WavePlan plan_waves(const prt_ctx* ctx, int spp)
     p.perPass = (long long)((ctx->W + 7) / 8) * ((ctx->H + 7) / 8) * 64;
     p.passes = passes_per_wave(ctx, spp);
     p.whole = whole_paths(p.passes * p.perPass, ctx->bvh.leafMax, ctx->cfg, nee, ctx->numSMs);
+    p.packet = ctx->cfg.packet;
+    if (!p.packet && p.passes >= kPacketPasses && p.passes * p.perPass >= kPacketPaths * ctx->numSMs) p.packet = 1;
     // without queues nothing but the item counter bounds a wave
     if (nee && ctx->cfg.pathsPerWave == 0) p.passes = (int)std::max<long long>(1, std::min<long long>(spp, kMaxItems / p.perPass));
     p.waves = (spp + p.passes - 1) / p.passes;
@@ -346,6 +357,8 @@ int record_render(prt_ctx* ctx, const WavePlan& plan, int spp, int maxDepth, int
     const int W = ctx->W, H = ctx->H;
     const int tilesX = (W + 7) / 8, tilesY = (H + 7) / 8;
     const int passesPerWave = plan.passes, waves = plan.waves, chains = plan.chains;
+    LaunchCfg cfg = ctx->cfg;
+    cfg.packet = plan.packet;
     const bool albedo = ctx->dAlbedo != nullptr;
     const bool nee = ctx->integrator == PRT_INTEGRATOR_DIFFUSE2;
     if (!plan.whole && (ctx->queueCap < passesPerWave * plan.perPass || ctx->queueChains < chains ||
@@ -387,19 +400,19 @@ int record_render(prt_ctx* ctx, const WavePlan& plan, int spp, int maxDepth, int
         a.thrConst = const_throughput(0);
         if (plan.whole)
         {
-            launches += launch_whole(a, albedo, nee, ctx->cfg, ctx->numSMs, s);
+            launches += launch_whole(a, albedo, nee, cfg, ctx->numSMs, s);
             continue;
         }
         // depth 0 fills the chain's queue, one launch carries its paths to their ends
         a.qout = ctx->q[c][0];
         a.thrOut = albedo ? ctx->thr[c][0] : nullptr;
-        launches += launch_bounce(a, 0, ctx->cfg, ctx->numSMs, s);
+        launches += launch_bounce(a, 0, cfg, ctx->numSMs, s);
         if (maxDepth > 0)
         {
             a.qin = a.qout;
             a.thrIn = a.thrOut;
             a.thrConst = const_throughput(1);
-            launches += launch_paths(a, ctx->cfg, ctx->numSMs, s);
+            launches += launch_paths(a, cfg, ctx->numSMs, s);
         }
     }
     if (chains > 1)

@@ -114,7 +114,8 @@ typedef struct {
                              e.g. 1080p views; slower for coarse ones); 2: warp packets
                              traversed with interval bounds of the packet (one child test per
                              node; faster still where a packet's rays stay close, slower for
-                             long, often missing rays); 0: per-lane (default) */
+                             long, often missing rays); 0 (default): per-lane, and as 1 in
+                             large waves of many passes */
     double mray;          /* throughput measured for the winner */
 } prt_tune;
 

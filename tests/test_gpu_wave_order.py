@@ -42,3 +42,31 @@ def test_passes_in_one_call(small, packets, spp, size, depth, integrator, albedo
     terms = 2 * spp * (depth + 1)
     np.testing.assert_allclose(img[..., :3], ref[..., :3], rtol=0, atol=2.0 ** -23 * terms * 2 * spp)
     c.close()
+
+
+@pytest.mark.parametrize("spp", [7, 8, 9])
+def test_packets_of_large_waves(small, spp):
+    """Large waves of eight passes and more take packets where no setting says
+    otherwise: the same rays and sums as a launch per bounce in small waves."""
+    import prt
+    mesh, view = small
+    w, h = 1601, 1001   # 12.9M paths in eight passes
+    c = prt.Context(0)
+    c.load_mesh(mesh.indices, mesh.positions)
+    c.build()
+    c.init_frame(w, h)
+    c.set_view(view, w, h)
+    c.set_tune(128, 0, 1 << 24, 2, 0)
+    st = c.render(spp, 2, accumulate=False)
+    img = c.read_accum()
+    assert c.get_tune()["primaryPackets"] == 0
+    c.set_pass(0)
+    c.clear()
+    c.set_tune(128, 0, 2 * 1608 * 1008, 2, 0)
+    _, rays = c.render_profile(spp, 2)
+    ref = c.read_accum()
+    assert st["ray"] == rays.sum()
+    np.testing.assert_array_equal(img[..., 3], ref[..., 3])
+    # up to spp terms of at most 1 on each side
+    np.testing.assert_allclose(img[..., :3], ref[..., :3], rtol=0, atol=2.0 ** -23 * spp * spp)
+    c.close()
