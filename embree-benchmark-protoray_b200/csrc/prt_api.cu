@@ -331,8 +331,14 @@ struct WavePlan
 // waves of 16.6M paths), per lane -> packets: 82K triangles 6.30 -> 5.87 ms, 1.38M
 // 23.2 -> 21.5, 10.24M 16.7 -> 15.2, 2M in 2000 spheres 10.1 -> 9.9.  At 7.4M paths the
 // last is 5% slower with packets, at 1.6M 40%.
+// Batches likewise, by their passes on average: 32 requests (156M paths) 28.0 -> 24.8 ms.
 constexpr long long kPacketPaths = 81920;   // per SM
 constexpr int kPacketPasses = 8;
+
+bool default_packets(const prt_ctx* ctx, long long paths, long long pixels)
+{
+    return paths >= kPacketPaths * ctx->numSMs && paths >= kPacketPasses * pixels;
+}
 
 WavePlan plan_waves(const prt_ctx* ctx, int spp)
 {
@@ -342,7 +348,7 @@ WavePlan plan_waves(const prt_ctx* ctx, int spp)
     p.passes = passes_per_wave(ctx, spp);
     p.whole = whole_paths(p.passes * p.perPass, ctx->bvh.leafMax, ctx->cfg, nee, ctx->numSMs);
     p.packet = ctx->cfg.packet;
-    if (!p.packet && p.passes >= kPacketPasses && p.passes * p.perPass >= kPacketPaths * ctx->numSMs) p.packet = 1;
+    if (!p.packet && default_packets(ctx, p.passes * p.perPass, p.perPass)) p.packet = 1;
     // without queues nothing but the item counter bounds a wave
     if (nee && ctx->cfg.pathsPerWave == 0) p.passes = (int)std::max<long long>(1, std::min<long long>(spp, kMaxItems / p.perPass));
     p.waves = (spp + p.passes - 1) / p.passes;
@@ -1324,7 +1330,7 @@ int prt_render_batch(prt_ctx* ctx, const prt_request* reqs, int n, prt_render_st
     CK(cudaSetDevice(ctx->device));
     std::vector<BatchReq> table((size_t)n);
     std::vector<float4*> tmp((size_t)n, nullptr);
-    long long total = 0;
+    long long total = 0, items = 0;   // paths; pixels of one pass each
     int maxDepth = 0;
     int leaf1 = 1, leafOne = 1;
     std::ostringstream key;
@@ -1346,6 +1352,7 @@ int prt_render_batch(prt_ctx* ctx, const prt_request* reqs, int n, prt_render_st
         b.spp = q.spp;
         b.maxDepth = q.maxDepth;
         b.pathBegin = total;
+        items += (long long)b.tilesX * b.tilesY * 64;
         total += (long long)b.tilesX * b.tilesY * 64 * q.spp;
         if (!b.scene.deferTris) leaf1 = 0;
         if (b.scene.leafTris != 1) leafOne = 0;
@@ -1389,6 +1396,8 @@ int prt_render_batch(prt_ctx* ctx, const prt_request* reqs, int n, prt_render_st
                            ctx->stream));
     long long ppw = ctx->cfg.pathsPerWave > 0 ? ctx->cfg.pathsPerWave : default_paths_per_wave(ctx);
     const long long waves = total > 0 ? (total + ppw - 1) / ppw : 0;
+    LaunchCfg cfg = ctx->cfg;
+    if (!cfg.packet && default_packets(ctx, total, items)) cfg.packet = 1;
     // waves are dealt round-robin to concurrent chains, as record_render does,
     // so the tail of one wave's bounce launch overlaps another wave's work
     const int chains = (int)std::max<long long>(1, std::min<long long>(chains_for(ctx), waves));
@@ -1423,7 +1432,7 @@ int prt_render_batch(prt_ctx* ctx, const prt_request* reqs, int n, prt_render_st
             CK(clear_chain(ctx, c, s));
             a.qin = nullptr;
             a.qout = ctx->q[c][0];
-            launches += launch_batch_first(a, ctx->cfg, ctx->numSMs, s);
+            launches += launch_batch_first(a, cfg, ctx->numSMs, s);
             if (maxDepth > 0)
             {
                 a.qin = a.qout;

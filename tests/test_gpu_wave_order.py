@@ -70,3 +70,32 @@ def test_packets_of_large_waves(small, spp):
     # up to spp terms of at most 1 on each side
     np.testing.assert_allclose(img[..., :3], ref[..., :3], rtol=0, atol=2.0 ** -23 * spp * spp)
     c.close()
+
+
+def test_packets_of_large_batches(small):
+    """A batch above the size that takes packets by default, in two waves that part
+    inside a request, equals the requests one by one."""
+    import prt
+    mesh, view = small
+    main = prt.Context(0)
+    scene = prt.Context(0)
+    scene.load_mesh(mesh.indices, mesh.positions)
+    scene.build()
+    shapes = [(333, 257, 21), (1001, 701, 16), (97, 5, 1)]   # 13.1M paths
+    reqs = [dict(scene=scene, camera=prt.camera_from_view(view, w, h), width=w, height=h, spp=s, maxDepth=2,
+                 accum=np.zeros((h, w, 4), np.float32)) for w, h, s in shapes]
+    main.set_tune(128, 0, 1 << 23, 2, 0)
+    st = main.render_batch(reqs)
+    rays = 0
+    for q in reqs:
+        scene.init_frame(q["width"], q["height"])
+        scene.set_view(view, q["width"], q["height"])
+        scene.set_pass(0)
+        rays += scene.render(q["spp"], 2, accumulate=False)["ray"]
+        ref = scene.read_accum()
+        np.testing.assert_array_equal(q["accum"][..., 3], ref[..., 3])
+        # up to spp terms of at most 1 on each side
+        np.testing.assert_allclose(q["accum"][..., :3], ref[..., :3], rtol=0, atol=2.0 ** -23 * q["spp"] ** 2)
+    assert st["ray"] == rays
+    scene.close()
+    main.close()
