@@ -5,8 +5,9 @@
 // -> shadeRaysKernel -> cudaMemcpy(count) } per bounce.  Here a wave takes two
 // persistent kernels: the first generates, traces and shades the primary rays
 // and queues the paths that go on, the second (k_paths) carries those paths
-// to their ends; small waves and next-event estimation take one.  Queue sizes stay on the device, so a whole render is launched
-// without host synchronisation (and is captured as a CUDA graph by the API).
+// to their ends; small waves and next-event estimation take one.  Queue sizes
+// stay on the device, so a whole render is launched without host synchronisation
+// (and, of several waves, is captured as a CUDA graph by the API).
 // k_bounce and k_bounce_nee with kFirst = false do one bounce of all paths
 // per launch, for prt_render_profile's times per depth.
 #include <algorithm>
@@ -176,12 +177,13 @@ constexpr int kRefillMin = PRT_REFILL_MIN;
 #ifndef PRT_BOUNCE_MIN_BLOCKS
 #define PRT_BOUNCE_MIN_BLOCKS 8
 #endif
-// The kernels that carry more per lane (a batch's request, shadow rays,
-// gradients, barycentrics) spill at 64 registers and are faster with 72 and 7
-// blocks: 32-request batch 30.8 -> 29.9 ms, diffuse2 1080p 4 passes 11.08 -> 10.93,
-// 4M closest-hit queries 1.280 -> 1.265, adjoint 512x512 16 passes 1.95 -> 1.93.  The
-// others lose 0.2% (any hit 1.3%, packets 3.5%); 6 blocks lose 1-3%, 9 blocks (56
-// registers) 5%.
+// The kernels that carry more per lane (whole paths, a batch's request, shadow
+// rays, gradients, barycentrics, the first bounce) spill at 64 registers and are
+// faster with 72 and 7 blocks: 32-request batch 30.8 -> 29.9 ms, diffuse2 1080p 4
+// passes 11.08 -> 10.93, 4M closest-hit queries 1.280 -> 1.265, adjoint 512x512 16
+// passes 1.95 -> 1.93, the same with albedo forward 1.48 -> 1.44, 1080p 1 pass 1.83 ->
+// 1.79 (32 passes 38.6 either way).  The others lose (bounce by bounce 0.7%, any hit
+// 1.3%, packets 2%); 6 blocks lose 1-3%, 9 blocks (56 registers) 5%.
 constexpr int kWideBlocks = 7;
 
 // Words of shared memory per lane of the per-bounce kernels.
@@ -197,7 +199,7 @@ constexpr int bounce_words(bool first) { return kShearWords + (first || !PRT_REL
 // atomic per warp, and fetch fresh rays, so a few long rays do not idle the
 // rest of the warp.
 template <bool kFirst, bool kAlbedo>
-__global__ void __launch_bounds__(128, PRT_BOUNCE_MIN_BLOCKS) k_bounce(WaveArgs a, int depth)
+__global__ void __launch_bounds__(128, kFirst ? kWideBlocks : PRT_BOUNCE_MIN_BLOCKS) k_bounce(WaveArgs a, int depth)
 {
     extern __shared__ uint2 s_stack[];
     TravStack st;
@@ -472,7 +474,7 @@ __device__ __forceinline__ int stop_idle(unsigned act)
 }
 
 template <class Args, bool kBatch, bool kAlbedo, bool kPrimary>
-__global__ void __launch_bounds__(128, kBatch || kPrimary ? kWideBlocks : PRT_BOUNCE_MIN_BLOCKS) k_paths(Args a)
+__global__ void __launch_bounds__(128, kWideBlocks) k_paths(Args a)
 {
     static_assert(!(kBatch && kPrimary), "a batch's primary rays have their own kernels");
     extern __shared__ uint2 s_stack[];
@@ -623,20 +625,21 @@ __global__ void __launch_bounds__(128, kBatch || kPrimary ? kWideBlocks : PRT_BO
 }
 
 // Primary rays as warp packets (trees with one-triangle leaves).  A warp takes
-// 32 consecutive wave items, half of an 8x8 tile (an 8x4 pixel block of one
-// pass), and traverses the tree once for all of them: every lane tests its own
+// 32 consecutive wave items, the passes of few pixels (of one pass, half of an 8x8
+// tile), and traverses the tree once for all of them: every lane tests its own
 // ray against the node all lanes are at (one broadcast load of the node), the
 // node's child hits are OR-ed over the warp, and the children are visited in
 // the order of one ray octant shared by the warp, from a stack in shared
 // memory that the warp shares.  Each lane culls with its own closest hit and
 // tests the triangles of the leaves its own ray hits, so its result is its
 // closest hit, the same as per-lane traversal gives (exact ties go to the
-// lower primitive id either way).  Camera rays of a small pixel block visit
-// nearly the same nodes when pixels are fine, so the lanes stay busy together
-// where the per-lane traversal of k_bounce runs 20 of 32 lanes per instruction
-// at this depth; with coarse pixels the union of the rays' nodes grows and the
-// packet loses (measured: +1.8% at 1920x1080, -26% at 480x272 on the terrain),
-// so it is a launch option (LaunchCfg::packet) the autotuner chooses.
+// lower primitive id either way).  Camera rays of few pixels visit nearly the same
+// nodes, so the lanes stay busy together where the per-lane traversal of k_bounce
+// runs 20 of 32 lanes per instruction at this depth; with one pass and coarse
+// pixels the union of the rays' nodes grows and the packet loses, and so do small
+// waves, which end in the longest packet.  LaunchCfg::packet asks for packets (the
+// autotuner tries them); without it plan_waves takes them for large waves of many
+// passes.
 #ifndef PRT_PACKET_PRIMARY
 #define PRT_PACKET_PRIMARY 1
 #endif
