@@ -907,7 +907,7 @@ int build_bvh8_tree(const float* dPos, int nv, const int* dIdx, int nt, Bvh8Devi
         const size_t nodeBytes = (sizeof(Bvh8Node) * (size_t)nodeCapacity + 255) & ~(size_t)255;
         // a rebuild writes into the block of the last build if it fits: freeing
         // and allocating hundreds of MB costs up to milliseconds and a device
-        // synchronisation
+        // synchronisation (the caller has made `stream` wait for what reads it)
         const size_t need = nodeBytes + sizeof(TriRec) * (size_t)n;
         if (!out.block || out.bytes < need || out.bytes > 2 * need)
         {

@@ -45,6 +45,66 @@ constexpr int kDefaultLeafMax = PRT_LEAF_MAX;
 constexpr long long kMaxItems = 1LL << 30;
 constexpr int kCounterStride = 64 + 2;   // counters per chain: one per bounce depth (<= 64) + 2
 
+// Queries in flight on callers' streams: they read the tree, whose block a
+// rebuild writes again.  note() after a query's launch remembers it by an event of
+// its stream, order() makes a stream wait for all of them.  Work that no event
+// tells of (a captured query runs whenever its graph is launched) leaves it to the
+// caller to wait for the whole device.
+struct CallerQueries
+{
+    static constexpr int kStreams = 32;
+    cudaEvent_t last[kStreams] = {};
+    unsigned long long id[kStreams] = {};   // streams (their handles may be reused)
+    int n = 0;
+    bool unknown = false;
+
+    void note(cudaStream_t s)
+    {
+        if (!unknown && !record(s))
+        {
+            cudaGetLastError();
+            unknown = true;
+        }
+    }
+    // false: not all of them are known
+    bool order(cudaStream_t s)
+    {
+        bool ok = !unknown;
+        for (int i = 0; i < n && ok; ++i) ok = cudaStreamWaitEvent(s, last[i], 0) == cudaSuccess;
+        if (!ok) cudaGetLastError();
+        n = 0;
+        unknown = false;
+        return ok;
+    }
+    void release()
+    {
+        for (cudaEvent_t& e : last)
+        {
+            if (e) cudaEventDestroy(e);
+            e = nullptr;
+        }
+        n = 0;
+    }
+
+private:
+    bool record(cudaStream_t s)
+    {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        unsigned long long sid = 0;
+        if (cudaStreamIsCapturing(s, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone ||
+            cudaStreamGetId(s, &sid) != cudaSuccess)
+            return false;
+        int k = 0;
+        while (k < n && id[k] != sid) ++k;
+        if (k == kStreams) return false;
+        if (!last[k] && cudaEventCreateWithFlags(&last[k], cudaEventDisableTiming) != cudaSuccess) return false;
+        if (cudaEventRecord(last[k], s) != cudaSuccess) return false;
+        id[k] = sid;
+        n = std::max(n, k + 1);
+        return true;
+    }
+};
+
 struct prt_ctx
 {
     int device = 0;
@@ -102,6 +162,7 @@ struct prt_ctx
     static constexpr int kIsectSlots = 64;
     int* dIsect = nullptr;
     int isectNext = 0;
+    CallerQueries queries;
 
     // query scratch
     RayRec* dRay = nullptr;
@@ -767,6 +828,7 @@ prt_ctx::~prt_ctx()
     }
     if (forkEv) cudaEventDestroy(forkEv);
     cudaFree(dIsect);
+    queries.release();
     cudaFree(dRay);
     cudaFree(dHit);
     cudaFree(dPNg);
@@ -942,6 +1004,9 @@ int prt_build_accel(prt_ctx* ctx, prt_build_stats* stats)
     CK(cudaSetDevice(ctx->device));
     clear_graphs(ctx);
     ctx->built = false;
+    // queries on callers' streams may still read the block that the build writes
+    // again; freeing it waits for the device
+    if (!ctx->queries.order(ctx->stream)) ctx->bvh.release();
     BuildInfo info;
     std::string err;
     int st = build_bvh8(ctx->dPos, ctx->nv, ctx->dIdx, ctx->nt, ctx->bvh, ctx->stream, err, &info, ctx->leafMax,
@@ -1230,7 +1295,8 @@ int prt_intersect(prt_ctx* ctx, const prt_ray* rays, prt_hit* hits, int n, void*
     if (st != PRT_OK) return st;
     ctx->launches += launch_intersect(scene_dev(ctx), (const RayRec*)rays, (HitRec*)hits, n, false, nullptr, fetch, ctx->numSMs, s);
     CK(cudaGetLastError());
-    if (!stream) CK(cudaStreamSynchronize(ctx->stream));
+    if (stream) ctx->queries.note(s);
+    else CK(cudaStreamSynchronize(ctx->stream));
     return PRT_OK;
 }
 
@@ -1262,7 +1328,8 @@ int prt_occluded(prt_ctx* ctx, const prt_ray* rays, float* out, int n, void* str
     if (st != PRT_OK) return st;
     ctx->launches += launch_intersect(scene_dev(ctx), (const RayRec*)rays, nullptr, n, true, out, fetch, ctx->numSMs, s);
     CK(cudaGetLastError());
-    if (!stream) CK(cudaStreamSynchronize(ctx->stream));
+    if (stream) ctx->queries.note(s);
+    else CK(cudaStreamSynchronize(ctx->stream));
     return PRT_OK;
 }
 
