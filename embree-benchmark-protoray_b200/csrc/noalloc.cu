@@ -69,7 +69,6 @@ cudaError_t current_context_id(unsigned long long* id)
 namespace {
 
 constexpr long long kNoAllocMaxPaths = 1LL << 19;
-constexpr long long kNoAllocMaxItems = 1LL << 30;   // of one launch without a queue: its 32-bit counter
 constexpr int kNoAllocCounters = 64 + 2;   // one slot per bounce depth (max depth 64) + 2
 
 struct NoAllocScratch
@@ -176,7 +175,7 @@ extern "C" int prt_render_noalloc(prt_ctx* ctx, const prt_camera* cam, int width
         maxDepth > kNoAllocCounters - 2)
         return ctx_fail(ctx, PRT_EINVAL, "prt_render_noalloc: invalid argument");
     const int tilesX = (width + 7) / 8, tilesY = (height + 7) / 8;
-    const long long perPass = (long long)tilesX * tilesY * 64;
+    const long long perPass = frame_items(width, height);
     if (perPass > kNoAllocMaxPaths)
         return ctx_fail(ctx, PRT_EINVAL,
                         "prt_render_noalloc: frame too large (at most 524288 pixels after rounding to 8x8 tiles)");
@@ -193,7 +192,7 @@ extern "C" int prt_render_noalloc(prt_ctx* ctx, const prt_camera* cam, int width
 
     // packets need the queue; otherwise waves without one are as large as they come
     const bool whole = nee || !packet_primaries(scene.leafTris, cfg);
-    const int passesPerWave = (int)std::max<long long>(1, (whole ? kNoAllocMaxItems : kNoAllocMaxPaths) / perPass);
+    const int passesPerWave = wave_passes(whole ? kMaxItems : kNoAllocMaxPaths, perPass, std::max(spp, 1));
     WaveArgs a;
     a.scene = scene;
     a.cam.origin = make_float3(cam->origin[0], cam->origin[1], cam->origin[2]);

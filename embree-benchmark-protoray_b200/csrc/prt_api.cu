@@ -40,9 +40,6 @@ constexpr int kMaxChains = 4;
 #define PRT_LEAF_MAX 1
 #endif
 constexpr int kDefaultLeafMax = PRT_LEAF_MAX;
-// Items (pixels of all passes, rounded up to tiles) of one launch: its 32-bit
-// counter also takes the requests of every lane past the end.
-constexpr long long kMaxItems = 1LL << 30;
 constexpr int kCounterStride = 64 + 2;   // counters per chain: one per bounce depth (<= 64) + 2
 
 // Queries in flight on callers' streams: they read the tree, whose block a
@@ -372,9 +369,7 @@ int chains_for(const prt_ctx* ctx) { return std::max(1, std::min(kMaxChains, ctx
 
 int passes_per_wave(const prt_ctx* ctx, int spp)
 {
-    const long long perPass = (long long)((ctx->W + 7) / 8) * ((ctx->H + 7) / 8) * 64;
-    long long ppw = ctx->cfg.pathsPerWave > 0 ? ctx->cfg.pathsPerWave : default_paths_per_wave(ctx);
-    return (int)std::max<long long>(1, std::min<long long>(spp, ppw / perPass));
+    return wave_passes(wave_paths(ctx->cfg.pathsPerWave, default_paths_per_wave(ctx)), frame_items(ctx->W, ctx->H), spp);
 }
 
 // The waves of one render call.
@@ -405,14 +400,14 @@ WavePlan plan_waves(const prt_ctx* ctx, int spp)
 {
     WavePlan p;
     const bool nee = ctx->integrator == PRT_INTEGRATOR_DIFFUSE2;
-    p.perPass = (long long)((ctx->W + 7) / 8) * ((ctx->H + 7) / 8) * 64;
+    p.perPass = frame_items(ctx->W, ctx->H);
     p.passes = passes_per_wave(ctx, spp);
     p.whole = whole_paths(p.passes * p.perPass, ctx->bvh.leafMax, ctx->cfg, nee, ctx->numSMs);
     p.packet = ctx->cfg.packet;
     if (!p.packet && default_packets(ctx, p.passes * p.perPass, p.perPass)) p.packet = 1;
     // without queues nothing but the item counter bounds a wave
-    if (nee && ctx->cfg.pathsPerWave == 0) p.passes = (int)std::max<long long>(1, std::min<long long>(spp, kMaxItems / p.perPass));
-    p.waves = (spp + p.passes - 1) / p.passes;
+    if (nee && ctx->cfg.pathsPerWave == 0) p.passes = wave_passes(kMaxItems, p.perPass, spp);
+    p.waves = wave_count(spp, p.passes);
     p.chains = std::max(1, std::min(chains_for(ctx), p.waves));
     return p;
 }
@@ -549,6 +544,12 @@ int check_ready(prt_ctx* ctx, bool needFrame)
     if (!ctx->built) return fail(ctx, PRT_ESTATE, "acceleration structure not built (prt_build_accel)");
     if (needFrame && !ctx->dAccum) return fail(ctx, PRT_ESTATE, "frame not initialised (prt_init_frame)");
     if (needFrame && !ctx->haveCamera) return fail(ctx, PRT_ESTATE, "camera not set (prt_set_camera)");
+    return PRT_OK;
+}
+
+int check_frame_items(prt_ctx* ctx)
+{
+    if (frame_items(ctx->W, ctx->H) > kMaxFrameItems) return fail(ctx, PRT_EINVAL, "frame too long for its width");
     return PRT_OK;
 }
 
@@ -1150,6 +1151,8 @@ int prt_render(prt_ctx* ctx, int spp, int maxDepth, int accumulate, prt_render_s
     int st = check_ready(ctx, true);
     if (st != PRT_OK) return st;
     if (spp < 0 || maxDepth < 0 || maxDepth > kMaxDepthCap) return fail(ctx, PRT_EINVAL, "invalid spp or maxDepth");
+    if (spp > 0) st = check_frame_items(ctx);
+    if (st != PRT_OK) return st;
     CK(cudaSetDevice(ctx->device));
     WavePlan plan{};
     if (spp > 0)
@@ -1195,10 +1198,12 @@ int prt_render_profile(prt_ctx* ctx, int spp, int maxDepth, double* msPerDepth, 
     if (st != PRT_OK) return st;
     if (spp <= 0 || maxDepth < 0 || maxDepth > kMaxDepthCap || !msPerDepth || !raysPerDepth)
         return fail(ctx, PRT_EINVAL, "invalid spp, maxDepth or output arrays");
+    st = check_frame_items(ctx);
+    if (st != PRT_OK) return st;
     CK(cudaSetDevice(ctx->device));
     const int W = ctx->W, H = ctx->H;
     const int tilesX = (W + 7) / 8, tilesY = (H + 7) / 8;
-    const long long perPass = (long long)tilesX * tilesY * 64;
+    const long long perPass = frame_items(W, H);
     const int ppw = passes_per_wave(ctx, spp);
     const bool albedo = ctx->dAlbedo != nullptr;
     const bool nee = ctx->integrator == PRT_INTEGRATOR_DIFFUSE2;
@@ -1306,6 +1311,8 @@ int prt_primary_rays(prt_ctx* ctx, int pass, prt_ray* rays, void* stream)
     if (st != PRT_OK) return st;
     if (pass < 0 || !rays) return fail(ctx, PRT_EINVAL, "invalid pass or ray buffer");
     if (!is_device_ptr(rays)) return fail(ctx, PRT_EINVAL, "prt_primary_rays takes a device pointer");
+    st = check_frame_items(ctx);
+    if (st != PRT_OK) return st;
     CK(cudaSetDevice(ctx->device));
     cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
     ctx->launches += launch_primary_rays(camera_dev(ctx->cam, ctx->W, ctx->H), pass, (RayRec*)rays, s);
@@ -1461,7 +1468,7 @@ int prt_render_batch(prt_ctx* ctx, const prt_request* reqs, int n, prt_render_st
     for (int r = 0; r < n; ++r)
         CK(cudaMemsetAsync(table[(size_t)r].accum, 0, sizeof(float4) * (size_t)reqs[r].width * reqs[r].height,
                            ctx->stream));
-    long long ppw = ctx->cfg.pathsPerWave > 0 ? ctx->cfg.pathsPerWave : default_paths_per_wave(ctx);
+    const long long ppw = wave_paths(ctx->cfg.pathsPerWave, default_paths_per_wave(ctx));
     const long long waves = total > 0 ? (total + ppw - 1) / ppw : 0;
     LaunchCfg cfg = ctx->cfg;
     if (!cfg.packet && default_packets(ctx, total, items)) cfg.packet = 1;
@@ -1612,7 +1619,7 @@ int prt_autotune(prt_ctx* ctx, int spp, int maxDepth, prt_tune* best)
     if (spp <= 0 || maxDepth < 0 || maxDepth > kMaxDepthCap)
         return fail(ctx, PRT_EINVAL, "autotune needs spp > 0 and 0 <= maxDepth <= 64");
     CK(cudaSetDevice(ctx->device));
-    const long long perPass = (long long)((ctx->W + 7) / 8) * ((ctx->H + 7) / 8) * 64;
+    const long long perPass = frame_items(ctx->W, ctx->H);
     const LaunchCfg saved = ctx->cfg;
 
     // Throughput of one configuration: the best of three timed renders of the

@@ -11,6 +11,7 @@
 #include "../../include/prt_b200.h"
 #include "prt_device.cuh"
 #include "soup_view.h"
+#include "wave_plan.h"
 
 namespace prt_b200 {
 
