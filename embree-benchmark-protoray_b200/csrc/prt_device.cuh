@@ -790,6 +790,18 @@ __device__ __forceinline__ unsigned long long hit_key(float t, int prim)
     return ((unsigned long long)__float_as_uint(t) << 32) | (uint32_t)prim;
 }
 
+// The same for any t: negative ones order below positive ones, by value.
+__device__ __forceinline__ unsigned long long signed_hit_key(float t, int prim)
+{
+    const uint32_t b = __float_as_uint(t);
+    return ((unsigned long long)((b & 0x80000000u) ? ~b : (b | 0x80000000u)) << 32) | (uint32_t)prim;
+}
+__device__ __forceinline__ float signed_key_t(unsigned long long key)
+{
+    const uint32_t b = (uint32_t)(key >> 32);
+    return __uint_as_float((b & 0x80000000u) ? (b & 0x7fffffffu) : ~b);
+}
+
 // One node visit of the deferred mode: returns the node's hit triangles
 // (tbase and tbits, the hit leaf slots, with the node's leaf-slot mask in
 // leafMask) instead of testing them.

@@ -1483,11 +1483,12 @@ __global__ void __launch_bounds__(128, kAnyHit ? PRT_BOUNCE_MIN_BLOCKS : kWideBl
 // Closest or any hit of one ray by a group of 8 lanes, lane j testing child j of
 // the node the ray is at and the triangles of that child if it is a leaf (trees
 // of any leaf size).  Every lane of the group holds the ray and the traversal
-// state; stk: the group's kPacketStack entries of shared memory.  Returns the
+// state; stk: the group's kPacketStack entries of shared memory.  behind: hits at
+// negative t count too (a ray may begin behind its origin).  Returns the
 // leaf-order index of the hit triangle, or -1, in every lane.
 template <bool kAnyHit>
-__device__ __forceinline__ int group_trace(const SceneDev& sc, const TravRay& r, const Shear& sh, float tnear, uint2* stk,
-                                           unsigned lane, float& tHit, int& primHit, float& uHit, float& vHit)
+__device__ __forceinline__ int group_trace(const SceneDev& sc, const TravRay& r, const Shear& sh, float tnear, bool behind,
+                                           uint2* stk, unsigned lane, float& tHit, int& primHit, float& uHit, float& vHit)
 {
     const int j = (int)(lane & 7u);
     const unsigned gshift = lane & 24u, gmask = 0xffu << gshift;
@@ -1532,7 +1533,7 @@ __device__ __forceinline__ int group_trace(const SceneDev& sc, const TravRay& r,
         {
             // the hit leaves' triangles, each lane its own; the group keeps the
             // nearest (ties to the lower primitive id)
-            unsigned long long key = hit_key(tHit, primHit);
+            unsigned long long key = signed_hit_key(tHit, primHit);
             const unsigned long long before = key;
             float u = 0.f, v = 0.f;
             int ti = 0;
@@ -1550,12 +1551,13 @@ __device__ __forceinline__ int group_trace(const SceneDev& sc, const TravRay& r,
                     if (tri_test(r.org, sh, f3(v0.x, v0.y, v0.z), f3(v1.x, v1.y, v1.z), f3(v2.x, v2.y, v2.z), tnear, tb, prim,
                                  pb, t, uu, vv))
                     {
+                        if (!behind && __float_as_int(t) < 0) continue;
                         tb = t;
                         pb = prim;
                         u = uu;
                         v = vv;
                         ti = idx;
-                        key = hit_key(t, prim);
+                        key = signed_hit_key(t, prim);
                     }
                 }
             }
@@ -1569,7 +1571,7 @@ __device__ __forceinline__ int group_trace(const SceneDev& sc, const TravRay& r,
             if (key != before)
             {
                 const int win = __ffs(__ballot_sync(gmask, mine == key)) - 1;
-                tHit = __uint_as_float((uint32_t)(key >> 32));
+                tHit = signed_key_t(key);
                 primHit = (int)(uint32_t)key;
                 uHit = __shfl_sync(gmask, u, win);
                 vHit = __shfl_sync(gmask, v, win);
@@ -1593,7 +1595,9 @@ __device__ __forceinline__ int group_trace(const SceneDev& sc, const TravRay& r,
 // Few rays: a group of 8 lanes per ray.  One lane per ray leaves the chip idle
 // while the longest ray's chain of node visits runs, each some 300 dependent
 // instructions and a cache miss; eight lanes cut a visit to about a fifth of
-// that.  perWarp (1, 2 or 4) rays share a warp.
+// that.  perWarp (1, 2 or 4) rays share a warp.  As with many rays, hits at
+// negative t count where triangles are tested in the lane and not where the
+// tests are deferred.
 template <bool kAnyHit>
 __global__ void __launch_bounds__(128) k_intersect_few(SceneDev sc, const RayRec* __restrict__ rays,
                                                      HitRec* __restrict__ hits, float* __restrict__ anyOut, int n,
@@ -1611,7 +1615,8 @@ __global__ void __launch_bounds__(128) k_intersect_few(SceneDev sc, const RayRec
     trav_setup(r, f3(a.x, a.y, a.z), dir);
     float t = b.w, u = 0.f, v = 0.f;
     int prim = 0x7fffffff;
-    const int tri = group_trace<kAnyHit>(sc, r, shear_of(dir), a.w, s_stk + (threadIdx.x >> 3) * kPacketStack, lane, t, prim, u, v);
+    const int tri = group_trace<kAnyHit>(sc, r, shear_of(dir), a.w, !sc.deferTris, s_stk + (threadIdx.x >> 3) * kPacketStack, lane, t,
+                                          prim, u, v);
     if ((lane & 7u) != 0) return;
     if (kAnyHit) anyOut[i] = tri >= 0 ? t : -1.0f;
     else reinterpret_cast<float4*>(hits)[i] = tri >= 0 ? make_float4(t, __int_as_float(prim), u, v)
@@ -1629,7 +1634,7 @@ __global__ void k_query(SceneDev sc, const RayRec* ray, HitRec* hit, float* pNg)
     trav_setup(r, f3(rr.ox, rr.oy, rr.oz), dir);
     float t = rr.tfar, u = 0.f, v = 0.f;
     int prim = 0x7fffffff;
-    const int ti = group_trace<false>(sc, r, shear_of(dir), rr.tnear, s_stk, threadIdx.x, t, prim, u, v);
+    const int ti = group_trace<false>(sc, r, shear_of(dir), rr.tnear, true, s_stk, threadIdx.x, t, prim, u, v);
     if (threadIdx.x != 0) return;
     if (ti < 0)
     {
