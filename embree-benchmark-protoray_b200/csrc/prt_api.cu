@@ -382,20 +382,6 @@ struct WavePlan
     int packet;          // primary rays of a wave with queues, as LaunchCfg::packet
 };
 
-// Without a setting, large waves of many passes take packets, which then span few
-// pixels; smaller ones end in the longest packet.  A 1080p frame of 16 passes (two
-// waves of 16.6M paths), per lane -> packets: 82K triangles 6.30 -> 5.87 ms, 1.38M
-// 23.2 -> 21.5, 10.24M 16.7 -> 15.2, 2M in 2000 spheres 10.1 -> 9.9.  At 7.4M paths the
-// last is 5% slower with packets, at 1.6M 40%.
-// Batches likewise, by their passes on average: 32 requests (156M paths) 28.0 -> 24.8 ms.
-constexpr long long kPacketPaths = 81920;   // per SM
-constexpr int kPacketPasses = 8;
-
-bool default_packets(const prt_ctx* ctx, long long paths, long long pixels)
-{
-    return paths >= kPacketPaths * ctx->numSMs && paths >= kPacketPasses * pixels;
-}
-
 WavePlan plan_waves(const prt_ctx* ctx, int spp)
 {
     WavePlan p;
@@ -403,8 +389,7 @@ WavePlan plan_waves(const prt_ctx* ctx, int spp)
     p.perPass = frame_items(ctx->W, ctx->H);
     p.passes = passes_per_wave(ctx, spp);
     p.whole = whole_paths(p.passes * p.perPass, ctx->bvh.leafMax, ctx->cfg, nee, ctx->numSMs);
-    p.packet = ctx->cfg.packet;
-    if (!p.packet && default_packets(ctx, p.passes * p.perPass, p.perPass)) p.packet = 1;
+    p.packet = primary_packets(ctx->cfg.packet, ctx->numSMs, p.passes * p.perPass, p.perPass);
     // without queues nothing but the item counter bounds a wave
     if (nee && ctx->cfg.pathsPerWave == 0) p.passes = wave_passes(kMaxItems, p.perPass, spp);
     p.waves = wave_count(spp, p.passes);
@@ -1471,7 +1456,7 @@ int prt_render_batch(prt_ctx* ctx, const prt_request* reqs, int n, prt_render_st
     const long long ppw = wave_paths(ctx->cfg.pathsPerWave, default_paths_per_wave(ctx));
     const long long waves = total > 0 ? (total + ppw - 1) / ppw : 0;
     LaunchCfg cfg = ctx->cfg;
-    if (!cfg.packet && default_packets(ctx, total, items)) cfg.packet = 1;
+    cfg.packet = primary_packets(cfg.packet, ctx->numSMs, total, items);
     // waves are dealt round-robin to concurrent chains, as record_render does,
     // so the tail of one wave's bounce launch overlaps another wave's work
     const int chains = (int)std::max<long long>(1, std::min<long long>(chains_for(ctx), waves));
@@ -1589,7 +1574,7 @@ int prt_set_tune(prt_ctx* ctx, const prt_tune* t)
 {
     if (!ctx || !t) return PRT_EINVAL;
     if (t->blockSize < 32 || t->blockSize > 128 || (t->blockSize & 31) || t->blocksPerSM < 0 || t->blocksPerSM > 64 ||
-        t->pathsPerWave < 0 || t->concurrentWaves < 0 || t->primaryPackets < 0 || t->primaryPackets > 2)
+        t->pathsPerWave < 0 || t->concurrentWaves < 0 || t->primaryPackets < 0 || t->primaryPackets > kPrimaryLanes)
         return fail(ctx, PRT_EINVAL, "invalid launch configuration");
     ctx->cfg.packet = t->primaryPackets;
     ctx->cfg.block = t->blockSize;
@@ -1677,8 +1662,16 @@ int prt_autotune(prt_ctx* ctx, int spp, int maxDepth, prt_tune* best)
             }
             return s2;
         };
-        for (int pk = 0; pk <= 2 && st == PRT_OK; ++pk)
+        for (int pk = 0; pk <= kPrimaryLanes && st == PRT_OK; ++pk)
         {
+            if (pk == kPrimaryLanes)
+            {
+                // a choice of its own only where the library's is packets
+                ctx->cfg = cur;
+                ctx->cfg.packet = kPrimaryAuto;
+                const WavePlan p = plan_waves(ctx, spp);
+                if (p.whole || !p.packet || ctx->bvh.leafMax != 1) continue;
+            }
             LaunchCfg c = cur;
             c.packet = pk;
             st = consider(c);

@@ -637,9 +637,9 @@ __global__ void __launch_bounds__(128, kWideBlocks) k_paths(Args a)
 // nodes, so the lanes stay busy together where the per-lane traversal of k_bounce
 // runs 20 of 32 lanes per instruction at this depth; with one pass and coarse
 // pixels the union of the rays' nodes grows and the packet loses, and so do small
-// waves, which end in the longest packet.  LaunchCfg::packet asks for packets (the
-// autotuner tries them); without it plan_waves takes them for large waves of many
-// passes.
+// waves, which end in the longest packet.  prt_tune.primaryPackets asks for packets
+// or lanes (the autotuner tries both); without it large waves of many passes take
+// packets (primary_packets in wave_plan.h).
 #ifndef PRT_PACKET_PRIMARY
 #define PRT_PACKET_PRIMARY 1
 #endif
@@ -2143,7 +2143,7 @@ int launch_bounce(const WaveArgs& a, int depth, const LaunchCfg& cfg, int numSMs
             int grid = grid_for(kernel, cfg.block, pshmem, numSMs, cfg);
             kernel<<<grid, cfg.block, pshmem, s>>>(a);
         };
-        if (cfg.packet == 2)
+        if (cfg.packet == kPrimaryIntervals)
         {
             if (albedo) goPacket(k_primary_packet<true, true>);
             else goPacket(k_primary_packet<false, true>);
@@ -2190,7 +2190,10 @@ void run_paths(Kernel kernel, const Args& a, int words, bool deferred, const Lau
 
 } // namespace
 
-bool packet_primaries(int leafTris, const LaunchCfg& cfg) { return PRT_PACKET_PRIMARY && cfg.packet && leafTris == 1; }
+bool packet_primaries(int leafTris, const LaunchCfg& cfg)
+{
+    return PRT_PACKET_PRIMARY && (cfg.packet == kPrimaryPackets || cfg.packet == kPrimaryIntervals) && leafTris == 1;
+}
 
 bool whole_paths(long long paths, int leafTris, const LaunchCfg& cfg, bool nee, int numSMs)
 {
@@ -2234,7 +2237,7 @@ int launch_batch_first(const BatchArgs& a, const LaunchCfg& cfg, int numSMs, cud
             int grid = grid_for(kernel, cfg.block, pshmem, numSMs, cfg);
             kernel<<<grid, cfg.block, pshmem, s>>>(a);
         };
-        if (cfg.packet == 2) goPacket(k_batch_primary_packet<true>);
+        if (cfg.packet == kPrimaryIntervals) goPacket(k_batch_primary_packet<true>);
         else goPacket(k_batch_primary_packet<false>);
         return 1;
     }

@@ -110,12 +110,13 @@ typedef struct {
     int blocksPerSM;      /* resident blocks per SM of the persistent grid */
     int pathsPerWave;     /* queue capacity (paths in flight per wave); 0 = automatic */
     int concurrentWaves;  /* waves in flight at once, 1..4 (0 keeps the current value) */
-    int primaryPackets;   /* 1: primary rays traced as warp packets (faster for fine pixels,
-                             e.g. 1080p views; slower for coarse ones); 2: warp packets
-                             traversed with interval bounds of the packet (one child test per
-                             node; faster still where a packet's rays stay close, slower for
-                             long, often missing rays); 0 (default): per-lane, and as 1 in
-                             large waves of many passes */
+    int primaryPackets;   /* 0 (default): the library chooses, warp packets (as 1) in large waves
+                             of many passes and per lane elsewhere; 1: primary rays traced as
+                             warp packets (faster for fine pixels, e.g. 1080p views; slower for
+                             coarse ones); 2: warp packets traversed with interval bounds of the
+                             packet (one child test per node; faster still where a packet's rays
+                             stay close, slower for long, often missing rays); 3: per lane
+                             everywhere.  prt_get_tune reports the setting */
     double mray;          /* throughput measured for the winner */
 } prt_tune;
 

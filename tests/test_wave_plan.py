@@ -23,7 +23,9 @@ int main()
     {
         const long long per = frame_items(w, h), paths = wave_paths(setting, 1 << 24);
         const int passes = wave_passes(paths, per, spp);
-        std::printf("%lld %lld %d %d %d\n", per, paths, passes, wave_count(spp, passes), per <= kMaxFrameItems);
+        std::printf("%lld %lld %d %d %d", per, paths, passes, wave_count(spp, passes), per <= kMaxFrameItems);
+        for (int mode = 0; mode < 4; ++mode) std::printf(" %d", primary_packets(mode, 148, passes * per, per));
+        std::printf("\n");
     }
 }
 """
@@ -47,7 +49,7 @@ def plan(tmp_path_factory):
 @pytest.mark.parametrize("w,h", [(1, 1), (8, 8), (1920, 1080), (1001, 563), (16384, 16384), (1, 1 << 27), (1 << 27, 2)])
 @pytest.mark.parametrize("spp", [1, 7, 1028, 1 << 20, INT_MAX])
 def test_items_of_a_launch(plan, w, h, spp, setting):
-    per, paths, passes, waves, frame_ok = plan(w, h, spp, setting)
+    per, paths, passes, waves, frame_ok = plan(w, h, spp, setting)[:5]
     assert per == (w + 7) // 8 * ((h + 7) // 8) * 64
     assert frame_ok
     assert 1 <= passes <= spp
@@ -60,3 +62,10 @@ def test_items_of_a_launch(plan, w, h, spp, setting):
 def test_frames_beyond_the_counter(plan):
     assert plan(1, 1 << 28, 1, 0)[4] == 0 and plan(1 << 28, 1, 1, 0)[4] == 0
     assert plan(2, 1 << 27, 1, 0)[4] == 1
+
+
+def test_camera_rays_per_lane_or_packets(plan):
+    """Settings 1 and 2 ask for packets, 3 for lanes, 0 leaves it to the wave's size."""
+    for w, h, spp, auto in ((256, 256, 16, 0), (1920, 1080, 1, 0), (1920, 1080, 7, 0), (1920, 1080, 8, 1),
+                            (1920, 1080, 64, 1), (640, 480, 64, 1), (4096, 4096, 4, 0)):
+        assert plan(w, h, spp, 0)[5:] == [auto, 1, 2, 0]
