@@ -1190,6 +1190,8 @@ int prt_render_profile(prt_ctx* ctx, int spp, int maxDepth, double* msPerDepth, 
     const int tilesX = (W + 7) / 8, tilesY = (H + 7) / 8;
     const long long perPass = frame_items(W, H);
     const int ppw = passes_per_wave(ctx, spp);
+    LaunchCfg cfg = ctx->cfg;
+    cfg.packet = plan_waves(ctx, spp).packet;   // camera rays as prt_render traces them in waves with a queue
     const bool albedo = ctx->dAlbedo != nullptr;
     const bool nee = ctx->integrator == PRT_INTEGRATOR_DIFFUSE2;
     st = ensure_queues(ctx, (long long)ppw * perPass, albedo, 1, nee, 2);
@@ -1230,7 +1232,7 @@ int prt_render_profile(prt_ctx* ctx, int spp, int maxDepth, double* msPerDepth, 
             a.Lin = nee && d > 0 ? ctx->Lq[0][(d - 1) & 1] : nullptr;
             a.Lout = nee ? ctx->Lq[0][d & 1] : nullptr;
             a.thrConst = const_throughput(d);
-            ctx->launches += launch_bounce(a, d, ctx->cfg, ctx->numSMs, ctx->stream);
+            ctx->launches += launch_bounce(a, d, cfg, ctx->numSMs, ctx->stream);
             CK(cudaEventRecord(ev[(size_t)d + 1], ctx->stream));
         }
         CK(cudaGetLastError());

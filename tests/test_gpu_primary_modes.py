@@ -40,3 +40,24 @@ def test_per_lane_setting(small):
         assert batch[-1][0] == frames[0][0]
         np.testing.assert_allclose(batch[-1][1], frames[0][1], rtol=0, atol=2.0 ** -23 * spp * spp)
     c.close()
+
+
+def test_profile_traces_camera_rays_as_the_renderer(small):
+    """prt_render_profile's first bounce is the kernel prt_render takes in large
+    waves: without a setting its time is that of packets, not of lanes."""
+    import prt
+    mesh, view = small
+    w, h, spp = 1601, 1001, 8
+    c = prt.Context(0)
+    c.load_mesh(mesh.indices, mesh.positions)
+    c.build()
+    c.init_frame(w, h)
+    c.set_view(view, w, h)
+    ms = {0: [], 1: [], 3: []}
+    for _ in range(6):
+        for mode in ms:
+            c.set_tune(128, 0, 1 << 24, 2, mode)
+            ms[mode].append(c.render_profile(spp, 2)[0][0])
+    library, packets, lanes = (min(ms[m][1:]) for m in (0, 1, 3))
+    assert abs(library - packets) < abs(library - lanes), ms
+    c.close()
