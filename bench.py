@@ -593,9 +593,10 @@ def run_kernel_tour(prt, torch, device):
     exceed L2 where the kernel reads bulk data, for profiler captures
     (`ncu ... python bench.py --kernel-tour`); prints one JSON line of
     CUDA-event times.  Phases: BVH build of 2000 level-4 icospheres (10.2M
-    triangles); 4M incoherent closest-hit and any-hit queries on the terrain;
+    triangles); 4M incoherent closest-hit and any-hit queries on the terrain, then 1000;
     one diffuse2 render (960x540, 4 spp); path-replay forward and backward
-    (small scene, 512x512, 4 spp, per-triangle albedo); a batch of 8 requests;
+    (small scene, 512x512, 4 spp, per-triangle albedo); a batch of 8 requests, then
+    of 1 spp each;
     the LDR resolve of a 3840x2160 frame; the mesh builder on the terrain as a
     soup (1.38M triangles, 138 MB)."""
     import scenes
@@ -634,6 +635,7 @@ def run_kernel_tour(prt, torch, device):
     occ = torch.zeros(n, dtype=torch.float32, device=dev)
     timed("intersect_4m", lambda: c.intersect(rays, hits, n))
     timed("occluded_4m", lambda: c.occluded(rays, occ, n))
+    timed("intersect_1k", lambda: c.intersect(rays, hits, 1000))
     c.set_integrator("diffuse2")
     c.init_frame(960, 540)
     c.set_view(tview, 960, 540)
@@ -665,6 +667,9 @@ def run_kernel_tour(prt, torch, device):
                      "spp": 1 + 3 * k, "maxDepth": 5,
                      "accum": torch.zeros((h, w, 4), dtype=torch.float32, device=dev)})
     timed("batch_8", lambda: c.render_batch(reqs))
+    for q in reqs:
+        q["spp"] = 1
+    timed("batch_8_1spp", lambda: c.render_batch(reqs))
     c.close()
 
     soup = np.zeros(terrain.tri_count, prt.SOUP_DTYPE)
@@ -831,7 +836,7 @@ def main():
                 "frac": round(achieved / hbm, 4), "peak_kind": peak_kind,
                 "traffic": None if tr is None else round(tr * rays_per_step),
                 "algorithmic_bytes_per_ray": ALGO_BYTES_PER_RAY,
-                "per": "render step (the k_bounce launches of one 64-spp frame, >99% of its device time)"}
+                "per": "render step (the camera-ray and path launches of one 64-spp frame, >99% of its device time)"}
     if tr is not None:
         roofline["traffic_bytes_per_ray"] = tr
     # The binding limit of the bounce kernel is instruction issue, not HBM:
