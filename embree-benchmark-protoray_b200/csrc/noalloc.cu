@@ -15,7 +15,7 @@
 //   * the frame may hold at most kNoAllocMaxPaths pixels after rounding up to
 //     8x8 tiles (524288, e.g. 1024x512 or 960x544); larger frames are
 //     rejected with PRT_EINVAL;
-//   * g_scratch occupies 20 MiB on every GPU that loads the library, until the
+//   * g_scratch occupies 18 MiB on every GPU that loads the library, until the
 //     process exits;
 //   * all calls on a device share g_scratch, which keeps the last call's
 //     contents: each call clears the counters it needs before using them, and

@@ -121,7 +121,8 @@ cudaError_t current_context_id(unsigned long long* id);
 // goes to cudaMemcpyAsync.
 void stage_retain(int device);    // a context on the device begins
 void stage_release(int device);   // and ends
-// returns when src has been read; the copies are enqueued on stream
+// the copies are enqueued on stream; returns when a pageable src has been read (a
+// pinned one is read when the stream gets there: wait for it before reusing src)
 cudaError_t stage_upload(void* dst, const void* src, size_t bytes, cudaStream_t stream);
 // returns when dst is complete
 cudaError_t stage_download(void* dst, const void* src, size_t bytes, cudaStream_t stream);

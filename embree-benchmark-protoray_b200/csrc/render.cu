@@ -158,16 +158,19 @@ constexpr int kRefillMin = PRT_REFILL_MIN;
 #define PRT_PAIRED_LATER 1
 #endif
 
-// Paired node test in the later bounces of the next-event-estimation kernel
-// (k_bounce_nee; diffuse2 on the terrain frame at 16 spp 2281 -> 2319 Mrays/s);
-// its first bounce keeps single FMAs (paired, it spills 128 bytes).
+// Paired node test of the next-event-estimation kernels: k_paths_nee and the later
+// bounces of k_bounce_nee (diffuse2 on the terrain frame at 16 spp 2281 -> 2319
+// Mrays/s); the first bounce of that one keeps single FMAs.
 #ifndef PRT_PAIRED_NEE
 #define PRT_PAIRED_NEE 1
 #endif
 
 // Paired node test in the any-hit ray-query kernel (k_intersect<true>): 4M
-// incoherent occlusion queries on the terrain 1.085 -> 1.024 ms; closest-hit
-// queries keep single FMAs (paired, they spill and took 1.358 instead of 1.305).
+// incoherent occlusion queries on the terrain 1.085 -> 1.024 ms.  Closest-hit
+// queries and k_batch_first have single FMAs: the former spilled with the paired test
+// while they had 64 registers and kept the shear terms in them.  At 72 without those
+// neither spills, and paired they would be 1% (4M closest hits 1.199 -> 1.188 ms) and
+// 2% faster (three requests of 1000x700 and 4 passes 1.236 -> 1.211 ms).
 #ifndef PRT_PAIRED_QUERY
 #define PRT_PAIRED_QUERY 1
 #endif
@@ -190,8 +193,8 @@ constexpr int kWideBlocks = 7;
 constexpr int bounce_words(bool first) { return kShearWords + (first || !PRT_RELOAD_PATH ? 5 : 0); }
 
 // One bounce of the wavefront over the queue of paths entering `depth`.
-// kFirst: the queue is implicit — item i is (pass, 8x8 tile, Morton index)
-// and the primary ray is generated in registers.
+// kFirst: the queue is implicit — item i is a pixel (8x8 tile, Morton index) and one
+// of its passes (wave_item) — and the primary ray is generated in registers.
 //
 // Each warp keeps 32 rays in flight.  Traversal advances one 8-wide node per
 // step; as soon as kRefillMin lanes have finished, the finished lanes shade

@@ -67,7 +67,7 @@ __device__ __forceinline__ float funord(uint32_t u)
 // The nodes of a depth are segments of the position range.  A warp walks its
 // axis' positions in windows of 32, with segmented shuffle scans inside a window
 // and a carry between windows, and windows whose segments are all single
-// triangles are skipped; the warps meet at five barriers per depth.  The scans'
+// triangles are skipped; the warps meet at six barriers per depth.  The scans'
 // shuffles and minima bound it (issue slots 70%, shared-memory pipe 74% in use);
 // element indices, segment ids and segment ends are bytes, so a subtree takes 15
 // KB of shared memory, and an SM holds 12 (by registers).

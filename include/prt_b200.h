@@ -151,7 +151,10 @@ int prt_set_integrator(prt_ctx* ctx, int integrator);
 
 /* --- acceleration structure (OptixIntersectorStreamCuda ctor, accel/optix/optix_intersector_stream_cuda.cpp:23-75) --- */
 /* The context keeps the build's device scratch (about 160 bytes per triangle)
- * for its later builds and mesh builds; prt_destroy frees it. */
+ * for its later builds and mesh builds; prt_destroy frees it.  A rebuild writes
+ * into the memory of the last tree where that fits (at most twice what it needs).
+ * Queries already issued on a caller's stream (prt_intersect, prt_occluded) finish
+ * on the tree they were issued on. */
 int prt_build_accel(prt_ctx* ctx, prt_build_stats* stats);
 /* Largest leaf of the 8-wide tree, 1..3 triangles, for the next build. */
 int prt_set_leaf_size(prt_ctx* ctx, int maxTrianglesPerLeaf);
@@ -210,7 +213,11 @@ int prt_query_ray(prt_ctx* ctx, const prt_ray* ray, prt_hit* hit, float p[3], fl
  * tfar FLT_MAX.  Needs a camera and a frame. */
 int prt_primary_rays(prt_ctx* ctx, int pass, prt_ray* rays, void* stream);
 
-/* --- intersector seam (IntersectorStreamCuda, core/intersector_stream_cuda.h:32-33) --- */
+/* --- intersector seam (IntersectorStreamCuda, core/intersector_stream_cuda.h:32-33) ---
+ * With stream NULL the call returns when the hits are written; on a caller's stream
+ * it returns at once.  Calls in flight at a time on several streams: at most 64 per
+ * context (each holds one of its work counters).  A hit at negative t (tnear < 0)
+ * is found only in trees with leaves of several triangles and by prt_query_ray. */
 /* Closest hit for n rays (device pointers); misses get t = -1. */
 int prt_intersect(prt_ctx* ctx, const prt_ray* rays, prt_hit* hits, int n, void* stream);
 /* Any hit for n rays (device pointers); out[i] = t of some hit, or -1 (AnyHitCuda). */
@@ -279,7 +286,7 @@ int prt_get_tune(prt_ctx* ctx, prt_tune* tune);
  * callers that cannot allocate device memory at render time (an application
  * that owns the GPU's memory through its own pool, or a frame loop that cannot
  * afford cudaMalloc's implicit synchronisation).  Its path queues live in one
- * fixed 20 MiB device array per GPU, so frames are limited to 524288 pixels
+ * fixed 18 MiB device array per GPU, so frames are limited to 524288 pixels
  * after rounding up to 8x8 tiles (larger ones return PRT_EINVAL).  `accum`
  * must be 16-byte aligned device (or managed) memory of the context's GPU,
  * else PRT_EINVAL.  All calls on a device share that array: calls that overlap
